@@ -499,7 +499,7 @@ extern "C" int mep_grouped_gemm(int mode, const void* a, int64_t a_rows, int64_t
   dim3 grid(num_ctas);
 #define MEP_GEMM_CASE(M)                                                                             \
   case M:                                                                                            \
-    MEP_CUDA_CHECK(cudaFuncSetAttribute(grouped_gemm_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmCfg<M>::kSmem)); \
+    if (allow_smem((const void*)grouped_gemm_kernel<M>, GemmCfg<M>::kSmem)) return -1; \
     grouped_gemm_kernel<M><<<grid, dim3(GemmCfg<M>::kThreads), GemmCfg<M>::kSmem, stream>>>(ma, mb0, mb1, mo, args);                       \
     break;
   switch (mode) {

@@ -594,7 +594,7 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   if (w2::make_map2(&ma, x, rows, args.M_w, x_ld, 64, 64, false)) return -1;
   if (w2::make_map2(&mb, dy, rows, args.N, dy_ld, 64, 64, false)) return -1;
   if (w2::make_map2(&mo, args.out, (int64_t)args.G * args.M_w, args.N, args.N, 32, 32, true)) return -1;
-  MEP_CUDA_CHECK(cudaFuncSetAttribute(w2::wgrad_2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w2::kSmem));
+  if (allow_smem((const void*)w2::wgrad_2cta_kernel, w2::kSmem)) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_ctas); cfg.blockDim = dim3(w2::kThreads); cfg.dynamicSmemBytes = w2::kSmem; cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -634,7 +634,7 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   cfg.attrs = attr; cfg.numAttrs = 1;
 #define MEP_T2_CASE(M)                                                                                                   \
   case M:                                                                                                                \
-    MEP_CUDA_CHECK(cudaFuncSetAttribute(t2::tok_2cta_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t2::kTokSmem)); \
+    if (allow_smem((const void*)t2::tok_2cta_kernel<M>, t2::kTokSmem)) return -1; \
     MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, t2::tok_2cta_kernel<M>, ma, mb0, mb1, mo, args));                              \
     break;
   switch (mode) {

@@ -1,0 +1,441 @@
+// Dispatch and combine of a group of ONE rank: plan, row scatter and padding in one launch; one gather-sum launch.
+//
+// With a single rank every expert is at home, a token's first entry is its primary row and all others are
+// duplicates on the same rank, so the whole exchange is a local permutation. The multi-rank kernels do it in
+// four dependent passes (planning, dispatch of the primaries, duplicate expansion from the primaries;
+// duplicate reduction into the primaries, combine), each with grid barriers and half of them on `num_sms` SMs.
+// Here the traffic is the minimum: dispatch reads every token row once and writes its K rows, combine reads the
+// K rows and writes one. Both are HBM bound; the tables they leave are the ones the multi-rank kernels leave.
+//
+// Counterpart of the reference's dispatch / combine for num_ep_ranks = 1 (moonep/dispatch.py:50-692,
+// moonep/combine.py:40-511), which has no separate path for it.
+#include "prims.cuh"
+#include "../host/launch.h"
+
+namespace mep {
+
+struct LocalDispatchArgs {
+  const __nv_bfloat16* hidden;   // [S, H]
+  const float* weights;          // [S, K] or null
+  __nv_bfloat16* out_hidden;     // [NvS, H]
+  float* out_weights;            // [NvS]
+  int32_t* out_srcinfo;          // [NvS] provenance table or null
+  int32_t* dst;                  // [N]   plan (written when fresh, read otherwise)
+  int32_t* zero_fill;            // [2E, 2]
+  // fresh only
+  const int32_t* topk;           // [N]
+  const int32_t* tpe;            // [E]
+  int32_t* cu_seqlens;           // [2E]
+  int32_t* experts_to_copy;      // [1, E]
+  int32_t* remote_stats;         // [2]
+  int32_t* dup_groups;           // [NvS, 3]
+  int32_t* dup_loffs;            // [NvS]
+  int32_t* dup_counts;           // [2]
+  uint32_t* sync;                // [0] launches completed, [1] start tickets, [2] finished CTAs, [16 + b] flag of CTA b
+  int32_t* hist;                 // [grid, E] expert histogram of each CTA's tokens
+};
+
+constexpr int kLocThreads = 256, kLocWarps = kLocThreads / 32;
+constexpr int kLocEntries = 1024;          // top-k entries ranked and copied at a time by one CTA
+constexpr int kLocZeroBytes = 4096;        // zeroed shared memory the padding rows are stored from
+constexpr int kLocMaxSlots = 8;            // row slots per copying warp
+
+// Exclusive prefix of padded group sizes: start[e] = first row of expert e; padpre[e] = padding rows of
+// experts < e. 256 threads, E / 256 consecutive experts each. Returns the number of padding rows.
+__device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, int* start, int* padpre, int* s_warp) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (E + kLocThreads - 1) / kLocThreads, e0 = tid * per, e1 = min(e0 + per, E);
+  int rows = 0, pads = 0;
+  for (int e = e0; e < e1; ++e) { const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad; rows += p; pads += p - n; }
+  int ri = warp_incl_scan(rows), pi = warp_incl_scan(pads);
+  if (lane == 31) { s_warp[warp] = ri; s_warp[kLocWarps + warp] = pi; }
+  __syncthreads();
+  int rb = 0, pb = 0, total = 0;
+  for (int w = 0; w < kLocWarps; ++w) {
+    if (w < warp) { rb += s_warp[w]; pb += s_warp[kLocWarps + w]; }
+    total += s_warp[kLocWarps + w];
+  }
+  rb += ri - rows; pb += pi - pads;
+  for (int e = e0; e < e1; ++e) {
+    const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad;
+    start[e] = rb; padpre[e] = pb; rb += p; pb += p - n;
+  }
+  return total;
+}
+
+// One CTA owns a contiguous range of tokens. FRESH: their entries are ranked among the same-expert entries of
+// the whole batch -- CTAs publish the histogram of their tokens and add up those of the CTAs before them, so
+// the order is the flat entry order and nothing is sorted -- and the plan tables are written. CTAs number
+// themselves in the order in which they start, so a CTA only ever waits for CTAs that are already running and
+// no cooperative launch is needed. Then, from `dst` alone, each row goes through a warp's slot in shared memory
+// with one bulk load and K bulk stores (lane k issues the store of entry k); rows of the next tokens are in
+// flight meanwhile, in the fresh case already during the ranking.
+// Bound by HBM: (1 + K) rows per token. 
+template <bool FRESH>
+__global__ void __launch_bounds__(kLocThreads, 1)
+local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, int copy_warps, int slots) {
+  const MepRankCtx c = *cp;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_bar[kLocWarps * kLocMaxSlots];
+  __shared__ int s_slot[kLocEntries];        // row of each entry of the current chunk (-1: bad entry, skipped)
+  __shared__ int s_warp[2 * kLocWarps];
+  __shared__ int s_vb, s_fail;
+  const int nb = gridDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int K = c.K, S = c.S, E = c.E, NvS = c.NvS, pad = c.token_padding;
+  const uint32_t row_bytes = (uint32_t)c.H * 2u;
+  unsigned char* s_zero = smem;
+  unsigned char* s_ring = smem + kLocZeroBytes;
+  const int ngroups = FRESH ? E : 2 * E;
+  int* s_start = reinterpret_cast<int*>(s_ring + (size_t)copy_warps * slots * row_bytes);   // FRESH: first row of expert e; else: first padding row of group g
+  int* s_padpre = s_start + ngroups;
+  int* s_cnt = s_padpre + ngroups;           // FRESH [E]: histogram, then next free row of expert e for this CTA's entries
+
+  if (tid == 0) {
+    s_fail = 0;
+    s_vb = FRESH ? (int)atomicAdd(&a.sync[1], 1u) : (int)blockIdx.x;
+    trace_mark(c, MEP_K_DISPATCH, 1);
+  }
+  if (tid < kLocWarps * kLocMaxSlots) mbar_init(&s_bar[tid], 1);
+  fence_mbar_init();
+  for (int i = tid; i < kLocZeroBytes / 16; i += kLocThreads) reinterpret_cast<int4*>(s_zero)[i] = make_int4(0, 0, 0, 0);
+  fence_proxy_async();
+  if (FRESH) for (int e = tid; e < E; e += kLocThreads) s_cnt[e] = 0;
+  __syncthreads();
+  const int vb = s_vb;
+  const uint32_t ep = FRESH ? *(volatile uint32_t*)&a.sync[0] + 1u : 0u;
+  const int tb = min(nb, S), tpb = (S + tb - 1) / tb;
+  const int t0 = min(vb * tpb, S), t1 = min(t0 + tpb, S);
+
+  // ---- the copying warps' first rows are on their way before anything else
+  const int chunk_tok = kLocEntries / K;
+  unsigned char* ring = s_ring + (size_t)warp * slots * row_bytes;
+  uint64_t* bars = s_bar + warp * kLocMaxSlots;
+  const bool copier = warp < copy_warps;
+  const int ntok = copier && t0 + warp < t1 ? (t1 - t0 - warp + copy_warps - 1) / copy_warps : 0;   // tokens t0 + warp + i * copy_warps
+  int issued = 0;
+  auto load = [&](int i) {       // lane 0
+    issued = i + 1;
+    mbar_expect_tx(&bars[i % slots], row_bytes);
+    bulk_g2s(ring + (size_t)(i % slots) * row_bytes, a.hidden + (size_t)(t0 + warp + i * copy_warps) * c.H, row_bytes, &bars[i % slots]);
+  };
+  if (lane == 0) for (int i = 0; i < slots - 1 && i < ntok; ++i) load(i);
+
+  // ---- layout, histogram of this CTA's entries
+  int total_pad;
+  if (FRESH) {
+    for (int i = t0 * K + tid; i < t1 * K; i += kLocThreads) {
+      const int e = __ldg(a.topk + i);
+      if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
+      else report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, i, (uint32_t)e, (uint32_t)E);
+    }
+    total_pad = local_layout(a.tpe, E, pad, s_start, s_padpre, s_warp);
+    __syncthreads();
+    if (t0 < t1) {
+      for (int e = tid; e < E; e += kLocThreads) a.hist[(size_t)vb * E + e] = s_cnt[e];
+      __syncthreads();
+      if (tid == 0) { __threadfence(); st_release_gpu(a.sync + 16 + vb, ep); }
+    }
+    if (vb == nb - 1) {          // the CTA with the least to copy writes the tables that only depend on the counts
+      for (int g = tid; g < 2 * E; g += kLocThreads) {
+        const int e = g < E ? g : E - 1;
+        const int n = __ldg(a.tpe + e), p = (n + pad - 1) / pad * pad;
+        a.cu_seqlens[g] = s_start[e] + p;
+        const bool has = g < E && p > n;
+        a.zero_fill[2 * g] = has ? s_start[e] + n : 0;
+        a.zero_fill[2 * g + 1] = has ? p - n : 0;
+        if (g < E) a.experts_to_copy[g] = -1;
+      }
+      if (tid < 2) { a.remote_stats[tid] = 0; a.dup_counts[tid] = K > 1 ? (tid ? S * (K - 1) : S) : 0; }
+    }
+  } else {
+    // padding rows of the saved plan: group g owns flat indices [padpre[g], padpre[g + 1])
+    int run = 0;
+    for (int g0 = 0; g0 < ngroups; g0 += kLocThreads) {
+      const int g = g0 + tid;
+      const int n = g < ngroups ? __ldg(a.zero_fill + 2 * g + 1) : 0;
+      if (g < ngroups) s_start[g] = __ldg(a.zero_fill + 2 * g);
+      const int incl = warp_incl_scan(n);
+      if (lane == 31) s_warp[warp] = incl;
+      __syncthreads();
+      int base = run;
+      for (int w = 0; w < kLocWarps; ++w) { if (w < warp) base += s_warp[w]; run += s_warp[w]; }
+      if (g < ngroups) s_padpre[g] = base + incl - n;
+      __syncthreads();
+    }
+    total_pad = run;
+  }
+
+  // ---- padding rows, one thread each; neighbours in the flat order go to different CTAs and warps
+  {
+    for (int z = (lane * kLocWarps + warp) * nb + vb; z < total_pad; z += kLocThreads * nb) {
+      int lo = 0, hi = ngroups - 1;          // last group with padpre <= z
+      while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (s_padpre[mid] <= z) lo = mid; else hi = mid - 1; }
+      int row = s_start[lo] + (z - s_padpre[lo]);
+      if (FRESH) row += __ldg(a.tpe + lo);
+      if ((unsigned)row >= (unsigned)NvS) report(c, MEP_ERR_BOUNDS, MEP_K_DISPATCH, 40, lo, (uint32_t)row, (uint32_t)NvS);
+      else {
+        char* p = (char*)a.out_hidden + (size_t)row * row_bytes;
+        for (uint32_t b = 0; b < row_bytes; b += kLocZeroBytes) bulk_s2g(p + b, s_zero, min((uint32_t)kLocZeroBytes, row_bytes - b));
+        if (a.weights) a.out_weights[row] = 0.f;
+        if (a.out_srcinfo) a.out_srcinfo[row] = -1;
+      }
+    }
+  }
+  bulk_commit();
+
+  // ---- entries of earlier CTAs
+  if (FRESH && t0 < t1) {
+    for (int u = tid; u < vb; u += kLocThreads) {
+      uint32_t seen = 0;
+      const bool ok = bounded_wait(c, [&] { seen = ld_acquire_gpu(a.sync + 16 + u); return (int32_t)(seen - ep) >= 0; });
+      if (!ok) { report(c, MEP_ERR_GRID_SYNC_TIMEOUT, MEP_K_PLANNING, 12, u, seen, ep); s_fail = 1; }
+    }
+    for (int e = tid; e < E; e += kLocThreads) s_cnt[e] = s_start[e];
+    __syncthreads();
+    if (E <= kLocThreads) {      // several threads per expert, each over every `parts`-th CTA
+      int w = 1; while (w < E) w <<= 1;
+      const int parts = kLocThreads / w, e = tid & (w - 1), part = tid / w;
+      if (e < E) {
+        int sum = 0;
+#pragma unroll 8
+        for (int u = part; u < vb; u += parts) sum += __ldcg(a.hist + (size_t)u * E + e);
+        if (sum) atomicAdd(&s_cnt[e], sum);
+      }
+    } else {
+      for (int e = tid; e < E; e += kLocThreads) {
+        int sum = 0;
+#pragma unroll 8
+        for (int u = 0; u < vb; ++u) sum += __ldcg(a.hist + (size_t)u * E + e);
+        s_cnt[e] += sum;
+      }
+    }
+    __syncthreads();
+  }
+
+  // ---- chunk by chunk: rank (fresh), tables, rows
+  int it = 0, arrived = 0;                     // tokens this warp has copied / whose load it has waited for
+  uint32_t phases = 0;                         // parity of each slot's barrier
+  bool ok = !(FRESH && s_fail);
+  for (int c0 = t0; c0 < t1 && ok; c0 += chunk_tok) {
+    const int c1 = min(c0 + chunk_tok, t1), n = (c1 - c0) * K;
+    if (FRESH) {
+      for (int i0 = 0; i0 < n; i0 += kLocThreads) {
+        const int i = i0 + tid;
+        int e = i < n ? __ldg(a.topk + (size_t)c0 * K + i) : -1;
+        if ((unsigned)e >= (unsigned)E) e = -1;
+        const unsigned m = __match_any_sync(0xffffffffu, e);
+        const int before = __popc(m & lanemask_lt());
+        int row = -1;
+        const int nw = min(kLocWarps, (n - i0 + 31) >> 5);
+        for (int w = 0; w < nw; ++w) {         // warps in order: the rank is stable
+          if (warp == w && e >= 0) {
+            const int leader = __ffs(m) - 1;
+            int old = 0;
+            if (lane == leader) { old = s_cnt[e]; s_cnt[e] = old + __popc(m); }
+            row = __shfl_sync(m, old, leader) + before;
+          }
+          __syncthreads();
+        }
+        if (i < n) {
+          if (e >= 0 && (row >= s_start[e] + __ldg(a.tpe + e) || (unsigned)row >= (unsigned)NvS)) {   // counts that are not those of topk
+            report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 2, c0 * K + i, (uint32_t)row, (uint32_t)NvS);
+            row = -1;
+          }
+          s_slot[i] = row;
+        }
+      }
+    } else {
+      for (int i = tid; i < n; i += kLocThreads) {
+        const int d = __ldg(a.dst + (size_t)c0 * K + i);
+        int row = d >= 0 ? d : -d - 1;
+        if (row >= NvS) { report(c, MEP_ERR_BOUNDS, MEP_K_DISPATCH, 41, c0 + i / K, (uint32_t)row, (uint32_t)NvS); row = -1; }
+        s_slot[i] = row;
+      }
+    }
+    __syncthreads();
+    // rows: warp w copies tokens t0 + w + i * copy_warps of this chunk
+    for (; it < ntok && ok; ++it) {
+      const int s = t0 + warp + it * copy_warps;
+      if (s >= c1) break;
+      const int st = it % slots;
+      if (it + slots - 1 < ntok) {             // refill the slot of the token before: its stores must have been read
+        bulk_wait_read<0>();
+        __syncwarp();
+        if (lane == 0) load(it + slots - 1);
+      }
+      bool got = true;
+      if (lane == 0) got = mbar_wait_bounded(&bars[st], (phases >> st) & 1u, c.wait_budget_ns);
+      got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
+      if (!got) { if (lane == 0) report(c, MEP_ERR_MBAR_TIMEOUT, MEP_K_DISPATCH, 20, s, 0, 0); ++arrived; phases ^= 1u << st; ok = false; break; }
+      phases ^= 1u << st;
+      ++arrived;
+      for (int k = lane; k < K; k += 32) {
+        const int row = s_slot[(s - c0) * K + k];
+        if (row >= 0) bulk_s2g((char*)a.out_hidden + (size_t)row * row_bytes, ring + (size_t)st * row_bytes, row_bytes);
+      }
+      bulk_commit();
+    }
+    for (int i = tid; i < n; i += kLocThreads) {
+      const int row = s_slot[i], j = c0 * K + i;
+      const int s = j / K, k = j - s * K;
+      if (FRESH) {
+        const int r = row < 0 ? 0 : row;
+        a.dst[j] = k == 0 ? r : -r - 1;
+        if (K > 1) {
+          if (k == 0) { a.dup_groups[3 * s] = r; a.dup_groups[3 * s + 1] = s * (K - 1); a.dup_groups[3 * s + 2] = K - 1; }
+          else a.dup_loffs[s * (K - 1) + k - 1] = r;
+        }
+      }
+      if (row >= 0) {
+        if (a.weights) a.out_weights[row] = a.weights[j];
+        if (a.out_srcinfo) a.out_srcinfo[row] = j;
+      }
+    }
+    __syncthreads();                           // s_slot is free again
+  }
+  if (!ok && lane == 0)                        // do not leave while loads into this CTA's memory are in flight
+    for (int i = arrived; i < issued; ++i) {
+      mbar_wait_bounded(&bars[i % slots], (phases >> (i % slots)) & 1u, c.wait_budget_ns);
+      phases ^= 1u << (i % slots);
+    }
+  bulk_wait_all<0>();
+  if (vb == 0 && tid == 0) {
+    count(c, MEP_CNT_DISPATCHES, 1); count(c, MEP_CNT_ROWS_SENT, (unsigned long long)S); count(c, MEP_CNT_PEER_ROWS, (unsigned long long)S);
+    trace_mark(c, MEP_K_DISPATCH, 5);
+  }
+  if (FRESH) {                                 // the last CTA out closes the launch
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      if (atomicAdd(&a.sync[2], 1u) == (uint32_t)nb - 1u) { a.sync[1] = 0u; a.sync[2] = 0u; a.sync[0] = ep; __threadfence(); }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ combine
+struct LocalCombineArgs {
+  const int32_t* dst;            // [N] plan
+  const __nv_bfloat16* rows;     // [NvS, H]
+  const float* weights;          // [NvS] or null
+  __nv_bfloat16* out;            // [S, H]
+  float* out_weights;            // [S, K] or null
+};
+
+__device__ __forceinline__ void add_bf16x8(float* acc, const int4& x) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); acc[2 * i] += f.x; acc[2 * i + 1] += f.y; }
+}
+
+// out[s] = sum over k, ascending, of the rows of token s, in fp32, rounded once: what the duplicate reduction
+// followed by the combine computes, without the intermediate row. A warp works on (token, column part) units: one
+// bulk load per row brings a unit into one half of the warp's stage while the other half is summed, and the plan
+// entries of the unit behind that one are already being fetched.
+// Bound by HBM: (K + 1) rows per token. Loading into registers instead kept too little in flight: 138 us at
+// S=4096, H=7168, K=8 with 32 warps per SM and 218 us with 8 (twice the loads per lane).
+constexpr int kLcWarps = 12, kLcHalf = 8192;
+
+__global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_bar[kLcWarps * 2];
+  const int K = cp->K, NvS = cp->NvS, nvec = cp->H >> 3;
+  const uint64_t budget = cp->wait_budget_ns;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < kLcWarps * 2) mbar_init(&s_bar[tid], 1);
+  fence_mbar_init();
+  __syncthreads();
+  unsigned char* stage = smem + (size_t)warp * 2 * kLcHalf;
+  uint64_t* bars = s_bar + warp * 2;
+  const int units = cp->S * nparts, step = gridDim.x * kLcWarps;
+  int u = blockIdx.x * kLcWarps + warp;
+  auto fetch = [&](int x) { return x < units && lane < K ? __ldg(a.dst + (size_t)(x / nparts) * K + lane) : 0; };
+  // loads of unit x (plan entry d in lane k) into half h; returns the lanes whose entry names a row
+  auto issue = [&](int x, int d, int h) {
+    const int part = x % nparts, vb = part * part_vecs;
+    const uint32_t bytes = (uint32_t)min(part_vecs, nvec - vb) * 16u;
+    const int row = d >= 0 ? d : -d - 1;
+    const unsigned valid = __ballot_sync(0xffffffffu, lane < K && row < NvS);
+    if (a.out_weights && part == 0 && lane < K) a.out_weights[(size_t)(x / nparts) * K + lane] = row < NvS ? __ldg(a.weights + row) : 0.f;
+    if (lane == 0) mbar_expect_tx(&bars[h], bytes * (uint32_t)__popc(valid));
+    __syncwarp();                              // also: every lane has finished reading this half
+    if ((valid >> lane) & 1u)
+      bulk_g2s(stage + (size_t)h * kLcHalf + (size_t)lane * part_vecs * 16, reinterpret_cast<const int4*>(a.rows) + (size_t)row * nvec + vb, bytes, &bars[h]);
+    return valid;
+  };
+  const unsigned all = K >= 32 ? 0xffffffffu : (1u << K) - 1u;
+  unsigned cur = 0, nxt = 0;
+  int h = 0, bad = -1;
+  uint32_t phase = 0;                          // parity of both halves: they are used in turn
+  if (u < units) cur = issue(u, fetch(u), 0);
+  int dn = fetch(u + step);
+  bool ok = true;
+  for (; u < units; u += step) {
+    const int un = u + step;
+    if (un < units) nxt = issue(un, dn, h ^ 1);
+    dn = fetch(un + step);
+    if (cur != all) bad = u / nparts;
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[h], phase, budget))) { ok = false; break; }
+    const int part = u % nparts, vb = part * part_vecs, n = min(part_vecs, nvec - vb);
+    const unsigned char* base = stage + (size_t)h * kLcHalf;
+    int4* orow = reinterpret_cast<int4*>(a.out) + (size_t)(u / nparts) * nvec + vb;
+    for (int v = lane; v < n; v += 32) {
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+      for (int k = 0; k < K; ++k)
+        if ((cur >> k) & 1u) add_bf16x8(acc, *reinterpret_cast<const int4*>(base + ((size_t)k * part_vecs + v) * 16));
+      int4 o; __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+      st_na_v4(orow + v, o);
+    }
+    cur = nxt; phase ^= (uint32_t)h; h ^= 1;
+  }
+  if (!ok) {                                   // the other half's copies get their time too before the stage goes away
+    if (u + step < units) mbar_wait_bounded(&bars[h ^ 1], phase ^ (uint32_t)h, budget);
+    if (lane == 0) report(*cp, MEP_ERR_MBAR_TIMEOUT, MEP_K_COMBINE, 22, u, 0, 0);
+  }
+  if (bad >= 0 && lane == 0) report(*cp, MEP_ERR_BOUNDS, MEP_K_COMBINE, 20, bad, (uint32_t)NvS, (uint32_t)NvS);   // corrupt or foreign plan
+  if (blockIdx.x == 0 && tid == 0) {
+    trace_mark(*cp, MEP_K_COMBINE, 1);
+    count(*cp, MEP_CNT_COMBINES, 1); count(*cp, MEP_CNT_ROWS_PULLED, (unsigned long long)cp->S * K);
+  }
+}
+
+}  // namespace mep
+
+// `num_blocks`: CTAs (one per SM). fresh: plan from topk / tpe as well; else a.dst / a.zero_fill are read.
+extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::LocalDispatchArgs* args, int fresh,
+                                         int num_blocks, int H, int E, cudaStream_t stream) {
+  using namespace mep;
+  const size_t row = (size_t)H * 2;
+  const size_t tables = (size_t)(fresh ? 3 : 4) * E * sizeof(int);
+  const size_t budget = 208 * 1024;
+  MEP_REQUIRE(tables + kLocZeroBytes + 2 * row <= budget, "dispatch: H=%d rows (%zu B) with E=%d do not fit shared memory", H, row, E);
+  const int all = (int)((budget - tables - kLocZeroBytes) / row);           // row slots that fit
+  int warps = all / 2 < kLocWarps ? all / 2 : kLocWarps;
+  int slots = all / warps < kLocMaxSlots ? all / warps : kLocMaxSlots;
+  // more than 64 KB of rows in flight per SM buys nothing; a smaller footprint starts sooner
+  while (slots > 2 && (size_t)warps * (slots - 1) * row >= 96 * 1024) --slots;
+  const size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
+  if (fresh) return launch_plain(local_dispatch_kernel<true>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+  return launch_plain(local_dispatch_kernel<false>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+}
+
+extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalCombineArgs* args, int num_blocks,
+                                        int S, int H, int K, cudaStream_t stream) {
+  using namespace mep;
+  const int nvec = H / 8;
+  // a unit is what fits half a warp's stage, or less while that leaves warps without work
+  int part = kLcHalf / 16 / K;
+  if (part > 32) part &= ~31;
+  if (part > nvec) part = nvec;
+  while (part > 32 && (long long)S * ((nvec + part - 1) / part) < (long long)num_blocks * kLcWarps) part = (part / 2 + 31) & ~31;
+  const int nparts = (nvec + part - 1) / part;
+  MEP_REQUIRE((long long)S * nparts < (1ll << 30), "combine: S=%d, H=%d is too large", S, H);
+  const int grid = (int)(((long long)S * nparts + kLcWarps - 1) / kLcWarps);
+  return launch_plain(local_combine_kernel, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
+                      stream, ctx, *args, part, nparts);
+}
+
+MEP_EXPORT_SIZEOF(LocalDispatchArgs, mep::LocalDispatchArgs)
+MEP_EXPORT_SIZEOF(LocalCombineArgs, mep::LocalCombineArgs)

@@ -6,7 +6,9 @@
 #include <stdarg.h>
 #include <stdio.h>
 #include <atomic>
+#include <mutex>
 #include <string>
+#include <vector>
 #include "../mep_types.h"
 
 // Exports sizeof(type) as mep_sizeof_<name>() so that the Python side can check its ctypes
@@ -32,6 +34,28 @@ int set_error(const char* fmt, ...);
     if (!(cond)) return ::mep::set_error(__VA_ARGS__);          \
   } while (0)
 
+// Raise a kernel's dynamic shared memory limit, once per kernel, device and size: the runtime call costs more than
+// the rest of a small launch's host work.
+inline int allow_smem(const void* kernel, size_t smem) {
+  if (smem <= 16 * 1024) return 0;
+  struct Seen { const void* k; int dev; size_t smem; };
+  static std::vector<Seen> seen;
+  static std::mutex guard;            // one table for all threads: the limit only ever rises
+  int dev = 0;
+  MEP_CUDA_CHECK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(guard);
+  for (Seen& s : seen)
+    if (s.k == kernel && s.dev == dev) {
+      if (s.smem >= smem) return 0;
+      MEP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      s.smem = smem;
+      return 0;
+    }
+  MEP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  seen.push_back({kernel, dev, smem});
+  return 0;
+}
+
 // Launch `kernel` with CTAs guaranteed co-resident (needed by the software barriers).
 template <class... KArgs, class... Args>
 int launch_cooperative(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
@@ -44,8 +68,7 @@ int launch_cooperative(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   if (pdl) { attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
              attr[n].val.programmaticStreamSerializationAllowed = 1; ++n; }
   cfg.attrs = attr; cfg.numAttrs = n;
-  if (smem > 16 * 1024)
-    MEP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (allow_smem((const void*)kernel, smem)) return -1;
   MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
@@ -57,8 +80,7 @@ int launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cfg.attrs = nullptr; cfg.numAttrs = 0;
-  if (smem > 16 * 1024)
-    MEP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (allow_smem((const void*)kernel, smem)) return -1;
   MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
@@ -76,8 +98,7 @@ int launch_plain_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = pdl ? attr : nullptr; cfg.numAttrs = pdl ? 1 : 0;
-  if (smem > 16 * 1024)
-    MEP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (allow_smem((const void*)kernel, smem)) return -1;
   MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;

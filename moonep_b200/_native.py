@@ -66,6 +66,16 @@ class DispatchArgs(C.Structure):
                 ("send_list", C.c_void_p), ("send_meta", C.c_void_p)]
 
 
+class LocalDispatchArgs(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("hidden", "weights", "out_hidden", "out_weights", "out_srcinfo", "dst", "zero_fill",
+                                          "topk", "tpe", "cu_seqlens", "experts_to_copy", "remote_stats", "dup_groups",
+                                          "dup_loffs", "dup_counts", "sync", "hist")]
+
+
+class LocalCombineArgs(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("dst", "rows", "weights", "out", "out_weights")]
+
+
 class SendOrderArgs(C.Structure):
     _fields_ = [("dst", C.c_void_p), ("cu_seqlens", C.c_void_p), ("send_list", C.c_void_p), ("send_meta", C.c_void_p),
                 ("hist", C.c_void_p), ("bucket", C.c_void_p)]
@@ -161,4 +171,4 @@ def ctx_array(ctx_ptrs):
 
 
 def cur_stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))

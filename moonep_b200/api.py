@@ -121,22 +121,12 @@ class OpsMixin:
         st, g, n = self._states, self.geo, len(self._states)
         fresh = plans is None
         for i in range(n):
-            h = hidden[i]
-            assert h.dtype == torch.bfloat16 and h.is_contiguous() and tuple(h.shape) == (g.S, g.H), \
-                f"hidden_sh must be a contiguous [S={g.S}, H={g.H}] bf16 tensor"
-            if weights is not None:
-                w = weights[i]
-                assert w.dtype == torch.float32 and w.is_contiguous() and w.numel() == g.N, \
-                    "route_weights_sk must be a contiguous [S, K] fp32 tensor"
+            self._check_hidden(hidden[i], None if weights is None else weights[i])
         cus = [None] * n
         if fresh:
             plans, cus = [], []
             for i in range(n):
-                t, c = topk[i].reshape(-1), tpe[i]
-                assert t.dtype == torch.int32 and t.numel() == g.N and t.is_contiguous(), \
-                    "topk_experts_sk must be a contiguous [S, K] int32 tensor"
-                assert c.dtype == torch.int32 and c.numel() == g.E and c.is_contiguous(), \
-                    "tokens_per_expert must be a contiguous [E] int32 tensor"
+                self._check_topk(topk[i].reshape(-1), tpe[i])
                 p, cu = engine.allocate_plan(st[i], with_send_list=True)
                 plans.append(p)
                 cus.append(cu)
@@ -144,8 +134,7 @@ class OpsMixin:
             engine.launch_send_order(st, plans, cus)
         else:
             for p in plans:
-                assert isinstance(p, MoonEPCommPlan), "plan must be a MoonEPCommPlan"
-                assert (p.N, p.R, p.E, p.NvS, p.K) == (g.N, g.R, g.E, g.NvS, g.K), "plan belongs to another Buffer geometry"
+                self._check_plan(p)
                 assert p.send_list is not None, "dispatch_ready needs a plan made by dispatch_ready (it carries the send list)"
         engine.launch_flag_epoch_bump(st)
         main = torch.cuda.current_stream()
@@ -178,20 +167,54 @@ class OpsMixin:
         return TileReady(st.scratch["tile_done"].data_ptr(), st.scratch["flag_epoch"].data_ptr(),
                          total - len(self._states) * self.geo.num_sms)
 
+    def _check_hidden(self, h, w):
+        g = self.geo
+        assert h.dtype == torch.bfloat16 and h.is_contiguous() and h.shape == (g.S, g.H), \
+            f"hidden_sh must be a contiguous [S={g.S}, H={g.H}] bf16 tensor"
+        if w is not None:
+            assert w.dtype == torch.float32 and w.is_contiguous() and w.numel() == g.N, \
+                "route_weights_sk must be a contiguous [S, K] fp32 tensor"
+
+    def _check_topk(self, t, c):
+        g = self.geo
+        assert t.dtype == torch.int32 and t.numel() == g.N and t.is_contiguous(), \
+            "topk_experts_sk must be a contiguous [S, K] int32 tensor"
+        assert c.dtype == torch.int32 and c.numel() == g.E and c.is_contiguous(), \
+            "tokens_per_expert must be a contiguous [E] int32 tensor"
+
+    def _check_plan(self, p):
+        g = self.geo
+        assert isinstance(p, MoonEPCommPlan), "plan must be a MoonEPCommPlan"
+        assert (p.N, p.R, p.E, p.NvS, p.K) == (g.N, g.R, g.E, g.NvS, g.K), "plan belongs to another Buffer geometry"
+
     # ---- dispatch
+    def _dispatch_local(self, hidden, weights, topk, tpe, plan, zero_copy, w_zero_copy):
+        """Single rank: one kernel plans and scatters, straight into the private copies if those are wanted (rows
+        behind the last group's are not written there)."""
+        st = self._states[0]
+        cu = None
+        if plan is None:
+            topk = topk.reshape(-1)
+            self._check_topk(topk, tpe)
+            plan, cu = engine.allocate_plan(st)
+        else:
+            self._check_plan(plan)
+            topk = tpe = None
+        h = st.hidden_local if zero_copy else torch.empty_like(st.hidden_local)
+        w = None if weights is None else st.weights_local if w_zero_copy else torch.empty_like(st.weights_local)
+        engine.launch_local_dispatch(st, hidden, weights, plan, h, w, self._num_sms_dedup, topk, tpe, cu)
+        return h, w, cu, plan
+
     def _dispatch_lists(self, hidden, weights, topk, tpe, plans, *, inter_rank_sync, zero_copy, w_zero_copy):
         st = self._states
         g = self.geo
         n = len(st)
         fresh = plans is None
         for i in range(n):
-            h = hidden[i]
-            assert h.dtype == torch.bfloat16 and h.is_contiguous() and tuple(h.shape) == (g.S, g.H), \
-                f"hidden_sh must be a contiguous [S={g.S}, H={g.H}] bf16 tensor"
-            if weights is not None:
-                w = weights[i]
-                assert w.dtype == torch.float32 and w.is_contiguous() and w.numel() == g.N, \
-                    "route_weights_sk must be a contiguous [S, K] fp32 tensor"
+            self._check_hidden(hidden[i], None if weights is None else weights[i])
+        if n == 1 and st[0].local and _SLOT_ORDER != "1":
+            return [[x] for x in self._dispatch_local(hidden[0], None if weights is None else weights[0], topk and topk[0],
+                                                      tpe and tpe[0], plans and plans[0], zero_copy, w_zero_copy)]
         cus = [None] * n
         # MOONEP_DISPATCH_SLOT_ORDER=1: the plain call also uses the slot-ordered kernel that expands
         # duplicate rows itself while rows are still arriving (no separate expansion pass)
@@ -199,11 +222,7 @@ class OpsMixin:
         if fresh:
             plans, cus = [], []
             for i in range(n):
-                t, c = topk[i].reshape(-1), tpe[i]
-                assert t.dtype == torch.int32 and t.numel() == g.N and t.is_contiguous(), \
-                    "topk_experts_sk must be a contiguous [S, K] int32 tensor"
-                assert c.dtype == torch.int32 and c.numel() == g.E and c.is_contiguous(), \
-                    "tokens_per_expert must be a contiguous [E] int32 tensor"
+                self._check_topk(topk[i].reshape(-1), tpe[i])
                 p, cu = engine.allocate_plan(st[i], with_send_list=slot_order)
                 plans.append(p)
                 cus.append(cu)
@@ -212,8 +231,7 @@ class OpsMixin:
                 engine.launch_send_order(st, plans, cus)
         else:
             for p in plans:
-                assert isinstance(p, MoonEPCommPlan), "plan must be a MoonEPCommPlan"
-                assert (p.N, p.R, p.E, p.NvS, p.K) == (g.N, g.R, g.E, g.NvS, g.K), "plan belongs to another Buffer geometry"
+                self._check_plan(p)
             slot_order = slot_order and all(p.send_list is not None for p in plans)
         # planning's barrier already orders this op after every rank's previous one
         if slot_order:
@@ -245,27 +263,41 @@ class OpsMixin:
         return out_h, out_w, cus, plans
 
     # ---- combine
+    def _check_combine(self, st, plan, h, w, zero_copy, w_zero_copy):
+        g = self.geo
+        assert isinstance(plan, MoonEPCommPlan), "Buffer.combine: plan is required"
+        assert h is not None and h.dtype == torch.bfloat16 and h.is_contiguous()
+        assert h.shape == (g.NvS, g.H), f"hidden_nvsh must be [NvS={g.NvS}, H={g.H}]"
+        if w is not None:
+            assert w.dtype == torch.float32 and w.is_contiguous() and w.shape == (g.NvS,)
+        if zero_copy:
+            assert h.data_ptr() == st.hidden_local.data_ptr(), (
+                "combine(zero_copy=True): hidden_nvsh must alias the shard view returned by "
+                "dispatch(zero_copy=True)")
+        if w_zero_copy and w is not None:
+            assert w.data_ptr() == st.weights_local.data_ptr(), (
+                "combine(router_weights_zero_copy=True): route_weights_nvs must alias the weights "
+                "view returned by dispatch(router_weights_zero_copy=True)")
+
+    def _combine_local(self, plan, h, w):
+        """Single rank: nobody else reads this shard, so the rows are summed where they are (no staging, no pre-reduction)."""
+        st, g = self._states[0], self.geo
+        self._check_plan(plan)
+        out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=st.device)
+        ow = None if w is None else torch.empty((g.S, g.K), dtype=torch.float32, device=st.device)
+        engine.launch_local_combine(st, plan, h, w, out, ow, self._num_sms_dedup)
+        return out, ow
+
     def _combine_lists(self, plans, hidden_nvsh, weights_nvs, *, inter_rank_sync, zero_copy, w_zero_copy):
         st = self._states
         g = self.geo
         n = len(st)
         for i in range(n):
-            assert isinstance(plans[i], MoonEPCommPlan), "Buffer.combine: plan is required"
-            h = hidden_nvsh[i]
-            assert h is not None and h.dtype == torch.bfloat16 and h.is_contiguous()
-            assert tuple(h.shape) == (g.NvS, g.H), f"hidden_nvsh must be [NvS={g.NvS}, H={g.H}]"
-            if weights_nvs is not None and weights_nvs[i] is not None:
-                w = weights_nvs[i]
-                assert w.dtype == torch.float32 and w.is_contiguous() and tuple(w.shape) == (g.NvS,)
-            if zero_copy:
-                assert h.data_ptr() == st[i].hidden_local.data_ptr(), (
-                    "combine(zero_copy=True): hidden_nvsh must alias the shard view returned by "
-                    "dispatch(zero_copy=True)")
-            if w_zero_copy and weights_nvs is not None and weights_nvs[i] is not None:
-                assert weights_nvs[i].data_ptr() == st[i].weights_local.data_ptr(), (
-                    "combine(router_weights_zero_copy=True): route_weights_nvs must alias the weights "
-                    "view returned by dispatch(router_weights_zero_copy=True)")
+            self._check_combine(st[i], plans[i], hidden_nvsh[i], None if weights_nvs is None else weights_nvs[i], zero_copy, w_zero_copy)
         have_w = weights_nvs is not None and weights_nvs[0] is not None
+        if n == 1 and st[0].local:
+            out, ow = self._combine_local(plans[0], hidden_nvsh[0], weights_nvs[0] if have_w else None)
+            return [out], [ow] if have_w else None
         staging = (not zero_copy) or (have_w and not w_zero_copy)
         if inter_rank_sync and staging and g.R > 1:
             engine.launch_rank_sync(st)     # peers may still be reading the shard we are about to overwrite
@@ -432,8 +464,9 @@ class Buffer(OpsMixin):
         self._heap.view(st.rank, g.off_bar, (4 * 128,), torch.int32).zero_()
         self._heap.view(st.rank, g.off_ready, (g.ntiles,), torch.int32).zero_()
         self._heap.view(st.rank, g.off_slotflag, (g.epn,), torch.int32).zero_()
-        for name in ("grid_bar", "epoch", "send_cnt", "vb_flags", "tile_done", "flag_epoch", "slot_done", "pf_epoch"):
-            st.scratch[name].zero_()
+        for name in ("grid_bar", "epoch", "send_cnt", "vb_flags", "tile_done", "flag_epoch", "slot_done", "pf_epoch", "loc_sync"):
+            if name in st.scratch:
+                st.scratch[name].zero_()
         st.status.zero_()
         st.status_host.zero_()
         torch.cuda.synchronize()
@@ -509,10 +542,17 @@ class Buffer(OpsMixin):
         cu_seqlens[2*epn] int32 | None, plan)`` plus a CUDA event when ``async_finish``.
         With a saved ``plan`` (backward of combine) planning is skipped, ``cu_seqlens`` is
         None, the same plan object is returned and its tensors are not modified."""
-        self._st()
+        st = self._st()
         if plan is None:
             assert topk_experts_sk is not None and tokens_per_expert is not None, \
                 "dispatch needs topk_experts_sk and tokens_per_expert unless a plan is reused"
+        if st.local and not async_finish and _SLOT_ORDER != "1" and not _NVTX:     # one kernel: straight to it
+            self._check_hidden(hidden_sh, route_weights_sk)
+            h, w, cu, p = self._dispatch_local(hidden_sh, route_weights_sk, topk_experts_sk, tokens_per_expert, plan, zero_copy,
+                                               router_weights_zero_copy)
+            if plan is None and _VERIFY_PLANS and not torch.cuda.is_current_stream_capturing():
+                self.verify_plan(p)
+            return h, w, cu, p
 
         def body():
             oh, ow, cus, plans = self._dispatch_lists(
@@ -524,7 +564,7 @@ class Buffer(OpsMixin):
             return oh[0], ow[0], cus[0], plans[0]
 
         tensors = [hidden_sh, route_weights_sk, topk_experts_sk, tokens_per_expert]
-        if plan is not None:
+        if plan is not None and async_finish:
             tensors += list(plan.tensors())
         (h, w, cu, p), ev = self._run(async_finish, tensors, body, "moonep.dispatch")
         if async_finish:
@@ -614,7 +654,11 @@ class Buffer(OpsMixin):
                 inter_rank_sync: bool = True, *, zero_copy: bool = False, router_weights_zero_copy: bool = False):
         """Sum each token's K rows back to token-major ``[S, H]`` (unweighted; the FFN applies the
         route weights).  Returns ``(hidden_sh, route_weights_sk | None, event | None)``."""
-        self._st()
+        st = self._st()
+        if st.local and not async_finish and not _NVTX:
+            self._check_combine(st, plan, hidden_nvsh, route_weights_nvs, zero_copy, router_weights_zero_copy)
+            o, w = self._combine_local(plan, hidden_nvsh, route_weights_nvs)
+            return o, w, None
 
         def body():
             outs, outw = self._combine_lists(
@@ -622,7 +666,7 @@ class Buffer(OpsMixin):
                 inter_rank_sync=inter_rank_sync, zero_copy=zero_copy, w_zero_copy=router_weights_zero_copy)
             return outs[0], (outw[0] if outw is not None else None)
 
-        tensors = [hidden_nvsh, route_weights_nvs] + (list(plan.tensors()) if isinstance(plan, MoonEPCommPlan) else [])
+        tensors = [hidden_nvsh, route_weights_nvs] + (list(plan.tensors()) if async_finish and isinstance(plan, MoonEPCommPlan) else [])
         (o, w), ev = self._run(async_finish, tensors, body, "moonep.combine")
         if async_finish:
             for t in (o, w):

@@ -16,7 +16,7 @@ import torch
 
 from . import _native
 from ._native import (MepRankCtx, PlanArgs, DispatchArgs, DupFinalizeArgs, DupArgs, CombineArgs, PushReduceArgs,
-                      PrefetchArgs, GradReduceArgs, SendOrderArgs, ptr)
+                      PrefetchArgs, GradReduceArgs, SendOrderArgs, LocalDispatchArgs, LocalCombineArgs, ptr)
 from .geometry import Geometry
 from .plan import MoonEPCommPlan
 
@@ -27,6 +27,9 @@ ERROR_NAMES = {1: "grid barrier timed out (a CTA never arrived)",
                5: "mbarrier phase never completed"}
 KERNEL_NAMES = {1: "rank_sync", 2: "planning", 3: "dispatch", 4: "dup_expand", 5: "dup_reduce", 6: "combine",
                 7: "prefetch", 8: "grad_reduce", 9: "grouped_gemm", 10: "wait_probe"}
+
+
+LOCAL_MAX_E = 2048
 
 
 class MoonEPTimeout(RuntimeError):
@@ -60,6 +63,8 @@ class RankState:
     status: torch.Tensor = None           # int32[8] device
     status_host: torch.Tensor = None      # int32[1] pinned host memory the kernels mirror status[0] into
     plan_fast: bool = False
+    local: bool = False                   # single rank: dispatch / combine are one local kernel each
+    local_blocks: int = 0                 # CTAs the local dispatch has scratch for
 
     @property
     def ctx_ptr(self) -> int:
@@ -91,6 +96,14 @@ def make_rank_state(geo: Geometry, rank: int, heap, device, budget_ns: int | Non
     s["pf_epoch"] = torch.zeros(2, **i32)                     # prefetch launches issued
     if os.environ.get("MOONEP_COUNTERS", "1") != "0":
         s["counters"] = torch.zeros(_native.COUNTER_SLOTS, dtype=torch.int64, device=dev)
+    checked = os.environ.get("MOONEP_CHECKED") == "1"
+    # a group of one rank exchanges rows with nobody: see csrc/device/local_exchange.cu. The checked mode keeps the
+    # general kernels (its table checks sit between them); E is what the kernel's tables in shared memory hold.
+    st.local = R == 1 and E <= LOCAL_MAX_E and not checked
+    if st.local:
+        st.local_blocks = torch.cuda.get_device_properties(dev).multi_processor_count
+        s["loc_sync"] = torch.zeros(16 + st.local_blocks, **i32)
+        s["loc_hist"] = torch.empty(st.local_blocks * E, **i32)
     st.status = torch.zeros(8, **i32)
     # first failure code, mirrored by the kernels into host memory the device can write: the host
     # tests it without synchronising (see Buffer._st)
@@ -100,7 +113,7 @@ def make_rank_state(geo: Geometry, rank: int, heap, device, budget_ns: int | Non
     c.rank, c.R, c.S, c.H, c.K, c.E, c.epn, c.N, c.NvS = rank, R, geo.S, geo.H, geo.K, E, epn, geo.N, geo.NvS
     c.token_padding, c.vblock_entries, c.num_vblocks = geo.token_padding, geo.vblock_entries, geo.num_vblocks
     c.num_sms = geo.num_sms
-    c.checked = 1 if os.environ.get("MOONEP_CHECKED") == "1" else 0
+    c.checked = 1 if checked else 0
     c.heap_base, c.chunk_stride = heap.base, heap.chunk_bytes
     for name in ("off_hidden", "off_weights", "off_tpe", "off_bar", "off_dupcnt", "off_dupgroups",
                  "off_duploffs", "off_ready", "off_rowsrc", "off_slotflag"):
@@ -121,6 +134,7 @@ def make_rank_state(geo: Geometry, rank: int, heap, device, budget_ns: int | Non
         s["trace"] = torch.zeros(1 + 2 * cap, dtype=torch.int64, device=dev)
         c.trace, c.trace_cap = s["trace"].data_ptr(), cap
     st.ctx_host = c
+    st._failed_word = C.c_int32.from_address(st.status_host.data_ptr())
     raw = bytes(c)
     st.ctx_dev = torch.frombuffer(bytearray(raw), dtype=torch.uint8).to(dev)
     st.plan_fast = bool(_native.load().mep_planning_is_fast(E, R))
@@ -133,7 +147,7 @@ def make_rank_state(geo: Geometry, rank: int, heap, device, budget_ns: int | Non
 def failed(st: RankState) -> bool:
     """True once any kernel of this rank has recorded a failure. A plain read of host memory: no
     synchronisation, usable between launches and during CUDA-graph replays."""
-    return int(st.status_host[0]) != 0
+    return st._failed_word.value != 0
 
 
 def read_counters(st: RankState, reset: bool = False) -> dict:
@@ -179,23 +193,55 @@ def _pack(states):
 
 
 def allocate_plan(st: RankState, with_send_list: bool = False):
-    """Plan-owned tensors plus cu_seqlens for one rank (reference: planning.py:1168-1215)."""
+    """Plan-owned tensors plus cu_seqlens for one rank (reference: planning.py:1168-1215).  They are views of ONE
+    allocation, each starting on a 16-byte boundary: a plan costs one allocator call instead of eight, which is
+    what a small dispatch would otherwise wait for."""
     g = st.geo
-    i32 = dict(dtype=torch.int32, device=st.device)
-    extra = dict(send_list=torch.empty(g.N, **i32), send_meta=torch.zeros(4, **i32)) if with_send_list else {}
-    plan = MoonEPCommPlan(
-        dst=torch.empty(g.N, **i32),
-        experts_to_copy=torch.empty(g.R, g.epn, **i32),
-        zero_fill_ranges=torch.empty(2 * g.epn, 2, **i32),
-        remote_stats=torch.empty(2, **i32),
-        N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K,
-        dup_groups=torch.empty(g.NvS, 3, **i32),
-        dup_loffs=torch.empty(g.NvS, **i32),
-        dup_counts=torch.zeros(2, **i32),
-        **extra,
-    )
-    cu = torch.empty(2 * g.epn, **i32)
-    return plan, cu
+    key = "plan_layout_send" if with_send_list else "plan_layout"
+    lay = st.scratch.get(key)
+    if lay is None:
+        sizes = [g.N, g.R * g.epn, 4 * g.epn, 2, 3 * g.NvS, g.NvS, 2, 2 * g.epn] + ([g.N, 4] if with_send_list else [])
+        pad = [-n % 4 for n in sizes]
+        lay = st.scratch[key] = ([x for pair in zip(sizes, pad) for x in pair], sum(sizes) + sum(pad))
+    parts = torch.empty(lay[1], dtype=torch.int32, device=st.device).split(lay[0])[::2]
+    if not st.local:
+        parts[6].zero_()
+    extra = {}
+    if with_send_list:
+        parts[9].zero_()
+        extra = dict(send_list=parts[8], send_meta=parts[9])
+    plan = MoonEPCommPlan.of_parts(
+        dst=parts[0], experts_to_copy=parts[1].view(g.R, g.epn), zero_fill_ranges=parts[2].view(2 * g.epn, 2),
+        remote_stats=parts[3], N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K,
+        dup_groups=parts[4].view(g.NvS, 3), dup_loffs=parts[5], dup_counts=parts[6], **extra)
+    return plan, parts[7]
+
+
+def launch_local_dispatch(st: RankState, hidden, weights, plan, out_hidden, out_weights, num_blocks: int,
+                          topk=None, tpe=None, cu=None):
+    """Single rank: the plan (if ``topk`` is given), the K rows of every token and the padding rows, one launch.
+    ``out_hidden`` / ``out_weights``: this rank's shard or any tensors of its shape."""
+    g = st.geo
+    a = LocalDispatchArgs(hidden.data_ptr(), ptr(weights), out_hidden.data_ptr(), ptr(out_weights), ptr(st.srcinfo_local),
+                          plan.dst.data_ptr(), plan.zero_fill_ranges.data_ptr())
+    fresh = topk is not None
+    if fresh:
+        sc = st.scratch
+        a.topk, a.tpe, a.cu_seqlens = topk.data_ptr(), tpe.data_ptr(), cu.data_ptr()
+        a.experts_to_copy, a.remote_stats = plan.experts_to_copy.data_ptr(), plan.remote_stats.data_ptr()
+        a.dup_groups, a.dup_loffs, a.dup_counts = plan.dup_groups.data_ptr(), plan.dup_loffs.data_ptr(), plan.dup_counts.data_ptr()
+        a.sync, a.hist = sc["loc_sync"].data_ptr(), sc["loc_hist"].data_ptr()
+    _native.check(_native.load().mep_launch_local_dispatch(C.c_void_p(st.ctx_ptr), C.byref(a), 1 if fresh else 0,
+                                                           min(num_blocks, st.local_blocks), g.H, g.E, _native.cur_stream()), "dispatch")
+
+
+def launch_local_combine(st: RankState, plan, rows, weights, out, out_weights, num_blocks: int):
+    """Single rank: ``out[s]`` = sum of the K rows of token ``s``; ``rows`` / ``weights`` may be any tensors of the
+    shard's shape and are only read."""
+    g = st.geo
+    a = LocalCombineArgs(plan.dst.data_ptr(), rows.data_ptr(), ptr(weights), out.data_ptr(), ptr(out_weights))
+    _native.check(_native.load().mep_launch_local_combine(C.c_void_p(st.ctx_ptr), C.byref(a), num_blocks, g.S, g.H, g.K,
+                                                          _native.cur_stream()), "combine")
 
 
 def launch_planning(states, topk_list, tpe_list, plans, cu_list):

@@ -69,6 +69,13 @@ class MoonEPCommPlan:
             chk("send_list", (self.N,))
             chk("send_meta", (4,))
 
+    @classmethod
+    def of_parts(cls, **fields_):
+        """A plan from tensors whose shapes the caller has laid out itself (skips the checks of the constructor)."""
+        p = cls.__new__(cls)
+        p.__dict__.update(fields_)
+        return p
+
     def tensors(self):
         """The tensor fields, in declaration order (used for record_stream)."""
         return tuple(getattr(self, f.name) for f in fields(self)

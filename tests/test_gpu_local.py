@@ -1,0 +1,97 @@
+"""Single-rank dispatch / combine (one kernel each) against the CPU oracle, at the sizes where the kernels' splits
+end: fewer tokens than CTAs, chunks of 1024 entries, one to many experts per thread, rows from 16 bytes to several
+zero-fill stores, one to 32 entries per token."""
+import numpy as np
+import pytest
+import torch
+
+from moonep_b200 import Buffer
+from moonep_b200.sim import plan_cluster, ops as simops
+from gpu_helpers import make_topk, traceable_hidden, check_plans, defined_rows
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # S      K   E     H      pad  routing
+    (1,      1,  1,    8,     1,   "random"),
+    (3,      32, 32,   16,    16,  "random"),
+    (147,    8,  16,   2048,  128, "biased"),
+    (149,    7,  24,   2056,  16,  "random"),
+    (700,    4,  257,  256,   1,   "random"),
+    (512,    2,  2048, 64,    8,   "random"),
+    (333,    5,  5,    7168,  128, "single_expert"),
+    (64,     8,  8,    15360, 128, "biased"),
+    (20000,  8,  32,   64,    128, "biased"),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "S%d_K%d_E%d_H%d" % c[:4])
+def test_local_exchange(case, cuda_device):
+    S, K, E, H, pad, kind = case
+    topk, tpe = make_topk(kind, S, K, E, 1, seed=7)
+    cp = plan_cluster(np.stack([t.numpy() for t in topk]), E, pad)
+    buf = Buffer(S, H, K, E, 1, token_padding=pad)
+    hidden = traceable_hidden(S, H, 0)
+    w = (torch.arange(S * K, dtype=torch.int32) + 1).view(torch.float32).reshape(S, K)
+    eh, ew = simops.dispatch(cp, [hidden.view(torch.int16).float()], [w.view(torch.int32).float()], fill=-1.0)
+    m = defined_rows(cp, 0)
+    g = torch.Generator().manual_seed(3)
+    y = torch.randn(cp.NvS, H, generator=g).to(torch.bfloat16)
+    args = hidden.cuda(), w.cuda(), topk[0].cuda(), tpe[0].cuda()
+    for zero_copy in (True, False, True):           # the launch's counters reset themselves
+        buf.hidden_nvsh_buffer_view.view(torch.int16).fill_(0x5555)
+        buf.router_weight_buffer_view.view(torch.int32).fill_(0x55555555)
+        h, wn, cu, plan = buf.dispatch(*args, zero_copy=zero_copy, router_weights_zero_copy=zero_copy)
+        torch.cuda.synchronize()
+        buf.check()
+        check_plans([plan], [cu], cp, 1)
+        assert torch.equal(h.cpu().view(torch.int16).float()[m], eh[0][m])
+        assert torch.equal(wn.cpu().view(torch.int32).float()[m], ew[0][m])
+    assert bool((buf.hidden_nvsh_buffer_view.cpu().view(torch.int16)[~m] == 0x5555).all()), "rows of no group were written"
+    ydw = wn.clone()
+    # the saved plan brings the same rows, and nothing else
+    buf.hidden_nvsh_buffer_view.view(torch.int16).fill_(0x3333)
+    buf.router_weight_buffer_view.view(torch.int32).fill_(0x33333333)
+    h2, w2, cu2, plan2 = buf.dispatch(args[0], plan=plan, zero_copy=True)
+    torch.cuda.synchronize()
+    assert plan2 is plan and w2 is None and cu2 is None
+    assert torch.equal(h2.cpu().view(torch.int16).float()[m], eh[0][m])
+    assert bool((buf.router_weight_buffer_view.view(torch.int32) == 0x33333333).all())
+    # combine: fp32 sum in ascending k, rounded once
+    yd = y.cuda()
+    out, gw, _ = buf.combine(plan=plan, hidden_nvsh=yd, route_weights_nvs=ydw)
+    torch.cuda.synchronize()
+    buf.check()
+    eo, _ = simops.combine(cp, [y])
+    assert torch.equal(out.cpu(), eo[0])
+    assert torch.equal(gw.cpu().view(torch.int32), w.view(torch.int32)) and torch.equal(yd.cpu(), y)
+    buf.destroy()
+
+
+def test_local_exchange_reports_bad_tables(cuda_device):
+    """A foreign table must end in a status, not in an access outside the buffers: an expert id that does not exist,
+    counts that are not those of the table, rows of the saved plan outside the shard."""
+    from moonep_b200.engine import MoonEPTimeout
+    S, H, K, E = 40, 64, 4, 8
+    topk, tpe = (t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=5))
+    x = torch.zeros(S, H, dtype=torch.bfloat16, device="cuda")
+    for what in ("expert", "counts", "plan", "combine"):
+        buf = Buffer(S, H, K, E, 1, token_padding=8)
+        h, _, _, plan = buf.dispatch(x, None, topk, tpe, zero_copy=True)
+        if what == "expert":
+            bad = topk.clone(); bad[3, 1] = E + 5
+            buf.dispatch(x, None, bad, tpe)
+        elif what == "counts":
+            bad = tpe.clone(); bad[int(bad.argmax())] -= 3
+            buf.dispatch(x, None, topk, bad)
+        else:
+            plan.dst[7] = buf.NvS + 11
+            if what == "plan":
+                buf.dispatch(x, plan=plan)
+            else:
+                buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)
+        with pytest.raises(MoonEPTimeout) as ei:
+            buf.check()
+        assert ei.value.status["code"] == 3
+        buf.reset()
+        buf.destroy()
