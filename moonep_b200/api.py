@@ -188,9 +188,9 @@ class OpsMixin:
         assert (p.N, p.R, p.E, p.NvS, p.K) == (g.N, g.R, g.E, g.NvS, g.K), "plan belongs to another Buffer geometry"
 
     # ---- dispatch
-    def _dispatch_local(self, hidden, weights, topk, tpe, plan, zero_copy, w_zero_copy):
+    def _dispatch_local(self, hidden, weights, topk, tpe, plan, zero_copy=False, w_zero_copy=False, out=None):
         """Single rank: one kernel plans and scatters, straight into the private copies if those are wanted (rows
-        behind the last group's are not written there)."""
+        behind the last group's are not written there).  ``out``: tensors to fill instead."""
         st = self._states[0]
         cu = None
         if plan is None:
@@ -200,8 +200,11 @@ class OpsMixin:
         else:
             self._check_plan(plan)
             topk = tpe = None
-        h = st.hidden_local if zero_copy else torch.empty_like(st.hidden_local)
-        w = None if weights is None else st.weights_local if w_zero_copy else torch.empty_like(st.weights_local)
+        if out is not None:
+            h, w = out
+        else:
+            h = st.hidden_local if zero_copy else torch.empty_like(st.hidden_local)
+            w = None if weights is None else st.weights_local if w_zero_copy else torch.empty_like(st.weights_local)
         engine.launch_local_dispatch(st, hidden, weights, plan, h, w, self._num_sms_dedup, topk, tpe, cu)
         return h, w, cu, plan
 
@@ -213,8 +216,9 @@ class OpsMixin:
         for i in range(n):
             self._check_hidden(hidden[i], None if weights is None else weights[i])
         if n == 1 and st[0].local and _SLOT_ORDER != "1":
-            return [[x] for x in self._dispatch_local(hidden[0], None if weights is None else weights[0], topk and topk[0],
-                                                      tpe and tpe[0], plans and plans[0], zero_copy, w_zero_copy)]
+            w = None if weights is None else weights[0]
+            h, w, cu, p = self._dispatch_local(hidden[0], w, topk and topk[0], tpe and tpe[0], plans and plans[0], True, True)
+            return [h if zero_copy else h.clone()], [w if w is None or w_zero_copy else w.clone()], [cu], [p]
         cus = [None] * n
         # MOONEP_DISPATCH_SLOT_ORDER=1: the plain call also uses the slot-ordered kernel that expands
         # duplicate rows itself while rows are still arriving (no separate expansion pass)

@@ -130,6 +130,8 @@ class MoEBlock:
             moe.on_grad_ready = None
         elif moe.epilogue_lr is None:
             moe.on_grad_ready = lambda n: gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr)
+        elif self.world == 1:
+            moe.on_grad_ready = lambda n: None      # no replicas: the epilogues have updated every expert
         else:
             moe.on_grad_ready = lambda n: gg.sgd_step_groups(self.pools.local_weight(n), self.pools.local_grad(n), lr,
                                                              moe._upd_mask, want=False)

@@ -89,6 +89,7 @@ class ExpertParallelMoE:
         if ready_flags is None:             # MOONEP_READY_FLAGS=0: the GEMMs wait for the whole dispatch
             ready_flags = os.environ.get("MOONEP_READY_FLAGS", "1") != "0"
         self.ready_flags = ready_flags
+        self._local = buffer._states[0].local       # single rank: see _forward_local
         dev = buffer.hidden_nvsh_buffer_view.device
         self._side = torch.cuda.Stream(device=dev)
         self._opt = torch.cuda.Stream(device=dev)
@@ -116,10 +117,14 @@ class ExpertParallelMoE:
         self.epilogue_lr = None
         i32 = dict(dtype=torch.int32, device=dev)
         self._upd_mask = torch.zeros(2 * g.epn, **i32)
+        if g.R == 1:                    # nobody holds a replica: always the same mask
+            self._upd_mask[:g.epn] = 1
         self._upd_hit = torch.zeros(g.epn + 1, **i32)
         self._upd_ones = torch.ones(g.R * g.epn, **i32)
 
     def _update_mask(self, plan):
+        if self.geo.R == 1:
+            return self._upd_mask
         return update_mask(plan.experts_to_copy, self.buf.rank, self.geo.epn, self._upd_mask, self._upd_hit, self._upd_ones)
 
     # weights / grads as [2*epn, in, out]
@@ -134,6 +139,8 @@ class ExpertParallelMoE:
         self._join_deferred()
         if gg.failed(self._act.device):     # a GEMM of an earlier step gave up a wait (host-visible flag, no sync)
             gg.check_status(self._act.device)
+        if self._local:
+            return self._forward_local(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, need_backward)
         if self.ready_flags:
             return self._forward_flagged(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, need_backward)
         h_view, w_view, cu, plan = buf.dispatch(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert,
@@ -159,6 +166,18 @@ class ExpertParallelMoE:
         else:
             gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w)
         return self._forward_tail(plan, cu, stashed, need_backward)
+
+    def _forward_local(self, hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, need_backward):
+        """Single rank.  The dispatch is one local kernel at HBM rate on all SMs, so there is nothing to gain from
+        starting the GEMM on flagged tiles; it writes straight into the private buffers that the backward pass
+        reads (no stash), and the down GEMM's rows stay in the shard, where the combine gathers them."""
+        buf, st = self.buf, self.buf._st()
+        x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
+        _, _, cu, plan = buf._dispatch_local(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, None, out=(x, w))
+        gg.gate_up(x, self._W("gate"), self._W("up"), cu, self._act, self._gu if need_backward else None, row_scale=w)
+        gg.down(self._act, self._W("down"), cu, st.hidden_local)
+        out, _ = buf._combine_local(plan, st.hidden_local, None)
+        return out, MoEContext(plan, cu, x, w, self._act, self._gu) if need_backward else None
 
     def _forward_flagged(self, hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, need_backward):
         """Forward pass with tile-ready flags: see the module docstring."""
@@ -247,7 +266,7 @@ class ExpertParallelMoE:
         dgrad(gate/up), see below).  Replicated experts keep the stored-gradient path -- their gradients
         are reduced across ranks first -- and ``on_grad_ready`` is expected to update exactly those."""
         buf, g, epn, Hp = self.buf, self.geo, self.geo.epn, self.Hp
-        acc, ov, multi = self.accumulate_grads, self.overlap_backward, self.geo.R > 1
+        acc, ov, multi = self.accumulate_grads, self.overlap_backward and not self._local, self.geo.R > 1
         self._join_deferred()
         main = torch.cuda.current_stream()
         pools = self.pools
@@ -258,7 +277,11 @@ class ExpertParallelMoE:
         # (on the comm stream, behind the dispatch); the dgrad GEMMs wait per slot
         refetch = multi and getattr(pools, "shared", None) is not None
         slots, ev_pf = None, None
-        if self.ready_flags and ctx.plan.send_list is not None:
+        if self._local:
+            dy = shard
+            buf._dispatch_local(grad_out_sh, None, None, None, ctx.plan, out=(shard, None))
+            gg.dgrad(dy, Wd, ctx.cu, self._dA)
+        elif self.ready_flags and ctx.plan.send_list is not None:
             # dgrad(down) starts on the tiles of the re-dispatched output grad as they complete
             dy, _, _, _, ready, _ = buf.dispatch_ready(grad_out_sh, plan=ctx.plan)
             if refetch:
@@ -400,5 +423,8 @@ class _MoEFn(torch.autograd.Function):
 
 def moe_apply(layer: ExpertParallelMoE, hidden, route_weights, topk, tpe):
     """Autograd entry: differentiable w.r.t. ``hidden`` and ``route_weights``; expert weight grads
-    are written into the pools' fp32 grad views by the backward pass."""
+    are written into the pools' fp32 grad views by the backward pass.  Without gradients (``torch.no_grad``) the
+    forward pass keeps nothing for a backward pass."""
+    if not torch.is_grad_enabled():
+        return layer.forward(hidden, route_weights, topk, tpe, need_backward=False)[0]
     return _MoEFn.apply(hidden, route_weights, topk, tpe, layer)
