@@ -60,6 +60,9 @@ struct GemmArgs {
   const int32_t* upd_mask;
   float upd_lr;
   int32_t reserved1;
+  // optional [G, 2] table (first padding row, padding rows) of the groups, as a plan carries it: rows behind the real
+  // ones, rounded up to 32, are then neither computed nor read (null: all padded rows are). CTA-pair kernels only.
+  const int32_t* pad_rows;
 };
 
 }  // namespace mep

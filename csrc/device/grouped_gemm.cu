@@ -22,8 +22,7 @@
 #include "tcgen05.cuh"
 #include "tile_queue.cuh"
 #include "gemm_args.h"
-#include "../host/driver_api.h"
-#include "../host/launch.h"
+#include "tmap.h"
 
 namespace mep {
 
@@ -432,38 +431,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   if (threadIdx.x == 0) tq::scheduler_done(args.sched, args.sched_ctas > 0 ? args.sched_ctas : (int)gridDim.x);
 }
 
-static int make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_cols, int box_rows,
-                    bool f32 = false) {
-  const DriverApi* d = driver(); if (!d) return -1;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const int es_bytes = f32 ? 4 : 2;
-  cuuint64_t strides[1] = {(cuuint64_t)ld * es_bytes};
-  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  cuuint32_t es[2] = {1, 1};
-  MEP_REQUIRE(((uintptr_t)base & 15) == 0 && (ld * es_bytes) % 16 == 0 && ld >= cols,
-              "gemm: tensor base/stride must be 16-byte aligned");
-  MEP_CU_CHECK(d->TensorMapEncodeTiled(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
-                                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-  return 0;
-}
-
-// MN-major operand [rows (k), cols (m or n)] viewed as (64 elements, rows, cols/64): one box of
-// `atoms` 64-wide atoms x 64 rows lands in shared memory atom after atom.
-static int make_map_mn(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld, int atoms) {
-  const DriverApi* d = driver(); if (!d) return -1;
-  MEP_REQUIRE(cols % 64 == 0, "gemm: MN-major operand width %lld must be a multiple of 64", (long long)cols);
-  cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
-  cuuint64_t strides[2] = {(cuuint64_t)ld * 2, 128};
-  cuuint32_t box[3] = {64, 64, (cuuint32_t)atoms};
-  cuuint32_t es[3] = {1, 1, 1};
-  MEP_REQUIRE(((uintptr_t)base & 15) == 0 && (ld * 2) % 16 == 0 && ld >= cols, "gemm: tensor base/stride must be 16-byte aligned");
-  MEP_CU_CHECK(d->TensorMapEncodeTiled(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
-                                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-  return 0;
-}
-
 }  // namespace mep
 
 // One grouped GEMM launch. `a` is a row-major bf16 matrix [a_rows, a_cols]; `b0`/`b1` are the
@@ -480,22 +447,22 @@ extern "C" int mep_grouped_gemm(int mode, const void* a, int64_t a_rows, int64_t
   const bool b_mn = mode == GEMM_GATE_UP || mode == GEMM_DOWN || mode == GEMM_WGRAD;
   if (mode == GEMM_WGRAD) {
     MEP_REQUIRE(args.M_w % kBM == 0 && args.N % kBN == 0, "wgrad: weight shape [%d,%d] must be multiples of [128,256]", args.M_w, args.N);
-    if (make_map(&ma, a, a_rows, a_cols, a_ld, 64, 64)) return -1;
+    if (tmap_rows(&ma, a, a_rows, a_cols, a_ld, 64, 64)) return -1;
   } else {
     MEP_REQUIRE(args.K % kBK == 0, "gemm: K=%d must be a multiple of 64", args.K);
     MEP_REQUIRE(args.N % (mode == GEMM_GATE_UP ? 128 : kBN) == 0, "gemm: N=%d not tileable", args.N);
-    if (make_map(&ma, a, a_rows, a_cols, a_ld, 64, kBM)) return -1;
+    if (tmap_rows(&ma, a, a_rows, a_cols, a_ld, 64, kBM)) return -1;
   }
   const int b_atoms = mode == GEMM_GATE_UP ? 2 : 4;
-  if (mode == GEMM_WGRAD) { if (make_map(&mb0, b0, b_rows, b_cols, b_ld, 64, 64)) return -1; }   // token-major operands: 2-D boxes are faster
-  else if (b_mn) { if (make_map_mn(&mb0, b0, b_rows, b_cols, b_ld, b_atoms)) return -1; }
-  else      { if (make_map(&mb0, b0, b_rows, b_cols, b_ld, 64, kBN)) return -1; }
-  if (b1) { if (b_mn ? make_map_mn(&mb1, b1, b_rows, b_cols, b_ld, b_atoms) : make_map(&mb1, b1, b_rows, b_cols, b_ld, 64, kBN)) return -1; }
+  if (mode == GEMM_WGRAD) { if (tmap_rows(&mb0, b0, b_rows, b_cols, b_ld, 64, 64)) return -1; }   // token-major operands: 2-D boxes are faster
+  else if (b_mn) { if (tmap_atoms(&mb0, b0, b_rows, b_cols, b_ld, b_atoms)) return -1; }
+  else      { if (tmap_rows(&mb0, b0, b_rows, b_cols, b_ld, 64, kBN)) return -1; }
+  if (b1) { if (b_mn ? tmap_atoms(&mb1, b1, b_rows, b_cols, b_ld, b_atoms) : tmap_rows(&mb1, b1, b_rows, b_cols, b_ld, 64, kBN)) return -1; }
   else mb1 = mb0;
   // output map: one 32-row x 128-byte box per epilogue warp and chunk
-  if (mode == GEMM_WGRAD) { if (make_map(&mo, args.out, (int64_t)args.G * args.M_w, args.N, args.N, 32, 32, true)) return -1; }
+  if (mode == GEMM_WGRAD) { if (tmap_rows(&mo, args.out, (int64_t)args.G * args.M_w, args.N, args.N, 32, 32, true)) return -1; }
   else if (mode == GEMM_GATE_UP) mo = ma;
-  else { if (make_map(&mo, args.out, a_rows, args.N, args.ldo, 64, 32)) return -1; }
+  else { if (tmap_rows(&mo, args.out, a_rows, args.N, args.ldo, 64, 32)) return -1; }
   dim3 grid(num_ctas);
 #define MEP_GEMM_CASE(M)                                                                             \
   case M:                                                                                            \

@@ -1,0 +1,416 @@
+// Token-major grouped GEMMs on CTA pairs (tcgen05.mma.cta_group::2): GATE_UP, DOWN, DGRAD, DGRAD_GU.
+//
+// A pair computes out^T: the 256 rows of an MMA tile are WEIGHT columns (128 per CTA) and its N side is up to 256
+// token rows of ONE expert (half of them staged by each CTA). Three things follow.
+//   * A tile never straddles experts although groups are only multiples of 128 rows (with tokens on the M side, a pair
+//     wastes half a tile for every group with an odd number of 128-row blocks), and N takes the group's real size in
+//     steps of 32: padding rows cost nothing when the caller passes their table (GemmArgs.pad_rows).
+//   * A CTA fills 32 KB of shared memory per 64-deep k-block for the math of a 128 x 256 x 64 block; a single CTA
+//     needs 48 KB. The kernels run at the board's power limit, where the bytes that move through L2 per FLOP
+//     set the clock as well.
+//   * The accumulator arrives transposed. It is read in MMA-fragment layout and turned by stmatrix.trans on its way
+//     into 128-byte swizzled staging rows, from where TMA stores (or, for the push epilogue, 16-byte peer stores)
+//     write whole 128-byte runs of token rows.
+// Roles per CTA: warp 0 = TMA producer, warp 1 = TMEM allocation (+ MMA issue in the leader), warps 2-9 = epilogue: TMEM
+// lane quarter = warp % 4, the two sets of four take alternate 16-token chunks.
+// GATE_UP: the M side of a CTA is 64 gate columns and the same 64 up columns, so g and u of an output sit 64 TMEM
+// lanes apart: the up warps hand their fp32 fragments to the gate warps through shared memory.
+#include "pair.cuh"
+#include "tile_queue.cuh"
+#include "gemm_args.h"
+#include "tmap.h"
+
+namespace mep {
+namespace tp {
+using namespace pair;
+
+constexpr int kBK = 64, kRing = 6, kEpiWarps = 8, kThreads = 64 + 32 * kEpiWarps;
+constexpr int kHalfBytes = 128 * kBK * 2;              // 16 KB: weight columns, or up to 128 token rows, of one k-block
+constexpr int kStageBytes = 2 * kHalfBytes;
+constexpr int kAtomBytes = 64 * kBK * 2;
+constexpr int kChunk = 16;                             // tokens per epilogue step
+constexpr int kStgBytes = kChunk * 128;                // staging: 16 tokens x 64 columns
+constexpr int kXchBytes = 32 * 64;                     // one warp's fp32 fragments of a chunk (GATE_UP)
+constexpr int kMaxGroups = 192;
+constexpr size_t kEpiBytes = 2 * 3 * kStgBytes + 4 * kXchBytes > 2 * 4 * kStgBytes ? 2 * 3 * kStgBytes + 4 * kXchBytes : 2 * 4 * kStgBytes;
+constexpr size_t kSmem = (size_t)kRing * kStageBytes + kEpiBytes + 1024;
+
+struct Tile { int g, row0, n, n0; };                   // n tokens from row0 (a multiple of 32, at most 256)
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// Bounded poll of a ready flag (see GemmArgs.tile_done / group_flags); SYS: written by another GPU.
+template <bool SYS>
+__device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, uint64_t budget_ns) {
+  auto up = [&] { return (int32_t)((SYS ? ld_acquire_sys(flag) : ld_acquire_gpu(flag)) - epoch) >= 0; };
+  if (up()) return true;
+  const long long t0 = clock64(), lim = budget_cycles(budget_ns);
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i) { __nanosleep(SYS ? 200 : 100); if (up()) return true; }
+    if (clock64() - t0 > lim) return false;
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, 1)
+tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
+                const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out2, GemmArgs args) {
+  constexpr bool W_MN = MODE == GEMM_GATE_UP || MODE == GEMM_DOWN;      // weights [k, column]: the M side is contiguous
+  constexpr int kCols = MODE == GEMM_GATE_UP ? 128 : 256;               // output columns of a tile
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full_bar[kRing], empty_bar[kRing], tfull_bar[2], tempty_bar[2];
+  __shared__ uint32_t s_tmem_base;
+  __shared__ volatile int s_abort;
+  __shared__ tq::Ring s_ring;
+  __shared__ int s_beg[kMaxGroups], s_units[kMaxGroups], s_start[kMaxGroups + 1];   // first row, 32-token units, first tile of a group
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t cr = cluster_ctarank();
+  const bool leader = cr == 0;
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const int G = args.G, kblocks = args.K / kBK;
+
+  if (warp == 0) {                       // tile list: 32 groups at a time
+    const int nblk = args.N / kCols;
+    int run = 0;
+    for (int g0 = 0; g0 < G; g0 += 32) {
+      const int g = g0 + lane;
+      int beg = 0, units = 0;
+      if (g < G) {
+        beg = g ? args.cu_seqlens[g - 1] : 0;
+        int rows = args.cu_seqlens[g] - beg;
+        if (args.pad_rows) rows -= args.pad_rows[2 * g + 1];
+        if (g >= args.g_begin && g < args.g_end) units = (rows + 31) >> 5;
+      }
+      const int tiles = ((units + 7) >> 3) * nblk, incl = warp_incl_scan(tiles);
+      if (g < G) { s_beg[g] = beg; s_units[g] = units; s_start[g] = run + incl - tiles; }
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_start[G] = run;
+  } else if (warp == 1) {
+    tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2();
+  } else if (threadIdx.x == 64) {
+    s_abort = 0;
+    for (int i = 0; i < kRing; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&tfull_bar[i], 1); mbar_init(&tempty_bar[i], 2 * kEpiWarps); }
+    tq::init(&s_ring, 2 * kEpiWarps + 2);      // both CTAs' epilogue warps, the MMA issuer, the peer's producer
+    fence_mbar_init();
+    tc::prefetch_tmap(&tma_x); tc::prefetch_tmap(&tma_w0); tc::prefetch_tmap(&tma_w1); tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  cluster_sync();                        // both CTAs' barriers exist before anyone touches the peer's
+  tc::fence_after_sync();
+  const uint32_t tmem_base = s_tmem_base;
+  const int ntiles = s_start[G];
+  const bool dyn = args.sched != nullptr;
+
+  auto note = [&](int site, int tile, int code) {
+    if (atomicCAS(&args.status[0], 0, code) == 0) {
+      args.status[1] = 200 + site; args.status[2] = blockIdx.x; args.status[3] = tile;
+      if (args.status_host) { *(volatile int32_t*)args.status_host = code; __threadfence_system(); }
+    }
+  };
+  auto fail = [&](int site, int tile, int code = MEP_ERR_MBAR_TIMEOUT) { note(site, tile, code); s_abort = 1; };
+  // tile number -> tile; `g` is a monotone cursor. The tiles of a group share its tokens evenly (in units of 32), token
+  // tiles vary fastest: the weight columns they have in common are then in L2.
+  auto get_tile = [&](int t, int& g, Tile& ti) {
+    while (s_start[g + 1] <= t) ++g;
+    const int units = s_units[g], mt = (units + 7) >> 3, local = t - s_start[g];
+    const int cb = local / mt, pt = local - cb * mt, base = units / mt, rem = units - base * mt;
+    ti.g = g; ti.n0 = cb * kCols;
+    ti.row0 = s_beg[g] + 32 * (pt * base + min(pt, rem));
+    ti.n = 32 * (base + (pt < rem ? 1 : 0));
+  };
+
+  if (warp == 0) {
+    // ---------------- TMA producer: this CTA's halves; bytes are counted on the LEADER's barrier
+    if (lane == 0) {
+      int it = 0, gcur = 0; Tile ti;
+      tq::Scheduler<true> sched; tq::Consumer<true> follow;
+      if (dyn) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
+      tq::Strided seq{pair, npairs, ntiles};
+      const uint32_t tile_ep = args.tile_done ? *(volatile const uint32_t*)args.tile_epoch : 0u;
+      const uint32_t group_ep = args.group_flags ? *(volatile const uint32_t*)args.group_epoch : 0u;
+      int seen_row = -1, seen_group = -1;            // flags known to be up: 128-row blocks of the last tile, last group
+      for (int t; !s_abort && (t = !dyn ? seq.next() : leader ? sched.next(args.budget_ns) : follow.next(args.budget_ns)) != -1;) {
+        if (t == -2) { fail(5, it); break; }
+        get_tile(t, gcur, ti);
+        if (args.tile_done && ti.row0 != seen_row) {
+          // the rows come from a dispatch that may still be running: wait until they have all landed and the
+          // duplicates are expanded, then order the TMA engine's reads behind that
+          bool up = true;
+          for (int b = ti.row0 >> 7; up && b <= (ti.row0 + ti.n - 1) >> 7; ++b) up = wait_flag<false>(args.tile_done + b, tile_ep, args.budget_ns);
+          if (!up) { fail(9, t, MEP_ERR_FLAG_TIMEOUT); break; }
+          fence_proxy_async();
+          seen_row = ti.row0;
+        }
+        if (args.group_flags && ti.g >= args.group_first && ti.g != seen_group) {
+          // the weights of this group are a prefetched expert that may still be on its way
+          if (!wait_flag<true>(args.group_flags + (ti.g - args.group_first), group_ep, args.budget_ns)) { fail(9, t, MEP_ERR_FLAG_TIMEOUT); break; }
+          fence_proxy_async();
+          seen_group = ti.g;
+        }
+        const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
+        const bool two = half > 64;                  // token rows arrive in boxes of 64
+        const uint32_t bytes = (uint32_t)kHalfBytes + (two ? 16384u : 8192u);
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % kRing; const uint32_t ph = (uint32_t)(it / kRing) & 1u;
+          if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns)) { fail(1, t); break; }
+          const uint32_t sw = smem_u32(smem + (size_t)s * kStageBytes), sx = sw + kHalfBytes;
+          const uint32_t bar = mapa(smem_u32(&full_bar[s]), 0);
+          if (leader) mbar_expect_tx(&full_bar[s], 2 * bytes);
+          const int k0 = kb * kBK;
+          if (MODE == GEMM_GATE_UP) {
+            tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+            tma_load_3d_bar(sw + kAtomBytes, &tma_w1, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+          } else if (MODE == GEMM_DOWN) {
+            tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
+          } else {
+            const int kh = args.K / 2;               // DGRAD_GU: first half of K from Wg, second from Wu
+            const bool second = MODE == GEMM_DGRAD_GU && k0 >= kh;
+            tma_load_2d_bar(sw, second ? &tma_w1 : &tma_w0, second ? k0 - kh : k0, wrow + ti.n0 + (int)cr * 128, bar);
+          }
+          tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
+          if (two) tma_load_2d_bar(sx + 8192, &tma_x, k0, xrow + 64, bar);
+        }
+      }
+      // the leader's last barrier phase covers both CTAs' copies: nobody leaves before it (cluster_sync below)
+      if (leader && it > 0) mbar_wait_bounded(&full_bar[(it - 1) % kRing], (uint32_t)((it - 1) / kRing) & 1u, args.budget_ns);
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (leader CTA only): one instruction drives both SMs. The whole warp runs the loop so
+    // that stage, phase and descriptors are warp-uniform; one elected lane issues. With a single diverged thread the
+    // loop took 673 cycles per k-block, 512 of which the tensor cores need.
+    if (leader) {
+      const uint32_t smem0 = smem_u32(smem);
+      const uint64_t wdesc0 = W_MN ? tc::smem_desc(smem0, kAtomBytes, 1024) : tc::smem_desc(smem0, 16, 1024);
+      const uint64_t xdesc0 = tc::smem_desc(smem0 + kHalfBytes, 16, 1024);
+      constexpr uint32_t kWStep = W_MN ? 2048 >> 4 : 32 >> 4, kXStep = 32 >> 4;      // one 16-deep step in a descriptor's address field
+      int tcnt = 0, gcur = 0; Tile ti;
+      uint32_t stage = 0, phase = 0;
+      tq::Consumer<true> tiles; tiles.setup(&s_ring);
+      tq::Strided seq{pair, npairs, ntiles};
+      for (;; ++tcnt) {
+        int t = -1;
+        if (!dyn) { if (!s_abort) t = seq.next(); }
+        else if (lane == 0 && !s_abort) { t = tiles.next(args.budget_ns); if (t == -2) fail(6, tiles.n); }
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t < 0) break;
+        get_tile(t, gcur, ti);
+        const uint32_t idesc = tc::instr_desc_bf16(256, 0, W_MN, false) | ((uint32_t)(ti.n >> 3) << 17);
+        const int acc = tcnt & 1; const uint32_t aph = (uint32_t)(tcnt >> 1) & 1u;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, args.budget_ns))) { if (lane == 0) fail(2, t); break; }
+        tc::fence_after_sync();
+        const uint32_t d_tmem = tmem_base + (uint32_t)acc * 256;
+        bool ok = true;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) { if (lane == 0) fail(3, t); ok = false; break; }
+          tc::fence_after_sync();
+          if (elect_one()) {
+            const uint64_t wd = wdesc0 + stage * (kStageBytes >> 4), xd = xdesc0 + stage * (kStageBytes >> 4);
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) mma2_bf16(d_tmem, wd + k * kWStep, xd + k * kXStep, idesc, (kb | k) ? 1u : 0u);
+            mma2_commit_both(smem_u32(&empty_bar[stage]));
+          }
+          __syncwarp();
+          if (++stage == kRing) { stage = 0; phase ^= 1u; }
+        }
+        if (!ok) break;
+        if (elect_one()) mma2_commit_both(smem_u32(&tfull_bar[acc]));
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---------------- epilogue: this CTA's 128 weight columns (TMEM lanes) of every token of the tile
+    const int q = warp & 3, set = (warp - 2) >> 2, side = q >> 1;      // side: TMEM lanes 0-63 or 64-127 = one 64-column staging row
+    const uint32_t epi = smem_u32(smem + (size_t)kRing * kStageBytes);
+    const uint32_t tempty_leader[2] = {mapa(smem_u32(&tempty_bar[0]), 0), mapa(smem_u32(&tempty_bar[1]), 0)};
+    const bool issuer = lane == 0 && (q & 1) == 0;                      // one lane per (set, side) stores the staged rows
+    const bool push = MODE != GEMM_GATE_UP && args.push_info != nullptr;
+    // stmatrix: thread 8i + j addresses the 8-column block i of token row j; the 128-byte swizzle is xor by (row & 7)
+    const uint32_t st_row = (uint32_t)(lane & 7) * 128, st_col = (uint32_t)((((q & 1) * 4 + (lane >> 3)) ^ (lane & 7)) << 4);
+    int chunk_no = 0;
+    int tcnt = 0, gcur = 0; Tile ti;
+    tq::Consumer<true> tiles; tiles.setup(&s_ring);
+    tq::Strided seq{pair, npairs, ntiles};
+    auto stage = [&](uint32_t buf, const uint32_t* lo, const uint32_t* hi, float sc[4]) {
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const uint32_t* l = lo + 4 * b; const uint32_t* h = hi + 4 * b;
+        const float s0 = sc[2 * b], s1 = sc[2 * b + 1];
+        st_matrix_x4_trans(buf + (uint32_t)b * 1024 + st_row + st_col,
+                           pack2(__uint_as_float(l[0]) * s0, __uint_as_float(l[1]) * s1), pack2(__uint_as_float(l[2]) * s0, __uint_as_float(l[3]) * s1),
+                           pack2(__uint_as_float(h[0]) * s0, __uint_as_float(h[1]) * s1), pack2(__uint_as_float(h[2]) * s0, __uint_as_float(h[3]) * s1));
+      }
+    };
+    for (;; ++tcnt) {
+      int t = -1;
+      if (!dyn) { if (!s_abort) t = seq.next(); }
+      else {
+        if (lane == 0 && !s_abort) { t = tiles.next(args.budget_ns); if (t == -2) fail(7, tiles.n); }
+        t = __shfl_sync(0xffffffffu, t, 0);
+      }
+      const int acc = tcnt & 1; const uint32_t aph = (uint32_t)(tcnt >> 1) & 1u;
+      int ok = 0;
+      if (t >= 0) {
+        get_tile(t, gcur, ti);
+        if (lane == 0) { ok = mbar_wait_bounded(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0; if (!ok) fail(4, t); }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+      }
+      // the warps of a set stage rows together: they go on or stop together
+      if (!named_barrier_all(1 + 4 + set, 128, ok != 0)) break;
+      tc::fence_after_sync();
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * 256;
+      const int nchunks = ti.n / kChunk;
+      const int col0 = ti.n0 + (int)cr * (kCols / 2) + (MODE == GEMM_GATE_UP ? 0 : side * 64);
+      for (int c = set; c < nchunks; c += 2, ++chunk_no) {
+        const int row = ti.row0 + c * kChunk;
+        float sc[4] = {1.f, 1.f, 1.f, 1.f};          // row factors of this thread's four tokens
+        if ((MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) && args.row_scale) {
+          const float* rs = args.row_scale + row + 2 * (lane & 3);
+          sc[0] = __ldcg(rs); sc[1] = __ldcg(rs + 1); sc[2] = __ldcg(rs + 8); sc[3] = __ldcg(rs + 9);
+        }
+        uint32_t lo[8], hi[8];
+        tmem_ld_frag16(taddr + (uint32_t)c * kChunk, lo);
+        tmem_ld_frag16(taddr + (16u << 16) + (uint32_t)c * kChunk, hi);
+        tc::tmem_ld_wait();
+        if (c + 2 >= nchunks) {                      // this warp has read its last chunk: hand the accumulator back
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) remote_arrive(tempty_leader[acc]);
+        }
+        if (MODE == GEMM_GATE_UP) {
+          // staging of a set: [act | gate | up], one buffer each
+          const uint32_t b_act = epi + (uint32_t)set * 3 * kStgBytes, b_gate = b_act + kStgBytes, b_up = b_gate + kStgBytes;
+          const uint32_t xch = epi + 2 * 3 * kStgBytes + (uint32_t)(set * 2 + (q & 1)) * kXchBytes + (uint32_t)lane * 16;
+          if (side == 1) {
+            tc::st_shared_v4(xch, lo[0], lo[1], lo[2], lo[3]); tc::st_shared_v4(xch + 512, lo[4], lo[5], lo[6], lo[7]);
+            tc::st_shared_v4(xch + 1024, hi[0], hi[1], hi[2], hi[3]); tc::st_shared_v4(xch + 1536, hi[4], hi[5], hi[6], hi[7]);
+          }
+          if (issuer) bulk_wait_read<0>();           // the rows staged for the chunk before have left
+          named_barrier(1 + set, 128);
+          float one[4] = {1.f, 1.f, 1.f, 1.f};
+          if (side == 1) {
+            if (args.out2) stage(b_up, lo, hi, one);
+          } else {
+            if (args.out2) stage(b_gate, lo, hi, one);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                uint32_t* r = (h ? hi : lo) + 4 * b;
+                const int4 u4 = tc::ld_shared_v4(xch + h * 1024 + b * 512);
+                const float u[4] = {__int_as_float(u4.x), __int_as_float(u4.y), __int_as_float(u4.z), __int_as_float(u4.w)};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const float g = __uint_as_float(r[i]);
+                  r[i] = __float_as_uint(g / (1.f + __expf(-g)) * u[i]);
+                }
+              }
+            }
+            stage(b_act, lo, hi, sc);
+          }
+          tc::fence_async_smem();
+          named_barrier(1 + set, 128);
+          if (issuer) {
+            if (side == 0) {
+              tc::tma_store_2d(&tma_out, b_act, col0, row);
+              if (args.out2) tc::tma_store_2d(&tma_out2, b_gate, col0, row);
+            } else if (args.out2) {
+              tc::tma_store_2d(&tma_out2, b_up, args.N + col0, row);
+            }
+            bulk_commit();
+          }
+        } else {
+          const uint32_t buf = epi + (uint32_t)((set * 2 + side) * 2 + (chunk_no & 1)) * kStgBytes;
+          const int bar = 1 + set * 2 + side;
+          if (issuer) bulk_wait_read<1>();           // the store issued two chunks ago has read this buffer
+          named_barrier(bar, 64);
+          stage(buf, lo, hi, sc);
+          if (!push) {
+            tc::fence_async_smem();
+            named_barrier(bar, 64);
+            if (issuer) { tc::tma_store_2d(&tma_out, buf, col0, row); bulk_commit(); }
+          } else {
+            // "push": every row goes straight to the rank its token came from (peer memory, plain 16-byte stores, 8
+            // lanes per 128-byte run)
+            named_barrier(bar, 64);
+            const int tid = (q & 1) * 32 + lane, j = tid & 7;
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+              const int rr = p * 8 + (tid >> 3), info = args.push_info[row + rr];
+              if (info < 0) continue;
+              const int src = info / args.push_rows, idx = info - src * args.push_rows;
+              if (src >= args.push_ranks) { if (j == 0) note(8, row + rr, MEP_ERR_BOUNDS); continue; }
+              unsigned char* base = args.push_base + (size_t)src * args.push_stride;
+              st_v4(base + ((size_t)idx * args.N + col0) * 2 + j * 16, tc::ld_shared_v4(buf + rr * 128 + ((j ^ (rr & 7)) << 4)));
+              if (args.push_wsrc && col0 == 0 && j == 0)
+                *reinterpret_cast<float*>(args.push_wbase + (size_t)src * args.push_stride + (size_t)idx * 4) = args.push_wsrc[row + rr];
+            }
+          }
+        }
+      }
+    }
+    if (lane == 0) bulk_wait_all<0>();       // shared memory must outlive the stores reading it
+  }
+
+  // ---------------- teardown: nobody leaves while the peer may still signal into this CTA
+  tc::fence_before_sync();
+  __syncthreads();
+  cluster_sync();
+  tc::fence_after_sync();
+  if (warp == 1) tmem_dealloc2(tmem_base, 512);
+  if (leader && threadIdx.x == 0) tq::scheduler_done(args.sched, args.sched_ctas > 0 ? args.sched_ctas / 2 : npairs);
+}
+
+}  // namespace tp
+}  // namespace mep
+
+// One grouped GEMM launch on CTA pairs; same contract as mep_grouped_gemm for modes 0-3.
+extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, int64_t a_cols, int64_t a_ld,
+                                     const void* b0, const void* b1, int64_t b_rows, int64_t b_cols, int64_t b_ld,
+                                     const mep::GemmArgs* args_in, int num_ctas, cudaStream_t stream) {
+  using namespace mep;
+  const GemmArgs& args = *args_in;
+  MEP_REQUIRE(mode >= GEMM_GATE_UP && mode <= GEMM_DGRAD_GU, "gemm (CTA pairs): mode %d not supported", mode);
+  MEP_REQUIRE(args.G >= 1 && args.G <= tp::kMaxGroups, "gemm: G=%d out of range [1,%d]", args.G, tp::kMaxGroups);
+  MEP_REQUIRE(args.K % 64 == 0 && args.N % (mode == GEMM_GATE_UP ? 128 : 256) == 0, "gemm (CTA pairs): K=%d N=%d not tileable", args.K, args.N);
+  num_ctas &= ~1;
+  MEP_REQUIRE(num_ctas >= 2, "gemm (CTA pairs): needs at least two CTAs");
+  CUtensorMap mx, mw0, mw1, mo, mo2;
+  if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 64)) return -1;
+  auto weights = [&](CUtensorMap* m, const void* b) {
+    if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1);
+    if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2);
+    return tmap_rows(m, b, b_rows, b_cols, b_ld, 64, 128);
+  };
+  if (weights(&mw0, b0)) return -1;
+  if (b1) { if (weights(&mw1, b1)) return -1; } else mw1 = mw0;
+  if (args.push_info) mo = mx;
+  else if (tmap_rows(&mo, args.out, a_rows, args.N, args.ldo, 64, tp::kChunk)) return -1;
+  if (mode == GEMM_GATE_UP && args.out2) { if (tmap_rows(&mo2, args.out2, a_rows, 2 * (int64_t)args.N, 2 * (int64_t)args.N, 64, tp::kChunk)) return -1; }
+  else mo2 = mo;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(num_ctas); cfg.blockDim = dim3(tp::kThreads); cfg.dynamicSmemBytes = tp::kSmem; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+#define MEP_TP_CASE(M)                                                                             \
+  case M:                                                                                          \
+    if (allow_smem((const void*)tp::tok_pair_kernel<M>, tp::kSmem)) return -1;                       \
+    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tp::tok_pair_kernel<M>, mx, mw0, mw1, mo, mo2, args));   \
+    break;
+  switch (mode) {
+    MEP_TP_CASE(GEMM_GATE_UP) MEP_TP_CASE(GEMM_DOWN) MEP_TP_CASE(GEMM_DGRAD) MEP_TP_CASE(GEMM_DGRAD_GU)
+    default: return set_error("gemm (CTA pairs): unknown mode %d", mode);
+  }
+#undef MEP_TP_CASE
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return 0;
+}

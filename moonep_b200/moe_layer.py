@@ -89,6 +89,7 @@ class ExpertParallelMoE:
         if ready_flags is None:             # MOONEP_READY_FLAGS=0: the GEMMs wait for the whole dispatch
             ready_flags = os.environ.get("MOONEP_READY_FLAGS", "1") != "0"
         self.ready_flags = ready_flags
+        self._skip_pad = gg.skips_padding() and self.H % 256 == 0 and self.Hp % 256 == 0
         self._local = buffer._states[0].local       # single rank: see _forward_local
         dev = buffer.hidden_nvsh_buffer_view.device
         self._side = torch.cuda.Stream(device=dev)
@@ -127,6 +128,10 @@ class ExpertParallelMoE:
             return self._upd_mask
         return update_mask(plan.experts_to_copy, self.buf.rank, self.geo.epn, self._upd_mask, self._upd_hit, self._upd_ones)
 
+    def _pad(self, plan):
+        """The plan's table of padding rows, for GEMMs that skip them."""
+        return plan.zero_fill_ranges if self._skip_pad else None
+
     # weights / grads as [2*epn, in, out]
     def _W(self, n):
         return self.pools.compute_weight(n)
@@ -158,13 +163,13 @@ class ExpertParallelMoE:
                 self._w.copy_(w_view)
                 stashed = self._side.record_event()
         gu = self._gu if need_backward else None
-        Wg, Wu, Wd = self._W("gate"), self._W("up"), self._W("down")
+        Wg, Wu, pad = self._W("gate"), self._W("up"), self._pad(plan)
         if ev is not None:
-            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(0, epn))
+            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(0, epn), pad=pad)
             torch.cuda.current_stream().wait_event(ev)
-            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(epn, 2 * epn))
+            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(epn, 2 * epn), pad=pad)
         else:
-            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w)
+            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, pad=pad)
         return self._forward_tail(plan, cu, stashed, need_backward)
 
     def _forward_local(self, hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, need_backward):
@@ -174,8 +179,9 @@ class ExpertParallelMoE:
         buf, st = self.buf, self.buf._st()
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
         _, _, cu, plan = buf._dispatch_local(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, None, out=(x, w))
-        gg.gate_up(x, self._W("gate"), self._W("up"), cu, self._act, self._gu if need_backward else None, row_scale=w)
-        gg.down(self._act, self._W("down"), cu, st.hidden_local)
+        pad = self._pad(plan)
+        gg.gate_up(x, self._W("gate"), self._W("up"), cu, self._act, self._gu if need_backward else None, row_scale=w, pad=pad)
+        gg.down(self._act, self._W("down"), cu, st.hidden_local, pad=pad)
         out, _ = buf._combine_local(plan, st.hidden_local, None)
         return out, MoEContext(plan, cu, x, w, self._act, self._gu) if need_backward else None
 
@@ -201,11 +207,12 @@ class ExpertParallelMoE:
         # in tile order) additionally wait for their slot's flag, not for the whole prefetch.
         slots = buf.slot_ready() if g.R > 1 else None
         tk = gg.Ticket(self._act.device, self._total_sms)
-        free = min(ready.free_sms, self._total_sms - self._comm_sms)
-        gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, num_ctas=free, ticket=tk, ready=ready, slots=slots)
+        free = min(ready.free_sms, self._total_sms - self._comm_sms) & ~1      # CTA pairs
+        gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, num_ctas=free, ticket=tk, ready=ready, slots=slots,
+                   pad=self._pad(plan))
         with torch.cuda.stream(comm):
             gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, num_ctas=self._total_sms - free, ticket=tk,
-                       ready=ready, slots=slots)
+                       ready=ready, slots=slots, pad=self._pad(plan))
             joined = comm.record_event()
         main.wait_event(joined)
         return self._forward_tail(plan, cu, stashed, need_backward)
@@ -218,10 +225,10 @@ class ExpertParallelMoE:
         if g.off_push:
             # push-combine: the down GEMM's epilogue sends every row to its source rank while the
             # GEMM is still running; what is left of the combine is a barrier and a local sum
-            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, push=buf.push_target())
+            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, push=buf.push_target(), pad=self._pad(plan))
             out, _, _ = buf.combine_pushed()
         else:
-            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view)
+            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, pad=self._pad(plan))
             out, _, _ = buf.combine(plan=plan, hidden_nvsh=buf.hidden_nvsh_buffer_view, zero_copy=True)
         ctx = MoEContext(plan, cu, self._x, self._w, self._act, self._gu) if need_backward else None
         return out, ctx
@@ -272,7 +279,7 @@ class ExpertParallelMoE:
         pools = self.pools
         pair = lambda n: (pools.local_grad(n), pools.reduce_view(n))      # noqa: E731
         Wg, Wu, Wd = self._W("gate"), self._W("up"), self._W("down")
-        shard = buf.hidden_nvsh_buffer_view
+        shard, pad = buf.hidden_nvsh_buffer_view, self._pad(ctx.plan)
         # slots shared with other layers hold someone else's experts by now: fetch this layer's again
         # (on the comm stream, behind the dispatch); the dgrad GEMMs wait per slot
         refetch = multi and getattr(pools, "shared", None) is not None
@@ -280,7 +287,7 @@ class ExpertParallelMoE:
         if self._local:
             dy = shard
             buf._dispatch_local(grad_out_sh, None, None, None, ctx.plan, out=(shard, None))
-            gg.dgrad(dy, Wd, ctx.cu, self._dA)
+            gg.dgrad(dy, Wd, ctx.cu, self._dA, pad=pad)
         elif self.ready_flags and ctx.plan.send_list is not None:
             # dgrad(down) starts on the tiles of the re-dispatched output grad as they complete
             dy, _, _, _, ready, _ = buf.dispatch_ready(grad_out_sh, plan=ctx.plan)
@@ -288,10 +295,10 @@ class ExpertParallelMoE:
                 ev_pf = buf.prefetch_weight(plan=ctx.plan, async_finish=True, **pools.prefetch_kwargs())
                 slots = buf.slot_ready()
             tk = gg.Ticket(self._act.device, self._total_sms)
-            free = min(ready.free_sms, self._total_sms - self._comm_sms)
-            gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=free, ticket=tk, ready=ready, slots=slots)
+            free = min(ready.free_sms, self._total_sms - self._comm_sms) & ~1      # CTA pairs
+            gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=free, ticket=tk, ready=ready, slots=slots, pad=pad)
             with torch.cuda.stream(buf.comm_stream):
-                gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=self._total_sms - free, ticket=tk, ready=ready, slots=slots)
+                gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=self._total_sms - free, ticket=tk, ready=ready, slots=slots, pad=pad)
                 joined = buf.comm_stream.record_event()
             main.wait_event(joined)
         else:
@@ -299,7 +306,7 @@ class ExpertParallelMoE:
             if refetch:
                 ev_pf = buf.prefetch_weight(plan=ctx.plan, async_finish=True, **pools.prefetch_kwargs())
                 slots = buf.slot_ready()
-            gg.dgrad(dy, Wd, ctx.cu, self._dA, slots=slots)
+            gg.dgrad(dy, Wd, ctx.cu, self._dA, slots=slots, pad=pad)
         if ev_pf is not None:
             main.wait_event(ev_pf)      # dgrad(gate/up) further down reads the other two projections' slots
         dw_view = buf.router_weight_buffer_view
@@ -311,7 +318,7 @@ class ExpertParallelMoE:
             assert not acc, "the optimizer cannot sit in the GEMM epilogue while gradients are accumulated"
             mask, lr_e = self._update_mask(ctx.plan), self.epilogue_lr
             upd = lambda n: (self._W(n), lr_e, mask)      # noqa: E731
-        gg.wgrad(ctx.act, dy, ctx.cu, self._dW("down"), accumulate=acc, zero_empty_below=epn, update=upd("down"))
+        gg.wgrad(ctx.act, dy, ctx.cu, self._dW("down"), accumulate=acc, zero_empty_below=epn, pad=pad, update=upd("down"))
         if not multi:
             self._optimizer("down", main)
         dW_gate, dG = self._dW("gate"), self._dgu[:, :Hp]
@@ -320,7 +327,7 @@ class ExpertParallelMoE:
         # wgrad(up),  reduce(up)  -- every communication kernel still has a GEMM to run beside, except the last.
         gate_late = self.epilogue_lr is not None
         if not gate_late:
-            gg.wgrad(ctx.x, dG, ctx.cu, dW_gate, accumulate=acc, zero_empty_below=epn)
+            gg.wgrad(ctx.x, dG, ctx.cu, dW_gate, accumulate=acc, zero_empty_below=epn, pad=pad)
         ev_red = None
         if multi:
             # the weight-gradient GEMMs overwrite the slots they use, so consumed slots need no zeroing
@@ -329,10 +336,10 @@ class ExpertParallelMoE:
             ev_red = buf.reduce_grad_subset(ctx.plan, first, async_finish=ov, clear_slots=acc)
             self._optimizer("down", ev_red if ov else main)
         if ov and multi:
-            ev = self._beside_comm(lambda n, tk: gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, num_ctas=n, ticket=tk))
+            ev = self._beside_comm(lambda n, tk: gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, num_ctas=n, ticket=tk, pad=pad))
             main.wait_event(ev)
         else:
-            gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard)
+            gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, pad=pad)
         if not gate_late:
             self._optimizer("gate", main, *([ev_red] if ev_red is not None else []))
         grad_hidden, grad_w, ev_comb = buf.combine(plan=ctx.plan, hidden_nvsh=shard, route_weights_nvs=dw_view,
@@ -340,20 +347,20 @@ class ExpertParallelMoE:
         if gate_late:
             if ov:
                 ev = self._beside_comm(lambda n, tk: gg.wgrad(ctx.x, dG, ctx.cu, dW_gate, accumulate=acc, zero_empty_below=epn,
-                                                              num_ctas=n, ticket=tk, update=upd("gate")))
+                                                              num_ctas=n, ticket=tk, pad=pad, update=upd("gate")))
                 main.wait_event(ev)   # also covers the combine, which precedes that launch on the comm stream
             else:
-                gg.wgrad(ctx.x, dG, ctx.cu, dW_gate, accumulate=acc, zero_empty_below=epn, update=upd("gate"))
+                gg.wgrad(ctx.x, dG, ctx.cu, dW_gate, accumulate=acc, zero_empty_below=epn, pad=pad, update=upd("gate"))
             ev_red_g = None
             if multi:
                 ev_red_g = buf.reduce_grad_subset(ctx.plan, [pair("gate")], async_finish=ov, clear_slots=acc)
         dW_up, dU = self._dW("up"), self._dgu[:, Hp:]
         if ov and (multi or not gate_late):      # a communication kernel was just queued on the comm stream
             ev = self._beside_comm(lambda n, tk: gg.wgrad(ctx.x, dU, ctx.cu, dW_up, accumulate=acc, zero_empty_below=epn,
-                                                          num_ctas=n, ticket=tk, update=upd("up")))
+                                                          num_ctas=n, ticket=tk, pad=pad, update=upd("up")))
             main.wait_event(ev)       # also covers the combine, which precedes that launch on the comm stream
         else:
-            gg.wgrad(ctx.x, dU, ctx.cu, dW_up, accumulate=acc, zero_empty_below=epn, update=upd("up"))
+            gg.wgrad(ctx.x, dU, ctx.cu, dW_up, accumulate=acc, zero_empty_below=epn, pad=pad, update=upd("up"))
         if gate_late:
             self._optimizer("gate", main, *([ev_red_g] if ev_red_g is not None else []))
         self.grads_pending = None

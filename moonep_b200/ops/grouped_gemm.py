@@ -36,7 +36,8 @@ class GemmArgs(C.Structure):
                 ("tile_done", C.c_void_p), ("tile_epoch", C.c_void_p), ("status_host", C.c_void_p),
                 ("group_flags", C.c_void_p), ("group_epoch", C.c_void_p),
                 ("push_rows", C.c_int32), ("push_ranks", C.c_int32), ("group_first", C.c_int32), ("sched_ctas", C.c_int32),
-                ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("reserved1", C.c_int32)]
+                ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("reserved1", C.c_int32),
+                ("pad_rows", C.c_void_p)]
 
 
 class PushTarget:
@@ -135,7 +136,7 @@ def check_status(device="cuda") -> None:
 
 def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=None, row_scale=None, ldo=0,
             accumulate=False, zero_empty_below=0, a_cols=None, b_rows=None, b_cols=None, b_ld=None, groups=None, num_ctas=None,
-            dynamic=False, ticket=None, push=None, push_w=None, ready=None, slots=None):
+            dynamic=False, ticket=None, push=None, push_w=None, ready=None, slots=None, pad=None):
     lib = _native.load()
     assert a.dtype == torch.bfloat16 and b0.dtype == torch.bfloat16
     assert cu.dtype == torch.int32 and cu.is_contiguous()
@@ -162,6 +163,7 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
         args.tile_done, args.tile_epoch = ready.done_ptr, ready.epoch_ptr
     if slots is not None:
         args.group_flags, args.group_epoch, args.group_first = slots.flags_ptr, slots.epoch_ptr, slots.first
+    args.pad_rows = _native.ptr(pad)
     if push is not None:
         assert mode in (DOWN, DGRAD, DGRAD_GU) and push.info.dtype == torch.int32 and push.info.numel() >= a.shape[0]
         args.push_info, args.push_base, args.push_stride = push.info.data_ptr(), push.base, push.stride
@@ -173,8 +175,9 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
     a_ld = a.stride(0)
     a_cols = a.shape[1] if a_cols is None else a_cols
     fn = lib.mep_grouped_gemm
-    if mode != WGRAD and push is None and ready is None and slots is None and os.environ.get("MOONEP_GEMM_2CTA", "0") == "1":
-        fn = lib.mep_grouped_gemm_2cta      # CTA-pair kernels (tcgen05 cta_group::2), 256-token tiles
+    # CTA pairs (tcgen05 cta_group::2) unless they are switched off or there is no pair to run on
+    if mode != WGRAD and (num_ctas or _num_sms(a.device)) >= 2 and os.environ.get("MOONEP_GEMM_2CTA", "1") == "1":
+        fn = lib.mep_grouped_gemm_2cta
     rc = fn(mode, C.c_void_p(a.data_ptr()), C.c_int64(a_rows), C.c_int64(a_cols), C.c_int64(a_ld),
                               C.c_void_p(b0.data_ptr()), C.c_void_p(_native.ptr(b1)), C.c_int64(b_rows),
                               C.c_int64(b_cols), C.c_int64(b_ld), C.byref(args),
@@ -188,43 +191,45 @@ def _w2d(w):
 
 
 def gate_up(x, wg, wu, cu, act_out, gu_out=None, row_scale=None, groups=None, num_ctas=None, dynamic=False, ticket=None,
-            ready=None, slots=None):
+            ready=None, slots=None, pad=None):
     """``act_out[r] = row_scale[r] * silu(x[r] Wg[g]) * (x[r] Wu[g])``; optionally stores the
     pre-activations ``gu_out = [x Wg | x Wu]`` (``[NvS, 2*out]``) for the backward pass.
     ``ready`` (a ``TileReady`` from ``Buffer.dispatch_ready``): ``x`` is still being filled by that
     dispatch; every 128-row tile is loaded only once its flag says it is complete.  Launch with
     ``num_ctas <= ready.free_sms`` while the dispatch kernel may still be running.
     ``slots`` (a ``SlotReady`` from ``Buffer.slot_ready``): the weights of the groups ``>= slots.first`` are
-    prefetched experts that may still be on their way; each such group is loaded once its slot is complete."""
+    prefetched experts that may still be on their way; each such group is loaded once its slot is complete.
+    ``pad`` (every GEMM of this module; int32 ``[G, 2]``, a plan's ``zero_fill_ranges``): rows behind a group's real ones,
+    rounded up to 32, are then neither computed nor read."""
     G, K, N = wg.shape
     assert wu.shape == wg.shape and x.shape[1] == K and N % 128 == 0 and K % 64 == 0
     rows, cols = _w2d(wg)
     _launch(GATE_UP, x, wg, wu, cu, N=N, K=K, b_group_rows=K, out=act_out, out2=gu_out, row_scale=row_scale,
             ldo=act_out.stride(0), b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket,
-            ready=ready, slots=slots)
+            ready=ready, slots=slots, pad=pad)
 
 
-def down(act, wd, cu, out, row_scale=None, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None):
+def down(act, wd, cu, out, row_scale=None, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, pad=None):
     """``out[r] = row_scale[r] * (act[r] Wd[g])`` with ``Wd [G, inner, hidden]``.  With ``push`` (a
     ``PushTarget``) the rows are not written to ``out`` but sent to the ranks their tokens came from."""
     G, K, N = wd.shape
     assert act.shape[1] == K and N % 256 == 0 and K % 64 == 0
     rows, cols = _w2d(wd)
     _launch(DOWN, act, wd, None, cu, N=N, K=K, b_group_rows=K, out=out, row_scale=row_scale, ldo=out.stride(0),
-            b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, push=push)
+            b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, push=push, pad=pad)
 
 
-def dgrad(dy, w, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, ready=None, slots=None):
+def dgrad(dy, w, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, ready=None, slots=None, pad=None):
     """``out[r] = dy[r] W[g]^T`` with ``W [G, in, out]`` -> ``out [NvS, in]``.  ``ready`` / ``slots``: as in ``gate_up``."""
     G, N, K = w.shape
     assert dy.shape[1] == K and N % 256 == 0 and K % 64 == 0
     rows, cols = _w2d(w)
     _launch(DGRAD, dy, w, None, cu, N=N, K=K, b_group_rows=N, out=out, ldo=out.stride(0),
             b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, ready=ready,
-            slots=slots)
+            slots=slots, pad=pad)
 
 
-def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, push_w=None):
+def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, push_w=None, pad=None):
     """``out[r] = dG[r] Wg[g]^T + dU[r] Wu[g]^T`` with ``dgu = [dG | dU]`` (``[NvS, 2*inner]``).  With
     ``push`` the rows (and ``push_w[r]``, e.g. the route-weight grads) go to their source ranks."""
     G, N, Kh = wg.shape
@@ -232,7 +237,13 @@ def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=Fals
     rows, cols = _w2d(wg)
     _launch(DGRAD_GU, dgu, wg, wu, cu, N=N, K=2 * Kh, b_group_rows=N, out=out, ldo=out.stride(0),
             b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket,
-            push=push, push_w=push_w)
+            push=push, push_w=push_w, pad=pad)
+
+
+def skips_padding() -> bool:
+    """Whether every GEMM of a layer runs on the CTA-pair kernels, which honour ``pad``: only then may one leave
+    padding rows unwritten that another would otherwise read."""
+    return os.environ.get("MOONEP_GEMM_2CTA", "1") == "1" and os.environ.get("MOONEP_WGRAD_2CTA", "1") != "0"
 
 
 def wgrad_update_supported(M: int, N: int) -> bool:
@@ -241,7 +252,7 @@ def wgrad_update_supported(M: int, N: int) -> bool:
 
 
 def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num_ctas=None, dynamic=False, ticket=None,
-          update=None):
+          update=None, pad=None):
     """``out[g] (+)= x_g^T dy_g`` in fp32; ``out [G, in, out_dim]``.  ``dy`` may be a column slice
     of a wider matrix (row pitch = ``dy.stride(0)``).  Groups without rows are left untouched,
     except that with ``accumulate=False`` empty groups ``g < zero_empty_below`` are zeroed (local
@@ -265,6 +276,7 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
         args.G, args.N, args.K, args.M_w = G, N, 0, M
         args.accumulate, args.g_begin, args.g_end = (1 if accumulate else 0), G0, G1
         args.zero_empty_below = zero_empty_below
+        args.pad_rows = _native.ptr(pad)
         args.out = out.data_ptr()
         args.status = _status(x.device).data_ptr()
         args.status_host = _status_host(x.device).data_ptr()
@@ -286,7 +298,7 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
         return
     assert update is None, "wgrad(update=...) needs weight shapes that are multiples of 256"
     _launch(WGRAD, x, dy, None, cu, N=N, M_w=M, out=out, accumulate=accumulate, zero_empty_below=zero_empty_below,
-            b_rows=dy.shape[0], b_cols=N, b_ld=dy.stride(0), groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket)
+            b_rows=dy.shape[0], b_cols=N, b_ld=dy.stride(0), groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, pad=pad)
 
 
 def swiglu_bwd(dA, gu, w, dgu, dw, cu, num_blocks=None):

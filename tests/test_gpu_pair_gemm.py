@@ -1,0 +1,65 @@
+"""CTA-pair grouped GEMMs with a table of padding rows: groups whose real sizes lie around the kernels' steps (32-token
+units, 128-row halves, 256-row tiles, evenly shared tiles above that), against an fp32 reference."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = {"units": [1, 31, 32, 33, 64, 65, 0, 127], "tiles": [128, 129, 255, 256, 257, 0, 300, 511], "large": [513, 1000, 0, 1281]}
+
+
+def _rel(a, b):
+    return float((a.float() - b.float()).norm() / (b.float().norm() + 1e-12))
+
+
+@pytest.mark.parametrize("dynamic", [False, True], ids=["static", "dynamic"])
+@pytest.mark.parametrize("kn", [(256, 256), (320, 512)], ids=["256x256", "320x512"])
+@pytest.mark.parametrize("sizes", list(SIZES))
+def test_padding_rows_are_skipped(sizes, kn, dynamic, cuda_device):
+    from moonep_b200.ops import grouped_gemm as gg
+    n = SIZES[sizes]
+    (K, N), G = kn, len(n)
+    padded = [(r + 127) // 128 * 128 for r in n]
+    ends = torch.tensor(padded).cumsum(0)
+    cu = ends.to(torch.int32).cuda()
+    pad = torch.tensor([[int(e) - p + r, p - r] if p > r else [0, 0] for r, p, e in zip(n, padded, ends)], dtype=torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rows = int(ends[-1]) + 128
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, wg, wu, wd, scale = bf(rows, K, sc=0.5), bf(G, K, N, sc=0.05), bf(G, K, N, sc=0.05), bf(G, N, 256, sc=0.05), torch.rand(rows, device="cuda", generator=g) + 0.5
+    full = lambda c, dt=torch.bfloat16: torch.full((rows, c), float("nan"), dtype=dt, device="cuda")    # noqa: E731
+    act, gu, y, dA = full(N), full(2 * N), full(256), full(N)
+    kw = dict(pad=pad, dynamic=dynamic)
+    gg.gate_up(x, wg, wu, cu, act, gu, row_scale=scale, **kw)
+    gg.down(act, wd, cu, y, row_scale=scale, **kw)
+    if N % 256 == 0:
+        gg.dgrad(y, wd, cu, dA, **kw)
+    dW = torch.full((G, 256, N), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    gg.check_status()
+    written = torch.zeros(rows, dtype=torch.bool)
+    for i, (r, p, e) in enumerate(zip(n, padded, ends.tolist())):
+        a = e - p
+        written[a:a + (r + 31) // 32 * 32] = True
+        if r == 0:
+            continue
+        s = slice(a, a + r)
+        gr, ur = x[s].float() @ wg[i].float(), x[s].float() @ wu[i].float()
+        # bf16 results of fp32 sums: half a bf16 ulp is 2^-9
+        assert _rel(gu[s, :N], gr) < 4e-3 and _rel(gu[s, N:], ur) < 4e-3, f"group {i} ({r} rows): pre-activations"
+        assert _rel(act[s], torch.nn.functional.silu(gr) * ur * scale[s, None]) < 4e-3, f"group {i} ({r} rows): swiglu"
+        assert _rel(y[s], (act[s].float() @ wd[i].float()) * scale[s, None]) < 4e-3, f"group {i} ({r} rows): down"
+        assert _rel(dA[s], y[s].float() @ wd[i].float().T) < 4e-3, f"group {i} ({r} rows): dgrad"
+    for t in (act, gu, y, dA):
+        nan = torch.isnan(t.float()).any(dim=1).cpu()
+        assert not bool(nan[written].any()) and bool(nan[~written].all()), "rows behind the 32-row step were written"
+    # weight gradients read no row behind the step (NaN there); the rows up to it must be zero on one side, as a
+    # dispatch leaves them
+    for i, (r, p, e) in enumerate(zip(n, padded, ends.tolist())):
+        y[e - p + r:e - p + (r + 31) // 32 * 32] = 0
+    gg.wgrad(y, act, cu, dW, zero_empty_below=G, **kw)
+    torch.cuda.synchronize()
+    gg.check_status()
+    for i, (r, p, e) in enumerate(zip(n, padded, ends.tolist())):
+        ref = y[e - p:e - p + r].float().T @ act[e - p:e - p + r].float()
+        assert torch.equal(dW[i], torch.zeros_like(dW[i])) if r == 0 else _rel(dW[i], ref) < 1e-4, f"group {i} ({r} rows): wgrad"
