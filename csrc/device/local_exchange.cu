@@ -10,30 +10,10 @@
 // Counterpart of the reference's dispatch / combine for num_ep_ranks = 1 (moonep/dispatch.py:50-692,
 // moonep/combine.py:40-511), which has no separate path for it.
 #include "prims.cuh"
+#include "local_args.h"
 #include "../host/launch.h"
 
 namespace mep {
-
-struct LocalDispatchArgs {
-  const __nv_bfloat16* hidden;   // [S, H]
-  const float* weights;          // [S, K] or null
-  __nv_bfloat16* out_hidden;     // [NvS, H]
-  float* out_weights;            // [NvS]
-  int32_t* out_srcinfo;          // [NvS] provenance table or null
-  int32_t* dst;                  // [N]   plan (written when fresh, read otherwise)
-  int32_t* zero_fill;            // [2E, 2]
-  // fresh only
-  const int32_t* topk;           // [N]
-  const int32_t* tpe;            // [E]
-  int32_t* cu_seqlens;           // [2E]
-  int32_t* experts_to_copy;      // [1, E]
-  int32_t* remote_stats;         // [2]
-  int32_t* dup_groups;           // [NvS, 3]
-  int32_t* dup_loffs;            // [NvS]
-  int32_t* dup_counts;           // [2]
-  uint32_t* sync;                // [0] launches completed, [1] start tickets, [2] finished CTAs, [16 + b] flag of CTA b
-  int32_t* hist;                 // [grid, E] expert histogram of each CTA's tokens
-};
 
 constexpr int kLocThreads = 256, kLocWarps = kLocThreads / 32;
 constexpr int kLocEntries = 1024;          // top-k entries ranked and copied at a time by one CTA
@@ -313,14 +293,6 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
 }
 
 // ------------------------------------------------------------------ combine
-struct LocalCombineArgs {
-  const int32_t* dst;            // [N] plan
-  const __nv_bfloat16* rows;     // [NvS, H]
-  const float* weights;          // [NvS] or null
-  __nv_bfloat16* out;            // [S, H]
-  float* out_weights;            // [S, K] or null
-};
-
 __device__ __forceinline__ void add_bf16x8(float* acc, const int4& x) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&x);
 #pragma unroll

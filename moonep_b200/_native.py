@@ -76,6 +76,15 @@ class LocalCombineArgs(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("dst", "rows", "weights", "out", "out_weights")]
 
 
+class MoeLocal(C.Structure):
+    _fields_ = ([("ctx", C.c_void_p)] + [(n, C.c_int32) for n in ("S", "H", "Hp", "K", "E", "NvS", "blocks", "combine_blocks",
+                                                                 "num_ctas", "reserved")]
+                + [("plan_off", C.c_int64 * 8)]
+                + [(n, C.c_void_p) for n in ("w_gate", "w_up", "w_down", "shard", "shard_w", "srcinfo", "x", "w", "act", "gu", "dA",
+                                             "dgu", "dw_gate", "dw_up", "dw_down", "sync", "hist", "status", "status_host")]
+                + [("budget_ns", C.c_uint64)])
+
+
 class SendOrderArgs(C.Structure):
     _fields_ = [("dst", C.c_void_p), ("cu_seqlens", C.c_void_p), ("send_list", C.c_void_p), ("send_meta", C.c_void_p),
                 ("hist", C.c_void_p), ("bucket", C.c_void_p)]
@@ -150,6 +159,11 @@ def load(build_if_missing: bool = True):
     lib.mep_mc_add_device.argtypes = [vp]
     lib.mep_mc_bind_map.argtypes = [vp, vp, C.POINTER(C.c_ulonglong)]
     lib.mep_mc_destroy.argtypes = [vp]
+    lib.mep_route.argtypes = [vp] * 5 + [i32] * 3 + [vp]
+    lib.mep_route_bwd.argtypes = [vp] * 4 + [i32] * 3 + [vp]
+    lib.mep_swiglu.argtypes = [vp, vp, C.c_int64, i32, vp]
+    lib.mep_moe_local_forward.argtypes = [vp] * 7 + [i32, vp]
+    lib.mep_moe_local_backward.argtypes = [vp] * 5 + [i32, C.c_float, vp, vp]
     _LIB = lib
     return lib
 
@@ -170,5 +184,9 @@ def ctx_array(ctx_ptrs):
     return arr
 
 
+def raw_stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def cur_stream() -> C.c_void_p:
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return C.c_void_p(raw_stream())

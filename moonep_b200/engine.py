@@ -196,25 +196,86 @@ def allocate_plan(st: RankState, with_send_list: bool = False):
     """Plan-owned tensors plus cu_seqlens for one rank (reference: planning.py:1168-1215).  They are views of ONE
     allocation, each starting on a 16-byte boundary: a plan costs one allocator call instead of eight, which is
     what a small dispatch would otherwise wait for."""
-    g = st.geo
+    sizes, total, _ = _plan_layout(st, with_send_list)
+    parts = torch.empty(total, dtype=torch.int32, device=st.device).split(sizes)[::2]
+    if not st.local:
+        parts[6].zero_()
+    if with_send_list:
+        parts[9].zero_()
+    return _plan_of_parts(st.geo, parts, with_send_list)
+
+
+def _plan_layout(st: RankState, with_send_list: bool = False):
+    """``(sizes and gaps, total, first element of every field)`` of a plan's allocation."""
     key = "plan_layout_send" if with_send_list else "plan_layout"
     lay = st.scratch.get(key)
     if lay is None:
+        g = st.geo
         sizes = [g.N, g.R * g.epn, 4 * g.epn, 2, 3 * g.NvS, g.NvS, 2, 2 * g.epn] + ([g.N, 4] if with_send_list else [])
-        pad = [-n % 4 for n in sizes]
-        lay = st.scratch[key] = ([x for pair in zip(sizes, pad) for x in pair], sum(sizes) + sum(pad))
-    parts = torch.empty(lay[1], dtype=torch.int32, device=st.device).split(lay[0])[::2]
-    if not st.local:
-        parts[6].zero_()
-    extra = {}
-    if with_send_list:
-        parts[9].zero_()
-        extra = dict(send_list=parts[8], send_meta=parts[9])
+        both, first, off = [], [], 0
+        for n in sizes:
+            first.append(off)
+            both += [n, -n % 4]
+            off += n + -n % 4
+        lay = st.scratch[key] = (both, off, first)
+    return lay
+
+
+def _plan_of_parts(g: Geometry, parts, with_send_list: bool = False):
+    extra = dict(send_list=parts[8], send_meta=parts[9]) if with_send_list else {}
     plan = MoonEPCommPlan.of_parts(
         dst=parts[0], experts_to_copy=parts[1].view(g.R, g.epn), zero_fill_ranges=parts[2].view(2 * g.epn, 2),
         remote_stats=parts[3], N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K,
         dup_groups=parts[4].view(g.NvS, 3), dup_loffs=parts[5], dup_counts=parts[6], **extra)
     return plan, parts[7]
+
+
+class LocalLayer:
+    """A single-rank MoE layer's forward and backward pass as one native call each (csrc/host/moe_local.cc)."""
+
+    def __init__(self, st: RankState, Hp: int, weights, grads, work: dict, blocks: int, num_ctas: int, status, status_host, budget_ns: int):
+        g, a = st.geo, _native.MoeLocal()
+        a.ctx = st.ctx_ptr
+        a.S, a.H, a.Hp, a.K, a.E, a.NvS = g.S, g.H, Hp, g.K, g.E, g.NvS
+        a.blocks, a.combine_blocks, a.num_ctas = min(blocks, st.local_blocks), blocks, num_ctas
+        self._sizes, self._total, first = _plan_layout(st)
+        a.plan_off = (C.c_int64 * 8)(*first)
+        for name, t in zip(("w_gate", "w_up", "w_down"), weights):
+            setattr(a, name, t.data_ptr())
+        for name, t in zip(("dw_gate", "dw_up", "dw_down"), grads or ()):
+            setattr(a, name, t.data_ptr())
+        for name, t in work.items():
+            setattr(a, name, t.data_ptr())
+        a.shard, a.shard_w, a.srcinfo = st.hidden_local.data_ptr(), st.weights_local.data_ptr(), ptr(st.srcinfo_local)
+        a.sync, a.hist = st.scratch["loc_sync"].data_ptr(), st.scratch["loc_hist"].data_ptr()
+        a.status, a.status_host, a.budget_ns = status.data_ptr(), status_host.data_ptr(), budget_ns
+        self._geo, self._args, self._ref, self._dev = g, a, C.addressof(a), st.device
+        self._lib = _native.load()
+
+    def forward(self, hidden, route_w, topk, tpe, keep: bool):
+        """Returns ``(out, plan allocation)``."""
+        g = self._geo
+        slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
+        out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
+        rc = self._lib.mep_moe_local_forward(self._ref, hidden.data_ptr(), route_w.data_ptr(), topk.data_ptr(), tpe.data_ptr(),
+                                             slab.data_ptr(), out.data_ptr(), 1 if keep else 0, _native.raw_stream())
+        if rc:
+            _native.check(rc, "moe forward")
+        return out, slab
+
+    def backward(self, dy, slab, accumulate: bool, lr: float, mask):
+        g = self._geo
+        dx = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
+        dw = torch.empty((g.S, g.K), dtype=torch.float32, device=self._dev)
+        rc = self._lib.mep_moe_local_backward(self._ref, dy.data_ptr(), slab.data_ptr(), dx.data_ptr(), dw.data_ptr(),
+                                              1 if accumulate else 0, lr, ptr(mask), _native.raw_stream())
+        if rc:
+            _native.check(rc, "moe backward")
+        return dx, dw
+
+    def plan_of(self, slab):
+        """``(plan, cu_seqlens)`` of a forward pass."""
+        return _plan_of_parts(self._geo, slab.split(self._sizes)[::2])
 
 
 def launch_local_dispatch(st: RankState, hidden, weights, plan, out_hidden, out_weights, num_blocks: int,

@@ -45,7 +45,27 @@ class MoEContext:
     gu: torch.Tensor         # pre-activations [NvS, 2H']
 
 
+class _LocalContext:
+    """``MoEContext`` of a single-rank forward pass: the plan's allocation; its tensors are named when somebody asks."""
+
+    def __init__(self, layer, slab):
+        self._layer, self.slab, self._named = layer, slab, None
+        self.x, self.w_nvs, self.act, self.gu = layer._x, layer._w, layer._act, layer._gu
+
+    def _plan(self):
+        if self._named is None:
+            self._named = self._layer._native.plan_of(self.slab)
+        return self._named
+
+    plan = property(lambda self: self._plan()[0])
+    cu = property(lambda self: self._plan()[1])
+
+
 _DEFERRED: list = []       # layers whose last gradient reduction is still running (see wait_grads)
+
+
+def no_update(name: str) -> None:
+    """``on_grad_ready`` of a layer whose weight-gradient epilogues have updated every expert."""
 
 
 def update_mask(experts_to_copy, rank: int, epn: int, mask=None, hit=None, ones=None):
@@ -117,11 +137,21 @@ class ExpertParallelMoE:
         # optimizer in the weight-gradient GEMM's epilogue (see ``backward``): learning rate, or None
         self.epilogue_lr = None
         i32 = dict(dtype=torch.int32, device=dev)
+        self._native = self._native_layer() if self._local and self._skip_pad and "MOONEP_GEMM_DYNAMIC" not in os.environ else None
         self._upd_mask = torch.zeros(2 * g.epn, **i32)
         if g.R == 1:                    # nobody holds a replica: always the same mask
             self._upd_mask[:g.epn] = 1
         self._upd_hit = torch.zeros(g.epn + 1, **i32)
         self._upd_ones = torch.ones(g.R * g.epn, **i32)
+
+    def _native_layer(self):
+        from . import engine
+        names = ("gate", "up", "down")
+        return engine.LocalLayer(
+            self.buf._states[0], self.Hp, [self._W(n) for n in names],
+            [self._dW(n) for n in names] if self.pools.with_grads else None,
+            dict(x=self._x, w=self._w, act=self._act, gu=self._gu, dA=self._dA, dgu=self._dgu), self.buf._num_sms_dedup,
+            self._total_sms, gg._status(self._act.device), gg._status_host(self._act.device), engine.wait_budget_ns())
 
     def _update_mask(self, plan):
         if self.geo.R == 1:
@@ -177,6 +207,12 @@ class ExpertParallelMoE:
         starting the GEMM on flagged tiles; it writes straight into the private buffers that the backward pass
         reads (no stash), and the down GEMM's rows stay in the shard, where the combine gathers them."""
         buf, st = self.buf, self.buf._st()
+        if self._native is not None and route_weights_sk is not None:
+            topk = topk_sk.reshape(-1)
+            buf._check_hidden(hidden_sh, route_weights_sk)
+            buf._check_topk(topk, tokens_per_expert)
+            out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward)
+            return out, _LocalContext(self, slab) if need_backward else None
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
         _, _, cu, plan = buf._dispatch_local(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, None, out=(x, w))
         pad = self._pad(plan)
@@ -275,6 +311,14 @@ class ExpertParallelMoE:
         buf, g, epn, Hp = self.buf, self.geo, self.geo.epn, self.Hp
         acc, ov, multi = self.accumulate_grads, self.overlap_backward and not self._local, self.geo.R > 1
         self._join_deferred()
+        if (self._native is not None and isinstance(ctx, _LocalContext) and self.on_comm_quiet is None
+                and (self.on_grad_ready is None or self.on_grad_ready is no_update)):
+            buf._st()
+            buf._check_hidden(grad_out_sh, None)
+            lr = self.epilogue_lr
+            assert lr is None or not acc, "the optimizer cannot sit in the GEMM epilogue while gradients are accumulated"
+            self.grads_pending = None
+            return self._native.backward(grad_out_sh, ctx.slab, acc, lr or 0.0, None if lr is None else self._upd_mask)
         main = torch.cuda.current_stream()
         pools = self.pools
         pair = lambda n: (pools.local_grad(n), pools.reduce_view(n))      # noqa: E731

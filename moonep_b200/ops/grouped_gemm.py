@@ -19,6 +19,7 @@ import os
 import torch
 
 from .. import _native
+from ..engine import wait_budget_ns
 
 GATE_UP, DOWN, DGRAD, DGRAD_GU, WGRAD = range(5)
 _status_cache: dict = {}
@@ -50,6 +51,8 @@ class PushTarget:
 
 
 def _dev_index(device) -> int:
+    if isinstance(device, torch.device) and device.index is not None:
+        return device.index
     idx = torch.device(device).index
     return torch.cuda.current_device() if idx is None else idx
 
@@ -62,21 +65,41 @@ def _status(device) -> torch.Tensor:
 
 
 _status_host_cache: dict = {}
+_failed_word: dict = {}
 
 
 def _status_host(device) -> torch.Tensor:
     """Pinned host word the GEMM kernels mirror their failure code into (see ``failed``)."""
     key = _dev_index(device)
     if key not in _status_host_cache:
-        _status_host_cache[key] = torch.zeros(1, dtype=torch.int32).pin_memory()
+        t = _status_host_cache[key] = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _failed_word[key] = C.c_int32.from_address(t.data_ptr())
     return _status_host_cache[key]
 
 
 def failed(device="cuda") -> bool:
     """True once a grouped GEMM on ``device`` has given up a wait.  Reads host memory only (no
     synchronisation); ``check_status`` gives the details and clears the state."""
-    t = _status_host_cache.get(_dev_index(device))
-    return t is not None and int(t[0]) != 0
+    w = _failed_word.get(_dev_index(device))
+    return w is not None and w.value != 0
+
+
+_arg_template: dict = {}
+
+
+def _new_args(device, cu, pad) -> GemmArgs:
+    """An argument block with everything that does not depend on the call: one copy instead of a dozen assignments."""
+    key = _dev_index(device)
+    t = _arg_template.get(key)
+    if t is None:
+        t = GemmArgs()
+        t.status, t.status_host = _status(device).data_ptr(), _status_host(device).data_ptr()
+        _arg_template[key] = t
+    args = GemmArgs.from_buffer_copy(t)
+    args.cu_seqlens, args.budget_ns = cu.data_ptr(), wait_budget_ns()
+    if pad is not None:
+        args.pad_rows = pad.data_ptr()
+    return args
 
 
 _SCHED_SLOTS = 64
@@ -142,18 +165,13 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
     assert cu.dtype == torch.int32 and cu.is_contiguous()
     G = cu.numel()
     g0, g1 = (0, G) if groups is None else groups
-    args = GemmArgs()
-    args.cu_seqlens = cu.data_ptr()
+    args = _new_args(a.device, cu, pad)
     args.G, args.N, args.K, args.M_w = G, N, K, M_w
     args.b_group_rows, args.accumulate = b_group_rows, 1 if accumulate else 0
     args.g_begin, args.g_end = g0, g1
     args.zero_empty_below = zero_empty_below
     args.out, args.out2 = out.data_ptr(), _native.ptr(out2)
     args.row_scale, args.ldo = _native.ptr(row_scale), ldo
-    args.status = _status(a.device).data_ptr()
-    args.status_host = _status_host(a.device).data_ptr()
-    from ..engine import wait_budget_ns
-    args.budget_ns = wait_budget_ns()
     if ticket is not None:
         args.sched, args.sched_ctas = ticket.ptr, ticket.total_ctas
     else:
@@ -163,7 +181,6 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
         args.tile_done, args.tile_epoch = ready.done_ptr, ready.epoch_ptr
     if slots is not None:
         args.group_flags, args.group_epoch, args.group_first = slots.flags_ptr, slots.epoch_ptr, slots.first
-    args.pad_rows = _native.ptr(pad)
     if push is not None:
         assert mode in (DOWN, DGRAD, DGRAD_GU) and push.info.dtype == torch.int32 and push.info.numel() >= a.shape[0]
         args.push_info, args.push_base, args.push_stride = push.info.data_ptr(), push.base, push.stride
@@ -271,17 +288,11 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
         # CTA-pair kernel (tcgen05 cta_group::2): a third less operand traffic per SM
         lib = _native.load()
         G0, G1 = (0, G) if groups is None else groups
-        args = GemmArgs()
-        args.cu_seqlens = cu.data_ptr()
+        args = _new_args(x.device, cu, pad)
         args.G, args.N, args.K, args.M_w = G, N, 0, M
         args.accumulate, args.g_begin, args.g_end = (1 if accumulate else 0), G0, G1
         args.zero_empty_below = zero_empty_below
-        args.pad_rows = _native.ptr(pad)
         args.out = out.data_ptr()
-        args.status = _status(x.device).data_ptr()
-        args.status_host = _status_host(x.device).data_ptr()
-        from ..engine import wait_budget_ns
-        args.budget_ns = wait_budget_ns()
         if ticket is not None:
             args.sched, args.sched_ctas = ticket.ptr, ticket.total_ctas
         else:
@@ -330,3 +341,16 @@ def sgd_step(p, g, lr, num_blocks=None):
     nb = num_blocks or 8 * _num_sms(p.device)
     _native.check(lib.mep_sgd_step(C.c_void_p(p.data_ptr()), C.c_void_p(g.data_ptr()), C.c_float(lr),
                                    C.c_int64(p.numel()), nb, _native.cur_stream()), "sgd_step")
+
+
+def sgd_step_many(ps, gs, lr, num_blocks=None):
+    """``sgd_step`` of up to four tensors in one launch."""
+    lib = _native.load()
+    n = len(ps)
+    for p, g in zip(ps, gs):
+        assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.numel() == g.numel()
+        assert p.is_contiguous() and g.is_contiguous()
+    nb = num_blocks or 8 * _num_sms(ps[0].device)
+    P, N = C.c_void_p * n, C.c_int64 * n
+    _native.check(lib.mep_sgd_step_many(n, P(*[p.data_ptr() for p in ps]), P(*[g.data_ptr() for g in gs]), N(*[p.numel() for p in ps]),
+                                        C.c_float(lr), nb, _native.cur_stream()), "sgd_step_many")

@@ -144,7 +144,7 @@ class ExpertPools:
                 world, rank = 1, 0
         self.world, self.rank, self._group = world, rank, group
         self.shared = shared
-        self._aliases, self._wview, self._gview = [], {}, {}
+        self._aliases, self._wview, self._gview, self._views = [], {}, {}, {}
         if shared is not None:
             assert heap is None and shared.world == world and shared.epn == epn and shared.dtype == dtype
             assert shared.shapes == self._shapes and (shared.with_grads or not with_grads)
@@ -196,17 +196,25 @@ class ExpertPools:
         rank = self.rank if rank is None else rank
         return self.heap.view(rank, off + first * r * c * es, (count, r, c), dtype)
 
+    def _cached(self, what, name, rank, make):
+        """Views are asked for at every step and never change: each is built once."""
+        key = (what, name, rank)
+        v = self._views.get(key)
+        if v is None:
+            v = self._views[key] = make()
+        return v
+
     # ---- weights
     def local_weight(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._wview[name][:self.epn]
-        return self._view(self._woff[name], name, self.dtype, 0, self.epn, rank)
+        return self._cached("local_weight", name, rank, lambda: self._view(self._woff[name], name, self.dtype, 0, self.epn, rank))
 
     def compute_weight(self, name, rank=None) -> torch.Tensor:
         """``[2*epn, rows, cols]``: local experts then this rank's prefetch slots."""
         if self.shared is not None:
             return self._wview[name]
-        return self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank)
+        return self._cached("compute_weight", name, rank, lambda: self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank))
 
     def prefetch_view(self, name) -> torch.Tensor:
         """``[R, epn, rows, cols]`` view of every rank's prefetch slots."""
@@ -220,12 +228,12 @@ class ExpertPools:
     def local_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name][:self.epn]
-        return self._view(self._goff[name], name, torch.float32, 0, self.epn, rank)
+        return self._cached("local_grad", name, rank, lambda: self._view(self._goff[name], name, torch.float32, 0, self.epn, rank))
 
     def compute_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name]
-        return self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank)
+        return self._cached("compute_grad", name, rank, lambda: self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank))
 
     def reduce_view(self, name) -> torch.Tensor:
         if self.shared is not None:
@@ -249,6 +257,7 @@ class ExpertPools:
         return kw
 
     def destroy(self) -> None:
+        self._views = {}
         if self._aliases:
             torch.cuda.synchronize()
             self._wview, self._gview = {}, {}
