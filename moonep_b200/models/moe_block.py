@@ -20,8 +20,9 @@ import torch
 import torch.distributed as dist
 
 from ..api import Buffer
-from ..moe_layer import ExpertParallelMoE, moe_apply
+from ..moe_layer import ExpertParallelMoE, moe_apply, no_update
 from ..ops import grouped_gemm as gg
+from ..ops import router as rt
 from ..pools import ExpertPools
 
 
@@ -43,6 +44,67 @@ CONFIGS = {
     "qwen3_30b_a3b": MoEConfig("qwen3_30b_a3b", 2048, 768, 8, 16, S=8192),
     "tiny": MoEConfig("tiny", 256, 256, 2, 2, shared_experts=1, S=128),
 }
+
+
+class _RouteFn(torch.autograd.Function):
+    """``MoEBlock.route``: the weights are differentiable, table and counts are not."""
+
+    @staticmethod
+    def forward(ctx, hidden, router, blk):
+        w, topk, tpe = rt.route(hidden @ router, blk.router_bias, blk.cfg.K)
+        ctx.save_for_backward(hidden, router, w, topk)
+        ctx.mark_non_differentiable(topk, tpe)
+        return w, topk, tpe
+
+    @staticmethod
+    def backward(ctx, dw, _topk, _tpe):
+        hidden, router, w, topk = ctx.saved_tensors
+        dl = rt.route_bwd(w, dw.contiguous(), topk, router.shape[1])
+        return (dl @ router.t() if ctx.needs_input_grad[0] else None, hidden.t() @ dl if ctx.needs_input_grad[1] else None, None)
+
+
+def _block_forward(blk, hidden, router, s0, s1, keep: bool):
+    """Output, and with ``keep`` what the backward pass needs: (MoE context, route weights, table, shared gate/up, activation)."""
+    w, topk, tpe = rt.route(hidden @ router, blk.router_bias, blk.cfg.K)
+    out, mctx = blk.moe.forward(hidden, w, topk, tpe, need_backward=keep)
+    gu = act = None
+    if s0 is not None:
+        gu = hidden @ s0
+        act = rt.swiglu(gu)
+        out.addmm_(act, s1)                     # added in the GEMM's fp32 accumulator, rounded once
+    return out, mctx, w, topk, gu, act
+
+
+class _BlockFn(torch.autograd.Function):
+    """A whole block as one autograd node: the three contributions to the input gradient (experts, router, shared
+    expert) are accumulated by the GEMMs that produce them instead of by additions over ``[S, H]``."""
+
+    @staticmethod
+    def forward(ctx, hidden, router, s0, s1, blk):
+        out, ctx.mctx, w, topk, gu, act = _block_forward(blk, hidden, router, s0, s1, True)
+        ctx.blk = blk
+        ctx.save_for_backward(hidden, router, s0, s1, w, topk, gu, act)
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        hidden, router, s0, s1, w, topk, gu, act = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        dy = dy.contiguous()
+        dx, dw = ctx.blk.moe.backward(ctx.mctx, dy)
+        dl = rt.route_bwd(w, dw, topk, router.shape[1])
+        drouter = hidden.t() @ dl if need[1] else None
+        if need[0]:
+            dx.addmm_(dl, router.t())
+        ds0 = ds1 = None
+        if s0 is not None:
+            dgu = torch.empty_like(gu)
+            gg.swiglu_bwd(dy @ s1.t(), gu, None, dgu, None, ctx.blk._rows)
+            ds1 = act.t() @ dy if need[3] else None
+            ds0 = hidden.t() @ dgu if need[2] else None
+            if need[0]:
+                dx.addmm_(dgu, s0.t())
+        return dx if need[0] else None, drouter, ds0, ds1, None
 
 
 class MoEBlock:
@@ -74,6 +136,10 @@ class MoEBlock:
         self.router = (torch.randn(cfg.H, self.E, device=dev, generator=gs) * 0.02).to(torch.bfloat16).requires_grad_(True)
         # a per-expert bias added to the logits skews the routing (maxvio sweeps)
         self.router_bias = (torch.randn(self.E, device=dev, generator=gs) * router_skew).float()
+        # router, experts and shared expert as one autograd node with fused element-wise kernels; sizes those do not
+        # cover take the plain torch operators
+        self._fused_route = rt.supported(self.E, cfg.K)
+        self._rows = torch.tensor([cfg.S], dtype=torch.int32, device=dev)
         self.shared = None
         if cfg.shared_experts:
             hs = cfg.Hp * cfg.shared_experts
@@ -87,6 +153,8 @@ class MoEBlock:
             dist.barrier(group=group)
 
     def route(self, hidden):
+        if self._fused_route:
+            return _RouteFn.apply(hidden, self.router, self)
         cfg = self.cfg
         logits = (hidden @ self.router).float() + self.router_bias
         probs = torch.softmax(logits, dim=-1)
@@ -98,6 +166,11 @@ class MoEBlock:
         return w, topk, tpe
 
     def forward(self, hidden):
+        if self._fused_route and hidden.dtype == torch.bfloat16 and hidden.is_contiguous():
+            shared = self.shared or (None, None)
+            if not torch.is_grad_enabled():
+                return _block_forward(self, hidden, self.router, *shared, False)[0]
+            return _BlockFn.apply(hidden, self.router, *shared, self)
         w, topk, tpe = self.route(hidden)
         out = moe_apply(self.moe, hidden, w, topk, tpe)
         if self.shared is not None:
@@ -131,23 +204,28 @@ class MoEBlock:
         elif moe.epilogue_lr is None:
             moe.on_grad_ready = lambda n: gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr)
         elif self.world == 1:
-            moe.on_grad_ready = lambda n: None      # no replicas: the epilogues have updated every expert
+            moe.on_grad_ready = no_update           # no replicas: the epilogues have updated every expert
         else:
             moe.on_grad_ready = lambda n: gg.sgd_step_groups(self.pools.local_weight(n), self.pools.local_grad(n), lr,
                                                              moe._upd_mask, want=False)
 
     def sgd_step(self, lr: float):
         if self.moe.on_grad_ready is None:
-            for n in ("down", "gate", "up"):     # ``up`` last: its cross-rank reduction may still be running
-                self.moe.wait_grads(n)
-                gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr)
+            names = ("down", "gate", "up")
+            if self.moe.grads_pending is None:
+                gg.sgd_step_many([self.pools.local_weight(n) for n in names], [self.pools.local_grad(n) for n in names], lr)
+            else:
+                for n in names:                  # ``up`` last: its cross-rank reduction may still be running
+                    self.moe.wait_grads(n)
+                    gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr)
         else:
             assert lr == self._fused_lr, "the experts were already updated with another learning rate"
             self.moe.wait_grads()       # the last reduction and the update behind it may still be running
         with torch.no_grad():
-            for p in self.parameters():
-                if p.grad is not None:
-                    p.add_(p.grad.to(p.dtype), alpha=-lr)
+            ps = [p for p in self.parameters() if p.grad is not None]
+            if ps:
+                torch._foreach_add_(ps, [p.grad.to(p.dtype) for p in ps], alpha=-lr)
+                for p in ps:
                     p.grad = None
 
     def destroy(self):
