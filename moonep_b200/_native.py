@@ -159,7 +159,8 @@ def load(build_if_missing: bool = True):
     lib.mep_mc_add_device.argtypes = [vp]
     lib.mep_mc_bind_map.argtypes = [vp, vp, C.POINTER(C.c_ulonglong)]
     lib.mep_mc_destroy.argtypes = [vp]
-    lib.mep_route.argtypes = [vp] * 5 + [i32] * 3 + [vp]
+    lib.mep_route.argtypes = [vp] * 6 + [i32] * 3 + [vp]
+    lib.mep_swiglu_dense_bwd.argtypes = [vp, vp, vp, C.c_int64, i32, vp]
     lib.mep_route_bwd.argtypes = [vp] * 4 + [i32] * 3 + [vp]
     lib.mep_swiglu.argtypes = [vp, vp, C.c_int64, i32, vp]
     lib.mep_moe_local_forward.argtypes = [vp] * 7 + [i32, vp]

@@ -51,28 +51,28 @@ class _RouteFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, router, blk):
-        w, topk, tpe = rt.route(hidden @ router, blk.router_bias, blk.cfg.K)
-        ctx.save_for_backward(hidden, router, w, topk)
+        w, topk, tpe, probs = rt.route(hidden @ router, blk.router_bias, blk.cfg.K, with_probs=True)
+        ctx.save_for_backward(hidden, router, probs, topk)
         ctx.mark_non_differentiable(topk, tpe)
         return w, topk, tpe
 
     @staticmethod
     def backward(ctx, dw, _topk, _tpe):
-        hidden, router, w, topk = ctx.saved_tensors
-        dl = rt.route_bwd(w, dw.contiguous(), topk, router.shape[1])
+        hidden, router, probs, topk = ctx.saved_tensors
+        dl = rt.route_bwd(probs, dw.contiguous(), topk)
         return (dl @ router.t() if ctx.needs_input_grad[0] else None, hidden.t() @ dl if ctx.needs_input_grad[1] else None, None)
 
 
 def _block_forward(blk, hidden, router, s0, s1, keep: bool):
-    """Output, and with ``keep`` what the backward pass needs: (MoE context, route weights, table, shared gate/up, activation)."""
-    w, topk, tpe = rt.route(hidden @ router, blk.router_bias, blk.cfg.K)
+    """Output, and with ``keep`` what the backward pass needs: (MoE context, probabilities, table, shared gate/up, activation)."""
+    w, topk, tpe, probs = rt.route(hidden @ router, blk.router_bias, blk.cfg.K, with_probs=keep)
     out, mctx = blk.moe.forward(hidden, w, topk, tpe, need_backward=keep)
     gu = act = None
     if s0 is not None:
         gu = hidden @ s0
         act = rt.swiglu(gu)
-        out.addmm_(act, s1)                     # added in the GEMM's fp32 accumulator, rounded once
-    return out, mctx, w, topk, gu, act
+        out.add_(act @ s1)
+    return out, mctx, probs, topk, gu, act
 
 
 class _BlockFn(torch.autograd.Function):
@@ -81,25 +81,24 @@ class _BlockFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, router, s0, s1, blk):
-        out, ctx.mctx, w, topk, gu, act = _block_forward(blk, hidden, router, s0, s1, True)
+        out, ctx.mctx, probs, topk, gu, act = _block_forward(blk, hidden, router, s0, s1, True)
         ctx.blk = blk
-        ctx.save_for_backward(hidden, router, s0, s1, w, topk, gu, act)
+        ctx.save_for_backward(hidden, router, s0, s1, probs, topk, gu, act)
         return out
 
     @staticmethod
     def backward(ctx, dy):
-        hidden, router, s0, s1, w, topk, gu, act = ctx.saved_tensors
+        hidden, router, s0, s1, probs, topk, gu, act = ctx.saved_tensors
         need = ctx.needs_input_grad
         dy = dy.contiguous()
         dx, dw = ctx.blk.moe.backward(ctx.mctx, dy)
-        dl = rt.route_bwd(w, dw, topk, router.shape[1])
+        dl = rt.route_bwd(probs, dw, topk)
         drouter = hidden.t() @ dl if need[1] else None
         if need[0]:
             dx.addmm_(dl, router.t())
         ds0 = ds1 = None
         if s0 is not None:
-            dgu = torch.empty_like(gu)
-            gg.swiglu_bwd(dy @ s1.t(), gu, None, dgu, None, ctx.blk._rows)
+            dgu = rt.swiglu_bwd(dy @ s1.t(), gu)
             ds1 = act.t() @ dy if need[3] else None
             ds0 = hidden.t() @ dgu if need[2] else None
             if need[0]:
@@ -139,7 +138,6 @@ class MoEBlock:
         # router, experts and shared expert as one autograd node with fused element-wise kernels; sizes those do not
         # cover take the plain torch operators
         self._fused_route = rt.supported(self.E, cfg.K)
-        self._rows = torch.tensor([cfg.S], dtype=torch.int32, device=dev)
         self.shared = None
         if cfg.shared_experts:
             hs = cfg.Hp * cfg.shared_experts

@@ -10,33 +10,41 @@ pytestmark = pytest.mark.gpu
 def test_route_matches_torch(S, E, K, cuda_device):
     from moonep_b200.ops import router as rt
     g = torch.Generator(device="cuda").manual_seed(S + E)
-    # distinct sums of logit and bias: the order of equal ones is anybody's
+    # the bias makes the sums distinct: the order of equal ones is anybody's
     logits = torch.randn(S, E, device="cuda", generator=g).to(torch.bfloat16)
     bias = torch.randn(E, device="cuda", generator=g)
-    w, topk, tpe = rt.route(logits, bias, K)
-    x = (logits.float() + bias).requires_grad_(True)
-    wr, tr = torch.topk(torch.softmax(x, -1), K, -1)
+    w, topk, tpe, probs = rt.route(logits, bias, K, with_probs=True)
+    lf = logits.clone().requires_grad_(True)
+    pr = torch.softmax(lf.float() + bias, -1)
+    wr, tr = torch.topk(pr, K, -1)
     wr = wr / wr.sum(-1, keepdim=True)
-    torch.cuda.synchronize()
-    chosen = (logits.float() + bias).gather(1, topk.long())
-    assert torch.equal(chosen, (logits.float() + bias).gather(1, tr)) and all(len(set(r)) == K for r in topk.tolist())
-    assert torch.equal(tpe.long(), torch.bincount(topk.flatten().long(), minlength=E))
-    assert torch.allclose(w, wr, rtol=1e-5, atol=1e-7)        # a handful of fp32 roundings and expf's two ulp
     dw = torch.randn(S, K, device="cuda", generator=g)
     wr.backward(dw)
-    dl = rt.route_bwd(w, dw, topk, E)
-    ref = x.grad
-    assert float((dl.float() - ref).norm()) <= 4e-3 * float(ref.norm()) + 1e-6 * S ** 0.5      # rounded to bf16 once
+    torch.cuda.synchronize()
+    assert torch.equal(probs, pr) and torch.equal(topk.long(), tr) and torch.equal(w, wr)
+    assert torch.equal(tpe.long(), torch.bincount(topk.flatten().long(), minlength=E))
+    assert torch.equal(rt.route_bwd(probs, dw, topk), lf.grad)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (130, 256), (33, 2056)])
+def test_dense_swiglu_matches_torch(rows, n, cuda_device):
+    from moonep_b200.ops import router as rt
+    g = torch.Generator(device="cuda").manual_seed(n)
+    gu = (torch.randn(rows, 2 * n, device="cuda", generator=g) * 3).to(torch.bfloat16).requires_grad_(True)
+    d = torch.randn(rows, n, device="cuda", generator=g).to(torch.bfloat16)
+    act = torch.nn.functional.silu(gu[:, :n]) * gu[:, n:]
+    act.backward(d)
+    assert torch.equal(rt.swiglu(gu.detach()), act) and torch.equal(rt.swiglu_bwd(d, gu.detach()), gu.grad)
 
 
 def test_route_of_nans_names_existing_experts(cuda_device):
     from moonep_b200.ops import router as rt
     logits = torch.full((5, 48), float("nan"), device="cuda").to(torch.bfloat16)
-    logits[1, :40] = 1.0
-    w, topk, tpe = rt.route(logits, torch.zeros(48, device="cuda"), 8)
+    logits[1, :40] = 1.0          # one NaN makes every probability of its row NaN
+    w, topk, tpe, _ = rt.route(logits, torch.zeros(48, device="cuda"), 8)
     t = topk.cpu()
     assert int(t.min()) >= 0 and int(t.max()) < 48 and all(len(set(r)) == 8 for r in t.tolist()) and int(tpe.sum()) == 40
-    assert sorted(t[1].tolist()) == list(range(40, 48)), "NaN counts as the largest value"
+    assert bool(torch.isnan(w).all())
 
 
 @pytest.mark.parametrize("shared", [0, 1])
@@ -62,5 +70,7 @@ def test_block_node_matches_torch_operators(shared, cuda_device):
         got.append([y.detach(), x.grad] + [p.grad for p in blk.parameters()] + [blk.pools.local_grad(n).clone() for n in ("gate", "up", "down")])
         blk.destroy()
     for i, (a, b) in enumerate(zip(*got)):
-        # the operators round every intermediate to bf16 (2^-9 each, a few in a row), the node does not
-        assert float((a.float() - b.float()).norm() / b.float().norm()) < 1e-2, i
+        if i == 1:      # the input gradient: the node adds its parts in fp32, the operators in bf16 (2^-9 for each addition)
+            assert float((a.float() - b.float()).norm() / b.float().norm()) < 8e-3
+        else:
+            assert torch.equal(a, b), i
