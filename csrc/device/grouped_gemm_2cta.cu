@@ -48,6 +48,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   const bool leader = cr == 0;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int G = args.G;
+  pdl_trigger();
 
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -58,6 +59,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     tc::prefetch_tmap(&tma_a); tc::prefetch_tmap(&tma_b); tc::prefetch_tmap(&tma_out);
   }
   if (warp == 1) { tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2(); }
+  pdl_wait();                           // everything below reads what kernels before this one wrote
   if (warp == 2) {                      // tile list: 32 groups at a time
     int n = 0;
     for (int g0 = 0; g0 < G; g0 += 32) {
@@ -306,10 +308,12 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   if (allow_smem((const void*)w2::wgrad_2cta_kernel, w2::kSmem)) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_ctas); cfg.blockDim = dim3(w2::kThreads); cfg.dynamicSmemBytes = w2::kSmem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
   MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, w2::wgrad_2cta_kernel, ma, mb, mo, args));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;

@@ -24,16 +24,17 @@ namespace mep {
 namespace tp {
 using namespace pair;
 
-constexpr int kBK = 64, kRing = 6, kEpiWarps = 8, kThreads = 64 + 32 * kEpiWarps;
-constexpr int kHalfBytes = 128 * kBK * 2;              // 16 KB: weight columns, or up to 128 token rows, of one k-block
-constexpr int kStageBytes = 2 * kHalfBytes;
+constexpr int kBK = 64, kEpiWarps = 8, kThreads = 64 + 32 * kEpiWarps;
+constexpr int kWBytes = 128 * kBK * 2;                 // 16 KB: a CTA's weight columns of one k-block
+constexpr int kRingBytes = 6 * 2 * kWBytes, kMaxRing = 11;
 constexpr int kAtomBytes = 64 * kBK * 2;
 constexpr int kChunk = 16;                             // tokens per epilogue step
 constexpr int kStgBytes = kChunk * 128;                // staging: 16 tokens x 64 columns
-constexpr int kXchBytes = 32 * 64;                     // one warp's fp32 fragments of a chunk (GATE_UP)
+constexpr int kXchBytes = 32 * 32;                     // half of a warp's fp32 fragments of a chunk (GATE_UP)
 constexpr int kMaxGroups = 192;
-constexpr size_t kEpiBytes = 2 * 3 * kStgBytes + 4 * kXchBytes > 2 * 4 * kStgBytes ? 2 * 3 * kStgBytes + 4 * kXchBytes : 2 * 4 * kStgBytes;
-constexpr size_t kSmem = (size_t)kRing * kStageBytes + kEpiBytes + 1024;
+constexpr int kStgSet = 4 * kStgBytes;                 // GATE_UP: act twice, gate, up; else: two buffers for each 64-column side
+constexpr size_t kEpiBytes = 2 * kStgSet + kEpiWarps * kXchBytes;
+constexpr size_t kSmem = (size_t)kRingBytes + kEpiBytes + 1024;
 
 struct Tile { int g, row0, n, n0; };                   // n tokens from row0 (a multiple of 32, at most 256)
 
@@ -57,13 +58,13 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, 
 
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
-tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
+tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_x16, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
                 const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out2, GemmArgs args) {
   constexpr bool W_MN = MODE == GEMM_GATE_UP || MODE == GEMM_DOWN;      // weights [k, column]: the M side is contiguous
   constexpr int kCols = MODE == GEMM_GATE_UP ? 128 : 256;               // output columns of a tile
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full_bar[kRing], empty_bar[kRing], tfull_bar[2], tempty_bar[2];
+  __shared__ __align__(8) uint64_t full_bar[kMaxRing], empty_bar[kMaxRing], tfull_bar[2], tempty_bar[2];
   __shared__ uint32_t s_tmem_base;
   __shared__ volatile int s_abort;
   __shared__ tq::Ring s_ring;
@@ -72,11 +73,27 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   const uint32_t cr = cluster_ctarank();
   const bool leader = cr == 0;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  __shared__ float s_scale[2][2][128];   // [set][accumulator]: row factors of the set's chunks
+  __shared__ int s_half;                 // most token rows a CTA stages for a tile of this launch
   const int G = args.G, kblocks = args.K / kBK;
+  pdl_trigger();
 
+  if (warp == 1) {
+    tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2();
+  } else if (threadIdx.x == 64) {
+    s_abort = 0;
+    for (int i = 0; i < kMaxRing; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&tfull_bar[i], 1); mbar_init(&tempty_bar[i], 2 * kEpiWarps); }
+    tq::init(&s_ring, 2 * kEpiWarps + 2);      // both CTAs' epilogue warps, the MMA issuer, the peer's producer
+    fence_mbar_init();
+  } else if (threadIdx.x == 96) {
+    tc::prefetch_tmap(&tma_x); tc::prefetch_tmap(&tma_x16); tc::prefetch_tmap(&tma_w0); tc::prefetch_tmap(&tma_w1);
+    tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
+  }
+  pdl_wait();                            // everything below reads what kernels before this one wrote
   if (warp == 0) {                       // tile list: 32 groups at a time
     const int nblk = args.N / kCols;
-    int run = 0;
+    int run = 0, most = 0;
     for (int g0 = 0; g0 < G; g0 += 32) {
       const int g = g0 + lane;
       int beg = 0, units = 0;
@@ -86,20 +103,13 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         if (args.pad_rows) rows -= args.pad_rows[2 * g + 1];
         if (g >= args.g_begin && g < args.g_end) units = (rows + 31) >> 5;
       }
-      const int tiles = ((units + 7) >> 3) * nblk, incl = warp_incl_scan(tiles);
+      const int mt = (units + 7) >> 3, tiles = mt * nblk, incl = warp_incl_scan(tiles);
+      if (units) most = max(most, (units + mt - 1) / mt);
       if (g < G) { s_beg[g] = beg; s_units[g] = units; s_start[g] = run + incl - tiles; }
       run += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) s_start[G] = run;
-  } else if (warp == 1) {
-    tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2();
-  } else if (threadIdx.x == 64) {
-    s_abort = 0;
-    for (int i = 0; i < kRing; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&tfull_bar[i], 1); mbar_init(&tempty_bar[i], 2 * kEpiWarps); }
-    tq::init(&s_ring, 2 * kEpiWarps + 2);      // both CTAs' epilogue warps, the MMA issuer, the peer's producer
-    fence_mbar_init();
-    tc::prefetch_tmap(&tma_x); tc::prefetch_tmap(&tma_w0); tc::prefetch_tmap(&tma_w1); tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
+    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    if (lane == 0) { s_start[G] = run; s_half = 16 * most; }
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -108,6 +118,13 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   const uint32_t tmem_base = s_tmem_base;
   const int ntiles = s_start[G];
   const bool dyn = args.sched != nullptr;
+  // Token rows arrive in boxes of 64, or of 16 where no tile of the launch has more than 48 for a CTA: a stage is then
+  // little more than its weights and up to eleven fit instead of six. With few tokens per expert the kernel streams
+  // weights, and what an SM has in flight is its bandwidth.
+  const bool small = s_half <= 48;
+  const uint32_t x_bytes = small ? max(s_half, 16) * 128u : s_half <= 64 ? 8192u : 16384u;
+  const uint32_t stage_bytes = ((uint32_t)kWBytes + x_bytes + 1023u) & ~1023u;
+  const uint32_t nstages = min((uint32_t)kMaxRing, (uint32_t)kRingBytes / stage_bytes);
 
   auto note = [&](int site, int tile, int code) {
     if (atomicCAS(&args.status[0], 0, code) == 0) {
@@ -131,6 +148,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     // ---------------- TMA producer: this CTA's halves; bytes are counted on the LEADER's barrier
     if (lane == 0) {
       int it = 0, gcur = 0; Tile ti;
+      uint32_t s = 0, ph = 0;
       tq::Scheduler<true> sched; tq::Consumer<true> follow;
       if (dyn) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
       tq::Strided seq{pair, npairs, ntiles};
@@ -156,12 +174,11 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
           seen_group = ti.g;
         }
         const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
-        const bool two = half > 64;                  // token rows arrive in boxes of 64
-        const uint32_t bytes = (uint32_t)kHalfBytes + (two ? 16384u : 8192u);
+        const int boxes = small ? half >> 4 : (half + 63) >> 6;
+        const uint32_t bytes = (uint32_t)kWBytes + (uint32_t)boxes * (small ? 2048u : 8192u);
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % kRing; const uint32_t ph = (uint32_t)(it / kRing) & 1u;
           if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns)) { fail(1, t); break; }
-          const uint32_t sw = smem_u32(smem + (size_t)s * kStageBytes), sx = sw + kHalfBytes;
+          const uint32_t sw = smem_u32(smem) + s * stage_bytes, sx = sw + kWBytes;
           const uint32_t bar = mapa(smem_u32(&full_bar[s]), 0);
           if (leader) mbar_expect_tx(&full_bar[s], 2 * bytes);
           const int k0 = kb * kBK;
@@ -175,12 +192,17 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
             const bool second = MODE == GEMM_DGRAD_GU && k0 >= kh;
             tma_load_2d_bar(sw, second ? &tma_w1 : &tma_w0, second ? k0 - kh : k0, wrow + ti.n0 + (int)cr * 128, bar);
           }
-          tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
-          if (two) tma_load_2d_bar(sx + 8192, &tma_x, k0, xrow + 64, bar);
+          if (small) {
+            for (int i = 0; i < boxes; ++i) tma_load_2d_bar(sx + i * 2048, &tma_x16, k0, xrow + 16 * i, bar);
+          } else {
+            tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
+            if (boxes > 1) tma_load_2d_bar(sx + 8192, &tma_x, k0, xrow + 64, bar);
+          }
+          if (++s == nstages) { s = 0; ph ^= 1u; }
         }
       }
       // the leader's last barrier phase covers both CTAs' copies: nobody leaves before it (cluster_sync below)
-      if (leader && it > 0) mbar_wait_bounded(&full_bar[(it - 1) % kRing], (uint32_t)((it - 1) / kRing) & 1u, args.budget_ns);
+      if (leader && it > 0) mbar_wait_bounded(&full_bar[s ? s - 1 : nstages - 1], s ? ph : ph ^ 1u, args.budget_ns);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only): one instruction drives both SMs. The whole warp runs the loop so
@@ -189,7 +211,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     if (leader) {
       const uint32_t smem0 = smem_u32(smem);
       const uint64_t wdesc0 = W_MN ? tc::smem_desc(smem0, kAtomBytes, 1024) : tc::smem_desc(smem0, 16, 1024);
-      const uint64_t xdesc0 = tc::smem_desc(smem0 + kHalfBytes, 16, 1024);
+      const uint64_t xdesc0 = tc::smem_desc(smem0 + kWBytes, 16, 1024);
       constexpr uint32_t kWStep = W_MN ? 2048 >> 4 : 32 >> 4, kXStep = 32 >> 4;      // one 16-deep step in a descriptor's address field
       int tcnt = 0, gcur = 0; Tile ti;
       uint32_t stage = 0, phase = 0;
@@ -212,13 +234,13 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
           if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) { if (lane == 0) fail(3, t); ok = false; break; }
           tc::fence_after_sync();
           if (elect_one()) {
-            const uint64_t wd = wdesc0 + stage * (kStageBytes >> 4), xd = xdesc0 + stage * (kStageBytes >> 4);
+            const uint64_t wd = wdesc0 + stage * (stage_bytes >> 4), xd = xdesc0 + stage * (stage_bytes >> 4);
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k) mma2_bf16(d_tmem, wd + k * kWStep, xd + k * kXStep, idesc, (kb | k) ? 1u : 0u);
             mma2_commit_both(smem_u32(&empty_bar[stage]));
           }
           __syncwarp();
-          if (++stage == kRing) { stage = 0; phase ^= 1u; }
+          if (++stage == nstages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         if (elect_one()) mma2_commit_both(smem_u32(&tfull_bar[acc]));
@@ -228,8 +250,9 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   } else {
     // ---------------- epilogue: this CTA's 128 weight columns (TMEM lanes) of every token of the tile
     const int q = warp & 3, set = (warp - 2) >> 2, side = q >> 1;      // side: TMEM lanes 0-63 or 64-127 = one 64-column staging row
-    const uint32_t epi = smem_u32(smem + (size_t)kRing * kStageBytes);
+    const uint32_t epi = smem_u32(smem + kRingBytes);
     const uint32_t tempty_leader[2] = {mapa(smem_u32(&tempty_bar[0]), 0), mapa(smem_u32(&tempty_bar[1]), 0)};
+    const int set_tid = (warp - 2 - 4 * set) * 32 + lane;
     const bool issuer = lane == 0 && (q & 1) == 0;                      // one lane per (set, side) stores the staged rows
     const bool push = MODE != GEMM_GATE_UP && args.push_info != nullptr;
     // stmatrix: thread 8i + j addresses the 8-column block i of token row j; the 128-byte swizzle is xor by (row & 7)
@@ -257,11 +280,17 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       }
       const int acc = tcnt & 1; const uint32_t aph = (uint32_t)(tcnt >> 1) & 1u;
       int ok = 0;
+      float rs = 1.f;
       if (t >= 0) {
         get_tile(t, gcur, ti);
+        if ((MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) && args.row_scale) {      // in flight while the tile's MMAs finish
+          const int i = ((set_tid >> 4) * 2 + set) * kChunk + (set_tid & 15);
+          if (i < ti.n) rs = __ldcg(args.row_scale + ti.row0 + i);
+        }
         if (lane == 0) { ok = mbar_wait_bounded(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0; if (!ok) fail(4, t); }
         ok = __shfl_sync(0xffffffffu, ok, 0);
       }
+      if (MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) s_scale[set][acc][set_tid] = rs;
       // the warps of a set stage rows together: they go on or stop together
       if (!named_barrier_all(1 + 4 + set, 128, ok != 0)) break;
       tc::fence_after_sync();
@@ -271,9 +300,9 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       for (int c = set; c < nchunks; c += 2, ++chunk_no) {
         const int row = ti.row0 + c * kChunk;
         float sc[4] = {1.f, 1.f, 1.f, 1.f};          // row factors of this thread's four tokens
-        if ((MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) && args.row_scale) {
-          const float* rs = args.row_scale + row + 2 * (lane & 3);
-          sc[0] = __ldcg(rs); sc[1] = __ldcg(rs + 1); sc[2] = __ldcg(rs + 8); sc[3] = __ldcg(rs + 9);
+        if (MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) {
+          const float* f = &s_scale[set][acc][(c >> 1) * kChunk + 2 * (lane & 3)];
+          sc[0] = f[0]; sc[1] = f[1]; sc[2] = f[8]; sc[3] = f[9];
         }
         uint32_t lo[8], hi[8];
         tmem_ld_frag16(taddr + (uint32_t)c * kChunk, lo);
@@ -285,45 +314,38 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
           if (lane == 0) remote_arrive(tempty_leader[acc]);
         }
         if (MODE == GEMM_GATE_UP) {
-          // staging of a set: [act | gate | up], one buffer each
-          const uint32_t b_act = epi + (uint32_t)set * 3 * kStgBytes, b_gate = b_act + kStgBytes, b_up = b_gate + kStgBytes;
-          const uint32_t xch = epi + 2 * 3 * kStgBytes + (uint32_t)(set * 2 + (q & 1)) * kXchBytes + (uint32_t)lane * 16;
-          if (side == 1) {
-            tc::st_shared_v4(xch, lo[0], lo[1], lo[2], lo[3]); tc::st_shared_v4(xch + 512, lo[4], lo[5], lo[6], lo[7]);
-            tc::st_shared_v4(xch + 1024, hi[0], hi[1], hi[2], hi[3]); tc::st_shared_v4(xch + 1536, hi[4], hi[5], hi[6], hi[7]);
-          }
-          if (issuer) bulk_wait_read<0>();           // the rows staged for the chunk before have left
+          // The gate warps compute the first eight tokens of the chunk, the up warps the other eight: each hands the
+          // partner warp (same columns, other side) the half that it needs.
+          const uint32_t base = epi + (uint32_t)set * kStgSet, b_act = base + (uint32_t)(chunk_no & 1) * kStgBytes;
+          const uint32_t b_mine = base + (uint32_t)(2 + side) * kStgBytes;           // gate or up
+          const uint32_t xch = epi + 2 * kStgSet + (uint32_t)(set * 2 + (q & 1)) * 2 * kXchBytes + (uint32_t)lane * 16;
+          uint32_t keep[8];                          // this side's eight tokens: columns 0-15, then 16-31 of the warp
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { keep[i] = side ? lo[4 + i] : lo[i]; keep[4 + i] = side ? hi[4 + i] : hi[i]; }
+          tc::st_shared_v4(xch + (uint32_t)side * kXchBytes, side ? lo[0] : lo[4], side ? lo[1] : lo[5], side ? lo[2] : lo[6], side ? lo[3] : lo[7]);
+          tc::st_shared_v4(xch + (uint32_t)side * kXchBytes + 512, side ? hi[0] : hi[4], side ? hi[1] : hi[5], side ? hi[2] : hi[6], side ? hi[3] : hi[7]);
+          if (issuer) { if (args.out2) bulk_wait_read<0>(); else bulk_wait_read<1>(); }     // the buffers written below have left
           named_barrier(1 + set, 128);
-          float one[4] = {1.f, 1.f, 1.f, 1.f};
-          if (side == 1) {
-            if (args.out2) stage(b_up, lo, hi, one);
-          } else {
-            if (args.out2) stage(b_gate, lo, hi, one);
+          if (args.out2) { float one[4] = {1.f, 1.f, 1.f, 1.f}; stage(b_mine, lo, hi, one); }
+          uint32_t o[4];
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
+          for (int h = 0; h < 2; ++h) {
+            const int4 p4 = tc::ld_shared_v4(xch + (uint32_t)(side ^ 1) * kXchBytes + h * 512);
+            const float p[4] = {__int_as_float(p4.x), __int_as_float(p4.y), __int_as_float(p4.z), __int_as_float(p4.w)};
+            float v[4];
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                uint32_t* r = (h ? hi : lo) + 4 * b;
-                const int4 u4 = tc::ld_shared_v4(xch + h * 1024 + b * 512);
-                const float u[4] = {__int_as_float(u4.x), __int_as_float(u4.y), __int_as_float(u4.z), __int_as_float(u4.w)};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float g = __uint_as_float(r[i]);
-                  r[i] = __float_as_uint(g / (1.f + __expf(-g)) * u[i]);
-                }
-              }
+            for (int i = 0; i < 4; ++i) {
+              const float m = __uint_as_float(keep[4 * h + i]), g = side ? p[i] : m, u = side ? m : p[i];
+              v[i] = g / (1.f + __expf(-g)) * u * sc[2 * side + (i & 1)];
             }
-            stage(b_act, lo, hi, sc);
+            o[2 * h] = pack2(v[0], v[1]); o[2 * h + 1] = pack2(v[2], v[3]);
           }
+          st_matrix_x4_trans(b_act + (uint32_t)side * 1024 + st_row + st_col, o[0], o[1], o[2], o[3]);
           tc::fence_async_smem();
           named_barrier(1 + set, 128);
           if (issuer) {
-            if (side == 0) {
-              tc::tma_store_2d(&tma_out, b_act, col0, row);
-              if (args.out2) tc::tma_store_2d(&tma_out2, b_gate, col0, row);
-            } else if (args.out2) {
-              tc::tma_store_2d(&tma_out2, b_up, args.N + col0, row);
-            }
+            if (side == 0) tc::tma_store_2d(&tma_out, b_act, col0, row);
+            if (args.out2) tc::tma_store_2d(&tma_out2, b_mine, side * args.N + col0, row);
             bulk_commit();
           }
         } else {
@@ -382,8 +404,8 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   MEP_REQUIRE(args.K % 64 == 0 && args.N % (mode == GEMM_GATE_UP ? 128 : 256) == 0, "gemm (CTA pairs): K=%d N=%d not tileable", args.K, args.N);
   num_ctas &= ~1;
   MEP_REQUIRE(num_ctas >= 2, "gemm (CTA pairs): needs at least two CTAs");
-  CUtensorMap mx, mw0, mw1, mo, mo2;
-  if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 64)) return -1;
+  CUtensorMap mx, mx16, mw0, mw1, mo, mo2;
+  if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 64) || tmap_rows(&mx16, a, a_rows, a_cols, a_ld, 64, 16)) return -1;
   auto weights = [&](CUtensorMap* m, const void* b) {
     if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1);
     if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2);
@@ -397,14 +419,16 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   else mo2 = mo;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_ctas); cfg.blockDim = dim3(tp::kThreads); cfg.dynamicSmemBytes = tp::kSmem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
 #define MEP_TP_CASE(M)                                                                             \
   case M:                                                                                          \
     if (allow_smem((const void*)tp::tok_pair_kernel<M>, tp::kSmem)) return -1;                       \
-    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tp::tok_pair_kernel<M>, mx, mw0, mw1, mo, mo2, args));   \
+    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tp::tok_pair_kernel<M>, mx, mx16, mw0, mw1, mo, mo2, args));   \
     break;
   switch (mode) {
     MEP_TP_CASE(GEMM_GATE_UP) MEP_TP_CASE(GEMM_DOWN) MEP_TP_CASE(GEMM_DGRAD) MEP_TP_CASE(GEMM_DGRAD_GU)

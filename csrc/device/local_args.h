@@ -25,6 +25,9 @@ struct LocalDispatchArgs {
   int32_t* dup_counts;           // [2]
   uint32_t* sync;                // [0] launches completed, [1] start tickets, [2] finished CTAs, [16 + b] flag of CTA b
   int32_t* hist;                 // [grid, E] expert histogram of each CTA's tokens
+  int32_t pad_step;              // 0: every padding row is cleared; else those up to the next multiple of this (a power of
+                                 // two that divides token_padding), which is as far as the CTA-pair GEMMs read
+  int32_t reserved;
 };
 
 struct LocalCombineArgs {

@@ -20,13 +20,18 @@ constexpr int kLocEntries = 1024;          // top-k entries ranked and copied at
 constexpr int kLocZeroBytes = 4096;        // zeroed shared memory the padding rows are stored from
 constexpr int kLocMaxSlots = 8;            // row slots per copying warp
 
+constexpr int kLocDirect = 8192;           // up to this many entries every CTA counts all entries before its own by itself
+
+// Padding rows that are cleared behind row `first` of a group's `n` (see LocalDispatchArgs.pad_step).
+__device__ __forceinline__ int local_pads(int first, int n, int step) { return step ? min(n, -first & (step - 1)) : n; }
+
 // Exclusive prefix of padded group sizes: start[e] = first row of expert e; padpre[e] = padding rows of
 // experts < e. 256 threads, E / 256 consecutive experts each. Returns the number of padding rows.
-__device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, int* start, int* padpre, int* s_warp) {
+__device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, int step, int* start, int* padpre, int* s_warp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int per = (E + kLocThreads - 1) / kLocThreads, e0 = tid * per, e1 = min(e0 + per, E);
   int rows = 0, pads = 0;
-  for (int e = e0; e < e1; ++e) { const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad; rows += p; pads += p - n; }
+  for (int e = e0; e < e1; ++e) { const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad; rows += p; pads += local_pads(n, p - n, step); }
   int ri = warp_incl_scan(rows), pi = warp_incl_scan(pads);
   if (lane == 31) { s_warp[warp] = ri; s_warp[kLocWarps + warp] = pi; }
   __syncthreads();
@@ -38,22 +43,25 @@ __device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, 
   rb += ri - rows; pb += pi - pads;
   for (int e = e0; e < e1; ++e) {
     const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad;
-    start[e] = rb; padpre[e] = pb; rb += p; pb += p - n;
+    start[e] = rb; padpre[e] = pb; rb += p; pb += local_pads(n, p - n, step);
   }
   return total;
 }
 
 // One CTA owns a contiguous range of tokens. FRESH: their entries are ranked among the same-expert entries of
-// the whole batch -- CTAs publish the histogram of their tokens and add up those of the CTAs before them, so
-// the order is the flat entry order and nothing is sorted -- and the plan tables are written. CTAs number
-// themselves in the order in which they start, so a CTA only ever waits for CTAs that are already running and
-// no cooperative launch is needed. Then, from `dst` alone, each row goes through a warp's slot in shared memory
+// the whole batch, in flat entry order, and the plan tables are written. Up to kLocDirect entries (MODE 1) a CTA
+// counts the entries before its own itself: reading them is quicker than a hand-over between CTAs, which costs two
+// round trips to L2. Above that (MODE 2) CTAs publish the histogram of their tokens and add up those of the CTAs
+// before them; they number themselves in the order in which they start, so a CTA only ever waits for CTAs that are
+// already running and no cooperative launch is needed. Then, from `dst` alone, each row goes through a warp's slot in shared memory
 // with one bulk load and K bulk stores (lane k issues the store of entry k); rows of the next tokens are in
 // flight meanwhile, in the fresh case already during the ranking.
 // Bound by HBM: (1 + K) rows per token. 
-template <bool FRESH>
+template <int MODE>                        // 0: saved plan
 __global__ void __launch_bounds__(kLocThreads, 1)
 local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, int copy_warps, int slots) {
+  constexpr bool FRESH = MODE != 0, SHARED = MODE == 2;
+  pdl_trigger();                             // a GEMM behind this kernel may set itself up meanwhile
   const MepRankCtx c = *cp;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLocWarps * kLocMaxSlots];
@@ -72,7 +80,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
 
   if (tid == 0) {
     s_fail = 0;
-    s_vb = FRESH ? (int)atomicAdd(&a.sync[1], 1u) : (int)blockIdx.x;
+    s_vb = SHARED ? (int)atomicAdd(&a.sync[1], 1u) : (int)blockIdx.x;
     trace_mark(c, MEP_K_DISPATCH, 1);
   }
   if (tid < kLocWarps * kLocMaxSlots) mbar_init(&s_bar[tid], 1);
@@ -82,7 +90,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   if (FRESH) for (int e = tid; e < E; e += kLocThreads) s_cnt[e] = 0;
   __syncthreads();
   const int vb = s_vb;
-  const uint32_t ep = FRESH ? *(volatile uint32_t*)&a.sync[0] + 1u : 0u;
+  const uint32_t ep = SHARED ? *(volatile uint32_t*)&a.sync[0] + 1u : 0u;
   const int tb = min(nb, S), tpb = (S + tb - 1) / tb;
   const int t0 = min(vb * tpb, S), t1 = min(t0 + tpb, S);
 
@@ -103,14 +111,22 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   // ---- layout, histogram of this CTA's entries
   int total_pad;
   if (FRESH) {
-    for (int i = t0 * K + tid; i < t1 * K; i += kLocThreads) {
-      const int e = __ldg(a.topk + i);
-      if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
-      else report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, i, (uint32_t)e, (uint32_t)E);
+    if (SHARED) {                            // own entries
+      for (int i = t0 * K + tid; i < t1 * K; i += kLocThreads) {
+        const int e = __ldg(a.topk + i);
+        if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
+        else report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, i, (uint32_t)e, (uint32_t)E);
+      }
+    } else if (t0 < t1) {                    // all entries before them
+#pragma unroll 8
+      for (int i = tid; i < t0 * K; i += kLocThreads) {
+        const int e = __ldg(a.topk + i);
+        if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
+      }
     }
-    total_pad = local_layout(a.tpe, E, pad, s_start, s_padpre, s_warp);
+    total_pad = local_layout(a.tpe, E, pad, a.pad_step, s_start, s_padpre, s_warp);
     __syncthreads();
-    if (t0 < t1) {
+    if (SHARED && t0 < t1) {
       for (int e = tid; e < E; e += kLocThreads) a.hist[(size_t)vb * E + e] = s_cnt[e];
       __syncthreads();
       if (tid == 0) { __threadfence(); st_release_gpu(a.sync + 16 + vb, ep); }
@@ -132,8 +148,9 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
     int run = 0;
     for (int g0 = 0; g0 < ngroups; g0 += kLocThreads) {
       const int g = g0 + tid;
-      const int n = g < ngroups ? __ldg(a.zero_fill + 2 * g + 1) : 0;
-      if (g < ngroups) s_start[g] = __ldg(a.zero_fill + 2 * g);
+      const int first = g < ngroups ? __ldg(a.zero_fill + 2 * g) : 0;
+      const int n = g < ngroups ? local_pads(first, __ldg(a.zero_fill + 2 * g + 1), a.pad_step) : 0;
+      if (g < ngroups) s_start[g] = first;
       const int incl = warp_incl_scan(n);
       if (lane == 31) s_warp[warp] = incl;
       __syncthreads();
@@ -164,7 +181,10 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   bulk_commit();
 
   // ---- entries of earlier CTAs
-  if (FRESH && t0 < t1) {
+  if (MODE == 1) {
+    for (int e = tid; e < E; e += kLocThreads) s_cnt[e] += s_start[e];
+    __syncthreads();
+  } else if (SHARED && t0 < t1) {
     for (int u = tid; u < vb; u += kLocThreads) {
       uint32_t seen = 0;
       const bool ok = bounded_wait(c, [&] { seen = ld_acquire_gpu(a.sync + 16 + u); return (int32_t)(seen - ep) >= 0; });
@@ -195,14 +215,17 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   // ---- chunk by chunk: rank (fresh), tables, rows
   int it = 0, arrived = 0;                     // tokens this warp has copied / whose load it has waited for
   uint32_t phases = 0;                         // parity of each slot's barrier
-  bool ok = !(FRESH && s_fail);
+  bool ok = !(SHARED && s_fail);
   for (int c0 = t0; c0 < t1 && ok; c0 += chunk_tok) {
     const int c1 = min(c0 + chunk_tok, t1), n = (c1 - c0) * K;
     if (FRESH) {
       for (int i0 = 0; i0 < n; i0 += kLocThreads) {
         const int i = i0 + tid;
         int e = i < n ? __ldg(a.topk + (size_t)c0 * K + i) : -1;
-        if ((unsigned)e >= (unsigned)E) e = -1;
+        if ((unsigned)e >= (unsigned)E) {
+          if (MODE == 1 && i < n) report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, c0 * K + i, (uint32_t)e, (uint32_t)E);
+          e = -1;
+        }
         const unsigned m = __match_any_sync(0xffffffffu, e);
         const int before = __popc(m & lanemask_lt());
         int row = -1;
@@ -283,7 +306,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
     count(c, MEP_CNT_DISPATCHES, 1); count(c, MEP_CNT_ROWS_SENT, (unsigned long long)S); count(c, MEP_CNT_PEER_ROWS, (unsigned long long)S);
     trace_mark(c, MEP_K_DISPATCH, 5);
   }
-  if (FRESH) {                                 // the last CTA out closes the launch
+  if (SHARED) {                                // the last CTA out closes the launch
     __syncthreads();
     if (tid == 0) {
       __threadfence();
@@ -308,6 +331,7 @@ __device__ __forceinline__ void add_bf16x8(float* acc, const int4& x) {
 constexpr int kLcWarps = 12, kLcHalf = 8192;
 
 __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts) {
+  pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLcWarps * 2];
   const int K = cp->K, NvS = cp->NvS, nvec = cp->H >> 3;
@@ -315,6 +339,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid < kLcWarps * 2) mbar_init(&s_bar[tid], 1);
   fence_mbar_init();
+  pdl_wait();                                  // the rows may come from the kernel right before
   __syncthreads();
   unsigned char* stage = smem + (size_t)warp * 2 * kLcHalf;
   uint64_t* bars = s_bar + warp * 2;
@@ -377,7 +402,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
 
 // `num_blocks`: CTAs (one per SM). fresh: plan from topk / tpe as well; else a.dst / a.zero_fill are read.
 extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::LocalDispatchArgs* args, int fresh,
-                                         int num_blocks, int H, int E, cudaStream_t stream) {
+                                         int num_blocks, int S, int K, int H, int E, cudaStream_t stream) {
   using namespace mep;
   const size_t row = (size_t)H * 2;
   const size_t tables = (size_t)(fresh ? 3 : 4) * E * sizeof(int);
@@ -389,12 +414,13 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
   // more than 64 KB of rows in flight per SM buys nothing; a smaller footprint starts sooner
   while (slots > 2 && (size_t)warps * (slots - 1) * row >= 96 * 1024) --slots;
   const size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
-  if (fresh) return launch_plain(local_dispatch_kernel<true>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
-  return launch_plain(local_dispatch_kernel<false>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+  if (fresh && S * K <= kLocDirect) return launch_plain(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+  if (fresh) return launch_plain(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+  return launch_plain(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
 }
 
 extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalCombineArgs* args, int num_blocks,
-                                        int S, int H, int K, cudaStream_t stream) {
+                                        int S, int H, int K, int pdl, cudaStream_t stream) {
   using namespace mep;
   const int nvec = H / 8;
   // a unit is what fits half a warp's stage, or less while that leaves warps without work
@@ -405,8 +431,8 @@ extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalC
   const int nparts = (nvec + part - 1) / part;
   MEP_REQUIRE((long long)S * nparts < (1ll << 30), "combine: S=%d, H=%d is too large", S, H);
   const int grid = (int)(((long long)S * nparts + kLcWarps - 1) / kLcWarps);
-  return launch_plain(local_combine_kernel, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
-                      stream, ctx, *args, part, nparts);
+  return launch_plain_pdl(local_combine_kernel, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
+                          stream, pdl != 0, ctx, *args, part, nparts);
 }
 
 MEP_EXPORT_SIZEOF(LocalDispatchArgs, mep::LocalDispatchArgs)

@@ -13,6 +13,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
                                                          const float* __restrict__ w, __nv_bfloat16* __restrict__ dgu,
                                                          float* __restrict__ dw, const int32_t* __restrict__ cu_seqlens,
                                                          int G, int Hp) {
+  pdl_trigger();
+  pdl_wait();
   const int nrows = cu_seqlens[G - 1];
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int nvec = Hp >> 3;
@@ -90,9 +92,9 @@ __global__ void __launch_bounds__(256) sgd_groups_kernel(__nv_bfloat16* __restri
 }  // namespace mep
 
 extern "C" int mep_swiglu_bwd(const void* dA, const void* gu, const float* w, void* dgu, float* dw,
-                              const int32_t* cu_seqlens, int G, int Hp, int num_blocks, cudaStream_t stream) {
+                              const int32_t* cu_seqlens, int G, int Hp, int num_blocks, int pdl, cudaStream_t stream) {
   MEP_REQUIRE(Hp % 8 == 0, "swiglu_bwd: inner size %d must be a multiple of 8", Hp);
-  return mep::launch_plain(mep::swiglu_bwd_kernel, dim3(num_blocks), dim3(256), 0, stream,
+  return mep::launch_plain_pdl(mep::swiglu_bwd_kernel, dim3(num_blocks), dim3(256), 0, stream, pdl != 0,
                            (const __nv_bfloat16*)dA, (const __nv_bfloat16*)gu, w, (__nv_bfloat16*)dgu, dw, cu_seqlens, G, Hp);
 }
 

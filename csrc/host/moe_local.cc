@@ -5,12 +5,12 @@
 #include "launch.h"
 
 extern "C" {
-int mep_launch_local_dispatch(const MepRankCtx*, const mep::LocalDispatchArgs*, int, int, int, int, cudaStream_t);
-int mep_launch_local_combine(const MepRankCtx*, const mep::LocalCombineArgs*, int, int, int, int, cudaStream_t);
+int mep_launch_local_dispatch(const MepRankCtx*, const mep::LocalDispatchArgs*, int, int, int, int, int, int, cudaStream_t);
+int mep_launch_local_combine(const MepRankCtx*, const mep::LocalCombineArgs*, int, int, int, int, int, cudaStream_t);
 int mep_grouped_gemm_2cta(int, const void*, int64_t, int64_t, int64_t, const void*, const void*, int64_t, int64_t, int64_t,
                           const mep::GemmArgs*, int, cudaStream_t);
 int mep_grouped_wgrad_2cta(const void*, int64_t, int64_t, const void*, int64_t, const mep::GemmArgs*, int, cudaStream_t);
-int mep_swiglu_bwd(const void*, const void*, const float*, void*, float*, const int32_t*, int, int, int, cudaStream_t);
+int mep_swiglu_bwd(const void*, const void*, const float*, void*, float*, const int32_t*, int, int, int, int, cudaStream_t);
 }
 
 namespace mep {
@@ -20,6 +20,7 @@ static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab) {
   a.cu_seqlens = slab + m.plan_off[7];
   a.pad_rows = slab + m.plan_off[2];
   a.G = 2 * m.E; a.g_end = 2 * m.E;
+  a.pdl = 1;                     // behind another kernel of the same call
   a.status = m.status; a.status_host = m.status_host; a.budget_ns = m.budget_ns;
   return a;
 }
@@ -27,6 +28,7 @@ static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab) {
 static LocalDispatchArgs dispatch_args(const MoeLocal& m, const void* hidden, int32_t* slab) {
   LocalDispatchArgs d = {};
   d.hidden = (const __nv_bfloat16*)hidden;
+  d.pad_step = 32;               // no GEMM of this layer reads further
   d.out_srcinfo = m.srcinfo;
   d.dst = slab + m.plan_off[0]; d.zero_fill = slab + m.plan_off[2];
   return d;
@@ -54,7 +56,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   d.dup_groups = slab + m.plan_off[4]; d.dup_loffs = slab + m.plan_off[5]; d.dup_counts = slab + m.plan_off[6];
   d.cu_seqlens = slab + m.plan_off[7];
   d.sync = m.sync; d.hist = m.hist;
-  if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.H, m.E, stream)) return -1;
+  if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.S, m.K, m.H, m.E, stream)) return -1;
   GemmArgs g = gemm_args(m, slab);
   g.N = m.Hp; g.K = m.H; g.out = m.act; g.out2 = keep ? m.gu : nullptr; g.row_scale = w; g.ldo = m.Hp;
   if (gemm(m, GEMM_GATE_UP, x, m.H, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
@@ -62,7 +64,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   g.N = m.H; g.K = m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DOWN, m.act, m.Hp, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, nullptr, (__nv_bfloat16*)out, nullptr};
-  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, stream);
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 1, stream);
 }
 
 // `update`: lr and the group mask of the update in the weight-gradient epilogues, or mask = null (gradients are stored).
@@ -72,12 +74,12 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   const MoeLocal& m = *mp;
   LocalDispatchArgs d = dispatch_args(m, dy, slab);
   d.out_hidden = m.shard;
-  if (mep_launch_local_dispatch(m.ctx, &d, 0, m.blocks, m.H, m.E, stream)) return -1;
+  if (mep_launch_local_dispatch(m.ctx, &d, 0, m.blocks, m.S, m.K, m.H, m.E, stream)) return -1;
   GemmArgs g = gemm_args(m, slab);
   g.N = m.Hp; g.K = m.H; g.out = m.dA; g.ldo = m.Hp;
   if (gemm(m, GEMM_DGRAD, m.shard, m.H, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
   const int32_t* cu = slab + m.plan_off[7];
-  if (mep_swiglu_bwd(m.dA, m.gu, m.w, m.dgu, m.shard_w, cu, 2 * m.E, m.Hp, 4 * m.num_ctas, stream)) return -1;
+  if (mep_swiglu_bwd(m.dA, m.gu, m.w, m.dgu, m.shard_w, cu, 2 * m.E, m.Hp, 4 * m.num_ctas, 1, stream)) return -1;
   auto wgrad = [&](const void* x, int64_t in, const void* dyc, int64_t ld, int64_t out, float* dw, const void* w) {
     GemmArgs a = gemm_args(m, slab);
     a.N = (int32_t)out; a.M_w = (int32_t)in; a.accumulate = accumulate; a.zero_empty_below = m.E; a.out = dw;
@@ -91,7 +93,7 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   g.N = m.H; g.K = 2 * m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DGRAD_GU, m.dgu, 2 * (int64_t)m.Hp, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, m.shard_w, (__nv_bfloat16*)dx, d_route_w};
-  if (mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, stream)) return -1;
+  if (mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 1, stream)) return -1;
   if (mask && wgrad(m.x, m.H, m.dgu, 2 * (int64_t)m.Hp, m.Hp, m.dw_gate, m.w_gate)) return -1;
   return wgrad(m.x, m.H, m.dgu + m.Hp, 2 * (int64_t)m.Hp, m.Hp, m.dw_up, m.w_up);
 }

@@ -69,7 +69,7 @@ class DispatchArgs(C.Structure):
 class LocalDispatchArgs(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("hidden", "weights", "out_hidden", "out_weights", "out_srcinfo", "dst", "zero_fill",
                                           "topk", "tpe", "cu_seqlens", "experts_to_copy", "remote_stats", "dup_groups",
-                                          "dup_loffs", "dup_counts", "sync", "hist")]
+                                          "dup_loffs", "dup_counts", "sync", "hist")] + [("pad_step", C.c_int32), ("reserved", C.c_int32)]
 
 
 class LocalCombineArgs(C.Structure):

@@ -293,7 +293,7 @@ def launch_local_dispatch(st: RankState, hidden, weights, plan, out_hidden, out_
         a.dup_groups, a.dup_loffs, a.dup_counts = plan.dup_groups.data_ptr(), plan.dup_loffs.data_ptr(), plan.dup_counts.data_ptr()
         a.sync, a.hist = sc["loc_sync"].data_ptr(), sc["loc_hist"].data_ptr()
     _native.check(_native.load().mep_launch_local_dispatch(C.c_void_p(st.ctx_ptr), C.byref(a), 1 if fresh else 0,
-                                                           min(num_blocks, st.local_blocks), g.H, g.E, _native.cur_stream()), "dispatch")
+                                                           min(num_blocks, st.local_blocks), g.S, g.K, g.H, g.E, _native.cur_stream()), "dispatch")
 
 
 def launch_local_combine(st: RankState, plan, rows, weights, out, out_weights, num_blocks: int):
@@ -301,7 +301,7 @@ def launch_local_combine(st: RankState, plan, rows, weights, out, out_weights, n
     shard's shape and are only read."""
     g = st.geo
     a = LocalCombineArgs(plan.dst.data_ptr(), rows.data_ptr(), ptr(weights), out.data_ptr(), ptr(out_weights))
-    _native.check(_native.load().mep_launch_local_combine(C.c_void_p(st.ctx_ptr), C.byref(a), num_blocks, g.S, g.H, g.K,
+    _native.check(_native.load().mep_launch_local_combine(C.c_void_p(st.ctx_ptr), C.byref(a), num_blocks, g.S, g.H, g.K, 0,
                                                           _native.cur_stream()), "combine")
 
 

@@ -29,7 +29,7 @@ _sm_cache: dict = {}
 class GemmArgs(C.Structure):
     _fields_ = [("cu_seqlens", C.c_void_p), ("G", C.c_int32), ("N", C.c_int32), ("K", C.c_int32),
                 ("M_w", C.c_int32), ("b_group_rows", C.c_int32), ("accumulate", C.c_int32),
-                ("g_begin", C.c_int32), ("g_end", C.c_int32), ("zero_empty_below", C.c_int32), ("reserved0", C.c_int32),
+                ("g_begin", C.c_int32), ("g_end", C.c_int32), ("zero_empty_below", C.c_int32), ("pdl", C.c_int32),
                 ("out", C.c_void_p), ("out2", C.c_void_p), ("row_scale", C.c_void_p), ("ldo", C.c_int64),
                 ("status", C.c_void_p), ("budget_ns", C.c_uint64), ("sched", C.c_void_p),
                 ("push_info", C.c_void_p), ("push_base", C.c_void_p), ("push_wbase", C.c_void_p),
@@ -319,7 +319,7 @@ def swiglu_bwd(dA, gu, w, dgu, dw, cu, num_blocks=None):
     nb = num_blocks or 4 * _num_sms(dA.device)
     _native.check(lib.mep_swiglu_bwd(C.c_void_p(dA.data_ptr()), C.c_void_p(gu.data_ptr()), C.c_void_p(_native.ptr(w)),
                                      C.c_void_p(dgu.data_ptr()), C.c_void_p(_native.ptr(dw)), C.c_void_p(cu.data_ptr()),
-                                     cu.numel(), Hp, nb, _native.cur_stream()), "swiglu_bwd")
+                                     cu.numel(), Hp, nb, 0, _native.cur_stream()), "swiglu_bwd")
 
 
 def sgd_step_groups(p, g, lr, mask, want: bool, num_blocks=None):
