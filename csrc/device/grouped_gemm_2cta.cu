@@ -101,30 +101,40 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   };
 
   if (warp == 0) {
-    // ---------------- TMA producer: this CTA's halves; bytes are counted on the LEADER's barrier
-    if (lane == 0) {
-      int it = 0; Tile ti;
-      tq::Scheduler<true> sched; tq::Consumer<true> follow;
-      if (dyn) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
-      tq::Strided seq{pair, npairs, ntiles};
-      for (int t; !s_abort && (t = !dyn ? seq.next() : leader ? sched.next(args.budget_ns) : follow.next(args.budget_ns)) != -1;) {
-        if (t == -2) { fail(5, it); break; }
-        get_tile(t, ti);
-        for (int kb = 0; kb < ti.kblocks; ++kb, ++it) {
-          const int s = it % kRing; const uint32_t ph = (uint32_t)(it / kRing) & 1u;
-          if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns)) { fail(1, t); break; }
-          const uint32_t sa = smem_u32(smem + (size_t)s * kStageBytes), sb = sa + kHalfBytes;
-          const uint32_t bar = mapa(smem_u32(&full_bar[s]), 0);
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);     // both CTAs' bytes
+    // ---------------- TMA producer: this CTA's halves; bytes are counted on the LEADER's barrier. The whole warp runs the
+    // loop and one elected lane issues (see grouped_gemm_pair.cu).
+    Tile ti;
+    uint32_t s = 0, ph = 0;
+    bool any = false, ready = true;      // ready: the stage is known to be free
+    tq::Scheduler<true> sched; tq::Consumer<true> follow;
+    if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
+    tq::Strided seq{pair, npairs, ntiles};
+    const uint32_t smem0 = smem_u32(smem), full0 = mapa(smem_u32(&full_bar[0]), 0);
+    for (;;) {
+      int t = -1;
+      if (!dyn) { if (!s_abort) t = seq.next(); }
+      else if (lane == 0 && !s_abort) { t = leader ? sched.next(args.budget_ns) : follow.next(args.budget_ns); if (t == -2) fail(5, -1); }
+      t = __shfl_sync(0xffffffffu, t, 0);
+      if (t < 0) break;
+      get_tile(t, ti);
+      const int am = ti.m0 + (int)cr * 128, bn = ti.n0 + (int)cr * 128;
+      for (int kb = 0; kb < ti.kblocks; ++kb) {
+        if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
+        const uint32_t sn = s + 1 == kRing ? 0u : s + 1, phn = sn ? ph : ph ^ 1u;
+        ready = mbar_test(&empty_bar[sn], phn ^ 1u);
+        if (elect_one()) {
+          const uint32_t sa = smem0 + s * kStageBytes, bar = full0 + s * 8u;
           const int k = ti.row0 + kb * kBK;
-          const int am = ti.m0 + (int)cr * 128, bn = ti.n0 + (int)cr * 128;
-          tma_load_2d_bar(sa, &tma_a, am, k, bar);
-          tma_load_2d_bar(sa + kAtomBytes, &tma_a, am + 64, k, bar);
-          tma_load_2d_bar(sb, &tma_b, bn, k, bar);
-          tma_load_2d_bar(sb + kAtomBytes, &tma_b, bn + 64, k, bar);
+          if (leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);     // both CTAs' bytes
+          tma_load_3d_bar(sa, &tma_a, 0, k, am / 64, bar);
+          tma_load_3d_bar(sa + kHalfBytes, &tma_b, 0, k, bn / 64, bar);
         }
+        __syncwarp();
+        any = true;
+        s = sn; ph = phn;
       }
     }
+    if (leader && any) mbar_wait_bounded(&full_bar[s ? s - 1 : kRing - 1], s ? ph : ph ^ 1u, args.budget_ns);     // no copy outlives the pair
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only): one instruction drives both SMs. The whole warp runs the loop so
     // that stage, phase and descriptors are warp-uniform (see grouped_gemm_pair.cu); one elected lane issues.
@@ -133,6 +143,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       const uint64_t adesc0 = tc::smem_desc(smem_u32(smem), kAtomBytes, 1024), bdesc0 = tc::smem_desc(smem_u32(smem) + kHalfBytes, kAtomBytes, 1024);
       int tcnt = 0; Tile ti;
       uint32_t stage = 0, phase = 0;
+      bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
       tq::Strided seq{pair, npairs, ntiles};
       for (;; ++tcnt) {
@@ -149,7 +160,12 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * 256;
         bool ok = true;
         for (int kb = 0; kb < ti.kblocks; ++kb) {
-          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) { if (lane == 0) fail(3, t); ok = false; break; }
+          if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) {
+            if (lane == 0) fail(3, t);
+            ok = false; break;
+          }
+          const uint32_t sn = stage + 1 == kRing ? 0u : stage + 1, phn = sn ? phase : phase ^ 1u;
+          ready = mbar_test(&full_bar[sn], phn);
           tc::fence_after_sync();
           const int steps = ti.ksteps - 4 * kb;
           if (elect_one()) {
@@ -160,7 +176,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             mma2_commit_both(smem_u32(&empty_bar[stage]));
           }
           __syncwarp();
-          if (++stage == kRing) { stage = 0; phase ^= 1u; }
+          stage = sn; phase = phn;
         }
         if (!ok) break;
         if (elect_one()) mma2_commit_both(smem_u32(&tfull_bar[acc]));
@@ -302,8 +318,8 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   num_ctas &= ~1;
   MEP_REQUIRE(num_ctas >= 2, "wgrad (2-CTA): needs at least two CTAs");
   CUtensorMap ma, mb, mo;
-  if (tmap_rows(&ma, x, rows, args.M_w, x_ld, 64, 64, false)) return -1;
-  if (tmap_rows(&mb, dy, rows, args.N, dy_ld, 64, 64, false)) return -1;
+  if (tmap_atoms(&ma, x, rows, args.M_w, x_ld, 2)) return -1;
+  if (tmap_atoms(&mb, dy, rows, args.N, dy_ld, 2)) return -1;
   if (tmap_rows(&mo, args.out, (int64_t)args.G * args.M_w, args.N, args.N, 32, 32, true)) return -1;
   if (allow_smem((const void*)w2::wgrad_2cta_kernel, w2::kSmem)) return -1;
   cudaLaunchConfig_t cfg = {};

@@ -58,7 +58,8 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, 
 
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
-tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_x16, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
+tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_x64,
+                const __grid_constant__ CUtensorMap tma_x16, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
                 const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out2, GemmArgs args) {
   constexpr bool W_MN = MODE == GEMM_GATE_UP || MODE == GEMM_DOWN;      // weights [k, column]: the M side is contiguous
   constexpr int kCols = MODE == GEMM_GATE_UP ? 128 : 256;               // output columns of a tile
@@ -87,7 +88,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     tq::init(&s_ring, 2 * kEpiWarps + 2);      // both CTAs' epilogue warps, the MMA issuer, the peer's producer
     fence_mbar_init();
   } else if (threadIdx.x == 96) {
-    tc::prefetch_tmap(&tma_x); tc::prefetch_tmap(&tma_x16); tc::prefetch_tmap(&tma_w0); tc::prefetch_tmap(&tma_w1);
+    tc::prefetch_tmap(&tma_x); tc::prefetch_tmap(&tma_x64); tc::prefetch_tmap(&tma_x16); tc::prefetch_tmap(&tma_w0); tc::prefetch_tmap(&tma_w1);
     tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
   }
   pdl_wait();                            // everything below reads what kernels before this one wrote
@@ -118,7 +119,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   const uint32_t tmem_base = s_tmem_base;
   const int ntiles = s_start[G];
   const bool dyn = args.sched != nullptr;
-  // Token rows arrive in boxes of 64, or of 16 where no tile of the launch has more than 48 for a CTA: a stage is then
+  // Token rows arrive in one box of 128 or 64, or in boxes of 16 where no tile of the launch has more than 48 for a CTA: a stage is then
   // little more than its weights and up to eleven fit instead of six. With few tokens per expert the kernel streams
   // weights, and what an SM has in flight is its bandwidth.
   const bool small = s_half <= 48;
@@ -145,43 +146,54 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   };
 
   if (warp == 0) {
-    // ---------------- TMA producer: this CTA's halves; bytes are counted on the LEADER's barrier
-    if (lane == 0) {
-      int it = 0, gcur = 0; Tile ti;
-      uint32_t s = 0, ph = 0;
-      tq::Scheduler<true> sched; tq::Consumer<true> follow;
-      if (dyn) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
-      tq::Strided seq{pair, npairs, ntiles};
-      const uint32_t tile_ep = args.tile_done ? *(volatile const uint32_t*)args.tile_epoch : 0u;
-      const uint32_t group_ep = args.group_flags ? *(volatile const uint32_t*)args.group_epoch : 0u;
-      int seen_row = -1, seen_group = -1;            // flags known to be up: 128-row blocks of the last tile, last group
-      for (int t; !s_abort && (t = !dyn ? seq.next() : leader ? sched.next(args.budget_ns) : follow.next(args.budget_ns)) != -1;) {
-        if (t == -2) { fail(5, it); break; }
-        get_tile(t, gcur, ti);
-        if (args.tile_done && ti.row0 != seen_row) {
-          // the rows come from a dispatch that may still be running: wait until they have all landed and the
-          // duplicates are expanded, then order the TMA engine's reads behind that
-          bool up = true;
-          for (int b = ti.row0 >> 7; up && b <= (ti.row0 + ti.n - 1) >> 7; ++b) up = wait_flag<false>(args.tile_done + b, tile_ep, args.budget_ns);
-          if (!up) { fail(9, t, MEP_ERR_FLAG_TIMEOUT); break; }
-          fence_proxy_async();
-          seen_row = ti.row0;
-        }
-        if (args.group_flags && ti.g >= args.group_first && ti.g != seen_group) {
-          // the weights of this group are a prefetched expert that may still be on its way
-          if (!wait_flag<true>(args.group_flags + (ti.g - args.group_first), group_ep, args.budget_ns)) { fail(9, t, MEP_ERR_FLAG_TIMEOUT); break; }
-          fence_proxy_async();
-          seen_group = ti.g;
-        }
-        const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
-        const int boxes = small ? half >> 4 : (half + 63) >> 6;
-        const uint32_t bytes = (uint32_t)kWBytes + (uint32_t)boxes * (small ? 2048u : 8192u);
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns)) { fail(1, t); break; }
-          const uint32_t sw = smem_u32(smem) + s * stage_bytes, sx = sw + kWBytes;
-          const uint32_t bar = mapa(smem_u32(&full_bar[s]), 0);
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * bytes);
+    // ---------------- TMA producer: this CTA's halves; bytes are counted on the LEADER's barrier. Like the MMA issuer the
+    // whole warp runs the loop and one elected lane issues: with a single diverged thread a k-block cost 640 cycles of
+    // issue alone, which held an SM to 46 GB/s of weights and the tensor cores to 80 % of their rate.
+    int gcur = 0; Tile ti;
+    uint32_t s = 0, ph = 0;
+    bool any = false, ready = true;      // ready: the stage is known to be free
+    tq::Scheduler<true> sched; tq::Consumer<true> follow;
+    if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
+    tq::Strided seq{pair, npairs, ntiles};
+    const uint32_t tile_ep = args.tile_done ? *(volatile const uint32_t*)args.tile_epoch : 0u;
+    const uint32_t group_ep = args.group_flags ? *(volatile const uint32_t*)args.group_epoch : 0u;
+    int seen_row = -1, seen_group = -1;              // flags known to be up: first row of the last tile, last group
+    const uint32_t smem0 = smem_u32(smem), full0 = mapa(smem_u32(&full_bar[0]), 0);
+    for (;;) {
+      int t = -1;
+      if (!dyn) { if (!s_abort) t = seq.next(); }
+      else if (lane == 0 && !s_abort) { t = leader ? sched.next(args.budget_ns) : follow.next(args.budget_ns); if (t == -2) fail(5, -1); }
+      t = __shfl_sync(0xffffffffu, t, 0);
+      if (t < 0) break;
+      get_tile(t, gcur, ti);
+      int up = 1;
+      if (args.tile_done && ti.row0 != seen_row) {
+        // the rows come from a dispatch that may still be running: wait until they have all landed and the
+        // duplicates are expanded, then order the TMA engine's reads behind that
+        if (lane == 0)
+          for (int b = ti.row0 >> 7; up && b <= (ti.row0 + ti.n - 1) >> 7; ++b) up = wait_flag<false>(args.tile_done + b, tile_ep, args.budget_ns) ? 1 : 0;
+        seen_row = ti.row0;
+      }
+      if (args.group_flags && ti.g >= args.group_first && ti.g != seen_group) {
+        // the weights of this group are a prefetched expert that may still be on its way
+        if (lane == 0 && up) up = wait_flag<true>(args.group_flags + (ti.g - args.group_first), group_ep, args.budget_ns) ? 1 : 0;
+        seen_group = ti.g;
+      }
+      if (args.tile_done || args.group_flags) {
+        if (!__shfl_sync(0xffffffffu, up, 0)) { if (lane == 0) fail(9, t, MEP_ERR_FLAG_TIMEOUT); break; }
+        __syncwarp();
+        fence_proxy_async();
+      }
+      const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
+      const uint32_t bytes = (uint32_t)kWBytes + (small ? (uint32_t)half * 128u : half > 64 ? 16384u : 8192u);
+      for (int kb = 0; kb < kblocks; ++kb) {
+        if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
+        const uint32_t sn = s + 1 == nstages ? 0u : s + 1, phn = sn ? ph : ph ^ 1u;
+        ready = mbar_test(&empty_bar[sn], phn ^ 1u);
+        if (elect_one()) {
+          const uint32_t sw = smem0 + s * stage_bytes, sx = sw + kWBytes, bar = full0 + s * 8u;
           const int k0 = kb * kBK;
+          if (leader) mbar_expect_tx(&full_bar[s], 2 * bytes);
           if (MODE == GEMM_GATE_UP) {
             tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
             tma_load_3d_bar(sw + kAtomBytes, &tma_w1, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
@@ -189,21 +201,24 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
             tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
           } else {
             const int kh = args.K / 2;               // DGRAD_GU: first half of K from Wg, second from Wu
-            const bool second = MODE == GEMM_DGRAD_GU && k0 >= kh;
-            tma_load_2d_bar(sw, second ? &tma_w1 : &tma_w0, second ? k0 - kh : k0, wrow + ti.n0 + (int)cr * 128, bar);
+            if (MODE == GEMM_DGRAD_GU && k0 >= kh) tma_load_2d_bar(sw, &tma_w1, k0 - kh, wrow + ti.n0 + (int)cr * 128, bar);
+            else tma_load_2d_bar(sw, &tma_w0, k0, wrow + ti.n0 + (int)cr * 128, bar);
           }
           if (small) {
-            for (int i = 0; i < boxes; ++i) tma_load_2d_bar(sx + i * 2048, &tma_x16, k0, xrow + 16 * i, bar);
-          } else {
+            for (int i = 0; i < half; i += 16) tma_load_2d_bar(sx + i * 128, &tma_x16, k0, xrow + i, bar);
+          } else if (half > 64) {
             tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
-            if (boxes > 1) tma_load_2d_bar(sx + 8192, &tma_x, k0, xrow + 64, bar);
+          } else {
+            tma_load_2d_bar(sx, &tma_x64, k0, xrow, bar);
           }
-          if (++s == nstages) { s = 0; ph ^= 1u; }
         }
+        __syncwarp();
+        any = true;
+        s = sn; ph = phn;
       }
-      // the leader's last barrier phase covers both CTAs' copies: nobody leaves before it (cluster_sync below)
-      if (leader && it > 0) mbar_wait_bounded(&full_bar[s ? s - 1 : nstages - 1], s ? ph : ph ^ 1u, args.budget_ns);
     }
+    // the leader's last barrier phase covers both CTAs' copies: nobody leaves before it (cluster_sync below)
+    if (leader && any) mbar_wait_bounded(&full_bar[s ? s - 1 : nstages - 1], s ? ph : ph ^ 1u, args.budget_ns);
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only): one instruction drives both SMs. The whole warp runs the loop so
     // that stage, phase and descriptors are warp-uniform; one elected lane issues. With a single diverged thread the
@@ -215,6 +230,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       constexpr uint32_t kWStep = W_MN ? 2048 >> 4 : 32 >> 4, kXStep = 32 >> 4;      // one 16-deep step in a descriptor's address field
       int tcnt = 0, gcur = 0; Tile ti;
       uint32_t stage = 0, phase = 0;
+      bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
       tq::Strided seq{pair, npairs, ntiles};
       for (;; ++tcnt) {
@@ -231,7 +247,12 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * 256;
         bool ok = true;
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) { if (lane == 0) fail(3, t); ok = false; break; }
+          if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) {
+            if (lane == 0) fail(3, t);
+            ok = false; break;
+          }
+          const uint32_t sn = stage + 1 == nstages ? 0u : stage + 1, phn = sn ? phase : phase ^ 1u;
+          ready = mbar_test(&full_bar[sn], phn);
           tc::fence_after_sync();
           if (elect_one()) {
             const uint64_t wd = wdesc0 + stage * (stage_bytes >> 4), xd = xdesc0 + stage * (stage_bytes >> 4);
@@ -240,7 +261,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
             mma2_commit_both(smem_u32(&empty_bar[stage]));
           }
           __syncwarp();
-          if (++stage == nstages) { stage = 0; phase ^= 1u; }
+          stage = sn; phase = phn;
         }
         if (!ok) break;
         if (elect_one()) mma2_commit_both(smem_u32(&tfull_bar[acc]));
@@ -404,8 +425,9 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   MEP_REQUIRE(args.K % 64 == 0 && args.N % (mode == GEMM_GATE_UP ? 128 : 256) == 0, "gemm (CTA pairs): K=%d N=%d not tileable", args.K, args.N);
   num_ctas &= ~1;
   MEP_REQUIRE(num_ctas >= 2, "gemm (CTA pairs): needs at least two CTAs");
-  CUtensorMap mx, mx16, mw0, mw1, mo, mo2;
-  if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 64) || tmap_rows(&mx16, a, a_rows, a_cols, a_ld, 64, 16)) return -1;
+  CUtensorMap mx, mx64, mx16, mw0, mw1, mo, mo2;
+  if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 128) || tmap_rows(&mx64, a, a_rows, a_cols, a_ld, 64, 64) ||
+      tmap_rows(&mx16, a, a_rows, a_cols, a_ld, 64, 16)) return -1;
   auto weights = [&](CUtensorMap* m, const void* b) {
     if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1);
     if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2);
@@ -428,7 +450,7 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
 #define MEP_TP_CASE(M)                                                                             \
   case M:                                                                                          \
     if (allow_smem((const void*)tp::tok_pair_kernel<M>, tp::kSmem)) return -1;                       \
-    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tp::tok_pair_kernel<M>, mx, mx16, mw0, mw1, mo, mo2, args));   \
+    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tp::tok_pair_kernel<M>, mx, mx64, mx16, mw0, mw1, mo, mo2, args));   \
     break;
   switch (mode) {
     MEP_TP_CASE(GEMM_GATE_UP) MEP_TP_CASE(GEMM_DOWN) MEP_TP_CASE(GEMM_DGRAD) MEP_TP_CASE(GEMM_DGRAD_GU)
