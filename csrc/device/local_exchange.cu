@@ -434,6 +434,3 @@ extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalC
   return launch_plain_pdl(local_combine_kernel, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
                           stream, pdl != 0, ctx, *args, part, nparts);
 }
-
-MEP_EXPORT_SIZEOF(LocalDispatchArgs, mep::LocalDispatchArgs)
-MEP_EXPORT_SIZEOF(LocalCombineArgs, mep::LocalCombineArgs)

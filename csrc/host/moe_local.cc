@@ -34,6 +34,14 @@ static LocalDispatchArgs dispatch_args(const MoeLocal& m, const void* hidden, in
   return d;
 }
 
+static void plan_into(const MoeLocal& m, const int32_t* topk, const int32_t* tpe, int32_t* slab, LocalDispatchArgs* d) {
+  d->topk = topk; d->tpe = tpe;
+  d->dst = slab + m.plan_off[0]; d->experts_to_copy = slab + m.plan_off[1]; d->zero_fill = slab + m.plan_off[2];
+  d->remote_stats = slab + m.plan_off[3]; d->dup_groups = slab + m.plan_off[4]; d->dup_loffs = slab + m.plan_off[5];
+  d->dup_counts = slab + m.plan_off[6]; d->cu_seqlens = slab + m.plan_off[7];
+  d->sync = m.sync; d->hist = m.hist;
+}
+
 // x [NvS, in] times weights [2E, in, out] (or their transposes), see GemmMode
 static int gemm(const MoeLocal& m, GemmMode mode, const void* a, int64_t a_cols, const void* b0, const void* b1, int64_t in, int64_t out,
                 GemmArgs& g, cudaStream_t stream) {
@@ -43,6 +51,28 @@ static int gemm(const MoeLocal& m, GemmMode mode, const void* a, int64_t a_cols,
 
 }  // namespace mep
 
+// Dispatch and combine alone, for a Buffer whose caller computes the experts. Dispatch plans into `slab` when `topk` is
+// given and reads the plan from it otherwise; `dst` / `zero_fill` may come from another plan's tensors instead.
+extern "C" int mep_local_dispatch_call(const mep::MoeLocal* mp, const void* hidden, const float* route_w, const int32_t* topk, const int32_t* tpe,
+                                       int32_t* slab, int32_t* dst, int32_t* zero_fill, void* rows, float* row_w, cudaStream_t stream) {
+  using namespace mep;
+  const MoeLocal& m = *mp;
+  LocalDispatchArgs d = {};
+  d.hidden = (const __nv_bfloat16*)hidden; d.weights = route_w;
+  d.out_hidden = (__nv_bfloat16*)rows; d.out_weights = row_w; d.out_srcinfo = m.srcinfo;
+  d.dst = dst; d.zero_fill = zero_fill;
+  if (topk) plan_into(m, topk, tpe, slab, &d);
+  return mep_launch_local_dispatch(m.ctx, &d, topk ? 1 : 0, m.blocks, m.S, m.K, m.H, m.E, stream);
+}
+
+extern "C" int mep_local_combine_call(const mep::MoeLocal* mp, const int32_t* dst, const void* rows, const float* row_w, void* out, float* out_w,
+                                      cudaStream_t stream) {
+  using namespace mep;
+  const MoeLocal& m = *mp;
+  LocalCombineArgs c = {dst, (const __nv_bfloat16*)rows, row_w, (__nv_bfloat16*)out, out_w};
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 0, stream);
+}
+
 extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden, const float* route_w, const int32_t* topk,
                                      const int32_t* tpe, int32_t* slab, void* out, int keep, cudaStream_t stream) {
   using namespace mep;
@@ -51,11 +81,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   float* w = keep ? m.w : m.shard_w;
   LocalDispatchArgs d = dispatch_args(m, hidden, slab);
   d.weights = route_w; d.out_hidden = x; d.out_weights = w;
-  d.topk = topk; d.tpe = tpe;
-  d.experts_to_copy = slab + m.plan_off[1]; d.remote_stats = slab + m.plan_off[3];
-  d.dup_groups = slab + m.plan_off[4]; d.dup_loffs = slab + m.plan_off[5]; d.dup_counts = slab + m.plan_off[6];
-  d.cu_seqlens = slab + m.plan_off[7];
-  d.sync = m.sync; d.hist = m.hist;
+  plan_into(m, topk, tpe, slab, &d);
   if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.S, m.K, m.H, m.E, stream)) return -1;
   GemmArgs g = gemm_args(m, slab);
   g.N = m.Hp; g.K = m.H; g.out = m.act; g.out2 = keep ? m.gu : nullptr; g.row_scale = w; g.ldo = m.Hp;

@@ -66,16 +66,6 @@ class DispatchArgs(C.Structure):
                 ("send_list", C.c_void_p), ("send_meta", C.c_void_p)]
 
 
-class LocalDispatchArgs(C.Structure):
-    _fields_ = [(n, C.c_void_p) for n in ("hidden", "weights", "out_hidden", "out_weights", "out_srcinfo", "dst", "zero_fill",
-                                          "topk", "tpe", "cu_seqlens", "experts_to_copy", "remote_stats", "dup_groups",
-                                          "dup_loffs", "dup_counts", "sync", "hist")] + [("pad_step", C.c_int32), ("reserved", C.c_int32)]
-
-
-class LocalCombineArgs(C.Structure):
-    _fields_ = [(n, C.c_void_p) for n in ("dst", "rows", "weights", "out", "out_weights")]
-
-
 class MoeLocal(C.Structure):
     _fields_ = ([("ctx", C.c_void_p)] + [(n, C.c_int32) for n in ("S", "H", "Hp", "K", "E", "NvS", "blocks", "combine_blocks",
                                                                  "num_ctas", "reserved")]
@@ -163,6 +153,8 @@ def load(build_if_missing: bool = True):
     lib.mep_swiglu_dense_bwd.argtypes = [vp, vp, vp, C.c_int64, i32, vp]
     lib.mep_route_bwd.argtypes = [vp] * 4 + [i32] * 3 + [vp]
     lib.mep_swiglu.argtypes = [vp, vp, C.c_int64, i32, vp]
+    lib.mep_local_dispatch_call.argtypes = [vp] * 11
+    lib.mep_local_combine_call.argtypes = [vp] * 7
     lib.mep_moe_local_forward.argtypes = [vp] * 7 + [i32, vp]
     lib.mep_moe_local_backward.argtypes = [vp] * 5 + [i32, C.c_float, vp, vp]
     _LIB = lib

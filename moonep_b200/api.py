@@ -188,24 +188,30 @@ class OpsMixin:
         assert (p.N, p.R, p.E, p.NvS, p.K) == (g.N, g.R, g.E, g.NvS, g.K), "plan belongs to another Buffer geometry"
 
     # ---- dispatch
+    def _local_exchange(self) -> engine.LocalExchange:
+        ex = getattr(self, "_local_ex", None)
+        if ex is None:
+            ex = self._local_ex = engine.LocalExchange(self._states[0], self._num_sms_dedup)
+        return ex
+
     def _dispatch_local(self, hidden, weights, topk, tpe, plan, zero_copy=False, w_zero_copy=False, out=None):
         """Single rank: one kernel plans and scatters, straight into the private copies if those are wanted (rows
         behind the last group's are not written there).  ``out``: tensors to fill instead."""
         st = self._states[0]
-        cu = None
-        if plan is None:
-            topk = topk.reshape(-1)
-            self._check_topk(topk, tpe)
-            plan, cu = engine.allocate_plan(st)
-        else:
-            self._check_plan(plan)
-            topk = tpe = None
         if out is not None:
             h, w = out
         else:
             h = st.hidden_local if zero_copy else torch.empty_like(st.hidden_local)
             w = None if weights is None else st.weights_local if w_zero_copy else torch.empty_like(st.weights_local)
-        engine.launch_local_dispatch(st, hidden, weights, plan, h, w, self._num_sms_dedup, topk, tpe, cu)
+        ex = self._local_exchange()
+        if plan is not None:
+            self._check_plan(plan)
+            ex.dispatch_again(hidden, weights, plan, h, w)
+            return h, w, None, plan
+        if not topk.is_contiguous():
+            topk = topk.reshape(-1)
+        self._check_topk(topk, tpe)
+        plan, cu = ex.dispatch(hidden, weights, topk, tpe, h, w)
         return h, w, cu, plan
 
     def _dispatch_lists(self, hidden, weights, topk, tpe, plans, *, inter_rank_sync, zero_copy, w_zero_copy):
@@ -289,7 +295,7 @@ class OpsMixin:
         self._check_plan(plan)
         out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=st.device)
         ow = None if w is None else torch.empty((g.S, g.K), dtype=torch.float32, device=st.device)
-        engine.launch_local_combine(st, plan, h, w, out, ow, self._num_sms_dedup)
+        self._local_exchange().combine(plan, h, w, out, ow)
         return out, ow
 
     def _combine_lists(self, plans, hidden_nvsh, weights_nvs, *, inter_rank_sync, zero_copy, w_zero_copy):

@@ -16,7 +16,7 @@ import torch
 
 from . import _native
 from ._native import (MepRankCtx, PlanArgs, DispatchArgs, DupFinalizeArgs, DupArgs, CombineArgs, PushReduceArgs,
-                      PrefetchArgs, GradReduceArgs, SendOrderArgs, LocalDispatchArgs, LocalCombineArgs, ptr)
+                      PrefetchArgs, GradReduceArgs, SendOrderArgs, ptr)
 from .geometry import Geometry
 from .plan import MoonEPCommPlan
 
@@ -230,27 +230,83 @@ def _plan_of_parts(g: Geometry, parts, with_send_list: bool = False):
     return plan, parts[7]
 
 
-class LocalLayer:
+class LocalExchange:
+    """Single-rank dispatch and combine, one native call each (csrc/host/moe_local.cc)."""
+
+    def __init__(self, st: RankState, blocks: int):
+        g, a = st.geo, _native.MoeLocal()
+        a.ctx = st.ctx_ptr
+        a.S, a.H, a.K, a.E, a.NvS = g.S, g.H, g.K, g.E, g.NvS
+        a.blocks, a.combine_blocks = min(blocks, st.local_blocks), blocks
+        _, self._total, first = _plan_layout(st)
+        a.plan_off = (C.c_int64 * 8)(*first)
+        self._cu_first, self._cu_n = first[7], 2 * g.epn
+        a.shard, a.shard_w, a.srcinfo = st.hidden_local.data_ptr(), st.weights_local.data_ptr(), ptr(st.srcinfo_local)
+        a.sync, a.hist = st.scratch["loc_sync"].data_ptr(), st.scratch["loc_hist"].data_ptr()
+        self._geo, self._args, self._ref, self._dev = g, a, C.addressof(a), st.device
+        self._ints = dict(N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K)
+        self._fields = dict(dst=(first[0], g.N, None), experts_to_copy=(first[1], g.epn, (1, g.epn)),
+                            zero_fill_ranges=(first[2], 4 * g.epn, (2 * g.epn, 2)), remote_stats=(first[3], 2, None),
+                            dup_groups=(first[4], 3 * g.NvS, (g.NvS, 3)), dup_loffs=(first[5], g.NvS, None), dup_counts=(first[6], 2, None))
+        self._lib = _native.load()
+
+    def _name_part(self, slab, name):
+        f = self._fields.get(name)
+        if f is None:
+            return None
+        v = slab.narrow(0, f[0], f[1])
+        return v if f[2] is None else v.view(f[2])
+
+    def plan_of(self, slab):
+        """``(plan, cu_seqlens)`` of an allocation that a native call has planned into."""
+        return MoonEPCommPlan.of_slab(slab, self._name_part, self._ints), slab.narrow(0, self._cu_first, self._cu_n)
+
+    def dispatch(self, hidden, route_w, topk, tpe, out_hidden, out_w):
+        """A fresh plan (in one allocation: what a small dispatch would otherwise wait for) and the K rows of every
+        token; returns ``(plan, cu_seqlens)``.  ``out_hidden`` / ``out_w``: any tensors of the shard's shape."""
+        slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
+        rc = self._lib.mep_local_dispatch_call(self._ref, hidden.data_ptr(), None if route_w is None else route_w.data_ptr(),
+                                               topk.data_ptr(), tpe.data_ptr(), slab.data_ptr(), None, None, out_hidden.data_ptr(),
+                                               None if out_w is None else out_w.data_ptr(), _native.raw_stream())
+        if rc:
+            _native.check(rc, "dispatch")
+        return self.plan_of(slab)
+
+    def dispatch_again(self, hidden, route_w, plan, out_hidden, out_w):
+        """The rows of a saved plan."""
+        rc = self._lib.mep_local_dispatch_call(self._ref, hidden.data_ptr(), None if route_w is None else route_w.data_ptr(), None, None,
+                                               None, self._dst(plan), plan.zero_fill_ranges.data_ptr(), out_hidden.data_ptr(),
+                                               None if out_w is None else out_w.data_ptr(), _native.raw_stream())
+        if rc:
+            _native.check(rc, "dispatch")
+
+    @staticmethod
+    def _dst(plan) -> int:      # the first field of a plan's allocation
+        slab = plan.__dict__.get("_slab")
+        return plan.dst.data_ptr() if slab is None else slab.data_ptr()
+
+    def combine(self, plan, rows, row_w, out, out_w):
+        """``out[s]`` = sum of the K rows of token ``s``; ``rows`` / ``row_w`` are any tensors of the shard's shape and only read."""
+        rc = self._lib.mep_local_combine_call(self._ref, self._dst(plan), rows.data_ptr(), None if row_w is None else row_w.data_ptr(),
+                                              out.data_ptr(), None if out_w is None else out_w.data_ptr(), _native.raw_stream())
+        if rc:
+            _native.check(rc, "combine")
+
+
+class LocalLayer(LocalExchange):
     """A single-rank MoE layer's forward and backward pass as one native call each (csrc/host/moe_local.cc)."""
 
     def __init__(self, st: RankState, Hp: int, weights, grads, work: dict, blocks: int, num_ctas: int, status, status_host, budget_ns: int):
-        g, a = st.geo, _native.MoeLocal()
-        a.ctx = st.ctx_ptr
-        a.S, a.H, a.Hp, a.K, a.E, a.NvS = g.S, g.H, Hp, g.K, g.E, g.NvS
-        a.blocks, a.combine_blocks, a.num_ctas = min(blocks, st.local_blocks), blocks, num_ctas
-        self._sizes, self._total, first = _plan_layout(st)
-        a.plan_off = (C.c_int64 * 8)(*first)
+        super().__init__(st, blocks)
+        a = self._args
+        a.Hp, a.num_ctas = Hp, num_ctas
         for name, t in zip(("w_gate", "w_up", "w_down"), weights):
             setattr(a, name, t.data_ptr())
         for name, t in zip(("dw_gate", "dw_up", "dw_down"), grads or ()):
             setattr(a, name, t.data_ptr())
         for name, t in work.items():
             setattr(a, name, t.data_ptr())
-        a.shard, a.shard_w, a.srcinfo = st.hidden_local.data_ptr(), st.weights_local.data_ptr(), ptr(st.srcinfo_local)
-        a.sync, a.hist = st.scratch["loc_sync"].data_ptr(), st.scratch["loc_hist"].data_ptr()
         a.status, a.status_host, a.budget_ns = status.data_ptr(), status_host.data_ptr(), budget_ns
-        self._geo, self._args, self._ref, self._dev = g, a, C.addressof(a), st.device
-        self._lib = _native.load()
 
     def forward(self, hidden, route_w, topk, tpe, keep: bool):
         """Returns ``(out, plan allocation)``."""
@@ -272,37 +328,6 @@ class LocalLayer:
         if rc:
             _native.check(rc, "moe backward")
         return dx, dw
-
-    def plan_of(self, slab):
-        """``(plan, cu_seqlens)`` of a forward pass."""
-        return _plan_of_parts(self._geo, slab.split(self._sizes)[::2])
-
-
-def launch_local_dispatch(st: RankState, hidden, weights, plan, out_hidden, out_weights, num_blocks: int,
-                          topk=None, tpe=None, cu=None):
-    """Single rank: the plan (if ``topk`` is given), the K rows of every token and the padding rows, one launch.
-    ``out_hidden`` / ``out_weights``: this rank's shard or any tensors of its shape."""
-    g = st.geo
-    a = LocalDispatchArgs(hidden.data_ptr(), ptr(weights), out_hidden.data_ptr(), ptr(out_weights), ptr(st.srcinfo_local),
-                          plan.dst.data_ptr(), plan.zero_fill_ranges.data_ptr())
-    fresh = topk is not None
-    if fresh:
-        sc = st.scratch
-        a.topk, a.tpe, a.cu_seqlens = topk.data_ptr(), tpe.data_ptr(), cu.data_ptr()
-        a.experts_to_copy, a.remote_stats = plan.experts_to_copy.data_ptr(), plan.remote_stats.data_ptr()
-        a.dup_groups, a.dup_loffs, a.dup_counts = plan.dup_groups.data_ptr(), plan.dup_loffs.data_ptr(), plan.dup_counts.data_ptr()
-        a.sync, a.hist = sc["loc_sync"].data_ptr(), sc["loc_hist"].data_ptr()
-    _native.check(_native.load().mep_launch_local_dispatch(C.c_void_p(st.ctx_ptr), C.byref(a), 1 if fresh else 0,
-                                                           min(num_blocks, st.local_blocks), g.S, g.K, g.H, g.E, _native.cur_stream()), "dispatch")
-
-
-def launch_local_combine(st: RankState, plan, rows, weights, out, out_weights, num_blocks: int):
-    """Single rank: ``out[s]`` = sum of the K rows of token ``s``; ``rows`` / ``weights`` may be any tensors of the
-    shard's shape and are only read."""
-    g = st.geo
-    a = LocalCombineArgs(plan.dst.data_ptr(), rows.data_ptr(), ptr(weights), out.data_ptr(), ptr(out_weights))
-    _native.check(_native.load().mep_launch_local_combine(C.c_void_p(st.ctx_ptr), C.byref(a), num_blocks, g.S, g.H, g.K, 0,
-                                                          _native.cur_stream()), "combine")
 
 
 def launch_planning(states, topk_list, tpe_list, plans, cu_list):

@@ -343,14 +343,18 @@ def sgd_step(p, g, lr, num_blocks=None):
                                    C.c_int64(p.numel()), nb, _native.cur_stream()), "sgd_step")
 
 
-def sgd_step_many(ps, gs, lr, num_blocks=None):
-    """``sgd_step`` of up to four tensors in one launch."""
-    lib = _native.load()
-    n = len(ps)
-    for p, g in zip(ps, gs):
-        assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.numel() == g.numel()
-        assert p.is_contiguous() and g.is_contiguous()
-    nb = num_blocks or 8 * _num_sms(ps[0].device)
-    P, N = C.c_void_p * n, C.c_int64 * n
-    _native.check(lib.mep_sgd_step_many(n, P(*[p.data_ptr() for p in ps]), P(*[g.data_ptr() for g in gs]), N(*[p.numel() for p in ps]),
-                                        C.c_float(lr), nb, _native.cur_stream()), "sgd_step_many")
+class SgdMany:
+    """``sgd_step`` of up to four tensors in one launch; the tensors are fixed, so their addresses are gathered once."""
+
+    def __init__(self, ps, gs, num_blocks=None):
+        n = len(ps)
+        for p, g in zip(ps, gs):
+            assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.numel() == g.numel()
+            assert p.is_contiguous() and g.is_contiguous()
+        P, N = C.c_void_p * n, C.c_int64 * n
+        self._args = (n, P(*[p.data_ptr() for p in ps]), P(*[g.data_ptr() for g in gs]), N(*[p.numel() for p in ps]))
+        self._blocks = num_blocks or 8 * _num_sms(ps[0].device)
+        self._keep = (list(ps), list(gs))
+
+    def step(self, lr):
+        _native.check(_native.load().mep_sgd_step_many(*self._args, C.c_float(lr), self._blocks, _native.cur_stream()), "sgd_step_many")

@@ -76,6 +76,25 @@ class MoonEPCommPlan:
         p.__dict__.update(fields_)
         return p
 
+    @classmethod
+    def of_slab(cls, slab, name_part, sizes: dict):
+        """A plan whose tensors are views of ``slab``: ``name_part(slab, field)`` returns one (None: no such field).  Each is
+        made when it is first asked for; a plan that only travels from dispatch to combine never needs them."""
+        p = cls.__new__(cls)
+        d = p.__dict__
+        d.update(sizes)
+        d["_slab"], d["_name_part"] = slab, name_part
+        return p
+
+    def __getattr__(self, name):        # reached only for what is not set yet
+        d = self.__dict__
+        make = d.get("_name_part")
+        v = None if make is None else make(d["_slab"], name)
+        if v is None:
+            raise AttributeError(name)
+        d[name] = v
+        return v
+
     def tensors(self):
         """The tensor fields, in declaration order (used for record_stream)."""
         return tuple(getattr(self, f.name) for f in fields(self)
