@@ -253,9 +253,9 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
                : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded mbarrier wait (budget in nanoseconds, see budget_cycles).
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
+// Bounded mbarrier wait (budget in nanoseconds, see budget_cycles). The polling loop is kept out of line: a GEMM waits in
+// ten places, and every launch fetches its code anew.
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
   // Back off between polls. Measured on the CTA-pair wgrad kernel (10 polling threads per CTA):
   // 1106 TFLOP/s with this 40 ns pause, 875 without it -- threads spinning on barriers keep the
   // shared-memory pipe busy and slow down every other barrier / copy instruction of the CTA.
@@ -267,6 +267,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     for (int i = 0; i < 32; ++i) { __nanosleep(MEP_POLL_SLEEP_NS); if (mbar_try_wait(bar, parity)) return true; }
     if (clock64() - t0 > lim) return false;
   }
+}
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
+  return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, budget_ns);
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }

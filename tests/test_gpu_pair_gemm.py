@@ -63,3 +63,31 @@ def test_padding_rows_are_skipped(sizes, kn, dynamic, cuda_device):
     for i, (r, p, e) in enumerate(zip(n, padded, ends.tolist())):
         ref = y[e - p:e - p + r].float().T @ act[e - p:e - p + r].float()
         assert torch.equal(dW[i], torch.zeros_like(dW[i])) if r == 0 else _rel(dW[i], ref) < 1e-4, f"group {i} ({r} rows): wgrad"
+
+
+def test_swiglu_epilogue_of_extreme_pre_activations(cuda_device):
+    """Gate values outside the epilogue's branch-free range (|g| >= 60, tiny, zero, infinite, NaN) beside ordinary ones: with
+    a unit gate weight and an up weight of one the activation is g / (1 + exp(-g)) * 1, rounded to bf16 once."""
+    from moonep_b200.ops import grouped_gemm as gg
+    vals = [0.0, -0.0, 1.0, -1.0, 59.9, -59.9, 60.0, -60.0, 87.0, -87.0, 88.5, -88.5, 104.0, -104.0, 1e30, -1e30, 3e38, -3e38,
+            1e-30, -1e-30, 1e-37, -1e-37, 2.5, -2.5, float("inf"), float("-inf"), float("nan"), 17.0, -17.0, 30.0, -30.0, 0.5]
+    rows, K, N = 128, 64, 128
+    x = torch.zeros(rows, K, device="cuda")
+    v = torch.tensor(vals, device="cuda").repeat(4)
+    x[:, 1] = 1.0
+    finite = torch.isfinite(v)
+    wg, wu = torch.zeros(1, K, N, device="cuda"), torch.zeros(1, K, N, device="cuda")
+    wg[0, 0] = 1.0                       # gate = x[:, 0] in every column
+    wu[0, 1] = 1.0                       # up = 1
+    x[:, 0] = torch.where(finite, v, torch.zeros_like(v))
+    cu = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    x, wg, wu = x.to(torch.bfloat16), wg.to(torch.bfloat16), wu.to(torch.bfloat16)
+    act, gu = torch.empty(rows, N, dtype=torch.bfloat16, device="cuda"), torch.empty(rows, 2 * N, dtype=torch.bfloat16, device="cuda")
+    gg.gate_up(x, wg, wu, cu, act, gu)
+    torch.cuda.synchronize()
+    gg.check_status()
+    g = x[:, 0].double()
+    ref = (g / (1.0 + torch.exp(-g)))[:, None].expand(rows, N)
+    assert torch.equal(gu[:, :N], x[:, :1].expand(rows, N)) and bool((gu[:, N:] == 1).all())
+    # exp's two ulp and one bf16 rounding: within one bf16 ulp (2^-7); below the smallest normal number fp32 exp ends in zero
+    assert bool(((act.double() - ref).abs() <= 2.0 ** -7 * ref.abs() + 2e-36).all())
