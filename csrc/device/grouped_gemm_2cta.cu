@@ -119,7 +119,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       get_tile(t, ti);
       const int am = ti.m0 + (int)cr * 128, bn = ti.n0 + (int)cr * 128;
       for (int kb = 0; kb < ti.kblocks; ++kb) {
-        if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
+        if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_compact(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
         const uint32_t sn = s + 1 == kRing ? 0u : s + 1, phn = sn ? ph : ph ^ 1u;
         ready = mbar_test(&empty_bar[sn], phn ^ 1u);
         if (elect_one()) {
@@ -134,7 +134,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         s = sn; ph = phn;
       }
     }
-    if (leader && any) mbar_wait_bounded(&full_bar[s ? s - 1 : kRing - 1], s ? ph : ph ^ 1u, args.budget_ns);     // no copy outlives the pair
+    if (leader && any) mbar_wait_compact(&full_bar[s ? s - 1 : kRing - 1], s ? ph : ph ^ 1u, args.budget_ns);     // no copy outlives the pair
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only): one instruction drives both SMs. The whole warp runs the loop so
     // that stage, phase and descriptors are warp-uniform (see grouped_gemm_pair.cu); one elected lane issues.
@@ -155,12 +155,12 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         get_tile(t, ti);
         if (ti.kblocks == 0) { --tcnt; continue; }
         const int acc = tcnt & 1; const uint32_t aph = (uint32_t)(tcnt >> 1) & 1u;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, args.budget_ns))) { if (lane == 0) fail(2, t); break; }
+        if (!__all_sync(0xffffffffu, mbar_wait_compact(&tempty_bar[acc], aph ^ 1u, args.budget_ns))) { if (lane == 0) fail(2, t); break; }
         tc::fence_after_sync();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * 256;
         bool ok = true;
         for (int kb = 0; kb < ti.kblocks; ++kb) {
-          if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) {
+          if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_compact(&full_bar[stage], phase, args.budget_ns))) {
             if (lane == 0) fail(3, t);
             ok = false; break;
           }
@@ -227,7 +227,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       }
       const int acc = tcnt & 1; const uint32_t aph = (uint32_t)(tcnt >> 1) & 1u;
       int ok = 1;
-      if (lane == 0) ok = mbar_wait_bounded(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0;
+      if (lane == 0) ok = mbar_wait_compact(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) { if (lane == 0) fail(4, t); break; }
       tc::fence_after_sync();

@@ -202,7 +202,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
       const uint32_t bytes = (uint32_t)kWBytes + (small ? (uint32_t)half * 128u : half > 64 ? 16384u : 8192u);
       for (int kb = 0; kb < kblocks; ++kb) {
-        if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
+        if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_compact(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
         const uint32_t sn = s + 1 == nstages ? 0u : s + 1, phn = sn ? ph : ph ^ 1u;
         ready = mbar_test(&empty_bar[sn], phn ^ 1u);
         if (elect_one()) {
@@ -233,7 +233,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       }
     }
     // the leader's last barrier phase covers both CTAs' copies: nobody leaves before it (cluster_sync below)
-    if (leader && any) mbar_wait_bounded(&full_bar[s ? s - 1 : nstages - 1], s ? ph : ph ^ 1u, args.budget_ns);
+    if (leader && any) mbar_wait_compact(&full_bar[s ? s - 1 : nstages - 1], s ? ph : ph ^ 1u, args.budget_ns);
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only): one instruction drives both SMs. The whole warp runs the loop so
     // that stage, phase and descriptors are warp-uniform; one elected lane issues. With a single diverged thread the
@@ -257,12 +257,12 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         get_tile(t, gcur, ti);
         const uint32_t idesc = tc::instr_desc_bf16(256, 0, W_MN, false) | ((uint32_t)(ti.n >> 3) << 17);
         const int acc = tcnt & 1; const uint32_t aph = (uint32_t)(tcnt >> 1) & 1u;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, args.budget_ns))) { if (lane == 0) fail(2, t); break; }
+        if (!__all_sync(0xffffffffu, mbar_wait_compact(&tempty_bar[acc], aph ^ 1u, args.budget_ns))) { if (lane == 0) fail(2, t); break; }
         tc::fence_after_sync();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * 256;
         bool ok = true;
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], phase, args.budget_ns))) {
+          if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_compact(&full_bar[stage], phase, args.budget_ns))) {
             if (lane == 0) fail(3, t);
             ok = false; break;
           }
@@ -323,7 +323,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
           const int i = ((set_tid >> 4) * 2 + set) * kChunk + (set_tid & 15);
           if (i < ti.n) rs = __ldcg(args.row_scale + ti.row0 + i);
         }
-        if (lane == 0) { ok = mbar_wait_bounded(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0; if (!ok) fail(4, t); }
+        if (lane == 0) { ok = mbar_wait_compact(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0; if (!ok) fail(4, t); }
         ok = __shfl_sync(0xffffffffu, ok, 0);
       }
       if (MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) s_scale[set][acc][set_tid] = rs;

@@ -253,9 +253,8 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
                : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded mbarrier wait (budget in nanoseconds, see budget_cycles). The polling loop is kept out of line: a GEMM waits in
-// ten places, and every launch fetches its code anew.
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
+// Bounded mbarrier wait (budget in nanoseconds, see budget_cycles).
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
   // Back off between polls. Measured on the CTA-pair wgrad kernel (10 polling threads per CTA):
   // 1106 TFLOP/s with this 40 ns pause, 875 without it -- threads spinning on barriers keep the
   // shared-memory pipe busy and slow down every other barrier / copy instruction of the CTA.
@@ -269,7 +268,13 @@ static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parit
   }
 }
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
-  return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, budget_ns);
+  return mbar_try_wait(bar, parity) || mbar_poll(bar, parity, budget_ns);
+}
+// The same with the polling loop out of line, for the GEMMs: they wait in ten places, and every launch fetches its code
+// anew. (The streaming kernels keep theirs inline: the call cost the single-rank combine 9 %.)
+static __device__ __noinline__ bool mbar_poll_call(uint64_t* bar, uint32_t parity, uint64_t budget_ns) { return mbar_poll(bar, parity, budget_ns); }
+__device__ __forceinline__ bool mbar_wait_compact(uint64_t* bar, uint32_t parity, uint64_t budget_ns) {
+  return mbar_try_wait(bar, parity) || mbar_poll_call(bar, parity, budget_ns);
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }

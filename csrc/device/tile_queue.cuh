@@ -82,7 +82,7 @@ struct Scheduler {
   // Next tile, or -1 at the end of the sequence; -2 if the ring never drained (bounded wait expired).
   __device__ __forceinline__ int next(uint64_t budget_ns) {
     const int slot = n % kSlots; const uint32_t ph = (uint32_t)(n / kSlots) & 1u;
-    const bool ok = PAIR ? wait_cluster_bounded(&r->empty[slot], ph ^ 1u, budget_ns) : mbar_wait_bounded(&r->empty[slot], ph ^ 1u, budget_ns);
+    const bool ok = PAIR ? wait_cluster_bounded(&r->empty[slot], ph ^ 1u, budget_ns) : mbar_wait_compact(&r->empty[slot], ph ^ 1u, budget_ns);
     if (!ok) return -2;
     int t = (int)pending;
     if (t < ntiles) pending = atomicAdd(counter, 1u); else t = -1;
@@ -116,7 +116,7 @@ struct Consumer {
   // Next tile (>= 0), -1 at the end, -2 if the bounded wait expired. One thread per role calls this.
   __device__ __forceinline__ int next(uint64_t budget_ns) {
     const int slot = n % kSlots; const uint32_t ph = (uint32_t)(n / kSlots) & 1u;
-    const bool ok = PAIR ? wait_cluster_bounded(&r->full[slot], ph, budget_ns) : mbar_wait_bounded(&r->full[slot], ph, budget_ns);
+    const bool ok = PAIR ? wait_cluster_bounded(&r->full[slot], ph, budget_ns) : mbar_wait_compact(&r->full[slot], ph, budget_ns);
     if (!ok) return -2;
     const int t = *(volatile int*)&r->id[slot];
     if (PAIR) arrive_cluster(sched_empty + 8u * slot);
