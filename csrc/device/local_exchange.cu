@@ -20,7 +20,8 @@ constexpr int kLocEntries = 1024;          // top-k entries ranked and copied at
 constexpr int kLocZeroBytes = 4096;        // zeroed shared memory the padding rows are stored from
 constexpr int kLocMaxSlots = 8;            // row slots per copying warp
 
-constexpr int kLocDirect = 8192;           // up to this many entries every CTA counts all entries before its own by itself
+constexpr int kLocDirect = 24576;          // up to this many entries every CTA counts all entries before its own by itself (dispatch
+                                           // at 12248 entries 16.8 instead of 22.8 us, at 18006 35 instead of 40, at 32768 106 instead of 102)
 
 // Padding rows that are cleared behind row `first` of a group's `n` (see LocalDispatchArgs.pad_step).
 __device__ __forceinline__ int local_pads(int first, int n, int step) { return step ? min(n, -first & (step - 1)) : n; }
