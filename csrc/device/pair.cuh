@@ -34,10 +34,6 @@ __device__ __forceinline__ void mma2_bf16(uint32_t tmem_d, uint64_t adesc, uint6
                "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// arrives on ONE barrier (own or peer CTA, given as a cluster address) when the pair's MMAs are done
-__device__ __forceinline__ void mma2_commit(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar_cluster_addr) : "memory");
-}
 // arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair when the pair's MMAs are done
 __device__ __forceinline__ void mma2_commit_both(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" :: "r"(bar), "h"((uint16_t)3) : "memory");

@@ -71,7 +71,7 @@ def _block_forward(blk, hidden, router, s0, s1, keep: bool):
     if s0 is not None:
         gu = hidden @ s0
         act = rt.swiglu(gu)
-        out.add_(act @ s1)
+        out.addmm_(act, s1)
     return out, mctx, probs, topk, gu, act
 
 

@@ -22,6 +22,8 @@ CASES = [
     (333,    5,  5,    7168,  128, "single_expert"),
     (64,     8,  8,    15360, 128, "biased"),
     (20000,  8,  32,   64,    128, "biased"),
+    (3072,   8,  64,   128,   16,  "random"),     # 24576 entries: the last size at which every CTA counts for itself
+    (3511,   7,  64,   128,   16,  "random"),     # 24577: the first with the hand-over
 ]
 
 
