@@ -32,6 +32,12 @@ constexpr int kChunk = 16;                             // tokens per epilogue st
 constexpr int kStgBytes = kChunk * 128;                // staging: 16 tokens x 64 columns
 constexpr int kXchBytes = 32 * 32;                     // half of a warp's fp32 fragments of a chunk (GATE_UP)
 constexpr int kMaxGroups = 192;
+// BANDS: a group with more than kXBytes of token rows is walked in bands of at most kBand token tiles, all weight columns for
+// a band, then the next band. 74 pairs then read 8 + 9 operand slabs at a time and fetch each token row from DRAM once; DRAM
+// traffic also costs clock, the kernels being at the power limit. One group of 32768 tokens, 7168 x 2048: gate/up 1.85 ->
+// 1.55 ms, down 0.91 -> 0.74; groups of 4000, 4096 x 1024: gate/up 0.471 -> 0.440, dgrad 0.237 -> 0.226. Below the line the
+// weights would be read again for nothing (4096 tokens, 4096 deep, 32 MB: 1.445 -> 1.481).
+constexpr int kBand = 8, kXBytes = 36 << 20;
 constexpr int kStgSet = 4 * kStgBytes;                 // GATE_UP: act twice, gate, up; else: two buffers for each 64-column side
 constexpr size_t kEpiBytes = 2 * kStgSet + kEpiWarps * kXchBytes;
 constexpr size_t kSmem = (size_t)kRingBytes + kEpiBytes + 1024;
@@ -58,6 +64,13 @@ __device__ __forceinline__ float silu(float g) {
   return fmaf(fmaf(-d, q, g), r, q);
 }
 
+// a / b for a >= 0, b > 0 and results below 2^20, without the code of an integer division: __fdividef is off by 2 ulp at
+// most, so the quotient by one at most.
+__device__ __forceinline__ int quotient(int a, int b) {
+  const int q = (int)__fdividef((float)a + 0.5f, (float)b), r = a - q * b;
+  return q + (r >= b) - (r < 0);
+}
+
 // Bounded poll of a ready flag (see GemmArgs.tile_done / group_flags); SYS: written by another GPU.
 template <bool SYS>
 __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, uint64_t budget_ns) {
@@ -71,7 +84,7 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, 
   }
 }
 
-template <int MODE>
+template <int MODE, bool BANDS>
 __global__ void __launch_bounds__(kThreads, 1)
 tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_x64,
                 const __grid_constant__ CUtensorMap tma_x16, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
@@ -150,11 +163,19 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   };
   auto fail = [&](int site, int tile, int code = MEP_ERR_MBAR_TIMEOUT) { note(site, tile, code); s_abort = 1; };
   // tile number -> tile; `g` is a monotone cursor. The tiles of a group share its tokens evenly (in units of 32), token
-  // tiles vary fastest: the weight columns they have in common are then in L2.
+  // tiles vary fastest: the weight columns they have in common are then in L2 (within a band, see kBand).
   auto get_tile = [&](int t, int& g, Tile& ti) {
     while (s_start[g + 1] <= t) ++g;
     const int units = s_units[g], mt = (units + 7) >> 3, local = t - s_start[g];
-    const int cb = local / mt, pt = local - cb * mt, base = units / mt, rem = units - base * mt;
+    int cb, pt;
+    if (BANDS && (int64_t)mt * args.K > kXBytes / 512) {
+      const int nblk = args.N / kCols, bands = quotient(mt - 1, kBand) + 1, bw = quotient(mt - 1, bands) + 1;
+      const int b = quotient(local, bw * nblk), in = local - b * bw * nblk, w = min(bw, mt - b * bw);
+      cb = quotient(in, w); pt = b * bw + in - cb * w;
+    } else {
+      cb = local / mt; pt = local - cb * mt;
+    }
+    const int base = units / mt, rem = units - base * mt;
     ti.g = g; ti.n0 = cb * kCols;
     ti.row0 = s_beg[g] + 32 * (pt * base + min(pt, rem));
     ti.n = 32 * (base + (pt < rem ? 1 : 0));
@@ -474,11 +495,16 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
-#define MEP_TP_CASE(M)                                                                             \
-  case M:                                                                                          \
-    if (allow_smem((const void*)tp::tok_pair_kernel<M>, tp::kSmem)) return -1;                       \
-    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tp::tok_pair_kernel<M>, mx, mx64, mx16, mw0, mw1, mo, mo2, args));   \
-    break;
+  // Group sizes are only known on the device, and the code for bands costs a launch of few tiles 1 us of 20: it is there where
+  // groups are half as large as the line on average, so that some may be above it.
+  const bool bands = a_rows * args.K * 2 > (int64_t)args.G * (tp::kXBytes / 2);
+#define MEP_TP_CASE(M)                                                                                          \
+  case M: {                                                                                                     \
+    auto* kernel = bands ? tp::tok_pair_kernel<M, true> : tp::tok_pair_kernel<M, false>;                           \
+    if (allow_smem((const void*)kernel, tp::kSmem)) return -1;                                                  \
+    MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, mx, mx64, mx16, mw0, mw1, mo, mo2, args));                  \
+    break;                                                                                                      \
+  }
   switch (mode) {
     MEP_TP_CASE(GEMM_GATE_UP) MEP_TP_CASE(GEMM_DOWN) MEP_TP_CASE(GEMM_DGRAD) MEP_TP_CASE(GEMM_DGRAD_GU)
     default: return set_error("gemm (CTA pairs): unknown mode %d", mode);

@@ -65,6 +65,34 @@ def test_padding_rows_are_skipped(sizes, kn, dynamic, cuda_device):
         assert torch.equal(dW[i], torch.zeros_like(dW[i])) if r == 0 else _rel(dW[i], ref) < 1e-4, f"group {i} ({r} rows): wgrad"
 
 
+@pytest.mark.parametrize("dynamic", [False, True], ids=["static", "dynamic"])
+def test_large_groups_are_walked_in_bands(dynamic, cuda_device):
+    """4096 deep, a group of more than 18 token tiles (36 MB) is taken in bands of at most 8: the last size below the line,
+    the first above it, bands of unequal size, between small groups."""
+    from moonep_b200.ops import grouped_gemm as gg
+    K, N, n = 4096, 512, [128, 4608, 4736, 0, 6272, 256]
+    cu = torch.tensor(n).cumsum(0).to(torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, w, wu, wt = bf(sum(n), K), bf(len(n), K, N, sc=0.02), bf(len(n), K, N, sc=0.02), bf(len(n), N, K, sc=0.02)
+    full = lambda c: torch.full((sum(n), c), float("nan"), dtype=torch.bfloat16, device="cuda")    # noqa: E731
+    act, gu, y, dA = full(N), full(2 * N), full(N), full(N)
+    gg.gate_up(x, w, wu, cu, act, gu, dynamic=dynamic)
+    gg.down(x, w, cu, y, dynamic=dynamic)
+    gg.dgrad(x, wt, cu, dA, dynamic=dynamic)
+    torch.cuda.synchronize()
+    gg.check_status()
+    a = 0
+    for i, r in enumerate(n):
+        if r:
+            s = slice(a, a + r)
+            for got, ref in ((gu[s, :N], w[i]), (gu[s, N:], wu[i]), (y[s], w[i]), (dA[s], wt[i].T)):
+                # bf16 results of fp32 sums: half a bf16 ulp is 2^-9; rows one by one, so that a misplaced tile shows
+                d, f = x[s].float() @ ref.float(), got.float()
+                assert bool(((f - d).norm(dim=1) < 4e-3 * d.norm(dim=1)).all()), f"group {i} ({r} rows)"
+        a += r
+
+
 def test_swiglu_epilogue_of_extreme_pre_activations(cuda_device):
     """Gate values outside the epilogue's branch-free range (|g| >= 60, tiny, zero, infinite, NaN) beside ordinary ones: with
     a unit gate weight and an up weight of one the activation is g / (1 + exp(-g)) * 1, rounded to bf16 once."""
