@@ -38,6 +38,15 @@ __device__ __forceinline__ void mma2_bf16(uint32_t tmem_d, uint64_t adesc, uint6
 __device__ __forceinline__ void mma2_commit_both(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" :: "r"(bar), "h"((uint16_t)3) : "memory");
 }
+// Division of a >= 0 by a launch constant, results below 2^20: the product with the rounded reciprocal is off by one at most
+struct Divisor {
+  int b; float r;
+  __device__ __forceinline__ explicit Divisor(int d) : b(d), r(1.f / (float)d) {}
+  __device__ __forceinline__ int operator()(int a) const {
+    const int q = (int)(((float)a + 0.5f) * r), rem = a - q * b;
+    return q + (rem >= b) - (rem < 0);
+  }
+};
 // one lane of a converged warp; the others' registers stay warp-uniform, which keeps MMA descriptors out of the vector registers
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;

@@ -93,6 +93,27 @@ def test_large_groups_are_walked_in_bands(dynamic, cuda_device):
         a += r
 
 
+@pytest.mark.parametrize("M", [2048, 2816, 4352])
+def test_weight_gradient_of_large_groups(M, cuda_device):
+    """Above 9 M elements of x in a group on average the row blocks go in bands of at most 8: 8 in one, 6 + 5, 6 + 6 + 5."""
+    from moonep_b200.ops import grouped_gemm as gg
+    n, N = [6400, 128, 0, 14976], 512
+    cu = torch.tensor(n).cumsum(0).to(torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, dy = ((torch.randn(sum(n), c, device="cuda", generator=g)).to(torch.bfloat16) for c in (M, N))
+    dW = torch.full((len(n), M, N), 7.0, device="cuda")
+    gg.wgrad(x, dy, cu, dW, zero_empty_below=len(n))
+    torch.cuda.synchronize()
+    gg.check_status()
+    a = 0
+    for i, r in enumerate(n):
+        ref = x[a:a + r].float().T @ dy[a:a + r].float()
+        # fp32 sums of the same products in another order; 256 x 256 blocks one by one, so that a misplaced tile shows
+        for got, want in zip(dW[i].unfold(0, 256, 256).unfold(1, 256, 256).flatten(0, 1), ref.unfold(0, 256, 256).unfold(1, 256, 256).flatten(0, 1)):
+            assert bool((got == 0).all()) if r == 0 else _rel(got, want) < 1e-4, f"group {i} ({r} rows)"
+        a += r
+
+
 def test_swiglu_epilogue_of_extreme_pre_activations(cuda_device):
     """Gate values outside the epilogue's branch-free range (|g| >= 60, tiny, zero, infinite, NaN) beside ordinary ones: with
     a unit gate weight and an up weight of one the activation is g / (1 + exp(-g)) * 1, rounded to bf16 once."""
