@@ -517,9 +517,11 @@ def run_ours(args):
                   "launch": graph_note, "path": path_note,
                   "e2e_input_copy": (f"inside each step's graph, starting at the {copy_at} phase, into the other input buffer"
                                      if graphed_e2e[0] is not None else "on a side stream, issued before the step that precedes its use"),
-                  "dispatch": ("per-tile ready flags: gate/up and dgrad(down) GEMMs start while the dispatch kernel runs"
+                  "dispatch": ("one kernel: plan, rows and padding of a local permutation" if world == 1 else
+                               "per-tile ready flags: gate/up and dgrad(down) GEMMs start while the dispatch kernel runs"
                                if blk.moe.ready_flags else "the GEMMs start after the dispatch kernel's exit barrier"),
-                  "combine": ("pushed by the down GEMM's epilogue into the source ranks' memory, then a local sum"
+                  "combine": ("one kernel: local gather-sum" if world == 1 else
+                              "pushed by the down GEMM's epilogue into the source ranks' memory, then a local sum"
                               if blk.buf.geo.off_push else "pulled from the peers' shards after the down GEMM"),
                   "comm": "moonep_b200.Buffer", "expert_ffn": "moonep_b200 tcgen05 grouped GEMM"},
         "clocks": {"sm_mhz": clocks["sm_mhz"], "sm_max_mhz": clocks["sm_max_mhz"], "reasons": clocks["reasons"]},
