@@ -214,6 +214,9 @@ class ExpertParallelMoE:
             out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward)
             return out, _LocalContext(self, slab) if need_backward else None
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
+        if route_weights_sk is None:        # unscaled rows; the buffers hold the weights of an earlier call
+            assert not need_backward, "a forward pass without route weights has no backward pass"
+            w = None
         _, _, cu, plan = buf._dispatch_local(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, None, out=(x, w))
         pad = self._pad(plan)
         gg.gate_up(x, self._W("gate"), self._W("up"), cu, self._act, self._gu if need_backward else None, row_scale=w, pad=pad)

@@ -1,0 +1,35 @@
+"""Calls of a single-rank layer and block besides the plain training step: optional arguments, inputs of other forms,
+contexts and pools that the caller has changed."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def make_block(shared=0, H=256, Hp=256, **kw):
+    from moonep_b200.models.moe_block import MoEBlock, MoEConfig
+    cfg = MoEConfig("t", H=H, Hp=Hp, K=2, epn=4, shared_experts=shared, S=130)
+    return MoEBlock(cfg, num_sms=4, seed=3, router_skew=0.5, **kw)
+
+
+def normal(shape, seed, scale=0.5):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).to(torch.bfloat16)
+
+
+def test_layer_without_route_weights_is_unscaled(cuda_device):
+    """Without route weights the rows are not scaled, whatever an earlier call has left in the buffers of the weights."""
+    blk = make_block()
+    x = normal((130, 256), 1)
+    with torch.no_grad():
+        w, topk, tpe = blk.route(x)
+    ones = torch.ones_like(w)
+    ref, _ = blk.moe.forward(x, ones, topk, tpe, need_backward=False)
+    for keep in (False, True):
+        blk.moe.forward(x, w * 3, topk, tpe, need_backward=keep)
+        out, ctx = blk.moe.forward(x, None, topk, tpe, need_backward=False)
+        torch.cuda.synchronize()
+        assert ctx is None and torch.equal(out, ref)
+    with pytest.raises(AssertionError, match="route weights"):
+        blk.moe.forward(x, None, topk, tpe, need_backward=True)
+    blk.destroy()
