@@ -198,6 +198,7 @@ class OpsMixin:
         """Single rank: one kernel plans and scatters, straight into the private copies if those are wanted (rows
         behind the last group's are not written there).  ``out``: tensors to fill instead."""
         st = self._states[0]
+        self._check_hidden(hidden, weights)      # here, so that no caller hands an unchecked address to the kernel
         if out is not None:
             h, w = out
         else:
@@ -219,12 +220,12 @@ class OpsMixin:
         g = self.geo
         n = len(st)
         fresh = plans is None
-        for i in range(n):
-            self._check_hidden(hidden[i], None if weights is None else weights[i])
         if n == 1 and st[0].local and _SLOT_ORDER != "1":
             w = None if weights is None else weights[0]
             h, w, cu, p = self._dispatch_local(hidden[0], w, topk and topk[0], tpe and tpe[0], plans and plans[0], True, True)
             return [h if zero_copy else h.clone()], [w if w is None or w_zero_copy else w.clone()], [cu], [p]
+        for i in range(n):
+            self._check_hidden(hidden[i], None if weights is None else weights[i])
         cus = [None] * n
         # MOONEP_DISPATCH_SLOT_ORDER=1: the plain call also uses the slot-ordered kernel that expands
         # duplicate rows itself while rows are still arriving (no separate expansion pass)
@@ -557,7 +558,6 @@ class Buffer(OpsMixin):
             assert topk_experts_sk is not None and tokens_per_expert is not None, \
                 "dispatch needs topk_experts_sk and tokens_per_expert unless a plan is reused"
         if st.local and not async_finish and _SLOT_ORDER != "1" and not _NVTX:     # one kernel: straight to it
-            self._check_hidden(hidden_sh, route_weights_sk)
             h, w, cu, p = self._dispatch_local(hidden_sh, route_weights_sk, topk_experts_sk, tokens_per_expert, plan, zero_copy,
                                                router_weights_zero_copy)
             if plan is None and _VERIFY_PLANS and not torch.cuda.is_current_stream_capturing():

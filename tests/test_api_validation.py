@@ -168,3 +168,34 @@ def test_clock_sampler_with_a_fake_nvidia_smi(tmp_path, monkeypatch):
     # no usable power reading: fall back to the upper half of the clock samples
     assert under_load([300.0, 300.0, 1900.0, 1950.0], [None] * 4) == [1900.0, 1950.0]
     assert under_load([1965.0, 1400.0, 1420.0], [100.0, 990.0, 1000.0]) == [1400.0, 1420.0]
+
+
+@pytest.mark.parametrize("what", ["expanded", "dtype", "short", "weights", "weights_dtype"])
+def test_local_dispatch_checks_its_inputs_for_every_caller(what):
+    """The layer calls ``_dispatch_local`` itself, with tensors to fill: nothing unchecked may reach the kernel."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from moonep_b200.api import OpsMixin
+
+    class Calls(OpsMixin):
+        geo = Geometry.make(8, 64, 2, 4, 1)
+        _states = [SimpleNamespace(hidden_local=None, weights_local=None)]
+
+        def _local_exchange(self):
+            raise RuntimeError("the kernel would have been launched")
+
+    h, w = torch.zeros(8, 64, dtype=torch.bfloat16), torch.zeros(8, 2)
+    if what == "expanded":
+        h = torch.zeros(1, 64, dtype=torch.bfloat16).expand(8, 64)
+    elif what == "dtype":
+        h = h.float()
+    elif what == "short":
+        h = h[:7]
+    elif what == "weights":
+        w = w[:7]
+    else:
+        w = w.double()
+    with pytest.raises(AssertionError, match="contiguous"):
+        Calls()._dispatch_local(h, w, None, None, None, out=(None, None))

@@ -33,3 +33,21 @@ def test_layer_without_route_weights_is_unscaled(cuda_device):
     with pytest.raises(AssertionError, match="route weights"):
         blk.moe.forward(x, None, topk, tpe, need_backward=True)
     blk.destroy()
+
+
+def test_backward_with_a_hook_refuses_a_bad_gradient(cuda_device):
+    """With a hook between the launches the backward pass runs from Python; its gradient is checked there too."""
+    blk = make_block()
+    blk.moe.on_grad_ready = lambda n: None
+    x, dy = normal((130, 256), 1), normal((130, 256), 2)
+    with torch.no_grad():
+        w, topk, tpe = blk.route(x)
+    _, ctx = blk.moe.forward(x, w, topk, tpe)
+    for bad in (dy[:1].expand(130, 256), dy.float(), dy[:129]):
+        with pytest.raises(AssertionError, match="hidden_sh"):
+            blk.moe.backward(ctx, bad)
+    dx, _ = blk.moe.backward(ctx, dy)
+    torch.cuda.synchronize()
+    blk.buf.check()
+    assert bool(torch.isfinite(dx.float()).all())
+    blk.destroy()
