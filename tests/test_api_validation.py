@@ -199,3 +199,33 @@ def test_local_dispatch_checks_its_inputs_for_every_caller(what):
         w = w.double()
     with pytest.raises(AssertionError, match="contiguous"):
         Calls()._dispatch_local(h, w, None, None, None, out=(None, None))
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4, 8])
+def test_local_combine_takes_rows_of_any_alignment(offset):
+    """Private rows may start anywhere in their storage; what reaches the kernel's bulk loads lies on 16 bytes."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from moonep_b200.api import OpsMixin
+
+    seen = []
+
+    class Calls(OpsMixin):
+        geo = Geometry.make(8, 64, 2, 4, 1)
+        _states = [SimpleNamespace(device="cpu")]
+
+        def _check_plan(self, p):
+            pass
+
+        def _local_exchange(self):
+            return SimpleNamespace(combine=lambda plan, rows, *rest: seen.append(rows))
+
+    n = Calls.geo.NvS * 64
+    flat = torch.arange(n + 16, dtype=torch.int32).to(torch.bfloat16)
+    base = -flat.data_ptr() % 16 // 2
+    rows = flat[base + offset:base + offset + n].view(-1, 64)
+    Calls()._combine_local(None, rows, None)
+    assert seen[0].data_ptr() % 16 == 0 and torch.equal(seen[0], rows)
+    assert (seen[0].data_ptr() == rows.data_ptr()) == (offset % 8 == 0)

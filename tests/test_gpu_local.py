@@ -97,3 +97,19 @@ def test_local_exchange_reports_bad_tables(cuda_device):
         assert ei.value.status["code"] == 3
         buf.reset()
         buf.destroy()
+
+
+def test_combine_of_rows_that_start_off_a_16_byte_boundary(cuda_device):
+    S, H, K, E = 40, 64, 4, 8
+    topk, tpe = (t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=5))
+    x = torch.randn(S, H, device="cuda").to(torch.bfloat16)
+    buf = Buffer(S, H, K, E, 1, token_padding=8)
+    h, _, _, plan = buf.dispatch(x, None, topk, tpe)
+    rows = torch.empty(h.numel() + 1, dtype=h.dtype, device="cuda")[1:].view(h.shape)
+    rows.copy_(h)
+    a, _, _ = buf.combine(plan=plan, hidden_nvsh=h)
+    b, _, _ = buf.combine(plan=plan, hidden_nvsh=rows)
+    torch.cuda.synchronize()
+    buf.check()
+    assert rows.data_ptr() % 16 == 2 and torch.equal(a, b)
+    buf.destroy()
