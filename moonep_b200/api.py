@@ -171,6 +171,7 @@ class OpsMixin:
         g = self.geo
         assert h.dtype == torch.bfloat16 and h.is_contiguous() and h.shape == (g.S, g.H), \
             f"hidden_sh must be a contiguous [S={g.S}, H={g.H}] bf16 tensor"
+        assert h.data_ptr() % 16 == 0, "hidden_sh must start on a 16-byte boundary"      # bulk loads in every dispatch kernel
         if w is not None:
             assert w.dtype == torch.float32 and w.is_contiguous() and w.numel() == g.N, \
                 "route_weights_sk must be a contiguous [S, K] fp32 tensor"

@@ -170,7 +170,7 @@ def test_clock_sampler_with_a_fake_nvidia_smi(tmp_path, monkeypatch):
     assert under_load([1965.0, 1400.0, 1420.0], [100.0, 990.0, 1000.0]) == [1400.0, 1420.0]
 
 
-@pytest.mark.parametrize("what", ["expanded", "dtype", "short", "weights", "weights_dtype"])
+@pytest.mark.parametrize("what", ["expanded", "dtype", "short", "start", "weights", "weights_dtype"])
 def test_local_dispatch_checks_its_inputs_for_every_caller(what):
     """The layer calls ``_dispatch_local`` itself, with tensors to fill: nothing unchecked may reach the kernel."""
     from types import SimpleNamespace
@@ -193,11 +193,13 @@ def test_local_dispatch_checks_its_inputs_for_every_caller(what):
         h = h.float()
     elif what == "short":
         h = h[:7]
+    elif what == "start":
+        h = torch.zeros(8 * 64 + 8, dtype=torch.bfloat16)[1:8 * 64 + 1].view(8, 64)
     elif what == "weights":
         w = w[:7]
     else:
         w = w.double()
-    with pytest.raises(AssertionError, match="contiguous"):
+    with pytest.raises(AssertionError, match="contiguous|16-byte boundary"):
         Calls()._dispatch_local(h, w, None, None, None, out=(None, None))
 
 
