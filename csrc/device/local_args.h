@@ -46,7 +46,7 @@ struct MoeLocal {
   int32_t reserved;
   int64_t plan_off[8];           // elements from the start of a plan's allocation: dst, experts_to_copy, zero_fill,
                                  // remote_stats, dup_groups, dup_loffs, dup_counts, cu_seqlens
-  const void *w_gate, *w_up, *w_down;            // [2E, in, out] bf16
+  const void *w_gate, *w_up, *w_down;            // [2E, in, out] bf16; these and the gradients are set for each call
   __nv_bfloat16* shard;          // [NvS, H] the Buffer's shard
   float* shard_w;                // [NvS]
   int32_t* srcinfo;              // or null

@@ -294,23 +294,22 @@ class LocalExchange:
 
 
 class LocalLayer(LocalExchange):
-    """A single-rank MoE layer's forward and backward pass as one native call each (csrc/host/moe_local.cc)."""
+    """A single-rank MoE layer's forward and backward pass as one native call each (csrc/host/moe_local.cc).  ``work``:
+    the layer's own buffers.  The addresses of weights and gradients (gate, up, down) come with every call."""
 
-    def __init__(self, st: RankState, Hp: int, weights, grads, work: dict, blocks: int, num_ctas: int, status, status_host, budget_ns: int):
+    def __init__(self, st: RankState, Hp: int, work: dict, blocks: int, num_ctas: int, status, status_host, budget_ns: int):
         super().__init__(st, blocks)
+        self.state = st
         a = self._args
         a.Hp, a.num_ctas = Hp, num_ctas
-        for name, t in zip(("w_gate", "w_up", "w_down"), weights):
-            setattr(a, name, t.data_ptr())
-        for name, t in zip(("dw_gate", "dw_up", "dw_down"), grads or ()):
-            setattr(a, name, t.data_ptr())
         for name, t in work.items():
             setattr(a, name, t.data_ptr())
         a.status, a.status_host, a.budget_ns = status.data_ptr(), status_host.data_ptr(), budget_ns
 
-    def forward(self, hidden, route_w, topk, tpe, keep: bool):
+    def forward(self, hidden, route_w, topk, tpe, keep: bool, weights):
         """Returns ``(out, plan allocation)``."""
-        g = self._geo
+        g, a = self._geo, self._args
+        a.w_gate, a.w_up, a.w_down = weights
         slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
         out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
         rc = self._lib.mep_moe_local_forward(self._ref, hidden.data_ptr(), route_w.data_ptr(), topk.data_ptr(), tpe.data_ptr(),
@@ -319,8 +318,10 @@ class LocalLayer(LocalExchange):
             _native.check(rc, "moe forward")
         return out, slab
 
-    def backward(self, dy, slab, accumulate: bool, lr: float, mask):
-        g = self._geo
+    def backward(self, dy, slab, accumulate: bool, lr: float, mask, weights, grads):
+        g, a = self._geo, self._args
+        a.w_gate, a.w_up, a.w_down = weights
+        a.dw_gate, a.dw_up, a.dw_down = grads
         dx = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
         dw = torch.empty((g.S, g.K), dtype=torch.float32, device=self._dev)
         rc = self._lib.mep_moe_local_backward(self._ref, dy.data_ptr(), slab.data_ptr(), dx.data_ptr(), dw.data_ptr(),

@@ -144,7 +144,6 @@ class MoEBlock:
             self.shared = [(torch.randn(cfg.H, 2 * hs, device=dev, generator=g) * 0.02).to(torch.bfloat16).requires_grad_(True),
                            (torch.randn(hs, cfg.H, device=dev, generator=g) * 0.02).to(torch.bfloat16).requires_grad_(True)]
         self.moe = ExpertParallelMoE(self.buf, self.pools)
-        self._sgd = None
         # sgd_step() joins the last gradient reduction before it updates ``up``
         self.moe.defer_last_reduction = os.environ.get("MOONEP_DEFER_LAST_REDUCTION", "1") != "0"
         torch.cuda.synchronize()
@@ -212,9 +211,8 @@ class MoEBlock:
         if self.moe.on_grad_ready is None:
             names = ("down", "gate", "up")
             if self.moe.grads_pending is None:
-                if self._sgd is None:
-                    self._sgd = gg.SgdMany([self.pools.local_weight(n) for n in names], [self.pools.local_grad(n) for n in names])
-                self._sgd.step(lr)
+                ps = self.pools
+                ps.kept("sgd", lambda: gg.SgdMany([ps.local_weight(n) for n in names], [ps.local_grad(n) for n in names])).step(lr)
             else:
                 for n in names:                  # ``up`` last: its cross-rank reduction may still be running
                     self.moe.wait_grads(n)
@@ -230,7 +228,6 @@ class MoEBlock:
                     p.grad = None
 
     def destroy(self):
-        self._sgd = None
         self.moe.wait_grads()        # nothing of this layer may still be queued on the comm stream
         self.pools.destroy()
         if self._own_buffer:

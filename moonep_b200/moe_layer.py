@@ -146,12 +146,9 @@ class ExpertParallelMoE:
 
     def _native_layer(self):
         from . import engine
-        names = ("gate", "up", "down")
         return engine.LocalLayer(
-            self.buf._states[0], self.Hp, [self._W(n) for n in names],
-            [self._dW(n) for n in names] if self.pools.with_grads else None,
-            dict(x=self._x, w=self._w, act=self._act, gu=self._gu, dA=self._dA, dgu=self._dgu), self.buf._num_sms_dedup,
-            self._total_sms, gg._status(self._act.device), gg._status_host(self._act.device), engine.wait_budget_ns())
+            self.buf._states[0], self.Hp, dict(x=self._x, w=self._w, act=self._act, gu=self._gu, dA=self._dA, dgu=self._dgu),
+            self.buf._num_sms_dedup, self._total_sms, gg._status(self._act.device), gg._status_host(self._act.device), engine.wait_budget_ns())
 
     def _update_mask(self, plan):
         if self.geo.R == 1:
@@ -207,11 +204,12 @@ class ExpertParallelMoE:
         starting the GEMM on flagged tiles; it writes straight into the private buffers that the backward pass
         reads (no stash), and the down GEMM's rows stay in the shard, where the combine gathers them."""
         buf, st = self.buf, self.buf._st()
-        if self._native is not None and route_weights_sk is not None:
+        if self._native is not None and self._native.state is st and route_weights_sk is not None:
             topk = topk_sk.reshape(-1)
             buf._check_hidden(hidden_sh, route_weights_sk)
             buf._check_topk(topk, tokens_per_expert)
-            out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward)
+            out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward,
+                                             self.pools.addresses(self.geo.epn, self.H, self.Hp))
             return out, _LocalContext(self, slab) if need_backward else None
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
         if route_weights_sk is None:        # unscaled rows; the buffers hold the weights of an earlier call
@@ -314,14 +312,14 @@ class ExpertParallelMoE:
         buf, g, epn, Hp = self.buf, self.geo, self.geo.epn, self.Hp
         acc, ov, multi = self.accumulate_grads, self.overlap_backward and not self._local, self.geo.R > 1
         self._join_deferred()
-        if (self._native is not None and isinstance(ctx, _LocalContext) and self.on_comm_quiet is None
-                and (self.on_grad_ready is None or self.on_grad_ready is no_update)):
-            buf._st()
+        if (self._native is not None and self._native.state is buf._st() and isinstance(ctx, _LocalContext)
+                and self.on_comm_quiet is None and (self.on_grad_ready is None or self.on_grad_ready is no_update)):
             buf._check_hidden(grad_out_sh, None)
             lr = self.epilogue_lr
             assert lr is None or not acc, "the optimizer cannot sit in the GEMM epilogue while gradients are accumulated"
             self.grads_pending = None
-            return self._native.backward(grad_out_sh, ctx.slab, acc, lr or 0.0, None if lr is None else self._upd_mask)
+            return self._native.backward(grad_out_sh, ctx.slab, acc, lr or 0.0, None if lr is None else self._upd_mask,
+                                         self.pools.addresses(epn, self.H, Hp), self.pools.addresses(epn, self.H, Hp, grads=True))
         main = torch.cuda.current_stream()
         pools = self.pools
         pair = lambda n: (pools.local_grad(n), pools.reduce_view(n))      # noqa: E731

@@ -196,25 +196,34 @@ class ExpertPools:
         rank = self.rank if rank is None else rank
         return self.heap.view(rank, off + first * r * c * es, (count, r, c), dtype)
 
-    def _cached(self, what, name, rank, make):
-        """Views are asked for at every step and never change: each is built once."""
-        key = (what, name, rank)
+    def kept(self, key, make):
+        """What ``make()`` built for ``key`` out of this memory (views, addresses): made once, forgotten by ``destroy``."""
         v = self._views.get(key)
         if v is None:
             v = self._views[key] = make()
         return v
 
+    def addresses(self, epn: int, H: int, Hp: int, grads: bool = False) -> tuple:
+        """Addresses of the three compute views (gate, up, down) for a native call of a layer of that size."""
+        def make():
+            assert self.epn == epn, f"pools hold {self.epn} experts, the layer needs {epn}"
+            for n, s in zip(NAMES, ((H, Hp), (H, Hp), (Hp, H))):
+                assert self._shapes[n] == s, f"pools hold {n} {self._shapes[n]}, the layer needs {s}"
+            assert self.dtype == torch.bfloat16, "the layer computes in bf16"
+            return tuple((self.compute_grad(n) if grads else self.compute_weight(n)).data_ptr() for n in NAMES)
+        return self.kept(("addresses", epn, H, Hp, grads), make)
+
     # ---- weights
     def local_weight(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._wview[name][:self.epn]
-        return self._cached("local_weight", name, rank, lambda: self._view(self._woff[name], name, self.dtype, 0, self.epn, rank))
+        return self.kept(("local_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, self.epn, rank))
 
     def compute_weight(self, name, rank=None) -> torch.Tensor:
         """``[2*epn, rows, cols]``: local experts then this rank's prefetch slots."""
         if self.shared is not None:
             return self._wview[name]
-        return self._cached("compute_weight", name, rank, lambda: self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank))
+        return self.kept(("compute_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank))
 
     def prefetch_view(self, name) -> torch.Tensor:
         """``[R, epn, rows, cols]`` view of every rank's prefetch slots."""
@@ -228,12 +237,12 @@ class ExpertPools:
     def local_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name][:self.epn]
-        return self._cached("local_grad", name, rank, lambda: self._view(self._goff[name], name, torch.float32, 0, self.epn, rank))
+        return self.kept(("local_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, self.epn, rank))
 
     def compute_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name]
-        return self._cached("compute_grad", name, rank, lambda: self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank))
+        return self.kept(("compute_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank))
 
     def reduce_view(self, name) -> torch.Tensor:
         if self.shared is not None:

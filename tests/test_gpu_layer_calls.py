@@ -51,3 +51,38 @@ def test_backward_with_a_hook_refuses_a_bad_gradient(cuda_device):
     blk.buf.check()
     assert bool(torch.isfinite(dx.float()).all())
     blk.destroy()
+
+
+def test_layer_uses_the_pools_it_has(cuda_device):
+    """Weights and gradients are those of the layer's pools at the time of the call; pools without gradients have no
+    backward pass, destroyed ones no pass at all."""
+    from moonep_b200.pools import ExpertPools
+    a, b = make_block(), make_block()
+    for n in ("gate", "up", "down"):
+        b.pools.local_weight(n).mul_(-0.5)
+    x, dy = normal((130, 256), 1), normal((130, 256), 2)
+    with torch.no_grad():
+        w, topk, tpe = a.route(x)
+    want, ctx = b.moe.forward(x, w, topk, tpe)
+    b.moe.backward(ctx, dy)
+    grads = [b.pools.local_grad(n).clone() for n in ("gate", "up", "down")]
+    a.moe.forward(x, w, topk, tpe)
+    own, a.moe.pools = a.moe.pools, b.pools
+    out, ctx = a.moe.forward(x, w, topk, tpe)
+    for n in ("gate", "up", "down"):
+        b.pools.local_grad(n).zero_()
+    a.moe.backward(ctx, dy)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert all(torch.equal(b.pools.local_grad(n), g) for n, g in zip(("gate", "up", "down"), grads))
+    a.moe.pools = ExpertPools(4, (256, 256), (256, 256), (256, 256))
+    _, ctx = a.moe.forward(x, w, topk, tpe)
+    with pytest.raises(KeyError):
+        a.moe.backward(ctx, dy)
+    a.moe.pools = own
+    own.destroy()
+    for call in (lambda: a.moe.forward(x, w, topk, tpe), lambda: a.moe.backward(ctx, dy), lambda: a.sgd_step(0.1)):
+        with pytest.raises(AttributeError):
+            call()
+    a.destroy()
+    b.destroy()
