@@ -45,20 +45,29 @@ class MoEContext:
     gu: torch.Tensor         # pre-activations [NvS, 2H']
 
 
-class _LocalContext:
-    """``MoEContext`` of a single-rank forward pass: the plan's allocation; its tensors are named when somebody asks."""
+class _LocalContext(MoEContext):
+    """``MoEContext`` of a native single-rank forward pass: the plan's allocation; its tensors are named when somebody asks."""
 
-    def __init__(self, layer, slab):
-        self._layer, self.slab, self._named = layer, slab, None
-        self.x, self.w_nvs, self.act, self.gu = layer._x, layer._w, layer._act, layer._gu
+    def __init__(self, plan=None, cu=None, x=None, w_nvs=None, act=None, gu=None, *, native=None, slab=None):
+        self._native, self._slab, self._named = native, slab, (plan, cu)
+        self.x, self.w_nvs, self.act, self.gu = x, w_nvs, act, gu
 
     def _plan(self):
-        if self._named is None:
-            self._named = self._layer._native.plan_of(self.slab)
+        if self._named[0] is None:
+            self._named = self._native.plan_of(self._slab)
         return self._named
 
-    plan = property(lambda self: self._plan()[0])
-    cu = property(lambda self: self._plan()[1])
+    plan = property(lambda self: self._plan()[0], lambda self, v: self._rename(v, self._plan()[1]))
+    cu = property(lambda self: self._plan()[1], lambda self, v: self._rename(self._plan()[0], v))
+
+    def _rename(self, plan, cu):
+        self._named, self._slab = (plan, cu), None
+
+    def slab_of(self, layer):
+        """The plan's allocation if all else that the backward pass reads is still what ``layer``'s native call left in its
+        own buffers; else None (the caller has put copies or another plan in their place)."""
+        mine = self._native is layer._native and self.x is layer._x and self.w_nvs is layer._w and self.act is layer._act and self.gu is layer._gu
+        return self._slab if mine else None
 
 
 _DEFERRED: list = []       # layers whose last gradient reduction is still running (see wait_grads)
@@ -210,7 +219,8 @@ class ExpertParallelMoE:
             buf._check_topk(topk, tokens_per_expert)
             out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward,
                                              self.pools.addresses(self.geo.epn, self.H, self.Hp))
-            return out, _LocalContext(self, slab) if need_backward else None
+            return out, _LocalContext(x=self._x, w_nvs=self._w, act=self._act, gu=self._gu, native=self._native,
+                                      slab=slab) if need_backward else None
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
         if route_weights_sk is None:        # unscaled rows; the buffers hold the weights of an earlier call
             assert not need_backward, "a forward pass without route weights has no backward pass"
@@ -312,13 +322,14 @@ class ExpertParallelMoE:
         buf, g, epn, Hp = self.buf, self.geo, self.geo.epn, self.Hp
         acc, ov, multi = self.accumulate_grads, self.overlap_backward and not self._local, self.geo.R > 1
         self._join_deferred()
-        if (self._native is not None and self._native.state is buf._st() and isinstance(ctx, _LocalContext)
-                and self.on_comm_quiet is None and (self.on_grad_ready is None or self.on_grad_ready is no_update)):
+        slab = ctx.slab_of(self) if self._native is not None and isinstance(ctx, _LocalContext) else None
+        if (slab is not None and self._native.state is buf._st() and self.on_comm_quiet is None
+                and (self.on_grad_ready is None or self.on_grad_ready is no_update)):
             buf._check_hidden(grad_out_sh, None)
             lr = self.epilogue_lr
             assert lr is None or not acc, "the optimizer cannot sit in the GEMM epilogue while gradients are accumulated"
             self.grads_pending = None
-            return self._native.backward(grad_out_sh, ctx.slab, acc, lr or 0.0, None if lr is None else self._upd_mask,
+            return self._native.backward(grad_out_sh, slab, acc, lr or 0.0, None if lr is None else self._upd_mask,
                                          self.pools.addresses(epn, self.H, Hp), self.pools.addresses(epn, self.H, Hp, grads=True))
         main = torch.cuda.current_stream()
         pools = self.pools

@@ -86,3 +86,35 @@ def test_layer_uses_the_pools_it_has(cuda_device):
             call()
     a.destroy()
     b.destroy()
+
+
+@pytest.mark.parametrize("how", ["assign", "replace"])
+def test_context_with_private_copies_outlives_the_next_forward_pass(how, cuda_device):
+    """A caller with two batches in flight gives the first context copies of what the second pass overwrites."""
+    import dataclasses
+    from moonep_b200.moe_layer import MoEContext
+    blk = make_block()
+    xs, dy = [normal((130, 256), s) for s in (1, 2)], normal((130, 256), 3)
+    with torch.no_grad():
+        routes = [blk.route(x) for x in xs]
+    names = ("gate", "up", "down")
+    _, ctx = blk.moe.forward(xs[0], *routes[0])
+    dx, dw = blk.moe.backward(ctx, dy)
+    grads = [blk.pools.local_grad(n).clone() for n in names]
+    for n in names:
+        blk.pools.local_grad(n).zero_()
+    _, ctx = blk.moe.forward(xs[0], *routes[0])
+    assert isinstance(ctx, MoEContext)
+    kept = {f: getattr(ctx, f).clone() for f in ("x", "w_nvs", "act", "gu")}
+    if how == "replace":
+        ctx = dataclasses.replace(ctx, **kept)
+    else:
+        for f, t in kept.items():
+            setattr(ctx, f, t)
+    blk.moe.forward(xs[1], *routes[1])
+    dx2, dw2 = blk.moe.backward(ctx, dy)
+    torch.cuda.synchronize()
+    blk.buf.check()
+    assert torch.equal(dx, dx2) and torch.equal(dw, dw2)
+    assert all(torch.equal(blk.pools.local_grad(n), g) for n, g in zip(names, grads))
+    blk.destroy()
