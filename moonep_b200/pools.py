@@ -203,6 +203,11 @@ class ExpertPools:
             v = self._views[key] = make()
         return v
 
+    def _alias(self, key, make) -> torch.Tensor:
+        """A kept view under a tensor object of the caller's own: what the caller sets on it (``requires_grad_``, ``.grad``,
+        shape in place) is nobody else's."""
+        return self.kept(key, make).detach()
+
     def addresses(self, epn: int, H: int, Hp: int, grads: bool = False) -> tuple:
         """Addresses of the three compute views (gate, up, down) for a native call of a layer of that size."""
         def make():
@@ -217,13 +222,13 @@ class ExpertPools:
     def local_weight(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._wview[name][:self.epn]
-        return self.kept(("local_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, self.epn, rank))
+        return self._alias(("local_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, self.epn, rank))
 
     def compute_weight(self, name, rank=None) -> torch.Tensor:
         """``[2*epn, rows, cols]``: local experts then this rank's prefetch slots."""
         if self.shared is not None:
             return self._wview[name]
-        return self.kept(("compute_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank))
+        return self._alias(("compute_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank))
 
     def prefetch_view(self, name) -> torch.Tensor:
         """``[R, epn, rows, cols]`` view of every rank's prefetch slots."""
@@ -237,12 +242,12 @@ class ExpertPools:
     def local_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name][:self.epn]
-        return self.kept(("local_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, self.epn, rank))
+        return self._alias(("local_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, self.epn, rank))
 
     def compute_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name]
-        return self.kept(("compute_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank))
+        return self._alias(("compute_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank))
 
     def reduce_view(self, name) -> torch.Tensor:
         if self.shared is not None:

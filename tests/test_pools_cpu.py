@@ -35,3 +35,19 @@ def test_no_addresses_without_memory():
     for ask in (lambda: p.addresses(2, 64, 32), lambda: p.local_weight("up"), lambda: p.kept("anything", lambda: p.local_weight("up"))):
         with pytest.raises(AttributeError):
             ask()
+
+
+@pytest.mark.parametrize("view", ["local_weight", "compute_weight", "local_grad", "compute_grad"])
+def test_views_share_memory_and_nothing_else(view):
+    p = make_pools()
+    a = getattr(p, view)("gate")
+    shape = a.shape
+    a.requires_grad_(True)
+    (a * 2).sum().backward()
+    b = getattr(p, view)("gate")
+    assert b is not a and not b.requires_grad and b.grad is None and b.shape == shape
+    b[1].fill_(3)
+    c = getattr(p, view)("gate")
+    c.unsqueeze_(0)
+    d = getattr(p, view)("gate")
+    assert d.shape == shape and bool((d[1] == 3).all()) and bool((d[0] == 0).all())
