@@ -46,23 +46,6 @@ CONFIGS = {
 }
 
 
-class _RouteFn(torch.autograd.Function):
-    """``MoEBlock.route``: the weights are differentiable, table and counts are not."""
-
-    @staticmethod
-    def forward(ctx, hidden, router, blk):
-        w, topk, tpe, probs = rt.route(hidden @ router, blk.router_bias, blk.cfg.K, with_probs=True)
-        ctx.save_for_backward(hidden, router, probs, topk)
-        ctx.mark_non_differentiable(topk, tpe)
-        return w, topk, tpe
-
-    @staticmethod
-    def backward(ctx, dw, _topk, _tpe):
-        hidden, router, probs, topk = ctx.saved_tensors
-        dl = rt.route_bwd(probs, dw.contiguous(), topk)
-        return (dl @ router.t() if ctx.needs_input_grad[0] else None, hidden.t() @ dl if ctx.needs_input_grad[1] else None, None)
-
-
 def _block_forward(blk, hidden, router, s0, s1, keep: bool):
     """Output, and with ``keep`` what the backward pass needs: (MoE context, probabilities, table, shared gate/up, activation)."""
     w, topk, tpe, probs = rt.route(hidden @ router, blk.router_bias, blk.cfg.K, with_probs=keep)
@@ -151,8 +134,8 @@ class MoEBlock:
             dist.barrier(group=group)
 
     def route(self, hidden):
-        if self._fused_route:
-            return _RouteFn.apply(hidden, self.router, self)
+        """Weights (differentiable as often and by whatever transform the caller likes), table and counts, as torch operators;
+        a whole block's ``forward`` has them in one launch."""
         cfg = self.cfg
         logits = (hidden @ self.router).float() + self.router_bias
         probs = torch.softmax(logits, dim=-1)

@@ -118,3 +118,23 @@ def test_context_with_private_copies_outlives_the_next_forward_pass(how, cuda_de
     assert torch.equal(dx, dx2) and torch.equal(dw, dw2)
     assert all(torch.equal(blk.pools.local_grad(n), g) for n, g in zip(names, grads))
     blk.destroy()
+
+
+def test_route_goes_through_transforms(cuda_device):
+    """``MoEBlock.route`` alone is made of torch operators: leading dimensions, second derivatives, forward mode, autocast."""
+    blk = make_block()
+    x = normal((130, 256), 1)
+    w, topk, tpe = blk.route(x)
+    w3, topk3, tpe3 = blk.route(x.view(13, 10, 256))
+    assert torch.equal(w3.flatten(0, 1), w) and torch.equal(topk3.flatten(0, 1), topk) and torch.equal(tpe3, tpe)
+    xr = x.clone().requires_grad_(True)
+    c = torch.linspace(-1, 1, 260, device="cuda").view(130, 2)
+    (g,) = torch.autograd.grad((blk.route(xr)[0] * c).sum(), xr, create_graph=True)
+    (g2,) = torch.autograd.grad(g.float().square().sum(), blk.router)
+    assert bool(g2.abs().sum() > 0) and bool(torch.isfinite(g2.float()).all())
+    with torch.autograd.forward_ad.dual_level():
+        d = blk.route(torch.autograd.forward_ad.make_dual(x, x * 0.5))[0]
+        assert torch.autograd.forward_ad.unpack_dual(d).tangent.shape == w.shape
+    with torch.autocast("cuda", torch.float16):
+        assert float((blk.route(x)[0] - w).abs().max()) < 0.05
+    blk.destroy()
