@@ -146,8 +146,17 @@ class MoEBlock:
         tpe.scatter_add_(0, topk.reshape(-1).long(), torch.ones(topk.numel(), dtype=torch.int32, device=hidden.device))
         return w, topk, tpe
 
+    def _fused(self, hidden) -> bool:
+        """Whether the fused kernels compute what the torch operators would: bf16 operands in rows, a plain fp32 bias that
+        wants no gradient, no autocast to another type."""
+        b, bf = self.router_bias, torch.bfloat16
+        return (self._fused_route and hidden.dtype == bf and hidden.ndim == 2 and hidden.is_contiguous() and self.router.dtype == bf
+                and b.dtype == torch.float32 and b.shape == (self.E,) and b.is_contiguous() and not b.requires_grad
+                and (self.shared is None or self.shared[0].dtype == self.shared[1].dtype == bf and self.shared[0].shape[1] % 16 == 0)
+                and (not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") == bf))
+
     def forward(self, hidden):
-        if self._fused_route and hidden.dtype == torch.bfloat16 and hidden.is_contiguous():
+        if self._fused(hidden):
             shared = self.shared or (None, None)
             if not torch.is_grad_enabled():
                 return _block_forward(self, hidden, self.router, *shared, False)[0]
