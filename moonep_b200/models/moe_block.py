@@ -74,12 +74,13 @@ class _BlockFn(torch.autograd.Function):
         hidden, router, s0, s1, probs, topk, gu, act = ctx.saved_tensors
         need = ctx.needs_input_grad
         dy = dy.contiguous()
-        dx, dw = ctx.blk.moe.backward(ctx.mctx, dy)
-        dl = rt.route_bwd(probs, dw, topk)
-        drouter = hidden.t() @ dl if need[1] else None
-        if need[0]:
-            dx.addmm_(dl, router.t())
-        ds0 = ds1 = None
+        dx = drouter = ds0 = ds1 = None
+        if need[0] or need[1]:           # else nothing in front of the experts wants a gradient, and they are frozen with it
+            dx, dw = ctx.blk.moe.backward(ctx.mctx, dy)
+            dl = rt.route_bwd(probs, dw, topk)
+            drouter = hidden.t() @ dl if need[1] else None
+            if need[0]:
+                dx.addmm_(dl, router.t())
         if s0 is not None:
             dgu = rt.swiglu_bwd(dy @ s1.t(), gu)
             ds1 = act.t() @ dy if need[3] else None

@@ -176,3 +176,24 @@ def test_block_under_autocast(cuda_device):
             y = blk.forward(x)
     assert float((y.float() - y0.detach().float()).norm() / y0.detach().float().norm()) < 2e-2
     blk.destroy()
+
+
+def test_frozen_router_and_input_freeze_the_experts(cuda_device):
+    """Without a gradient for the input or the router the experts have no backward pass; the shared expert still has its own."""
+    blk = make_block(shared=1)
+    blk.router.requires_grad_(False)
+    x, dy = normal((130, 256), 1), normal((130, 256), 2)
+    got = []
+    for fused in (True, False):
+        blk._fused_route = fused
+        for n in ("gate", "up", "down"):
+            blk.pools.local_grad(n).fill_(7.0)
+        blk.forward(x).backward(dy)
+        torch.cuda.synchronize()
+        assert all(bool((blk.pools.local_grad(n) == 7.0).all()) for n in ("gate", "up", "down"))
+        assert blk.router.grad is None
+        got.append([p.grad for p in blk.shared])
+        for p in blk.shared:
+            p.grad = None
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    blk.destroy()
