@@ -73,6 +73,8 @@ class _BlockFn(torch.autograd.Function):
     def backward(ctx, dy):
         hidden, router, s0, s1, probs, topk, gu, act = ctx.saved_tensors
         need = ctx.needs_input_grad
+        if torch.is_grad_enabled():      # create_graph: what comes back has to have derivatives of its own
+            return _block_backward_graph(ctx, dy)
         dy = dy.contiguous()
         dx = drouter = ds0 = ds1 = None
         if need[0] or need[1]:           # else nothing in front of the experts wants a gradient, and they are frozen with it
@@ -88,6 +90,31 @@ class _BlockFn(torch.autograd.Function):
             if need[0]:
                 dx.addmm_(dgu, s0.t())
         return dx if need[0] else None, drouter, ds0, ds1, None
+
+
+def _block_backward_graph(ctx, dy):
+    """``_BlockFn.backward`` in torch operators around the experts, whose gradients are constants as they are behind
+    ``moe_apply``."""
+    hidden, router, s0, s1, probs, topk, _, _ = ctx.saved_tensors
+    need = ctx.needs_input_grad
+    outs, douts, dx = [], [], None
+    if need[0] or need[1]:
+        with torch.no_grad():
+            dx, dw = ctx.blk.moe.backward(ctx.mctx, dy.contiguous())
+        logits = (hidden @ router).float()
+        v = torch.softmax(probs.log() + (logits - logits.detach()), dim=-1).gather(1, topk.long())      # the saved ones, as functions of the logits
+        outs, douts = [v / v.sum(dim=-1, keepdim=True)], [dw]
+    if s0 is not None:
+        gu = hidden @ s0
+        hs = gu.shape[1] // 2
+        outs.append((torch.nn.functional.silu(gu[:, :hs]) * gu[:, hs:]) @ s1)
+        douts.append(dy)
+    ins = [t for t, n in zip((hidden, router, s0, s1), need) if n]
+    got = iter(torch.autograd.grad(outs, ins, douts, create_graph=True, allow_unused=True))
+    g = [next(got) if n else None for n in need[:4]]
+    if need[0]:
+        g[0] = dx if g[0] is None else dx + g[0]
+    return *g, None
 
 
 class MoEBlock:

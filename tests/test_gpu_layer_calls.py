@@ -197,3 +197,22 @@ def test_frozen_router_and_input_freeze_the_experts(cuda_device):
             p.grad = None
     assert all(torch.equal(a, b) for a, b in zip(*got))
     blk.destroy()
+
+
+@pytest.mark.parametrize("shared", [0, 1])
+def test_second_derivatives_of_a_block(shared, cuda_device):
+    """With ``create_graph`` the gradients can be differentiated as those of the operators can: the experts' part is a
+    constant, router and shared expert are not."""
+    blk = make_block(shared=shared)
+    x, dy = normal((130, 256), 1), normal((130, 256), 2)
+    got = []
+    for fused in (True, False):
+        blk._fused_route = fused
+        xr, d = x.clone().requires_grad_(True), dy.clone().requires_grad_(True)
+        ps = blk.parameters()
+        first = torch.autograd.grad(blk.forward(xr), [xr] + ps, d, create_graph=True)
+        second = torch.autograd.grad(sum(f.float().square().sum() for f in first), [xr] + ps + ([d] if shared else []))
+        got.append([t.detach().float() for t in (*first, *second)])
+    for i, (a, b) in enumerate(zip(*got)):      # bf16 operators on both sides: a few roundings of 2^-9
+        assert float(b.norm()) > 0 and float((a - b).norm() / b.norm()) < 1.5e-2, i
+    blk.destroy()
