@@ -43,7 +43,7 @@ struct MoeLocal {
   const MepRankCtx* ctx;         // device
   int32_t S, H, Hp, K, E, NvS;
   int32_t blocks, combine_blocks, num_ctas;      // CTAs of dispatch, combine (most) and of the GEMMs
-  int32_t reserved;
+  int32_t pdl;                   // 1: programmatic launches between the kernels of one call
   int64_t plan_off[8];           // elements from the start of a plan's allocation: dst, experts_to_copy, zero_fill,
                                  // remote_stats, dup_groups, dup_loffs, dup_counts, cu_seqlens
   const void *w_gate, *w_up, *w_down;            // [2E, in, out] bf16; these and the gradients are set for each call

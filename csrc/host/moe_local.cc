@@ -20,7 +20,7 @@ static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab) {
   a.cu_seqlens = slab + m.plan_off[7];
   a.pad_rows = slab + m.plan_off[2];
   a.G = 2 * m.E; a.g_end = 2 * m.E;
-  a.pdl = 1;                     // behind another kernel of the same call
+  a.pdl = m.pdl;                 // behind another kernel of the same call
   a.status = m.status; a.status_host = m.status_host; a.budget_ns = m.budget_ns;
   return a;
 }
@@ -90,7 +90,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   g.N = m.H; g.K = m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DOWN, m.act, m.Hp, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, nullptr, (__nv_bfloat16*)out, nullptr};
-  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 1, stream);
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, stream);
 }
 
 // `update`: lr and the group mask of the update in the weight-gradient epilogues, or mask = null (gradients are stored).
@@ -105,7 +105,7 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   g.N = m.Hp; g.K = m.H; g.out = m.dA; g.ldo = m.Hp;
   if (gemm(m, GEMM_DGRAD, m.shard, m.H, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
   const int32_t* cu = slab + m.plan_off[7];
-  if (mep_swiglu_bwd(m.dA, m.gu, m.w, m.dgu, m.shard_w, cu, 2 * m.E, m.Hp, 4 * m.num_ctas, 1, stream)) return -1;
+  if (mep_swiglu_bwd(m.dA, m.gu, m.w, m.dgu, m.shard_w, cu, 2 * m.E, m.Hp, 4 * m.num_ctas, m.pdl, stream)) return -1;
   auto wgrad = [&](const void* x, int64_t in, const void* dyc, int64_t ld, int64_t out, float* dw, const void* w) {
     GemmArgs a = gemm_args(m, slab);
     a.N = (int32_t)out; a.M_w = (int32_t)in; a.accumulate = accumulate; a.zero_empty_below = m.E; a.out = dw;
@@ -119,7 +119,7 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   g.N = m.H; g.K = 2 * m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DGRAD_GU, m.dgu, 2 * (int64_t)m.Hp, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, m.shard_w, (__nv_bfloat16*)dx, d_route_w};
-  if (mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 1, stream)) return -1;
+  if (mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, stream)) return -1;
   if (mask && wgrad(m.x, m.H, m.dgu, 2 * (int64_t)m.Hp, m.Hp, m.dw_gate, m.w_gate)) return -1;
   return wgrad(m.x, m.H, m.dgu + m.Hp, 2 * (int64_t)m.Hp, m.Hp, m.dw_up, m.w_up);
 }

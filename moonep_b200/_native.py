@@ -68,7 +68,7 @@ class DispatchArgs(C.Structure):
 
 class MoeLocal(C.Structure):
     _fields_ = ([("ctx", C.c_void_p)] + [(n, C.c_int32) for n in ("S", "H", "Hp", "K", "E", "NvS", "blocks", "combine_blocks",
-                                                                 "num_ctas", "reserved")]
+                                                                 "num_ctas", "pdl")]
                 + [("plan_off", C.c_int64 * 8)]
                 + [(n, C.c_void_p) for n in ("w_gate", "w_up", "w_down", "shard", "shard_w", "srcinfo", "x", "w", "act", "gu", "dA",
                                              "dgu", "dw_gate", "dw_up", "dw_down", "sync", "hist", "status", "status_host")]

@@ -306,10 +306,11 @@ class LocalLayer(LocalExchange):
             setattr(a, name, t.data_ptr())
         a.status, a.status_host, a.budget_ns = status.data_ptr(), status_host.data_ptr(), budget_ns
 
-    def forward(self, hidden, route_w, topk, tpe, keep: bool, weights):
+    def forward(self, hidden, route_w, topk, tpe, keep: bool, weights, pdl: bool):
         """Returns ``(out, plan allocation)``."""
         g, a = self._geo, self._args
         a.w_gate, a.w_up, a.w_down = weights
+        a.pdl = pdl
         slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
         out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
         rc = self._lib.mep_moe_local_forward(self._ref, hidden.data_ptr(), route_w.data_ptr(), topk.data_ptr(), tpe.data_ptr(),
@@ -318,9 +319,10 @@ class LocalLayer(LocalExchange):
             _native.check(rc, "moe forward")
         return out, slab
 
-    def backward(self, dy, slab, accumulate: bool, lr: float, mask, weights, grads):
+    def backward(self, dy, slab, accumulate: bool, lr: float, mask, weights, grads, pdl: bool):
         g, a = self._geo, self._args
         a.w_gate, a.w_up, a.w_down = weights
+        a.pdl = pdl
         a.dw_gate, a.dw_up, a.dw_down = grads
         dx = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
         dw = torch.empty((g.S, g.K), dtype=torch.float32, device=self._dev)

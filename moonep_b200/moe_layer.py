@@ -218,7 +218,7 @@ class ExpertParallelMoE:
             buf._check_hidden(hidden_sh, route_weights_sk)
             buf._check_topk(topk, tokens_per_expert)
             out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward,
-                                             self.pools.addresses(self.geo.epn, self.H, self.Hp))
+                                             self.pools.addresses(self.geo.epn, self.H, self.Hp), buf.enable_pdl)
             return out, _LocalContext(x=self._x, w_nvs=self._w, act=self._act, gu=self._gu, native=self._native,
                                       slab=slab) if need_backward else None
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
@@ -330,7 +330,8 @@ class ExpertParallelMoE:
             assert lr is None or not acc, "the optimizer cannot sit in the GEMM epilogue while gradients are accumulated"
             self.grads_pending = None
             return self._native.backward(grad_out_sh, slab, acc, lr or 0.0, None if lr is None else self._upd_mask,
-                                         self.pools.addresses(epn, self.H, Hp), self.pools.addresses(epn, self.H, Hp, grads=True))
+                                         self.pools.addresses(epn, self.H, Hp), self.pools.addresses(epn, self.H, Hp, grads=True),
+                                         buf.enable_pdl)
         main = torch.cuda.current_stream()
         pools = self.pools
         pair = lambda n: (pools.local_grad(n), pools.reduce_view(n))      # noqa: E731

@@ -216,3 +216,24 @@ def test_second_derivatives_of_a_block(shared, cuda_device):
     for i, (a, b) in enumerate(zip(*got)):      # bf16 operators on both sides: a few roundings of 2^-9
         assert float(b.norm()) > 0 and float((a - b).norm() / b.norm()) < 1.5e-2, i
     blk.destroy()
+
+
+def test_native_calls_follow_the_launch_switch(cuda_device):
+    """``Buffer.enable_pdl`` decides at every call how the layer's kernels are launched; the results are the same bits."""
+    blk = make_block()
+    x, dy = normal((130, 256), 1), normal((130, 256), 2)
+    with torch.no_grad():
+        route = blk.route(x)
+    got = []
+    for pdl in (True, False):
+        blk.buf.enable_pdl = pdl
+        y, ctx = blk.moe.forward(x, *route)
+        assert blk.moe._native._args.pdl == pdl
+        blk.moe._native._args.pdl = 2
+        dx, dw = blk.moe.backward(ctx, dy)
+        assert blk.moe._native._args.pdl == pdl
+        got.append([y, dx, dw] + [blk.pools.local_grad(n).clone() for n in ("gate", "up", "down")])
+    torch.cuda.synchronize()
+    blk.buf.check()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    blk.destroy()
