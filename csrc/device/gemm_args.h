@@ -60,10 +60,18 @@ struct GemmArgs {
   void* upd_w;
   const int32_t* upd_mask;
   float upd_lr;
-  int32_t reserved1;
+  int32_t sched_odd;           // CTA-pair launches on a shared counter: CTAs asked for beyond those of the grid (1: an odd number,
+                               // -1: a single one, which runs as a pair)
   // optional [G, 2] table (first padding row, padding rows) of the groups, as a plan carries it: rows behind the real
   // ones, rounded up to 32, are then neither computed nor read (null: all padded rows are). CTA-pair kernels only.
   const int32_t* pad_rows;
 };
+
+// CTAs of a pair launch that was asked for `n`. On a counter shared with other launches the grid accounts for all `n`.
+inline int pair_ctas(GemmArgs* a, int n) {
+  const int grid = a->sched_ctas > 0 && n == 1 ? 2 : n & ~1;
+  a->sched_odd = a->sched_ctas > 0 ? n - grid : 0;
+  return grid;
+}
 
 }  // namespace mep

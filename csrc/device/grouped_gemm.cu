@@ -428,7 +428,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   __syncthreads();
   tc::fence_after_sync();
   if (warp == 1) tc::tmem_dealloc(tmem_base, kTmemCols);
-  if (threadIdx.x == 0) tq::scheduler_done(args.sched, args.sched_ctas > 0 ? args.sched_ctas : (int)gridDim.x);
+  if (threadIdx.x == 0) tq::scheduler_done(args.sched, 1, args.sched_ctas > 0 ? args.sched_ctas : (int)gridDim.x);
 }
 
 }  // namespace mep

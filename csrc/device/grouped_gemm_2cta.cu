@@ -310,7 +310,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   cluster_sync();
   tc::fence_after_sync();
   if (warp == 1) tmem_dealloc2(tmem_base, 512);
-  if (leader && threadIdx.x == 0) tq::scheduler_done(args.sched, args.sched_ctas > 0 ? args.sched_ctas / 2 : npairs);
+  if (leader && threadIdx.x == 0) tq::scheduler_done(args.sched, pair == 0 ? 2 + args.sched_odd : 2, args.sched_ctas > 0 ? args.sched_ctas : (int)gridDim.x);
 }
 
 }  // namespace w2
@@ -325,7 +325,7 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   GemmArgs args = *args_in;
   MEP_REQUIRE(args.G >= 1 && args.G <= w2::kMaxGroups, "wgrad: G=%d out of range", args.G);
   MEP_REQUIRE(args.M_w % 256 == 0 && args.N % 256 == 0, "wgrad (2-CTA): weight shape [%d,%d] must be multiples of 256", args.M_w, args.N);
-  num_ctas &= ~1;
+  num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "wgrad (2-CTA): needs at least two CTAs");
   CUtensorMap ma, mb, mo;
   if (tmap_atoms(&ma, x, rows, args.M_w, x_ld, 2)) return -1;

@@ -456,7 +456,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   cluster_sync();
   tc::fence_after_sync();
   if (warp == 1) tmem_dealloc2(tmem_base, 512);
-  if (leader && threadIdx.x == 0) tq::scheduler_done(args.sched, args.sched_ctas > 0 ? args.sched_ctas / 2 : npairs);
+  if (leader && threadIdx.x == 0) tq::scheduler_done(args.sched, pair == 0 ? 2 + args.sched_odd : 2, args.sched_ctas > 0 ? args.sched_ctas : (int)gridDim.x);
 }
 
 }  // namespace tp
@@ -467,11 +467,11 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
                                      const void* b0, const void* b1, int64_t b_rows, int64_t b_cols, int64_t b_ld,
                                      const mep::GemmArgs* args_in, int num_ctas, cudaStream_t stream) {
   using namespace mep;
-  const GemmArgs& args = *args_in;
+  GemmArgs args = *args_in;
   MEP_REQUIRE(mode >= GEMM_GATE_UP && mode <= GEMM_DGRAD_GU, "gemm (CTA pairs): mode %d not supported", mode);
   MEP_REQUIRE(args.G >= 1 && args.G <= tp::kMaxGroups, "gemm: G=%d out of range [1,%d]", args.G, tp::kMaxGroups);
   MEP_REQUIRE(args.K % 64 == 0 && args.N % (mode == GEMM_GATE_UP ? 128 : 256) == 0, "gemm (CTA pairs): K=%d N=%d not tileable", args.K, args.N);
-  num_ctas &= ~1;
+  num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "gemm (CTA pairs): needs at least two CTAs");
   CUtensorMap mx, mx64, mx16, mw0, mw1, mo, mo2;
   if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 128) || tmap_rows(&mx64, a, a_rows, a_cols, a_ld, 64, 64) ||

@@ -9,8 +9,8 @@
 // (MMA issuer, epilogue warps) and, in a pair, to the peer CTA's ring through distributed shared
 // memory, so every role walks the same sequence. A negative number ends the sequence.
 //
-// Ticket counter protocol (two words: next ticket, finished schedulers): schedulers draw with
-// atomicAdd; at CTA teardown every scheduler CTA counts itself and the last one puts both words
+// Ticket counter protocol (two words: next ticket, finished CTAs): schedulers draw with
+// atomicAdd; at CTA teardown every scheduler counts its CTAs and the last one puts both words
 // back to zero, so back-to-back launches (and CUDA-graph replays) need no host-side reset, and a
 // kernel that gave up on a bounded wait still leaves the counter clean.
 #pragma once
@@ -95,11 +95,13 @@ struct Scheduler {
   }
 };
 
-// Teardown accounting of one scheduler CTA (call after every role of the CTA has left its loop).
-__device__ __forceinline__ void scheduler_done(uint32_t* counter, int nschedulers) {
+// Teardown accounting of a scheduler that stands for `ctas` of the `total` CTAs that share the counter (call after every
+// role of its CTAs has left its loop). CTAs and not schedulers are counted: launches of single CTAs and of pairs, and
+// pair launches that were asked for an odd number, then add up to what the ticket was made for.
+__device__ __forceinline__ void scheduler_done(uint32_t* counter, int ctas, int total) {
   if (!counter) return;
   __threadfence();
-  if (atomicAdd(counter + 1, 1u) == (uint32_t)nschedulers - 1u) {
+  if (atomicAdd(counter + 1, (uint32_t)ctas) + (uint32_t)ctas == (uint32_t)total) {
     counter[0] = 0u; counter[1] = 0u;
     __threadfence();
   }

@@ -37,7 +37,7 @@ class GemmArgs(C.Structure):
                 ("tile_done", C.c_void_p), ("tile_epoch", C.c_void_p), ("status_host", C.c_void_p),
                 ("group_flags", C.c_void_p), ("group_epoch", C.c_void_p),
                 ("push_rows", C.c_int32), ("push_ranks", C.c_int32), ("group_first", C.c_int32), ("sched_ctas", C.c_int32),
-                ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("reserved1", C.c_int32),
+                ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("sched_odd", C.c_int32),
                 ("pad_rows", C.c_void_p)]
 
 
@@ -192,8 +192,9 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
     a_ld = a.stride(0)
     a_cols = a.shape[1] if a_cols is None else a_cols
     fn = lib.mep_grouped_gemm
-    # CTA pairs (tcgen05 cta_group::2) unless they are switched off or there is no pair to run on
-    if mode != WGRAD and (num_ctas or _num_sms(a.device)) >= 2 and os.environ.get("MOONEP_GEMM_2CTA", "1") == "1":
+    # CTA pairs (tcgen05 cta_group::2) unless they are switched off or there is no pair to run on; the launches that share
+    # a ticket number their tiles alike and must all run on the same kernel
+    if mode != WGRAD and (ticket is not None or (num_ctas or _num_sms(a.device)) >= 2) and os.environ.get("MOONEP_GEMM_2CTA", "1") == "1":
         fn = lib.mep_grouped_gemm_2cta
     rc = fn(mode, C.c_void_p(a.data_ptr()), C.c_int64(a_rows), C.c_int64(a_cols), C.c_int64(a_ld),
                               C.c_void_p(b0.data_ptr()), C.c_void_p(_native.ptr(b1)), C.c_int64(b_rows),

@@ -140,3 +140,29 @@ def test_swiglu_epilogue_of_extreme_pre_activations(cuda_device):
     assert torch.equal(gu[:, :N], x[:, :1].expand(rows, N)) and bool((gu[:, N:] == 1).all())
     # exp's two ulp and one bf16 rounding: within one bf16 ulp (2^-7); below the smallest normal number fp32 exp ends in zero
     assert bool(((act.double() - ref).abs() <= 2.0 ** -7 * ref.abs() + 2e-36).all())
+
+
+@pytest.mark.parametrize("split", [(33, 115), (1, 147), (31, 33, 84)], ids=str)
+def test_launches_of_odd_size_share_a_ticket(split, cuda_device):
+    """The launches on one ticket divide the tiles among them whatever their sizes, and leave the counter clean."""
+    from moonep_b200.ops import grouped_gemm as gg
+    K, N, n = 256, 512, [256, 0, 640, 128]
+    cu = torch.tensor(n).cumsum(0).to(torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(4)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, w, wu, wt = bf(sum(n), K), bf(4, K, N, sc=0.05), bf(4, K, N, sc=0.05), bf(4, N, K, sc=0.05)
+    dy = bf(sum(n), N)
+    calls = {"gate_up": (lambda o, **kw: gg.gate_up(x, w, wu, cu, o, **kw), (sum(n), N), torch.bfloat16),
+             "down": (lambda o, **kw: gg.down(x, w, cu, o, **kw), (sum(n), N), torch.bfloat16),
+             "dgrad": (lambda o, **kw: gg.dgrad(x, wt, cu, o, **kw), (sum(n), N), torch.bfloat16),
+             "wgrad": (lambda o, **kw: gg.wgrad(x, dy, cu, o, zero_empty_below=4, **kw), (4, K, N), torch.float32)}
+    for name, (call, shape, dt) in calls.items():
+        want, got = torch.full(shape, 7.0, dtype=dt, device="cuda"), torch.full(shape, 9.0, dtype=dt, device="cuda")
+        call(want)
+        tk = gg.Ticket(x.device, sum(split))
+        for c in split:
+            call(got, num_ctas=c, ticket=tk)
+        torch.cuda.synchronize()
+        gg.check_status()
+        assert torch.equal(got, want), name
+        assert not bool(gg._sched_cache[gg._dev_index(x.device)][0].any()), f"{name}: the counter was left behind"
