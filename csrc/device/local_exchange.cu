@@ -271,7 +271,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
       bool got = true;
       if (lane == 0) got = mbar_wait_bounded(&bars[st], (phases >> st) & 1u, c.wait_budget_ns);
       got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
-      if (!got) { if (lane == 0) report(c, MEP_ERR_MBAR_TIMEOUT, MEP_K_DISPATCH, 20, s, 0, 0); ++arrived; phases ^= 1u << st; ok = false; break; }
+      if (!got) { if (lane == 0) report(c, MEP_ERR_MBAR_TIMEOUT, MEP_K_DISPATCH, 20, s, 0, 0); ok = false; break; }
       phases ^= 1u << st;
       ++arrived;
       for (int k = lane; k < K; k += 32) {
@@ -296,9 +296,9 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
         if (a.out_srcinfo) a.out_srcinfo[row] = j;
       }
     }
-    __syncthreads();                           // s_slot is free again
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;   // s_slot is free again; the warps go on or stop together
   }
-  if (!ok && lane == 0)                        // do not leave while loads into this CTA's memory are in flight
+  if (!ok && lane == 0)                        // do not leave while loads into this CTA's memory are in flight: they get their time (again)
     for (int i = arrived; i < issued; ++i) {
       mbar_wait_bounded(&bars[i % slots], (phases >> (i % slots)) & 1u, c.wait_budget_ns);
       phases ^= 1u << (i % slots);
