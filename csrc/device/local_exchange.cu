@@ -306,6 +306,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   bulk_wait_all<0>();
   if (vb == 0 && tid == 0) {
     count(c, MEP_CNT_DISPATCHES, 1); count(c, MEP_CNT_ROWS_SENT, (unsigned long long)S); count(c, MEP_CNT_PEER_ROWS, (unsigned long long)S);
+    count(c, MEP_CNT_PAD_ROWS, (unsigned long long)total_pad);
     trace_mark(c, MEP_K_DISPATCH, 5);
   }
   if (SHARED) {                                // the last CTA out closes the launch

@@ -498,8 +498,9 @@ class Buffer(OpsMixin):
     def counters(self, reset: bool = False) -> dict:
         """Device-side counters of this Buffer's kernels since creation or the last reset
         (synchronises): dispatch / combine launches, rows sent in total, to other ranks and per
-        destination rank, padding rows cleared, rows pulled by combine, duplicate rows expanded by
-        flagged dispatches, cross-rank barriers executed and the time spent waiting in them.
+        destination rank, padding rows cleared, rows pulled by combine (all K of a token in a group of
+        one rank, which reduces nothing before), duplicate rows expanded by flagged dispatches,
+        cross-rank barriers executed and the time spent waiting in them.
         ``MOONEP_COUNTERS=0`` at construction switches the accounting off (empty dict)."""
         return engine.read_counters(self._st(), reset)
 

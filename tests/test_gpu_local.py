@@ -113,3 +113,25 @@ def test_combine_of_rows_that_start_off_a_16_byte_boundary(cuda_device):
     buf.check()
     assert rows.data_ptr() % 16 == 2 and torch.equal(a, b)
     buf.destroy()
+
+
+def test_padding_rows_are_counted(cuda_device):
+    """A Buffer's dispatch clears every padding row, fresh or saved; a layer's those that its GEMMs read."""
+    from moonep_b200.models.moe_block import MoEBlock, MoEConfig
+    S, H, K, E = 700, 64, 4, 8
+    topk, tpe = (t[0].cuda() for t in make_topk("biased", S, K, E, 1, seed=5))
+    x = torch.zeros(S, H, dtype=torch.bfloat16, device="cuda")
+    buf = Buffer(S, H, K, E, 1)
+    _, _, _, plan = buf.dispatch(x, None, topk, tpe, zero_copy=True)
+    pads = buf.stats(plan)["padded_rows"]
+    assert pads > 0 and buf.counters()["padding_rows_cleared"] == pads
+    buf.dispatch(x, plan=plan, zero_copy=True)
+    assert buf.counters(reset=True)["padding_rows_cleared"] == 2 * pads
+    buf.destroy()
+    blk = MoEBlock(MoEConfig("t", H=256, Hp=256, K=2, epn=4, S=130), num_sms=4, seed=3)
+    y = torch.randn(130, 256, device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        _, _, tpe = blk.route(y)
+        blk.forward(y)
+    assert blk.buf.counters()["padding_rows_cleared"] == int((-tpe % 32).sum())
+    blk.destroy()
