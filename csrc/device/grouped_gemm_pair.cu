@@ -19,6 +19,7 @@
 #include "tile_queue.cuh"
 #include "gemm_args.h"
 #include "tmap.h"
+#include "silu.cuh"
 
 namespace mep {
 namespace tp {
@@ -47,21 +48,6 @@ struct Tile { int g, row0, n, n0; };                   // n tokens from row0 (a 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// g / (1 + exp(-g)) without a branch. The compiler's division tests for special operands and branches, so the eight of a
-// chunk ran one after the other (1100 cycles); these interleave. A Newton step on the approximate reciprocal and the
-// residual correction of P. Markstein (IBM J. Res. Dev. 34, 1990) round like `/` for every float with |g| < 60 that is not
-// tiny (compared exhaustively); `plain` says so, anything else takes the division.
-__device__ __forceinline__ bool silu_plain(float g) { const float m = fabsf(g); return m < 60.f && (m >= 1e-30f || m == 0.f); }
-__device__ __noinline__ float silu_any(float g) { return g / (1.f + __expf(-g)); }
-__device__ __forceinline__ float silu(float g) {
-  const float d = 1.f + __expf(-g);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(r, fmaf(-d, r, 1.f), r);
-  const float q = g * r;
-  return fmaf(fmaf(-d, q, g), r, q);
 }
 
 // a / b for a >= 0, b > 0 and results below 2^20, without the code of an integer division: __fdividef is off by 2 ulp at

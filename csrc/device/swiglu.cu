@@ -5,21 +5,10 @@
 //   sgd_step:   p -= lr * g for bf16 parameters with fp32 gradients (benchmark optimizer).
 // Only rows below cu_seqlens[G-1] are defined; rows beyond are skipped.
 #include "prims.cuh"
+#include "silu.cuh"
 #include "../host/launch.h"
 
 namespace mep {
-
-// 1 / (1 + exp(-g)) without the compiler's division branch, which keeps neighbouring elements from interleaving: a Newton
-// step and a residual correction (P. Markstein, IBM J. Res. Dev. 34, 1990). Rounds like the division for every float with
-// |g| < 60 (compared exhaustively).
-__device__ __forceinline__ float sigmoid(float g) {
-  const float d = 1.f + __expf(-g);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(r, fmaf(-d, r, 1.f), r);
-  return fmaf(fmaf(-d, r, 1.f), r, r);
-}
-__device__ __noinline__ float sigmoid_any(float g) { return 1.f / (1.f + __expf(-g)); }
 
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dA, const __nv_bfloat16* __restrict__ gu,
                                                          const float* __restrict__ w, __nv_bfloat16* __restrict__ dgu,
@@ -51,7 +40,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 #pragma unroll
       for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(pg[i]); gs[2 * i] = f.x; gs[2 * i + 1] = f.y; }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { plain = plain && fabsf(gs[i]) < 60.f; sg[i] = sigmoid(gs[i]); }
+      for (int i = 0; i < 8; ++i) { plain = plain && sigmoid_plain(gs[i]); sg[i] = sigmoid(gs[i]); }
       if (!plain) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) sg[i] = sigmoid_any(gs[i]);
@@ -111,7 +100,23 @@ __global__ void __launch_bounds__(256) sgd_groups_kernel(__nv_bfloat16* __restri
   sgd_range(p + (int64_t)grp * n8 * 8, g + (int64_t)grp * n8 * 8, lr, n8);
 }
 
+// For tests: compares the branch-free forms with the division for the `n` floats whose bits start at `first`;
+// bad[0] / bad[1] count the sigmoids / SiLUs that differ, seen[0] / seen[1] those that were compared.
+__global__ void __launch_bounds__(256) silu_sweep_kernel(uint32_t first, uint32_t n, unsigned long long* bad, unsigned long long* seen) {
+  unsigned b0 = 0, b1 = 0, s0 = 0, s1 = 0;
+  for (uint64_t i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) {
+    const float g = __uint_as_float(first + (uint32_t)i);
+    if (sigmoid_plain(g)) { ++s0; b0 += __float_as_uint(sigmoid(g)) != __float_as_uint(sigmoid_any(g)); }
+    if (silu_plain(g)) { ++s1; b1 += __float_as_uint(silu(g)) != __float_as_uint(silu_any(g)); }
+  }
+  atomicAdd(bad, b0); atomicAdd(bad + 1, b1); atomicAdd(seen, s0); atomicAdd(seen + 1, s1);
+}
+
 }  // namespace mep
+
+extern "C" int mep_silu_sweep(uint32_t first, uint32_t n, unsigned long long* bad, unsigned long long* seen, cudaStream_t stream) {
+  return mep::launch_plain(mep::silu_sweep_kernel, dim3(1184), dim3(256), 0, stream, first, n, bad, seen);
+}
 
 extern "C" int mep_swiglu_bwd(const void* dA, const void* gu, const float* w, void* dgu, float* dw,
                               const int32_t* cu_seqlens, int G, int Hp, int num_blocks, int pdl, cudaStream_t stream) {

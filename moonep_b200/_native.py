@@ -153,6 +153,7 @@ def load(build_if_missing: bool = True):
     lib.mep_swiglu_dense_bwd.argtypes = [vp, vp, vp, C.c_int64, i32, vp]
     lib.mep_route_bwd.argtypes = [vp] * 4 + [i32] * 3 + [vp]
     lib.mep_swiglu.argtypes = [vp, vp, C.c_int64, i32, vp]
+    lib.mep_silu_sweep.argtypes = [C.c_uint32, C.c_uint32, vp, vp, vp]
     lib.mep_local_dispatch_call.argtypes = [vp] * 11
     lib.mep_local_combine_call.argtypes = [vp] * 7
     lib.mep_moe_local_forward.argtypes = [vp] * 7 + [i32, vp]

@@ -115,7 +115,7 @@ def test_weight_gradient_of_large_groups(M, cuda_device):
 
 
 def test_swiglu_epilogue_of_extreme_pre_activations(cuda_device):
-    """Gate values outside the epilogue's branch-free range (|g| >= 60, tiny, zero, infinite, NaN) beside ordinary ones: with
+    """Gate values outside the epilogue's branch-free range (|g| >= 60, tiny) and zeros beside ordinary ones: with
     a unit gate weight and an up weight of one the activation is g / (1 + exp(-g)) * 1, rounded to bf16 once."""
     from moonep_b200.ops import grouped_gemm as gg
     vals = [0.0, -0.0, 1.0, -1.0, 59.9, -59.9, 60.0, -60.0, 87.0, -87.0, 88.5, -88.5, 104.0, -104.0, 1e30, -1e30, 3e38, -3e38,
