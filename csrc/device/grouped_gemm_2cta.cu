@@ -29,7 +29,7 @@ constexpr size_t kSmem = (size_t)kRing * kStageBytes + (size_t)kEpiWarps * 2 * k
 
 using namespace pair;
 
-constexpr int kBandElems = 9 << 20;                          // elements of the wider operand in a group on average: 18 MB
+constexpr int kBandElems = 9 << 20;                          // elements of x for a group, on average over all G: 18 MB
 
 struct Tile { int g, row0, m0, n0, kblocks, ksteps; };      // ksteps: 16-row steps (a k-block has four)
 
@@ -100,6 +100,8 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   // Row blocks vary fastest, all of them or, where groups are large on average, in bands of at most 8: 74 pairs then read few
   // distinct slabs of a group that L2 does not hold (8 groups of 4096 tokens, 7168 x 2048: 0.817 -> 0.793 ms, with the SGD
   // epilogue 0.806 -> 0.771). With 1024 tokens a group's rows stay in L2 anyway, and the epilogue's updates take 1 % longer in bands.
+  // The mean is over all G groups; a layer passes its slots for replicas too, which are empty on one rank, and there its
+  // experts have to average 36 MB.
   const int mblk = args.M_w / 256, nblk = args.N / 256, bands = s_bands, bw = (mblk + bands - 1) / bands;
   const Divisor by_group(mblk * nblk), by_band(bw * nblk), by_row(bw), by_last(mblk - (bands - 1) * bw);
   auto get_tile = [&](int t, Tile& ti) {

@@ -27,7 +27,7 @@ using namespace pair;
 
 constexpr int kBK = 64, kEpiWarps = 8, kThreads = 64 + 32 * kEpiWarps;
 constexpr int kWBytes = 128 * kBK * 2;                 // 16 KB: a CTA's weight columns of one k-block
-constexpr int kRingBytes = 6 * 2 * kWBytes, kMaxRing = 11;
+constexpr int kRingBytes = 6 * 2 * kWBytes, kMaxRing = 10;     // a stage is 18 KB at least
 constexpr int kAtomBytes = 64 * kBK * 2;
 constexpr int kChunk = 16;                             // tokens per epilogue step
 constexpr int kStgBytes = kChunk * 128;                // staging: 16 tokens x 64 columns
@@ -134,7 +134,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   const int ntiles = s_start[G];
   const bool dyn = args.sched != nullptr;
   // Token rows arrive in one box of 128 or 64, or in boxes of 16 where no tile of the launch has more than 48 for a CTA: a stage is then
-  // little more than its weights and up to eleven fit instead of six. With few tokens per expert the kernel streams
+  // little more than its weights and up to ten fit instead of six. With few tokens per expert the kernel streams
   // weights, and what an SM has in flight is its bandwidth.
   const bool small = s_half <= 48;
   const uint32_t x_bytes = small ? max(s_half, 16) * 128u : s_half <= 64 ? 8192u : 16384u;
@@ -482,7 +482,8 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
   // Group sizes are only known on the device, and the code for bands costs a launch of few tiles 1 us of 20: it is there where
-  // groups are half as large as the line on average, so that some may be above it.
+  // groups are half as large as the line on average, so that some may be above it. All G groups count: a layer passes its
+  // slots for replicas too, which hold no row on one rank, so that there the average expert has to reach the line itself.
   const bool bands = a_rows * args.K * 2 > (int64_t)args.G * (tp::kXBytes / 2);
 #define MEP_TP_CASE(M)                                                                                          \
   case M: {                                                                                                     \

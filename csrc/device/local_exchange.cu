@@ -20,8 +20,17 @@ constexpr int kLocEntries = 1024;          // top-k entries ranked and copied at
 constexpr int kLocZeroBytes = 4096;        // zeroed shared memory the padding rows are stored from
 constexpr int kLocMaxSlots = 8;            // row slots per copying warp
 
-constexpr int kLocDirect = 24576;          // up to this many entries every CTA counts all entries before its own by itself (dispatch
-                                           // at 12248 entries 16.8 instead of 22.8 us, at 18006 35 instead of 40, at 32768 106 instead of 102)
+// Up to this many entries every CTA counts all entries before its own by itself, above it the CTAs hand over their
+// histograms. Counting costs a CTA all entries before its own, the hand-over two round trips to L2 and CTAs x E counts. Own
+// count against hand-over (K=8, caches flushed), in us:
+//   entries                12288        20480        24576        28672        32768        49152
+//   H=512,  E=64        16.4 / 23.6  20.5 / 24.6  24.6 / 26.6  26.6 / 27.5  28.7 / 29.7  38.9 / 33.7
+//   H=2048, E=16        22.5 / 28.7  29.6 / 32.9  34.9 / 37.8  38.9 / 41.0  45.2 / 45.1  65.5 / 61.4
+//   H=2048, E=256       35.8 / 45.1  42.0 / 50.2  47.2 / 51.2  49.2 / 54.3  55.3 / 55.3  74.8 / 70.7
+//   H=7168, E=16        45.1 / 49.2  73.7 / 75.8  88.1 / 90.1   102 / 102    115 / 112    168 / 163
+//   H=7168, E=64        53.2 / 53.3  79.0 / 77.8  92.2 / 88.2   107 / 105    119 / 117    174 / 166
+// The two cross between 24576 and 32768 for short rows and between 16384 and 28672 for long ones, whatever E is.
+constexpr int kLocDirect = 24576;
 
 // Padding rows that are cleared behind row `first` of a group's `n` (see LocalDispatchArgs.pad_step).
 __device__ __forceinline__ int local_pads(int first, int n, int step) { return step ? min(n, -first & (step - 1)) : n; }
@@ -414,7 +423,7 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
   const int all = (int)((budget - tables - kLocZeroBytes) / row);           // row slots that fit
   int warps = all / 2 < kLocWarps ? all / 2 : kLocWarps;
   int slots = all / warps < kLocMaxSlots ? all / warps : kLocMaxSlots;
-  // more than 64 KB of rows in flight per SM buys nothing; a smaller footprint starts sooner
+  // the fewest slots that still hold 96 KB of rows per SM: more buys nothing, and a smaller footprint starts sooner
   while (slots > 2 && (size_t)warps * (slots - 1) * row >= 96 * 1024) --slots;
   const size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
   if (fresh && S * K <= kLocDirect) return launch_plain(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);

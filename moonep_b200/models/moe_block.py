@@ -60,7 +60,7 @@ def _block_forward(blk, hidden, router, s0, s1, keep: bool):
 
 class _BlockFn(torch.autograd.Function):
     """A whole block as one autograd node: the three contributions to the input gradient (experts, router, shared
-    expert) are accumulated by the GEMMs that produce them instead of by additions over ``[S, H]``."""
+    expert, added in this order) are accumulated by the GEMMs that produce them instead of by additions over ``[S, H]``."""
 
     @staticmethod
     def forward(ctx, hidden, router, s0, s1, blk):
