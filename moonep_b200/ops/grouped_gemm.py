@@ -157,6 +157,30 @@ def check_status(device="cuda") -> None:
         raise RuntimeError(f"grouped GEMM aborted: code {v[0]} at site {v[1]}, CTA {v[2]}, tile {v[3]}")
 
 
+def _on_pairs(mode, rows, ngroups, G, N, K, skips_pad, ctas, shared) -> bool:
+    """Whether a token-major GEMM runs on CTA pairs (tcgen05 cta_group::2) or on single CTAs; same results, bit for bit.
+    ``MOONEP_GEMM_2CTA`` = 0 / 1 decides for all; only pairs skip padding rows, and gate/up is 13 % faster on them on average.
+
+    The others take the shorter estimate, in units of a single CTA's 64-deep k-block with 128 tokens, groups taken as equal.
+    A pair's k-block costs less the fewer of its 256 tokens a tile has, but its tiles are twice as large, so that the last
+    of the rounds over the CTAs may be emptier; its epilogue takes longer, which tiles of few k-blocks show, and so does the
+    launch (2-4 us).  The constants are fitted to 1950 timings of down and dgrad (K, N from 256 to 7168, 1 to 96 groups of 128 to
+    3000 rows, equal and uneven ones, caches flushed): 5 % of the calls lose more than 3 % against the better kernel, most of
+    them with uneven groups; on pairs alone 38 % did.  Single CTAs / pairs in us: down of 16 groups of 384 rows, 2048 x 768, 30.7 /
+    38.9; 60 groups of 512, 256 x 2816, 64.5 / 87.0; 32 groups of 384, 7168 x 2048, 339 / 296."""
+    env = os.environ.get("MOONEP_GEMM_2CTA", "")
+    if ctas < 2 and not shared:
+        return False
+    if skips_pad or mode == GATE_UP or env in ("0", "1"):
+        return env != "0"
+    blocks, depth = -(-rows // (128 * G)), K // 64
+    tiles = -(-blocks // 2)
+    single = -(-ngroups * blocks * (N // 256) // ctas)
+    pairs = -(-ngroups * tiles * (N // 256) // max(1, ctas // 2))
+    tokens = 128 * blocks / max(1, tiles)
+    return single * (depth + 1.4) >= 11.4 + pairs * (depth * (0.1 + tokens / 556) + tokens / 53)
+
+
 def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=None, row_scale=None, ldo=0,
             accumulate=False, zero_empty_below=0, a_cols=None, b_rows=None, b_cols=None, b_ld=None, groups=None, num_ctas=None,
             dynamic=False, ticket=None, push=None, push_w=None, ready=None, slots=None, pad=None):
@@ -192,9 +216,9 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
     a_ld = a.stride(0)
     a_cols = a.shape[1] if a_cols is None else a_cols
     fn = lib.mep_grouped_gemm
-    # CTA pairs (tcgen05 cta_group::2) unless they are switched off or there is no pair to run on; the launches that share
-    # a ticket number their tiles alike and must all run on the same kernel
-    if mode != WGRAD and (ticket is not None or (num_ctas or _num_sms(a.device)) >= 2) and os.environ.get("MOONEP_GEMM_2CTA", "1") == "1":
+    # the launches that share a ticket number their tiles alike and must all run on the same kernel
+    if mode != WGRAD and _on_pairs(mode, a_rows, g1 - g0, G, N, K, pad is not None,
+                                   ticket.total_ctas if ticket is not None else num_ctas or _num_sms(a.device), ticket is not None):
         fn = lib.mep_grouped_gemm_2cta
     rc = fn(mode, C.c_void_p(a.data_ptr()), C.c_int64(a_rows), C.c_int64(a_cols), C.c_int64(a_ld),
                               C.c_void_p(b0.data_ptr()), C.c_void_p(_native.ptr(b1)), C.c_int64(b_rows),
@@ -261,7 +285,7 @@ def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=Fals
 def skips_padding() -> bool:
     """Whether every GEMM of a layer runs on the CTA-pair kernels, which honour ``pad``: only then may one leave
     padding rows unwritten that another would otherwise read."""
-    return os.environ.get("MOONEP_GEMM_2CTA", "1") == "1" and os.environ.get("MOONEP_WGRAD_2CTA", "1") != "0"
+    return os.environ.get("MOONEP_GEMM_2CTA", "") != "0" and os.environ.get("MOONEP_WGRAD_2CTA", "1") != "0"
 
 
 def wgrad_update_supported(M: int, N: int) -> bool:

@@ -1,0 +1,46 @@
+"""Which kernel a token-major grouped GEMM runs on: the rule's fixed points, without a GPU."""
+import pytest
+
+from moonep_b200.ops.grouped_gemm import DGRAD, DGRAD_GU, DOWN, GATE_UP, _on_pairs
+
+MODES = [GATE_UP, DOWN, DGRAD, DGRAD_GU]
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_the_switch_decides_for_all(mode, monkeypatch):
+    for env in ("0", "1"):
+        monkeypatch.setenv("MOONEP_GEMM_2CTA", env)
+        for pad in (False, True):
+            for rows in (128, 100000):
+                assert _on_pairs(mode, rows, 4, 4, 512, 512, pad, 148, False) == (env == "1")
+                assert not _on_pairs(mode, rows, 4, 4, 512, 512, pad, 1, False), "a single CTA is no pair"
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_padding_is_skipped_by_pairs_only(mode, monkeypatch):
+    monkeypatch.delenv("MOONEP_GEMM_2CTA", raising=False)
+    for rows in (1, 128, 5000, 100000):
+        for K in (64, 512, 7168):
+            assert _on_pairs(mode, rows, 16, 16, 512, K, True, 148, False)
+
+
+def test_measured_sides_of_the_line(monkeypatch):
+    """(mode, groups, rows of each, K, N) with the kernel that was measured to be faster by 5 % or more."""
+    monkeypatch.delenv("MOONEP_GEMM_2CTA", raising=False)
+    single = [(DOWN, 16, 384, 2048, 768), (DGRAD, 16, 384, 2048, 768), (DGRAD_GU, 16, 384, 4096, 768), (DOWN, 32, 128, 2048, 768),
+              (DOWN, 4, 2048, 1024, 256), (DGRAD, 4, 2048, 1024, 256), (DOWN, 96, 128, 512, 512), (DGRAD, 96, 256, 512, 512),
+              (DOWN, 60, 512, 256, 2816), (DGRAD, 68, 640, 512, 1792)]
+    pairs = [(DOWN, 32, 384, 7168, 2048), (DGRAD, 32, 384, 7168, 2048), (DGRAD_GU, 32, 384, 14336, 2048), (DOWN, 4, 128, 7168, 2048),
+             (DGRAD_GU, 16, 128, 4096, 768), (DOWN, 8, 4096, 7168, 2048), (GATE_UP, 32, 1024, 7168, 2048), (GATE_UP, 16, 128, 2048, 768)]
+    for want, cases in ((False, single), (True, pairs)):
+        for mode, G, r, K, N in cases:
+            assert _on_pairs(mode, G * r, G, G, N, K, False, 148, False) == want, (mode, G, r, K, N)
+
+
+@pytest.mark.parametrize("total", [1, 2, 3, 148])
+def test_a_ticket_of_any_size_has_a_kernel(total, monkeypatch):
+    """The rule is asked with the ticket's CTAs and not the launch's, so that all its launches run on one kernel."""
+    monkeypatch.delenv("MOONEP_GEMM_2CTA", raising=False)
+    for mode in MODES:
+        for rows, K in ((0, 64), (128, 64), (6144, 2048), (40000, 7168)):
+            assert _on_pairs(mode, rows, 16, 16, 768, K, False, total, True) in (True, False)

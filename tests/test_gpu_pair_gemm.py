@@ -143,9 +143,10 @@ def test_swiglu_epilogue_of_extreme_pre_activations(cuda_device):
 
 
 @pytest.mark.parametrize("split", [(33, 115), (1, 147), (31, 33, 84)], ids=str)
-def test_launches_of_odd_size_share_a_ticket(split, cuda_device):
+def test_launches_of_odd_size_share_a_ticket(split, cuda_device, monkeypatch):
     """The launches on one ticket divide the tiles among them whatever their sizes, and leave the counter clean."""
     from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
     K, N, n = 256, 512, [256, 0, 640, 128]
     cu = torch.tensor(n).cumsum(0).to(torch.int32).cuda()
     g = torch.Generator(device="cuda").manual_seed(4)
@@ -166,3 +167,25 @@ def test_launches_of_odd_size_share_a_ticket(split, cuda_device):
         gg.check_status()
         assert torch.equal(got, want), name
         assert not bool(gg._sched_cache[gg._dev_index(x.device)][0].any()), f"{name}: the counter was left behind"
+
+
+@pytest.mark.parametrize("G,r,K,N", [(1, 128, 64, 256), (16, 384, 2048, 768), (4, 128, 2048, 768), (3, 1152, 256, 512)])
+def test_both_kernels_give_the_same_bits(G, r, K, N, cuda_device, monkeypatch):
+    """Left alone, a GEMM runs on single CTAs or on pairs: the sizes lie on both sides of the rule."""
+    from moonep_b200.ops import grouped_gemm as gg
+    cu = (torch.arange(1, G + 1, device="cuda") * r).to(torch.int32)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, x2, w, wu, scale = bf(G * r, K), bf(G * r, 2 * K), bf(G, K, N, sc=0.05), bf(G, K, N, sc=0.05), torch.rand(G * r, device="cuda", generator=g)
+    got = []
+    for env in (None, "0", "1"):
+        monkeypatch.delenv("MOONEP_GEMM_2CTA", raising=False) if env is None else monkeypatch.setenv("MOONEP_GEMM_2CTA", env)
+        act, gu, y, dA, dx = (torch.full((G * r, c), float("nan"), dtype=torch.bfloat16, device="cuda") for c in (N, 2 * N, N, N, N))
+        gg.gate_up(x, w, wu, cu, act, gu, row_scale=scale)
+        gg.down(x, w, cu, y, row_scale=scale)
+        gg.dgrad(x, w.view(G, N, K), cu, dA)
+        gg.dgrad_gate_up(x2, w.view(G, N, K), wu.view(G, N, K), cu, dx)
+        torch.cuda.synchronize()
+        gg.check_status()
+        got.append((act, gu, y, dA, dx))
+    assert all(torch.equal(a, b) and torch.equal(a, c) for a, b, c in zip(*got))

@@ -19,10 +19,11 @@ def test_every_float_rounds_like_the_division(sign, cuda_device):
     assert bad.tolist() == [0, 0]
 
 
-def test_epilogue_of_infinite_and_nan_gates(cuda_device):
+def test_epilogue_of_infinite_and_nan_gates(cuda_device, monkeypatch):
     """Gates that overflow in the accumulator, with an up projection of one, and NaN tokens, beside finite ones: inf, -inf * 0 = NaN,
     NaN."""
     from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
     rows, K, N, big = 128, 64, 128, 3e38
     x, wg, wu = (torch.zeros(s, dtype=torch.bfloat16, device="cuda") for s in ((rows, K), (1, K, N), (1, K, N)))
     x[:, 0], wu[0, 0] = 1.0, 1.0
