@@ -138,8 +138,12 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           const uint32_t sa = smem0 + s * kStageBytes, bar = full0 + s * 8u;
           const int k = ti.row0 + kb * kBK;
           if (leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);     // both CTAs' bytes
-          tma_load_3d_bar(sa, &tma_a, 0, k, am / 64, bar);
-          tma_load_3d_bar(sa + kHalfBytes, &tma_b, 0, k, bn / 64, bar);
+          // one 2-D box for each 64-column atom: with one 3-D box for both, launches of short groups that store their gradients were
+          // slower (64 groups of 256 tokens, 2048 x 1536: 212 us, with these 200), deep ones the same
+          tma_load_2d_bar(sa, &tma_a, am, k, bar);
+          tma_load_2d_bar(sa + kAtomBytes, &tma_a, am + 64, k, bar);
+          tma_load_2d_bar(sa + kHalfBytes, &tma_b, bn, k, bar);
+          tma_load_2d_bar(sa + kHalfBytes + kAtomBytes, &tma_b, bn + 64, k, bar);
         }
         __syncwarp();
         any = true;
@@ -330,8 +334,8 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "wgrad (2-CTA): needs at least two CTAs");
   CUtensorMap ma, mb, mo;
-  if (tmap_atoms(&ma, x, rows, args.M_w, x_ld, 2)) return -1;
-  if (tmap_atoms(&mb, dy, rows, args.N, dy_ld, 2)) return -1;
+  if (tmap_rows(&ma, x, rows, args.M_w, x_ld, 64, 64)) return -1;
+  if (tmap_rows(&mb, dy, rows, args.N, dy_ld, 64, 64)) return -1;
   if (tmap_rows(&mo, args.out, (int64_t)args.G * args.M_w, args.N, args.N, 32, 32, true)) return -1;
   if (allow_smem((const void*)w2::wgrad_2cta_kernel, w2::kSmem)) return -1;
   cudaLaunchConfig_t cfg = {};
