@@ -326,12 +326,14 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       float rs = 1.f;
       if (t >= 0) {
         get_tile(t, gcur, ti);
-        if ((MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) && args.row_scale) {      // in flight while the tile's MMAs finish
-          const int i = ((set_tid >> 4) * 2 + set) * kChunk + (set_tid & 15);
-          if (i < ti.n) rs = __ldcg(args.row_scale + ti.row0 + i);
-        }
+        const int i = ((set_tid >> 4) * 2 + set) * kChunk + (set_tid & 15);
+        const bool scaled = (MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) && args.row_scale && i < ti.n;
+        // in flight while the tile's MMAs finish -- unless a dispatch may still be writing the factors together with the rows:
+        // then only the finished MMAs, whose loads waited for the tile's flag, say that they are there
+        if (scaled && !args.tile_done) rs = __ldcg(args.row_scale + ti.row0 + i);
         if (lane == 0) { ok = mbar_wait_compact(&tfull_bar[acc], aph, args.budget_ns) ? 1 : 0; if (!ok) fail(4, t); }
         ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (scaled && args.tile_done) rs = __ldcg(args.row_scale + ti.row0 + i);
       }
       if (MODE == GEMM_GATE_UP || MODE == GEMM_DOWN) s_scale[set][acc][set_tid] = rs;
       // the warps of a set stage rows together: they go on or stop together

@@ -302,3 +302,30 @@ def test_a_failed_wait_stops_the_next_public_call(cuda_device, monkeypatch):
     torch.cuda.synchronize()
     buf.check()
     buf.destroy()
+
+
+def test_row_factors_are_read_behind_the_tile_flag(cuda_device):
+    """The factors of a tile's rows arrive with the rows. A dispatch on few SMs and large enough to run for long after the
+    GEMM has started: nothing of the poison that lay in the factors before may end up in the result."""
+    from moonep_b200 import Buffer
+    from moonep_b200.ops import grouped_gemm as gg
+    S, H, K, E, N = 2048, 2048, 8, 8, 256
+    topk, tpe = (t[0].cuda() for t in make_topk("biased", S, K, E, 1, seed=3))
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=gen) * sc).to(torch.bfloat16)     # noqa: E731
+    x, w, wg, wu = rnd(S, H), torch.rand(S, K, device="cuda", generator=gen), rnd(2 * E, H, N, sc=0.02), rnd(2 * E, H, N, sc=0.02)
+    buf = Buffer(S, H, K, E, 1, num_sms=4)
+    for _ in range(3):
+        buf.router_weight_buffer_view.fill_(float("nan"))
+        torch.cuda.synchronize()
+        h, wn, cu, plan, ready, ev = buf.dispatch_ready(x, w, topk, tpe)
+        act, ref = (torch.zeros(h.shape[0], N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        gg.gate_up(h, wg, wu, cu, act, row_scale=wn, num_ctas=min(128, ready.free_sms), ready=ready)
+        torch.cuda.current_stream().wait_event(ev)
+        gg.gate_up(h, wg, wu, cu, ref, row_scale=wn)
+        torch.cuda.synchronize()
+        buf.check()
+        gg.check_status()
+        n = int(cu[-1])
+        assert bool(torch.isfinite(ref[:n].float()).all()) and torch.equal(act[:n], ref[:n])
+    buf.destroy()
