@@ -155,6 +155,9 @@ class ExpertParallelMoE:
 
     def _native_layer(self):
         from . import engine
+        if self.pools.dtype == torch.bfloat16:          # gathered here and not in the first pass
+            for grads in (False, True) if self.pools.with_grads else (False,):
+                self.pools.addresses(self.geo.epn, self.H, self.Hp, grads)
         return engine.LocalLayer(
             self.buf._states[0], self.Hp, dict(x=self._x, w=self._w, act=self._act, gu=self._gu, dA=self._dA, dgu=self._dgu),
             self.buf._num_sms_dedup, self._total_sms, gg._status(self._act.device), gg._status_host(self._act.device), engine.wait_budget_ns())
