@@ -189,3 +189,38 @@ def test_both_kernels_give_the_same_bits(G, r, K, N, cuda_device, monkeypatch):
         gg.check_status()
         got.append((act, gu, y, dA, dx))
     assert all(torch.equal(a, b) and torch.equal(a, c) for a, b, c in zip(*got))
+
+
+@pytest.mark.parametrize("pairs", ["0", "1"], ids=["single", "pairs"])
+def test_pushed_rows_and_flagged_tiles_on_both_kernels(pairs, cuda_device, monkeypatch):
+    """The push epilogues and the tile flags, at sizes that the rule gives to one kernel only, on either of them."""
+    from test_gpu_comm import test_push_combine_matches_sum_of_rows
+    from test_gpu_flags import test_gemm_consumes_tiles_while_dispatch_runs
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", pairs)
+    test_push_combine_matches_sum_of_rows(4, cuda_device)
+    test_gemm_consumes_tiles_while_dispatch_runs(2, "dgrad", cuda_device)
+    test_gemm_consumes_tiles_while_dispatch_runs(4, "gate_up", cuda_device)
+
+
+@pytest.mark.parametrize("pairs", ["0", "1"], ids=["single", "pairs"])
+def test_dgrad_pushes_rows_and_their_scalars(pairs, cuda_device, monkeypatch):
+    """dgrad(gate/up) with identity weights: every dispatched row and its scalar go back to the token that it came from."""
+    from moonep_b200 import Buffer, routing
+    from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", pairs)
+    S, H, K, E = 96, 256, 4, 4
+    topk, w, tpe = routing.softmax_topk(S, K, E, 1.0, 5, 0, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(S, H, device="cuda", generator=g).to(torch.bfloat16)
+    buf = Buffer(S, H, K, E, 1, push_combine=True)
+    h, wn, cu, _ = buf.dispatch(x, w, topk, tpe, zero_copy=True, router_weights_zero_copy=True)
+    eye, zero = torch.eye(H, dtype=torch.bfloat16, device="cuda").repeat(2 * E, 1, 1).contiguous(), torch.zeros(2 * E, H, H, dtype=torch.bfloat16, device="cuda")
+    dgu = torch.cat([h, torch.zeros_like(h)], 1).contiguous()
+    dgu[int(cu[-1]):] = 0
+    gg.dgrad_gate_up(dgu, eye, zero, cu, torch.empty_like(h), push=buf.push_target(), push_w=wn)
+    out, ow, _ = buf.combine_pushed(want_weights=True)
+    torch.cuda.synchronize()
+    buf.check()
+    gg.check_status()
+    assert torch.equal(out, (x.float() * K).to(torch.bfloat16)) and torch.equal(ow, w)
+    buf.destroy()
