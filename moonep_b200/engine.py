@@ -300,17 +300,24 @@ class LocalLayer(LocalExchange):
     def __init__(self, st: RankState, Hp: int, work: dict, blocks: int, num_ctas: int, status, status_host, budget_ns: int):
         super().__init__(st, blocks)
         self.state = st
+        self._weights, self._grads, self._pdl = (None,) * 3, (None,) * 3, None      # what the argument block holds
         a = self._args
         a.Hp, a.num_ctas = Hp, num_ctas
         for name, t in work.items():
             setattr(a, name, t.data_ptr())
         a.status, a.status_host, a.budget_ns = status.data_ptr(), status_host.data_ptr(), budget_ns
 
+    def _set(self, weights, grads, pdl):
+        if weights != self._weights or grads != self._grads or pdl != self._pdl:
+            a = self._args
+            a.w_gate, a.w_up, a.w_down = self._weights = weights
+            a.dw_gate, a.dw_up, a.dw_down = self._grads = grads
+            a.pdl = self._pdl = pdl
+
     def forward(self, hidden, route_w, topk, tpe, keep: bool, weights, pdl: bool):
         """Returns ``(out, plan allocation)``."""
-        g, a = self._geo, self._args
-        a.w_gate, a.w_up, a.w_down = weights
-        a.pdl = pdl
+        g = self._geo
+        self._set(weights, self._grads, pdl)
         slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
         out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
         rc = self._lib.mep_moe_local_forward(self._ref, hidden.data_ptr(), route_w.data_ptr(), topk.data_ptr(), tpe.data_ptr(),
@@ -320,10 +327,8 @@ class LocalLayer(LocalExchange):
         return out, slab
 
     def backward(self, dy, slab, accumulate: bool, lr: float, mask, weights, grads, pdl: bool):
-        g, a = self._geo, self._args
-        a.w_gate, a.w_up, a.w_down = weights
-        a.pdl = pdl
-        a.dw_gate, a.dw_up, a.dw_down = grads
+        g = self._geo
+        self._set(weights, grads, pdl)
         dx = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
         dw = torch.empty((g.S, g.K), dtype=torch.float32, device=self._dev)
         rc = self._lib.mep_moe_local_backward(self._ref, dy.data_ptr(), slab.data_ptr(), dx.data_ptr(), dw.data_ptr(),

@@ -48,20 +48,19 @@ class MoEContext:
 class _LocalContext(MoEContext):
     """``MoEContext`` of a native single-rank forward pass: the plan's allocation; its tensors are named when somebody asks."""
 
-    def __init__(self, plan=None, cu=None, x=None, w_nvs=None, act=None, gu=None, *, native=None, slab=None):
-        self._native, self._slab, self._named = native, slab, (plan, cu)
-        self.x, self.w_nvs, self.act, self.gu = x, w_nvs, act, gu
+    def __init__(self, plan, cu, x, w_nvs, act, gu, native=None, slab=None):
+        self._plan_cu, self.x, self.w_nvs, self.act, self.gu, self._native, self._slab = (plan, cu), x, w_nvs, act, gu, native, slab
 
     def _plan(self):
-        if self._named[0] is None:
-            self._named = self._native.plan_of(self._slab)
-        return self._named
+        if self._plan_cu[0] is None:
+            self._plan_cu = self._native.plan_of(self._slab)
+        return self._plan_cu
 
     plan = property(lambda self: self._plan()[0], lambda self, v: self._rename(v, self._plan()[1]))
     cu = property(lambda self: self._plan()[1], lambda self, v: self._rename(self._plan()[0], v))
 
     def _rename(self, plan, cu):
-        self._named, self._slab = (plan, cu), None
+        self._plan_cu, self._slab = (plan, cu), None
 
     def slab_of(self, layer):
         """The plan's allocation if all else that the backward pass reads is still what ``layer``'s native call left in its
@@ -222,8 +221,7 @@ class ExpertParallelMoE:
             buf._check_topk(topk, tokens_per_expert)
             out, slab = self._native.forward(hidden_sh, route_weights_sk, topk, tokens_per_expert, need_backward,
                                              self.pools.addresses(self.geo.epn, self.H, self.Hp), buf.enable_pdl)
-            return out, _LocalContext(x=self._x, w_nvs=self._w, act=self._act, gu=self._gu, native=self._native,
-                                      slab=slab) if need_backward else None
+            return out, _LocalContext(None, None, self._x, self._w, self._act, self._gu, self._native, slab) if need_backward else None
         x, w = (self._x, self._w) if need_backward else (st.hidden_local, st.weights_local)
         if route_weights_sk is None:        # unscaled rows; the buffers hold the weights of an earlier call
             assert not need_backward, "a forward pass without route weights has no backward pass"

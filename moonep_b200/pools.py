@@ -203,32 +203,38 @@ class ExpertPools:
             v = self._views[key] = make()
         return v
 
-    def _alias(self, key, make) -> torch.Tensor:
+    def _alias(self, what, offs, name, dtype, count, rank) -> torch.Tensor:
         """A kept view under a tensor object of the caller's own: what the caller sets on it (``requires_grad_``, ``.grad``,
         shape in place) is nobody else's."""
-        return self.kept(key, make).detach()
+        key = (what, name, rank)
+        v = self._views.get(key)
+        if v is None:
+            v = self._views[key] = self._view(offs[name], name, dtype, 0, count, rank)
+        return v.detach()
 
     def addresses(self, epn: int, H: int, Hp: int, grads: bool = False) -> tuple:
         """Addresses of the three compute views (gate, up, down) for a native call of a layer of that size."""
-        def make():
+        key = (epn, H, Hp, grads)
+        v = self._views.get(key)
+        if v is None:
             assert self.epn == epn, f"pools hold {self.epn} experts, the layer needs {epn}"
             for n, s in zip(NAMES, ((H, Hp), (H, Hp), (Hp, H))):
                 assert self._shapes[n] == s, f"pools hold {n} {self._shapes[n]}, the layer needs {s}"
             assert self.dtype == torch.bfloat16, "the layer computes in bf16"
-            return tuple((self.compute_grad(n) if grads else self.compute_weight(n)).data_ptr() for n in NAMES)
-        return self.kept(("addresses", epn, H, Hp, grads), make)
+            v = self._views[key] = tuple((self.compute_grad(n) if grads else self.compute_weight(n)).data_ptr() for n in NAMES)
+        return v
 
     # ---- weights
     def local_weight(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._wview[name][:self.epn]
-        return self._alias(("local_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, self.epn, rank))
+        return self._alias("local_weight", self._woff, name, self.dtype, self.epn, rank)
 
     def compute_weight(self, name, rank=None) -> torch.Tensor:
         """``[2*epn, rows, cols]``: local experts then this rank's prefetch slots."""
         if self.shared is not None:
             return self._wview[name]
-        return self._alias(("compute_weight", name, rank), lambda: self._view(self._woff[name], name, self.dtype, 0, 2 * self.epn, rank))
+        return self._alias("compute_weight", self._woff, name, self.dtype, 2 * self.epn, rank)
 
     def prefetch_view(self, name) -> torch.Tensor:
         """``[R, epn, rows, cols]`` view of every rank's prefetch slots."""
@@ -242,12 +248,12 @@ class ExpertPools:
     def local_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name][:self.epn]
-        return self._alias(("local_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, self.epn, rank))
+        return self._alias("local_grad", self._goff, name, torch.float32, self.epn, rank)
 
     def compute_grad(self, name, rank=None) -> torch.Tensor:
         if self.shared is not None:
             return self._gview[name]
-        return self._alias(("compute_grad", name, rank), lambda: self._view(self._goff[name], name, torch.float32, 0, 2 * self.epn, rank))
+        return self._alias("compute_grad", self._goff, name, torch.float32, 2 * self.epn, rank)
 
     def reduce_view(self, name) -> torch.Tensor:
         if self.shared is not None:

@@ -229,7 +229,7 @@ def test_native_calls_follow_the_launch_switch(cuda_device):
         blk.buf.enable_pdl = pdl
         y, ctx = blk.moe.forward(x, *route)
         assert blk.moe._native._args.pdl == pdl
-        blk.moe._native._args.pdl = 2
+        blk.moe._native._args.pdl = blk.moe._native._pdl = 2
         dx, dw = blk.moe.backward(ctx, dy)
         assert blk.moe._native._args.pdl == pdl
         got.append([y, dx, dw] + [blk.pools.local_grad(n).clone() for n in ("gate", "up", "down")])
