@@ -41,7 +41,6 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   __shared__ __align__(8) uint64_t full_bar[kRing], empty_bar[kRing], tfull_bar[2], tempty_bar[2];
   __shared__ uint32_t s_tmem_base;
   __shared__ volatile int s_abort;
-  __shared__ int s_ntiles, s_bands;
   __shared__ tq::Ring s_ring;
   __shared__ int s_cu[kMaxGroups], s_units[kMaxGroups];     // first row, 32-row units of a group
   __shared__ unsigned char s_act[kMaxGroups];               // groups with tiles
@@ -62,32 +61,30 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   }
   if (warp == 1) { tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2(); }
   pdl_wait();                           // everything below reads what kernels before this one wrote
-  if (warp == 2) {                      // tile list: 32 groups at a time
-    int n = 0;
-    for (int g0 = 0; g0 < G; g0 += 32) {
-      const int g = g0 + lane;
-      bool act = false;
-      if (g < G) {
-        const int beg = g ? args.cu_seqlens[g - 1] : 0, end = args.cu_seqlens[g];
-        s_cu[g] = beg;
-        s_units[g] = (end - beg - (args.pad_rows ? args.pad_rows[2 * g + 1] : 0) + 31) >> 5;
-        act = g >= args.g_begin && g < args.g_end && (end > beg || (!args.accumulate && g < args.zero_empty_below));
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, act);
-      if (act) s_act[n + __popc(m & lanemask_lt())] = (unsigned char)g;
-      n += __popc(m);
+  // Tile list: a thread for each group. Groups with more tokens come first, as their tiles take longer: a launch then ends with
+  // the shortest tiles, and the pairs finish together (48 groups of 20 to 1400 tokens, 7168 x 2048: XXX).
+  int* s_key = reinterpret_cast<int*>(smem);      // the ring is not in use yet
+  bool act = false;
+  const int tg = threadIdx.x;
+  if (tg < kMaxGroups) {
+    int key = -1;
+    if (tg < G) {
+      const int beg = tg ? args.cu_seqlens[tg - 1] : 0, end = args.cu_seqlens[tg];
+      const int units = (end - beg - (args.pad_rows ? args.pad_rows[2 * tg + 1] : 0) + 31) >> 5;
+      s_cu[tg] = beg; s_units[tg] = units;
+      act = tg >= args.g_begin && tg < args.g_end && (end > beg || (!args.accumulate && tg < args.zero_empty_below));
+      if (act) key = units * 256 + (255 - tg);
     }
-    if (lane == 0) {
-      s_ntiles = n * (args.M_w / 256) * (args.N / 256);
-      s_bands = (int64_t)args.cu_seqlens[G - 1] * args.M_w > (int64_t)G * kBandElems ? (args.M_w / 256 + 7) / 8 : 1;
-    }
+    s_key[tg] = key;
   }
+  const int nact = __syncthreads_count(act ? 1 : 0);
+  if (act) s_act[rank_of(s_key[tg], s_key, G)] = (unsigned char)tg;
   tc::fence_before_sync();
   __syncthreads();
   cluster_sync();                       // both CTAs' barriers exist before anyone touches the peer's
   tc::fence_after_sync();
   const uint32_t tmem_base = s_tmem_base;
-  const int ntiles = s_ntiles;
+  const int ntiles = nact * (args.M_w / 256) * (args.N / 256);
   const bool dyn = args.sched != nullptr;
 
   auto fail = [&](int site, int tile) {
@@ -102,7 +99,8 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   // epilogue 0.806 -> 0.771). With 1024 tokens a group's rows stay in L2 anyway, and the epilogue's updates take 1 % longer in bands.
   // The mean is over all G groups; a layer passes its slots for replicas too, which are empty on one rank, and there its
   // experts have to average 36 MB.
-  const int mblk = args.M_w / 256, nblk = args.N / 256, bands = s_bands, bw = (mblk + bands - 1) / bands;
+  const int bands = (int64_t)args.cu_seqlens[G - 1] * args.M_w > (int64_t)G * kBandElems ? (args.M_w / 256 + 7) / 8 : 1;
+  const int mblk = args.M_w / 256, nblk = args.N / 256, bw = (mblk + bands - 1) / bands;
   const Divisor by_group(mblk * nblk), by_band(bw * nblk), by_row(bw), by_last(mblk - (bands - 1) * bw);
   auto get_tile = [&](int t, Tile& ti) {
     const int ai = by_group(t), local = t - ai * by_group.b, band = by_band(local), in = local - band * by_band.b;
@@ -120,7 +118,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     bool any = false, ready = true;      // ready: the stage is known to be free
     tq::Scheduler<true> sched; tq::Consumer<true> follow;
     if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
-    tq::Strided seq{pair, npairs, ntiles};
+    tq::Snake seq(pair, npairs, ntiles);
     const uint32_t smem0 = smem_u32(smem), full0 = mapa(smem_u32(&full_bar[0]), 0);
     for (;;) {
       int t = -1;
@@ -161,7 +159,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       uint32_t stage = 0, phase = 0;
       bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
-      tq::Strided seq{pair, npairs, ntiles};
+      tq::Snake seq(pair, npairs, ntiles);
       for (;; ++tcnt) {
         int t = -1;
         if (!dyn) { if (!s_abort) t = seq.next(); }
@@ -206,7 +204,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     const uint32_t tempty_leader[2] = {mapa(smem_u32(&tempty_bar[0]), 0), mapa(smem_u32(&tempty_bar[1]), 0)};
     int tcnt = 0, chunk_no = 0; Tile ti;
     tq::Consumer<true> tiles; tiles.setup(&s_ring);
-    tq::Strided seq{pair, npairs, ntiles};
+    tq::Snake seq(pair, npairs, ntiles);
     for (;; ++tcnt) {
       int t = -1;
       if (!dyn) { if (!s_abort) t = seq.next(); }

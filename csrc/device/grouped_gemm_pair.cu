@@ -83,7 +83,9 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   __shared__ uint32_t s_tmem_base;
   __shared__ volatile int s_abort;
   __shared__ tq::Ring s_ring;
-  __shared__ int s_beg[kMaxGroups], s_units[kMaxGroups], s_start[kMaxGroups + 1];   // first row, 32-token units, first tile of a group
+  // groups in the order of the tile list: number, first row, 32-token units, first tile; what they are ordered by
+  __shared__ int s_grp[kMaxGroups], s_beg[kMaxGroups], s_units[kMaxGroups], s_start[kMaxGroups + 1];
+  __shared__ __align__(16) int s_key[kMaxGroups];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cr = cluster_ctarank();
   const bool leader = cr == 0;
@@ -106,21 +108,35 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
   }
   pdl_wait();                            // everything below reads what kernels before this one wrote
-  if (warp == 0) {                       // tile list: 32 groups at a time
+  // Tile list: a thread for each group. Groups with larger tiles come first, so that the launch ends with the shortest and the
+  // pairs finish together -- unless the rows or weights are still arriving, in the order of the groups.
+  const int tg = threadIdx.x;
+  int units = 0, beg = 0, key = -1;
+  if (tg < kMaxGroups) {
+    if (tg < G) {
+      beg = tg ? args.cu_seqlens[tg - 1] : 0;
+      int rows = args.cu_seqlens[tg] - beg;
+      if (args.pad_rows) rows -= args.pad_rows[2 * tg + 1];
+      if (tg >= args.g_begin && tg < args.g_end) units = (rows + 31) >> 5;
+      const int mt = (units + 7) >> 3;
+      key = (units && !args.tile_done && !args.group_flags ? (units + mt - 1) / mt : 0) * 256 + (255 - tg);
+    }
+    s_key[tg] = key;
+  }
+  __syncthreads();
+  if (tg < G) {
+    const int at = rank_of(key, s_key, G);
+    s_grp[at] = tg; s_beg[at] = beg; s_units[at] = units;
+  }
+  __syncthreads();
+  if (warp == 0) {                       // first tile of each: 32 groups at a time
     const int nblk = args.N / kCols;
     int run = 0, most = 0;
     for (int g0 = 0; g0 < G; g0 += 32) {
-      const int g = g0 + lane;
-      int beg = 0, units = 0;
-      if (g < G) {
-        beg = g ? args.cu_seqlens[g - 1] : 0;
-        int rows = args.cu_seqlens[g] - beg;
-        if (args.pad_rows) rows -= args.pad_rows[2 * g + 1];
-        if (g >= args.g_begin && g < args.g_end) units = (rows + 31) >> 5;
-      }
-      const int mt = (units + 7) >> 3, tiles = mt * nblk, incl = warp_incl_scan(tiles);
-      if (units) most = max(most, (units + mt - 1) / mt);
-      if (g < G) { s_beg[g] = beg; s_units[g] = units; s_start[g] = run + incl - tiles; }
+      const int i = g0 + lane, u = i < G ? s_units[i] : 0;
+      const int mt = (u + 7) >> 3, tiles = mt * nblk, incl = warp_incl_scan(tiles);
+      if (u) most = max(most, (u + mt - 1) / mt);
+      if (i < G) s_start[i] = run + incl - tiles;
       run += __shfl_sync(0xffffffffu, incl, 31);
     }
     for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
@@ -148,7 +164,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     }
   };
   auto fail = [&](int site, int tile, int code = MEP_ERR_MBAR_TIMEOUT) { note(site, tile, code); s_abort = 1; };
-  // tile number -> tile; `g` is a monotone cursor. The tiles of a group share its tokens evenly (in units of 32), token
+  // tile number -> tile; `g` is a monotone cursor over the ordered groups. The tiles of a group share its tokens evenly (in units of 32), token
   // tiles vary fastest: the weight columns they have in common are then in L2 (within a band, see kBand).
   auto get_tile = [&](int t, int& g, Tile& ti) {
     while (s_start[g + 1] <= t) ++g;
@@ -162,7 +178,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       cb = local / mt; pt = local - cb * mt;
     }
     const int base = units / mt, rem = units - base * mt;
-    ti.g = g; ti.n0 = cb * kCols;
+    ti.g = s_grp[g]; ti.n0 = cb * kCols;
     ti.row0 = s_beg[g] + 32 * (pt * base + min(pt, rem));
     ti.n = 32 * (base + (pt < rem ? 1 : 0));
   };
@@ -176,7 +192,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     bool any = false, ready = true;      // ready: the stage is known to be free
     tq::Scheduler<true> sched; tq::Consumer<true> follow;
     if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
-    tq::Strided seq{pair, npairs, ntiles};
+    tq::Snake seq(pair, npairs, ntiles);
     const uint32_t tile_ep = args.tile_done ? *(volatile const uint32_t*)args.tile_epoch : 0u;
     const uint32_t group_ep = args.group_flags ? *(volatile const uint32_t*)args.group_epoch : 0u;
     int seen_row = -1, seen_group = -1;              // flags known to be up: first row of the last tile, last group
@@ -254,7 +270,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       uint32_t stage = 0, phase = 0;
       bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
-      tq::Strided seq{pair, npairs, ntiles};
+      tq::Snake seq(pair, npairs, ntiles);
       for (;; ++tcnt) {
         int t = -1;
         if (!dyn) { if (!s_abort) t = seq.next(); }
@@ -303,7 +319,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     int chunk_no = 0;
     int tcnt = 0, gcur = 0; Tile ti;
     tq::Consumer<true> tiles; tiles.setup(&s_ring);
-    tq::Strided seq{pair, npairs, ntiles};
+    tq::Snake seq(pair, npairs, ntiles);
     auto stage = [&](uint32_t buf, const uint32_t* lo, const uint32_t* hi, float sc[4]) {
 #pragma unroll
       for (int b = 0; b < 2; ++b) {

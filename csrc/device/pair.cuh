@@ -47,6 +47,17 @@ struct Divisor {
     return q + (rem >= b) - (rem < 0);
   }
 };
+// Place of `key` among the first `n` of `keys` in falling order (keys differ, those of groups that do not count are negative;
+// `keys` 16-byte aligned and filled up to a multiple of four).
+__device__ __forceinline__ int rank_of(int key, const int* keys, int n) {
+  int r = 0;
+#pragma unroll 4
+  for (int j = 0; j < n; j += 4) {
+    const int4 k = *reinterpret_cast<const int4*>(keys + j);
+    r += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
+  }
+  return r;
+}
 // one lane of a converged warp; the others' registers stay warp-uniform, which keeps MMA descriptors out of the vector registers
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;

@@ -1,7 +1,7 @@
 // Tile hand-out for the persistent grouped-GEMM kernels.
 //
 // Static order: every role of a CTA walks the strided sequence first, first + stride, ... on its
-// own (`Strided`); nothing is shared.
+// own (`Strided`, `Snake`); nothing is shared.
 // Dynamic order (the launch passes a ticket counter): one thread per CTA (per CTA pair: one
 // thread of the leader CTA), the TMA producer, is the scheduler. It draws the next tile number
 // from the global counter -- CTAs that start late or run beside another kernel simply draw fewer
@@ -24,6 +24,18 @@ constexpr int kSlots = 8;
 struct Strided {
   int cur, step, n;
   __device__ __forceinline__ int next() { const int t = cur; cur += step; return t < n ? t : -1; }
+};
+
+// The same with every other round backwards. Where tiles come in order of falling cost, worker 0 has the longest tile of each
+// round in strided order; here the differences of two rounds cancel.
+struct Snake {
+  int cur, ahead, back, n;       // steps from an even round to the odd one behind it, and from there to the next even one
+  __device__ __forceinline__ Snake(int first, int workers, int n_) : cur(first), ahead(2 * (workers - 1 - first) + 1), back(2 * first + 1), n(n_) {}
+  __device__ __forceinline__ int next() {
+    const int t = cur, d = ahead;
+    cur += d; ahead = back; back = d;
+    return t < n ? t : -1;
+  }
 };
 
 struct Ring {
