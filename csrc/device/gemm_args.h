@@ -65,6 +65,13 @@ struct GemmArgs {
   // optional [G, 2] table (first padding row, padding rows) of the groups, as a plan carries it: rows behind the real
   // ones, rounded up to 32, are then neither computed nor read (null: all padded rows are). CTA-pair kernels only.
   const int32_t* pad_rows;
+  // CTA-pair kernels. early: everything a launch reads besides the rows of `a` (WGRAD: besides both operands) and row_scale was there
+  // before the kernel right before it in the stream BEGAN: the tables below or cu_seqlens and pad_rows, the weights, upd_mask. It then
+  // sets up its tiles and loads the first weights while that kernel still runs.
+  // tokens, optional: token counts of groups 0 to tokens_n - 1 (the others are empty), instead of cu_seqlens and pad_rows; groups are padded to
+  // multiples of token_padding rows.
+  const int32_t* tokens;
+  int32_t tokens_n, token_padding, early, reserved;
 };
 
 // CTAs of a pair launch that was asked for `n`. On a counter shared with other launches the grid accounts for all `n`.

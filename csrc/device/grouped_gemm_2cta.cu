@@ -44,6 +44,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   __shared__ tq::Ring s_ring;
   __shared__ int s_cu[kMaxGroups], s_units[kMaxGroups];     // first row, 32-row units of a group
   __shared__ unsigned char s_act[kMaxGroups];               // groups with tiles
+  __shared__ int s_total;                                   // rows of all groups
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cr = cluster_ctarank();
   const bool leader = cr == 0;
@@ -60,20 +61,21 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     tc::prefetch_tmap(&tma_a); tc::prefetch_tmap(&tma_b); tc::prefetch_tmap(&tma_out);
   }
   if (warp == 1) { tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2(); }
-  pdl_wait();                           // everything below reads what kernels before this one wrote
+  if (!args.early) pdl_wait();          // the tables below may come from the kernel right before
   // Tile list: a thread for each group. Groups with more tokens come first, as their tiles take longer: a launch then ends with
   // the shortest tiles, and the pairs finish together (16 groups of 4096 tokens on average and up to
   // three times as many, 2048 x 768: 164 -> 146 us).
   int* s_key = reinterpret_cast<int*>(smem);      // the ring is not in use yet
   bool act = false;
   const int tg = threadIdx.x;
+  int beg, rows, units;
+  group_rows(args, s_key, beg, rows, units);
   if (tg < kMaxGroups) {
     int key = -1;
     if (tg < G) {
-      const int beg = tg ? args.cu_seqlens[tg - 1] : 0, end = args.cu_seqlens[tg];
-      const int units = (end - beg - (args.pad_rows ? args.pad_rows[2 * tg + 1] : 0) + 31) >> 5;
       s_cu[tg] = beg; s_units[tg] = units;
-      act = tg >= args.g_begin && tg < args.g_end && (end > beg || (!args.accumulate && tg < args.zero_empty_below));
+      if (tg == G - 1) s_total = beg + rows;
+      act = tg >= args.g_begin && tg < args.g_end && (rows > 0 || (!args.accumulate && tg < args.zero_empty_below));
       if (act) key = units * 256 + (255 - tg);
     }
     s_key[tg] = key;
@@ -100,7 +102,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   // epilogue 0.806 -> 0.771). With 1024 tokens a group's rows stay in L2 anyway, and the epilogue's updates take 1 % longer in bands.
   // The mean is over all G groups; a layer passes its slots for replicas too, which are empty on one rank, and there its
   // experts have to average 36 MB.
-  const int bands = (int64_t)args.cu_seqlens[G - 1] * args.M_w > (int64_t)G * kBandElems ? (args.M_w / 256 + 7) / 8 : 1;
+  const int bands = (int64_t)s_total * args.M_w > (int64_t)G * kBandElems ? (args.M_w / 256 + 7) / 8 : 1;
   const int mblk = args.M_w / 256, nblk = args.N / 256, bw = (mblk + bands - 1) / bands;
   const Divisor by_group(mblk * nblk), by_band(bw * nblk), by_row(bw), by_last(mblk - (bands - 1) * bw);
   auto get_tile = [&](int t, Tile& ti) {
@@ -121,6 +123,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
     tq::Snake seq(pair, npairs, ntiles);
     const uint32_t smem0 = smem_u32(smem), full0 = mapa(smem_u32(&full_bar[0]), 0);
+    if (args.early) pdl_wait();
     for (;;) {
       int t = -1;
       if (!dyn) { if (!s_abort) t = seq.next(); }
@@ -206,6 +209,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     // Gradients are not read before the launch ends: with their lines first in line to leave L2, short groups, whose operands are
     // read again for every tile, took 550 us instead of 635 (48 groups of 256 tokens, 7168 x 2048), deep ones the same.
     const uint64_t streamed = tc::evict_first();
+    if (args.early) pdl_wait();         // gradients and weights are written from here, and the kernel before may read them
     int tcnt = 0, chunk_no = 0; Tile ti;
     tq::Consumer<true> tiles; tiles.setup(&s_ring);
     tq::Snake seq(pair, npairs, ntiles);

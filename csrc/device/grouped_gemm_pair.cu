@@ -107,17 +107,15 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     tc::prefetch_tmap(&tma_x); tc::prefetch_tmap(&tma_x64); tc::prefetch_tmap(&tma_x16); tc::prefetch_tmap(&tma_w0); tc::prefetch_tmap(&tma_w1);
     tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
   }
-  pdl_wait();                            // everything below reads what kernels before this one wrote
+  if (!args.early) pdl_wait();           // the tables below may come from the kernel right before
   // Tile list: a thread for each group. Groups with larger tiles come first, so that the launch ends with the shortest and the
   // pairs finish together -- unless the rows or weights are still arriving, in the order of the groups.
   const int tg = threadIdx.x;
-  int units = 0, beg = 0, key = -1;
+  int units, beg, rows, key = -1;
+  group_rows(args, s_key, beg, rows, units);
   if (tg < kMaxGroups) {
     if (tg < G) {
-      beg = tg ? args.cu_seqlens[tg - 1] : 0;
-      int rows = args.cu_seqlens[tg] - beg;
-      if (args.pad_rows) rows -= args.pad_rows[2 * tg + 1];
-      if (tg >= args.g_begin && tg < args.g_end) units = (rows + 31) >> 5;
+      if (tg < args.g_begin || tg >= args.g_end) units = 0;
       const int mt = (units + 7) >> 3;
       key = (units && !args.tile_done && !args.group_flags ? (units + mt - 1) / mt : 0) * 256 + (255 - tg);
     }
@@ -190,6 +188,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     int gcur = 0; Tile ti;
     uint32_t s = 0, ph = 0;
     bool any = false, ready = true;      // ready: the stage is known to be free
+    bool early = args.early != 0;        // the kernel before has not been waited for yet
     tq::Scheduler<true> sched; tq::Consumer<true> follow;
     if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
     tq::Snake seq(pair, npairs, ntiles);
@@ -224,37 +223,56 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       }
       const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
       const uint32_t bytes = (uint32_t)kWBytes + (small ? (uint32_t)half * 128u : half > 64 ? 16384u : 8192u);
-      for (int kb = 0; kb < kblocks; ++kb) {
+      auto load_w = [&](int kb, uint32_t st) {
+        const uint32_t sw = smem0 + st * stage_bytes, bar = full0 + st * 8u;
+        const int k0 = kb * kBK;
+        if (leader) mbar_expect_tx(&full_bar[st], 2 * bytes);
+        if (MODE == GEMM_GATE_UP) {
+          tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+          tma_load_3d_bar(sw + kAtomBytes, &tma_w1, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+        } else if (MODE == GEMM_DOWN) {
+          tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
+        } else {
+          const int kh = args.K / 2;               // DGRAD_GU: first half of K from Wg, second from Wu
+          if (MODE == GEMM_DGRAD_GU && k0 >= kh) tma_load_2d_bar(sw, &tma_w1, k0 - kh, wrow + ti.n0 + (int)cr * 128, bar);
+          else tma_load_2d_bar(sw, &tma_w0, k0, wrow + ti.n0 + (int)cr * 128, bar);
+        }
+      };
+      auto load_x = [&](int kb, uint32_t st) {
+        const uint32_t sx = smem0 + st * stage_bytes + kWBytes, bar = full0 + st * 8u;
+        const int k0 = kb * kBK;
+        if (small) {
+          for (int i = 0; i < half; i += 16) tma_load_2d_bar(sx + i * 128, &tma_x16, k0, xrow + i, bar);
+        } else if (half > 64) {
+          tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
+        } else {
+          tma_load_2d_bar(sx, &tma_x64, k0, xrow, bar);
+        }
+      };
+      int kb = 0;
+      if (early) {                         // fill the ring with weights, then wait for the rows
+        const int pre = min((int)nstages, kblocks);
+        if (elect_one()) for (int i = 0; i < pre; ++i) load_w(i, i);
+        __syncwarp();
+        pdl_wait();
+        early = false;
+        if (elect_one()) for (int i = 0; i < pre; ++i) load_x(i, i);
+        __syncwarp();
+        kb = pre; any = true;
+        if (pre == (int)nstages) { s = 0; ph = 1; } else s = pre;
+        ready = mbar_test(&empty_bar[s], ph ^ 1u);
+      }
+      for (; kb < kblocks; ++kb) {
         if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, mbar_wait_compact(&empty_bar[s], ph ^ 1u, args.budget_ns))) { if (lane == 0) fail(1, t); break; }
         const uint32_t sn = s + 1 == nstages ? 0u : s + 1, phn = sn ? ph : ph ^ 1u;
         ready = mbar_test(&empty_bar[sn], phn ^ 1u);
-        if (elect_one()) {
-          const uint32_t sw = smem0 + s * stage_bytes, sx = sw + kWBytes, bar = full0 + s * 8u;
-          const int k0 = kb * kBK;
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * bytes);
-          if (MODE == GEMM_GATE_UP) {
-            tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
-            tma_load_3d_bar(sw + kAtomBytes, &tma_w1, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
-          } else if (MODE == GEMM_DOWN) {
-            tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
-          } else {
-            const int kh = args.K / 2;               // DGRAD_GU: first half of K from Wg, second from Wu
-            if (MODE == GEMM_DGRAD_GU && k0 >= kh) tma_load_2d_bar(sw, &tma_w1, k0 - kh, wrow + ti.n0 + (int)cr * 128, bar);
-            else tma_load_2d_bar(sw, &tma_w0, k0, wrow + ti.n0 + (int)cr * 128, bar);
-          }
-          if (small) {
-            for (int i = 0; i < half; i += 16) tma_load_2d_bar(sx + i * 128, &tma_x16, k0, xrow + i, bar);
-          } else if (half > 64) {
-            tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
-          } else {
-            tma_load_2d_bar(sx, &tma_x64, k0, xrow, bar);
-          }
-        }
+        if (elect_one()) { load_w(kb, s); load_x(kb, s); }
         __syncwarp();
         any = true;
         s = sn; ph = phn;
       }
     }
+    if (early) pdl_wait();               // whoever waits for this launch waits for the kernel before, too
     // the leader's last barrier phase covers both CTAs' copies: nobody leaves before it (cluster_sync below)
     if (leader && any) mbar_wait_compact(&full_bar[s ? s - 1 : nstages - 1], s ? ph : ph ^ 1u, args.budget_ns);
   } else if (warp == 1) {
@@ -308,6 +326,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     }
   } else {
     // ---------------- epilogue: this CTA's 128 weight columns (TMEM lanes) of every token of the tile
+    if (args.early) pdl_wait();
     const int q = warp & 3, set = (warp - 2) >> 2, side = q >> 1;      // side: TMEM lanes 0-63 or 64-127 = one 64-column staging row
     const uint32_t epi = smem_u32(smem + kRingBytes);
     const uint32_t tempty_leader[2] = {mapa(smem_u32(&tempty_bar[0]), 0), mapa(smem_u32(&tempty_bar[1]), 0)};

@@ -59,6 +59,7 @@ struct MoeLocal {
   int32_t* status;
   int32_t* status_host;
   uint64_t budget_ns;
+  int32_t token_padding, reserved;
 };
 
 }  // namespace mep

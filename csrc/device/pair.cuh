@@ -3,6 +3,7 @@
 // CTA's own shared memory; only its byte count goes to the leader's barrier. No cluster-wide copy is used.
 #pragma once
 #include "tcgen05.cuh"
+#include "gemm_args.h"
 
 namespace mep {
 namespace pair {
@@ -61,6 +62,28 @@ __device__ __forceinline__ int rank_of(int key, const int* keys, int n) {
     r += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
   }
   return r;
+}
+// First row and 32-row units of the calling thread's group (threadIdx.x; of no use to threads from G on). All threads call it;
+// `scratch`: 192 ints, 16-byte aligned, free again after the next block barrier.
+__device__ __forceinline__ void group_rows(const GemmArgs& args, int* scratch, int& beg, int& rows, int& units) {
+  const int g = threadIdx.x, G = args.G;
+  beg = 0; rows = 0; units = 0;
+  if (args.tokens) {
+    int n = g < args.tokens_n ? __ldg(args.tokens + g) : 0;
+    rows = (n + args.token_padding - 1) / args.token_padding * args.token_padding;
+    if (g < 192) scratch[g] = rows;
+    __syncthreads();
+    for (int j = 0; j < G; j += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(scratch + j);
+      beg += (j < g ? v.x : 0) + (j + 1 < g ? v.y : 0) + (j + 2 < g ? v.z : 0) + (j + 3 < g ? v.w : 0);
+    }
+    units = (n + 31) >> 5;
+    __syncthreads();                     // before the scratch is used for something else
+  } else if (g < G) {
+    beg = g ? args.cu_seqlens[g - 1] : 0;
+    rows = args.cu_seqlens[g] - beg;
+    units = (rows - (args.pad_rows ? args.pad_rows[2 * g + 1] : 0) + 31) >> 5;
+  }
 }
 // one lane of a converged warp; the others' registers stay warp-uniform, which keeps MMA descriptors out of the vector registers
 __device__ __forceinline__ bool elect_one() {

@@ -15,11 +15,15 @@ int mep_swiglu_bwd(const void*, const void*, const float*, void*, float*, const 
 
 namespace mep {
 
-static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab) {
+// A pass begins with a dispatch, an ordinary launch that begins when everything before it in the stream is done. Weights, and the
+// plan of a backward pass, are therefore complete before any GEMM of the pass begins, and so are the token counts that a forward
+// pass is given (`tpe`; its plan is written by the dispatch).
+static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab, const int32_t* tpe = nullptr) {
   GemmArgs a = {};
   a.cu_seqlens = slab + m.plan_off[7];
   a.pad_rows = slab + m.plan_off[2];
   a.G = 2 * m.E; a.g_end = 2 * m.E;
+  a.early = 1; a.tokens = tpe; a.tokens_n = m.E; a.token_padding = m.token_padding;
   a.pdl = m.pdl;                 // behind another kernel of the same call
   a.status = m.status; a.status_host = m.status_host; a.budget_ns = m.budget_ns;
   return a;
@@ -83,10 +87,10 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   d.weights = route_w; d.out_hidden = x; d.out_weights = w;
   plan_into(m, topk, tpe, slab, &d);
   if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.S, m.K, m.H, m.E, stream)) return -1;
-  GemmArgs g = gemm_args(m, slab);
+  GemmArgs g = gemm_args(m, slab, tpe);
   g.N = m.Hp; g.K = m.H; g.out = m.act; g.out2 = keep ? m.gu : nullptr; g.row_scale = w; g.ldo = m.Hp;
   if (gemm(m, GEMM_GATE_UP, x, m.H, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
-  g = gemm_args(m, slab);
+  g = gemm_args(m, slab, tpe);
   g.N = m.H; g.K = m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DOWN, m.act, m.Hp, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, nullptr, (__nv_bfloat16*)out, nullptr};

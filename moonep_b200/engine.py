@@ -236,7 +236,7 @@ class LocalExchange:
     def __init__(self, st: RankState, blocks: int):
         g, a = st.geo, _native.MoeLocal()
         a.ctx = st.ctx_ptr
-        a.S, a.H, a.K, a.E, a.NvS = g.S, g.H, g.K, g.E, g.NvS
+        a.S, a.H, a.K, a.E, a.NvS, a.token_padding = g.S, g.H, g.K, g.E, g.NvS, g.token_padding
         a.blocks, a.combine_blocks = min(blocks, st.local_blocks), blocks
         _, self._total, first = _plan_layout(st)
         a.plan_off = (C.c_int64 * 8)(*first)

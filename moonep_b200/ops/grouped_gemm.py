@@ -38,7 +38,8 @@ class GemmArgs(C.Structure):
                 ("group_flags", C.c_void_p), ("group_epoch", C.c_void_p),
                 ("push_rows", C.c_int32), ("push_ranks", C.c_int32), ("group_first", C.c_int32), ("sched_ctas", C.c_int32),
                 ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("sched_odd", C.c_int32),
-                ("pad_rows", C.c_void_p)]
+                ("pad_rows", C.c_void_p), ("tokens", C.c_void_p), ("tokens_n", C.c_int32), ("token_padding", C.c_int32),
+                ("early", C.c_int32), ("reserved", C.c_int32)]
 
 
 class PushTarget:
