@@ -354,7 +354,7 @@ def sgd_step_groups(p, g, lr, mask, want: bool, num_blocks=None):
     lib = _native.load()
     assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.shape == g.shape
     assert p.is_contiguous() and g.is_contiguous() and mask.dtype == torch.int32 and mask.numel() >= p.shape[0]
-    nb = num_blocks or 2 * _num_sms(p.device)
+    nb = num_blocks or 0
     _native.check(lib.mep_sgd_step_groups(C.c_void_p(p.data_ptr()), C.c_void_p(g.data_ptr()), C.c_float(lr),
                                           C.c_int64(p[0].numel()), p.shape[0], C.c_void_p(mask.data_ptr()), 1 if want else 0,
                                           nb, _native.cur_stream()), "sgd_step_groups")
@@ -364,7 +364,7 @@ def sgd_step(p, g, lr, num_blocks=None):
     lib = _native.load()
     assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.numel() == g.numel()
     assert p.is_contiguous() and g.is_contiguous()
-    nb = num_blocks or 8 * _num_sms(p.device)
+    nb = num_blocks or 0
     _native.check(lib.mep_sgd_step(C.c_void_p(p.data_ptr()), C.c_void_p(g.data_ptr()), C.c_float(lr),
                                    C.c_int64(p.numel()), nb, _native.cur_stream()), "sgd_step")
 
@@ -379,7 +379,7 @@ class SgdMany:
             assert p.is_contiguous() and g.is_contiguous()
         P, N = C.c_void_p * n, C.c_int64 * n
         self._args = (n, P(*[p.data_ptr() for p in ps]), P(*[g.data_ptr() for g in gs]), N(*[p.numel() for p in ps]))
-        self._blocks = num_blocks or 8 * _num_sms(ps[0].device)
+        self._blocks = num_blocks or 0
         self._keep = (list(ps), list(gs))
 
     def step(self, lr):

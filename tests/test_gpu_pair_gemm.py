@@ -224,3 +224,27 @@ def test_dgrad_pushes_rows_and_their_scalars(pairs, cuda_device, monkeypatch):
     gg.check_status()
     assert torch.equal(out, (x.float() * K).to(torch.bfloat16)) and torch.equal(ow, w)
     buf.destroy()
+
+
+@pytest.mark.parametrize("blocks", [None, 1, 5])
+def test_sgd_at_the_edges_of_its_chunks(blocks, cuda_device):
+    """Chunks are 8192 parameters. One rounding to fp32 and one to bf16: what double precision gives for a rate with few bits."""
+    from moonep_b200.ops import grouped_gemm as gg
+    sizes = [8, 2040, 2048, 8184, 8192, 8200, 3 * 8192 + 2056, 40 * 8192]
+    g = torch.Generator(device="cuda").manual_seed(6)
+    ps = [(torch.randn(n, device="cuda", generator=g)).to(torch.bfloat16) for n in sizes]
+    gs = [torch.randn(n, device="cuda", generator=g) for n in sizes]
+    want = [(p.double() - 0.125 * d.double()).float().to(torch.bfloat16) for p, d in zip(ps, gs)]
+    for p, d, w in zip(ps, gs, want):
+        a = p.clone()
+        gg.sgd_step(a, d, 0.125, num_blocks=blocks)
+        assert torch.equal(a, w), f"{p.numel()} parameters"
+    many = [p.clone() for p in ps]
+    for i in (0, 4):
+        gg.SgdMany(many[i:i + 4], gs[i:i + 4], num_blocks=blocks).step(0.125)
+    assert all(torch.equal(a, w) for a, w in zip(many, want))
+    p, d = (torch.cat([t[5][:8200]] * 3).view(3, -1) for t in (ps, gs))
+    mask = torch.tensor([1, 0, 1], dtype=torch.int32, device="cuda")
+    got = p.clone()
+    gg.sgd_step_groups(got, d, 0.125, mask, True, num_blocks=blocks)
+    assert torch.equal(got[0], want[5]) and torch.equal(got[1], p[1]) and torch.equal(got[2], want[5])
