@@ -71,7 +71,11 @@ struct GemmArgs {
   // tokens, optional: token counts of groups 0 to tokens_n - 1 (the others are empty), instead of cu_seqlens and pad_rows; groups are padded to
   // multiples of token_padding rows.
   const int32_t* tokens;
-  int32_t tokens_n, token_padding, early, reserved;
+  int32_t tokens_n, token_padding, early;
+  // WGRAD (CTA-pair kernel): 0, or the columns of one weight matrix (a multiple of 256), N = 2 * n_each: the second half of dy's columns
+  // gives the gradient (update) of another matrix of the same shape, out_b (upd_w_b).
+  int32_t n_each;
+  void *out_b, *upd_w_b;
 };
 
 // CTAs of a pair launch that was asked for `n`. On a counter shared with other launches the grid accounts for all `n`.

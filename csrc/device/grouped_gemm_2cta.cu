@@ -35,7 +35,7 @@ struct Tile { int g, row0, m0, n0, kblocks, ksteps; };      // ksteps: 16-row st
 
 __global__ void __launch_bounds__(kThreads, 1)
 wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                  const __grid_constant__ CUtensorMap tma_out, GemmArgs args) {
+                  const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out_b, GemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full_bar[kRing], empty_bar[kRing], tfull_bar[2], tempty_bar[2];
@@ -59,6 +59,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     tq::init(&s_ring, 2 * kEpiWarps + 2);      // both CTAs' epilogue warps, the MMA issuer, the peer's producer
     fence_mbar_init();
     tc::prefetch_tmap(&tma_a); tc::prefetch_tmap(&tma_b); tc::prefetch_tmap(&tma_out);
+    tc::prefetch_tmap(&tma_out_b);
   }
   if (warp == 1) { tmem_alloc2(&s_tmem_base, 512); tmem_relinquish2(); }
   if (!args.early) pdl_wait();          // the tables below may come from the kernel right before
@@ -223,22 +224,25 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       if (t < 0) break;
       get_tile(t, ti);
       const int orow0 = ti.g * args.M_w + ti.m0 + (int)cr * 128 + q * 32;
+      const int pitch = args.n_each ? args.n_each : args.N;        // one launch may compute two matrices side by side
+      const bool b = ti.n0 >= pitch;
+      const int ocol0 = b ? ti.n0 - pitch : ti.n0;
       // optimizer in the epilogue: this group's weights are updated in place and no gradient is written
       const bool upd = args.upd_mask != nullptr && args.upd_mask[ti.g] != 0;
       if (ti.kblocks == 0) {           // empty group that must end with a zero gradient (nothing to update)
         if (!upd) {
           // whole 512-byte runs: with a lane per row this path ran at a third of the HBM rate
-          float4* o = reinterpret_cast<float4*>((float*)args.out + (size_t)orow0 * args.N + ti.n0 + half * 128) + lane;
-          for (int r = 0; r < 32; ++r) __stcs(o + (size_t)r * (args.N / 4), make_float4(0.f, 0.f, 0.f, 0.f));
+          float4* o = reinterpret_cast<float4*>((float*)(b ? args.out_b : args.out) + (size_t)orow0 * pitch + ocol0 + half * 128) + lane;
+          for (int r = 0; r < 32; ++r) __stcs(o + (size_t)r * (pitch / 4), make_float4(0.f, 0.f, 0.f, 0.f));
         }
         --tcnt; continue;
       }
       // A chunk is 32 rows x 32 columns. The accumulator arrives with lane = row; the weights are read and
       // written with four lanes per row instead (16 bytes each, eight rows per instruction: whole sectors),
       // so the chunk takes the same trip through the warp's shared-memory slab as a stored gradient does.
-      const __nv_bfloat16* wbase = upd ? (const __nv_bfloat16*)args.upd_w + (size_t)orow0 * args.N + ti.n0 + (half * 4) * 32 : nullptr;
+      const __nv_bfloat16* wbase = upd ? (const __nv_bfloat16*)(b ? args.upd_w_b : args.upd_w) + (size_t)orow0 * pitch + ocol0 + (half * 4) * 32 : nullptr;
       auto wptr = [&](int i, int k) {
-        return const_cast<__nv_bfloat16*>(wbase) + (size_t)((lane >> 2) + 8 * k) * args.N + i * 32 + (lane & 3) * 8;
+        return const_cast<__nv_bfloat16*>(wbase) + (size_t)((lane >> 2) + 8 * k) * pitch + i * 32 + (lane & 3) * 8;
       };
       int4 wv[4][4];
       if (upd) {                       // the tile's weights (this warp's 32 x 128 part): in flight while its MMAs finish
@@ -307,8 +311,8 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (args.accumulate) tc::tma_reduce_add_2d(&tma_out, buf, ti.n0 + c * 32, orow0);
-          else tc::tma_store_2d(&tma_out, buf, ti.n0 + c * 32, orow0, streamed);
+          if (args.accumulate) tc::tma_reduce_add_2d(b ? &tma_out_b : &tma_out, buf, ocol0 + c * 32, orow0);
+          else tc::tma_store_2d(b ? &tma_out_b : &tma_out, buf, ocol0 + c * 32, orow0, streamed);
           bulk_commit();
         }
       }
@@ -339,10 +343,14 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   MEP_REQUIRE(args.M_w % 256 == 0 && args.N % 256 == 0, "wgrad (2-CTA): weight shape [%d,%d] must be multiples of 256", args.M_w, args.N);
   num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "wgrad (2-CTA): needs at least two CTAs");
-  CUtensorMap ma, mb, mo;
+  MEP_REQUIRE(args.n_each == 0 || (args.N == 2 * args.n_each && args.n_each % 256 == 0 && args.out_b), "wgrad (2-CTA): two matrices of %d columns in %d", args.n_each, args.N);
+  const int pitch = args.n_each ? args.n_each : args.N;
+  CUtensorMap ma, mb, mo, mo_b;
   if (tmap_rows(&ma, x, rows, args.M_w, x_ld, 64, 64)) return -1;
   if (tmap_rows(&mb, dy, rows, args.N, dy_ld, 64, 64)) return -1;
-  if (tmap_rows(&mo, args.out, (int64_t)args.G * args.M_w, args.N, args.N, 32, 32, true)) return -1;
+  if (tmap_rows(&mo, args.out, (int64_t)args.G * args.M_w, pitch, pitch, 32, 32, true)) return -1;
+  if (!args.n_each) mo_b = mo;
+  else if (tmap_rows(&mo_b, args.out_b, (int64_t)args.G * args.M_w, pitch, pitch, 32, 32, true)) return -1;
   if (allow_smem((const void*)w2::wgrad_2cta_kernel, w2::kSmem)) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_ctas); cfg.blockDim = dim3(w2::kThreads); cfg.dynamicSmemBytes = w2::kSmem; cfg.stream = stream;
@@ -352,7 +360,7 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
-  MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, w2::wgrad_2cta_kernel, ma, mb, mo, args));
+  MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, w2::wgrad_2cta_kernel, ma, mb, mo, mo_b, args));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
 }

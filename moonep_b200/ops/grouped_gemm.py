@@ -39,7 +39,7 @@ class GemmArgs(C.Structure):
                 ("push_rows", C.c_int32), ("push_ranks", C.c_int32), ("group_first", C.c_int32), ("sched_ctas", C.c_int32),
                 ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("sched_odd", C.c_int32),
                 ("pad_rows", C.c_void_p), ("tokens", C.c_void_p), ("tokens_n", C.c_int32), ("token_padding", C.c_int32),
-                ("early", C.c_int32), ("reserved", C.c_int32)]
+                ("early", C.c_int32), ("n_each", C.c_int32), ("out_b", C.c_void_p), ("upd_w_b", C.c_void_p)]
 
 
 class PushTarget:
@@ -295,7 +295,7 @@ def wgrad_update_supported(M: int, N: int) -> bool:
 
 
 def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num_ctas=None, dynamic=False, ticket=None,
-          update=None, pad=None):
+          update=None, pad=None, out_b=None, update_b=None):
     """``out[g] (+)= x_g^T dy_g`` in fp32; ``out [G, in, out_dim]``.  ``dy`` may be a column slice
     of a wider matrix (row pitch = ``dy.stride(0)``).  Groups without rows are left untouched,
     except that with ``accumulate=False`` empty groups ``g < zero_empty_below`` are zeroed (local
@@ -305,9 +305,15 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
     (int32 ``[G]`` on the device) the gradient is not written; ``weights[g]`` (bf16, same shape as ``out``)
     becomes ``weights[g] - lr * dW`` instead, bit for bit what ``sgd_step`` computes from a stored gradient.
     Groups with ``mask[g] == 0`` are written to ``out`` as usual.  Needs weight shapes that are multiples
-    of 256 (the CTA-pair kernel)."""
+    of 256 (the CTA-pair kernel).
+
+    ``out_b``: a second tensor like ``out``, for the second half of ``dy``'s columns (gate and up in one launch);
+    ``update_b``: its weights, if ``update`` is given."""
     G, M, N = out.shape
     assert out.dtype == torch.float32 and out.is_contiguous()
+    if out_b is not None:
+        assert out_b.dtype == torch.float32 and out_b.is_contiguous() and out_b.shape == out.shape and wgrad_update_supported(M, N)
+        N *= 2
     assert x.shape[1] == M and dy.shape[1] == N and M % 128 == 0 and N % 256 == 0
     assert dy.stride(1) == 1 and x.stride(1) == 1
     if M % 256 == 0 and os.environ.get("MOONEP_WGRAD_2CTA", "1") != "0":
@@ -328,6 +334,12 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
             assert w.dtype == torch.bfloat16 and tuple(w.shape) == tuple(out.shape) and w.is_contiguous()
             assert mask.dtype == torch.int32 and mask.numel() == G and mask.is_cuda
             args.upd_w, args.upd_mask, args.upd_lr = w.data_ptr(), mask.data_ptr(), float(lr)
+            assert (update_b is None) == (out_b is None)
+        if out_b is not None:
+            args.n_each, args.out_b = N // 2, out_b.data_ptr()
+            if update is not None:
+                assert update_b.dtype == torch.bfloat16 and update_b.shape == out.shape and update_b.is_contiguous()
+                args.upd_w_b = update_b.data_ptr()
         rc = lib.mep_grouped_wgrad_2cta(C.c_void_p(x.data_ptr()), C.c_int64(x.shape[0]), C.c_int64(x.stride(0)),
                                         C.c_void_p(dy.data_ptr()), C.c_int64(dy.stride(0)), C.byref(args),
                                         num_ctas or _num_sms(x.device), _native.cur_stream())

@@ -226,6 +226,34 @@ def test_dgrad_pushes_rows_and_their_scalars(pairs, cuda_device, monkeypatch):
     buf.destroy()
 
 
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_two_weight_gradients_in_one_launch(accumulate, cuda_device):
+    """The halves of dy's columns give two matrices: the same bits as two launches, with an update in the epilogue for some groups,
+    groups without tokens and a group whose k-blocks do not fill the last one."""
+    from moonep_b200.ops import grouped_gemm as gg
+    n, M, N = [128, 0, 384, 256, 0], 512, 256
+    cu = torch.tensor(n).cumsum(0).to(torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, dy = ((torch.randn(sum(n), c, device="cuda", generator=g)).to(torch.bfloat16) for c in (M, 2 * N))
+    mask = None if accumulate else torch.tensor([1, 1, 0, 1, 0], dtype=torch.int32, device="cuda")
+    w0 = [(torch.randn(len(n), M, N, device="cuda", generator=g)).to(torch.bfloat16) for _ in range(2)]
+    runs = []
+    for together in (False, True):
+        out, w = [torch.full((len(n), M, N), 7.0, device="cuda") for _ in range(2)], [t.clone() for t in w0]
+        up = lambda i: None if accumulate else (w[i], 0.1, mask)     # noqa: E731
+        kw = dict(accumulate=accumulate, zero_empty_below=4)
+        if together:
+            gg.wgrad(x, dy, cu, out[0], update=up(0), out_b=out[1], update_b=None if accumulate else w[1], **kw)
+        else:
+            gg.wgrad(x, dy[:, :N], cu, out[0], update=up(0), **kw)
+            gg.wgrad(x, dy[:, N:], cu, out[1], update=up(1), **kw)
+        torch.cuda.synchronize()
+        gg.check_status()
+        runs.append(out + w)
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("blocks", [None, 1, 5])
 def test_sgd_at_the_edges_of_its_chunks(blocks, cuda_device):
     """Chunks are 8192 parameters. One rounding to fp32 and one to bf16: what double precision gives for a rate with few bits."""
