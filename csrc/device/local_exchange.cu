@@ -32,6 +32,14 @@ constexpr int kLocMaxSlots = 8;            // row slots per copying warp
 // The two cross between 24576 and 32768 for short rows and between 16384 and 28672 for long ones, whatever E is.
 constexpr int kLocDirect = 24576;
 
+// A large batch of a saved plan is copied by many short CTAs, two or three to an SM, that the hardware hands out as SMs come free: SMs
+// are not equally far from memory, and with one CTA for each the last was done 10 % after the average. Bytes that a CTA moves, times
+// 148, and least bytes of a large batch. One CTA per SM against short ones, in us: S=4096, H=7168, K=8 101.6 / 89.2; 8192, 7168, 4 109.2 /
+// 95.4; 8192, 2048, 8 58.8 / 53.8. Below 200 MB the gain is gone in a combine right behind, whose rows were in L2 (3001, 4096, 6 with its
+// combine 65.8 / 66.9). Not for a fresh plan: planners and copiers in one launch hand over in 10 us, which only the largest
+// batches win back (4096, 7168, 8 107.6 / 103.4; 1531, 7168, 8 48.1 / 55).
+constexpr long long kLocShort = 45ll << 20, kLocLarge = 200ll << 20;
+
 // Padding rows that are cleared behind row `first` of a group's `n` (see LocalDispatchArgs.pad_step).
 __device__ __forceinline__ int local_pads(int first, int n, int step) { return step ? min(n, -first & (step - 1)) : n; }
 
@@ -69,7 +77,7 @@ __device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, 
 // Bound by HBM: (1 + K) rows per token; 106 us at S=4096, H=7168, K=8 (5.0 TB/s, mostly stores) where planning, dispatch
 // and duplicate expansion took 185.
 template <int MODE>                        // 0: saved plan
-__global__ void __launch_bounds__(kLocThreads, 1)
+__global__ void __launch_bounds__(kLocThreads, MODE ? 1 : 3)
 local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, int copy_warps, int slots) {
   constexpr bool FRESH = MODE != 0, SHARED = MODE == 2;
   pdl_trigger();                             // a GEMM behind this kernel may set itself up meanwhile
@@ -337,12 +345,14 @@ __device__ __forceinline__ void add_bf16x8(float* acc, const int4& x) {
 // out[s] = sum over k, ascending, of the rows of token s, in fp32, rounded once: what the duplicate reduction
 // followed by the combine computes, without the intermediate row. A warp works on (token, column part) units: one
 // bulk load per row brings a unit into one half of the warp's stage while the other half is summed, and the plan
-// entries of the unit behind that one are already being fetched.
+// entries of the unit behind that one are already being fetched. `last_first`: units come from the last to the
+// first. Where nothing has touched the rows of a large batch since its dispatch, which goes through the tokens in order, the last
+// ones are still in L2: saved dispatch and combine of S=4096, H=7168, K=8 187.8 -> 182.3 us.
 // Bound by HBM: (K + 1) rows per token. Loading into registers instead kept too little in flight: 138 us at
 // S=4096, H=7168, K=8 with 32 warps per SM and 218 us with 8 (twice the loads per lane).
 constexpr int kLcWarps = 12, kLcHalf = 8192;
 
-__global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts) {
+__global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts, int last_first) {
   pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLcWarps * 2];
@@ -357,9 +367,11 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   uint64_t* bars = s_bar + warp * 2;
   const int units = cp->S * nparts, step = gridDim.x * kLcWarps;
   int u = blockIdx.x * kLcWarps + warp;
-  auto fetch = [&](int x) { return x < units && lane < K ? __ldg(a.dst + (size_t)(x / nparts) * K + lane) : 0; };
+  auto unit = [&](int x) { return last_first ? units - 1 - x : x; };
+  auto fetch = [&](int x) { return x < units && lane < K ? __ldg(a.dst + (size_t)(unit(x) / nparts) * K + lane) : 0; };
   // loads of unit x (plan entry d in lane k) into half h; returns the lanes whose entry names a row
-  auto issue = [&](int x, int d, int h) {
+  auto issue = [&](int at, int d, int h) {
+    const int x = unit(at);
     const int part = x % nparts, vb = part * part_vecs;
     const uint32_t bytes = (uint32_t)min(part_vecs, nvec - vb) * 16u;
     const int row = d >= 0 ? d : -d - 1;
@@ -382,11 +394,12 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
     const int un = u + step;
     if (un < units) nxt = issue(un, dn, h ^ 1);
     dn = fetch(un + step);
-    if (cur != all) bad = u / nparts;
+    const int x = unit(u);
+    if (cur != all) bad = x / nparts;
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[h], phase, budget))) { ok = false; break; }
-    const int part = u % nparts, vb = part * part_vecs, n = min(part_vecs, nvec - vb);
+    const int part = x % nparts, vb = part * part_vecs, n = min(part_vecs, nvec - vb);
     const unsigned char* base = stage + (size_t)h * kLcHalf;
-    int4* orow = reinterpret_cast<int4*>(a.out) + (size_t)(u / nparts) * nvec + vb;
+    int4* orow = reinterpret_cast<int4*>(a.out) + (size_t)(x / nparts) * nvec + vb;
     for (int v = lane; v < n; v += 32) {
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
@@ -418,14 +431,21 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
   using namespace mep;
   const size_t row = (size_t)H * 2;
   const size_t tables = (size_t)(fresh ? 3 : 4) * E * sizeof(int);
-  const size_t budget = 208 * 1024;
+  const long long bytes = (long long)S * (K + 1) * (long long)row;
+  const bool large = !fresh && bytes >= kLocLarge && tables + kLocZeroBytes + 2 * row <= 104 * 1024;
+  const size_t budget = (large ? 104 : 208) * 1024, ring = (large ? 52 : 96) * 1024;
   MEP_REQUIRE(tables + kLocZeroBytes + 2 * row <= budget, "dispatch: H=%d rows (%zu B) with E=%d do not fit shared memory", H, row, E);
   const int all = (int)((budget - tables - kLocZeroBytes) / row);           // row slots that fit
   int warps = all / 2 < kLocWarps ? all / 2 : kLocWarps;
   int slots = all / warps < kLocMaxSlots ? all / warps : kLocMaxSlots;
-  // the fewest slots that still hold 96 KB of rows per SM: more buys nothing, and a smaller footprint starts sooner
-  while (slots > 2 && (size_t)warps * (slots - 1) * row >= 96 * 1024) --slots;
+  // the fewest slots that still hold `ring` bytes of rows per CTA: more buys nothing, and a smaller footprint starts sooner
+  while (slots > 2 && (size_t)warps * (slots - 1) * row >= ring) --slots;
   const size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
+  if (large) {                               // the same number of tokens for each warp
+    const long long each = kLocShort / 148 / ((long long)row * (K + 1) * warps);
+    const int tokens = warps * (each < 1 ? 1 : (int)each);
+    num_blocks = (S + tokens - 1) / tokens;
+  }
   if (fresh && S * K <= kLocDirect) return launch_plain(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
   if (fresh) return launch_plain(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
   return launch_plain(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
@@ -444,5 +464,5 @@ extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalC
   MEP_REQUIRE((long long)S * nparts < (1ll << 30), "combine: S=%d, H=%d is too large", S, H);
   const int grid = (int)(((long long)S * nparts + kLcWarps - 1) / kLcWarps);
   return launch_plain_pdl(local_combine_kernel, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
-                          stream, pdl != 0, ctx, *args, part, nparts);
+                          stream, pdl != 0, ctx, *args, part, nparts, (long long)S * (K + 1) * H * 2 >= kLocLarge ? 1 : 0);
 }

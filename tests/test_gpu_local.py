@@ -135,3 +135,18 @@ def test_padding_rows_are_counted(cuda_device):
         blk.forward(y)
     assert blk.buf.counters()["padding_rows_cleared"] == int((-tpe % 32).sum())
     blk.destroy()
+
+
+# Large batches (200 MiB moved): the saved plan's rows come from many short CTAs and the combine begins with the last tokens. Just above
+# the line with fresh plans on both sides of the hand-over, one entry per token, fewer tokens than CTAs with rows of which three fit.
+LARGE_CASES = [
+    (2048, 8,  48,   5696,  16,  "random"),
+    (5003, 5,  40,   3496,  128, "biased"),
+    (9600, 1,  7,    5464,  1,   "random"),
+    (200,  32, 64,   15904, 16,  "random"),
+]
+
+
+@pytest.mark.parametrize("case", LARGE_CASES, ids=lambda c: "S%d_K%d_E%d_H%d" % c[:4])
+def test_local_exchange_of_large_batches(case, cuda_device):
+    test_local_exchange(case, cuda_device)
