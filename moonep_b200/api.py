@@ -293,14 +293,10 @@ class OpsMixin:
 
     def _combine_local(self, plan, h, w):
         """Single rank: nobody else reads this shard, so the rows are summed where they are (no staging, no pre-reduction)."""
-        st, g = self._states[0], self.geo
         self._check_plan(plan)
         if h.data_ptr() % 16:        # the kernel's bulk loads start on 16-byte boundaries
             h = h.clone()
-        out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=st.device)
-        ow = None if w is None else torch.empty((g.S, g.K), dtype=torch.float32, device=st.device)
-        self._local_exchange().combine(plan, h, w, out, ow)
-        return out, ow
+        return self._local_exchange().combine(plan, h, w)
 
     def _combine_lists(self, plans, hidden_nvsh, weights_nvs, *, inter_rank_sync, zero_copy, w_zero_copy):
         st = self._states

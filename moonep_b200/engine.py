@@ -240,26 +240,29 @@ class LocalExchange:
         a.blocks, a.combine_blocks = min(blocks, st.local_blocks), blocks
         _, self._total, first = _plan_layout(st)
         a.plan_off = (C.c_int64 * 8)(*first)
-        self._cu_first, self._cu_n = first[7], 2 * g.epn
+        self._cu_first, self._cu_shape = first[7], (2 * g.epn,)
         a.shard, a.shard_w, a.srcinfo = st.hidden_local.data_ptr(), st.weights_local.data_ptr(), ptr(st.srcinfo_local)
         a.sync, a.hist = st.scratch["loc_sync"].data_ptr(), st.scratch["loc_hist"].data_ptr()
-        self._geo, self._args, self._ref, self._dev = g, a, C.addressof(a), st.device
+        self._args, self._ref, self._dev = a, C.addressof(a), st.device
         self._ints = dict(N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K)
-        self._fields = dict(dst=(first[0], g.N, None), experts_to_copy=(first[1], g.epn, (1, g.epn)),
-                            zero_fill_ranges=(first[2], 4 * g.epn, (2 * g.epn, 2)), remote_stats=(first[3], 2, None),
-                            dup_groups=(first[4], 3 * g.NvS, (g.NvS, 3)), dup_loffs=(first[5], g.NvS, None), dup_counts=(first[6], 2, None))
+        # shape, strides and first element of each part: one as_strided call costs a third of narrow and view
+        self._fields = dict(dst=((g.N,), (1,), first[0]), experts_to_copy=((1, g.epn), (g.epn, 1), first[1]),
+                            zero_fill_ranges=((2 * g.epn, 2), (2, 1), first[2]), remote_stats=((2,), (1,), first[3]),
+                            dup_groups=((g.NvS, 3), (3, 1), first[4]), dup_loffs=((g.NvS,), (1,), first[5]), dup_counts=((2,), (1,), first[6]))
+        # what results are made like: half the cost of a size, a type and a device
+        self._rows_like = st.hidden_local.narrow(0, 0, g.S)
+        self._weights_like = st.weights_local.as_strided((g.S, g.K), (g.K, 1))
         self._lib = _native.load()
 
     def _name_part(self, slab, name):
         f = self._fields.get(name)
         if f is None:
             return None
-        v = slab.narrow(0, f[0], f[1])
-        return v if f[2] is None else v.view(f[2])
+        return slab.as_strided(*f)
 
     def plan_of(self, slab):
         """``(plan, cu_seqlens)`` of an allocation that a native call has planned into."""
-        return MoonEPCommPlan.of_slab(slab, self._name_part, self._ints), slab.narrow(0, self._cu_first, self._cu_n)
+        return MoonEPCommPlan.of_slab(slab, self._name_part, self._ints), slab.as_strided(self._cu_shape, (1,), self._cu_first)
 
     def dispatch(self, hidden, route_w, topk, tpe, out_hidden, out_w):
         """A fresh plan (in one allocation: what a small dispatch would otherwise wait for) and the K rows of every
@@ -285,12 +288,16 @@ class LocalExchange:
         slab = plan.__dict__.get("_slab")
         return plan.dst.data_ptr() if slab is None else slab.data_ptr()
 
-    def combine(self, plan, rows, row_w, out, out_w):
-        """``out[s]`` = sum of the K rows of token ``s``; ``rows`` / ``row_w`` are any tensors of the shard's shape and only read."""
+    def combine(self, plan, rows, row_w):
+        """``(out, out_w)``: ``out[s]`` = sum of the K rows of token ``s``; ``rows`` / ``row_w`` are any tensors of the shard's shape and only
+        read."""
+        out = torch.empty_like(self._rows_like)
+        out_w = None if row_w is None else torch.empty_like(self._weights_like)
         rc = self._lib.mep_local_combine_call(self._ref, self._dst(plan), rows.data_ptr(), None if row_w is None else row_w.data_ptr(),
                                               out.data_ptr(), None if out_w is None else out_w.data_ptr(), _native.raw_stream())
         if rc:
             _native.check(rc, "combine")
+        return out, out_w
 
 
 class LocalLayer(LocalExchange):
@@ -316,10 +323,9 @@ class LocalLayer(LocalExchange):
 
     def forward(self, hidden, route_w, topk, tpe, keep: bool, weights, pdl: bool):
         """Returns ``(out, plan allocation)``."""
-        g = self._geo
         self._set(weights, self._grads, pdl)
         slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
-        out = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
+        out = torch.empty_like(self._rows_like)
         rc = self._lib.mep_moe_local_forward(self._ref, hidden.data_ptr(), route_w.data_ptr(), topk.data_ptr(), tpe.data_ptr(),
                                              slab.data_ptr(), out.data_ptr(), 1 if keep else 0, _native.raw_stream())
         if rc:
@@ -327,10 +333,8 @@ class LocalLayer(LocalExchange):
         return out, slab
 
     def backward(self, dy, slab, accumulate: bool, lr: float, mask, weights, grads, pdl: bool):
-        g = self._geo
         self._set(weights, grads, pdl)
-        dx = torch.empty((g.S, g.H), dtype=torch.bfloat16, device=self._dev)
-        dw = torch.empty((g.S, g.K), dtype=torch.float32, device=self._dev)
+        dx, dw = torch.empty_like(self._rows_like), torch.empty_like(self._weights_like)
         rc = self._lib.mep_moe_local_backward(self._ref, dy.data_ptr(), slab.data_ptr(), dx.data_ptr(), dw.data_ptr(),
                                               1 if accumulate else 0, lr, ptr(mask), _native.raw_stream())
         if rc:
