@@ -77,12 +77,12 @@ __device__ __forceinline__ void group_rows(const GemmArgs& args, int* scratch, i
       const int4 v = *reinterpret_cast<const int4*>(scratch + j);
       beg += (j < g ? v.x : 0) + (j + 1 < g ? v.y : 0) + (j + 2 < g ? v.z : 0) + (j + 3 < g ? v.w : 0);
     }
-    units = (n + 31) >> 5;
+    units = max((n + 31) >> 5, 0);
     __syncthreads();                     // before the scratch is used for something else
   } else if (g < G) {
     beg = g ? args.cu_seqlens[g - 1] : 0;
     rows = args.cu_seqlens[g] - beg;
-    units = (rows - (args.pad_rows ? args.pad_rows[2 * g + 1] : 0) + 31) >> 5;
+    units = max((rows - (args.pad_rows ? args.pad_rows[2 * g + 1] : 0) + 31) >> 5, 0);
   }
 }
 // one lane of a converged warp; the others' registers stay warp-uniform, which keeps MMA descriptors out of the vector registers

@@ -73,16 +73,19 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 // A block's loads of a chunk are all in flight before the first is used, and by default a block has one chunk: short blocks
 // that the hardware hands out even out the SMs' unequal distance from memory. 3 x 705 M parameters: 2324 us (7.28 TB/s), where
 // 1184 blocks in a loop of single vectors took 2496; 3 x 34 M: 115 against 130. Two chunks a block take 2400, loads that are
-// marked as streaming 2480.
-constexpr int kSgdVecs = 4, kSgdChunk = 256 * kSgdVecs;      // vectors of eight parameters
+// marked as streaming 2480. Callers that name a number of blocks run beside a GEMM: single vectors in a loop need 32 registers
+// instead of 72 and find room next to its CTAs.
+constexpr int kSgdVecs = 4;                                  // vectors of eight parameters
 
+template <int VECS>
 __device__ __forceinline__ void sgd_range(__nv_bfloat16* __restrict__ p, const float* __restrict__ g, float lr, int64_t n8) {
+  constexpr int kSgdChunk = 256 * VECS;
   const int64_t chunks = (n8 + kSgdChunk - 1) / kSgdChunk;
   for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
     const int64_t base = c * kSgdChunk + threadIdx.x;
-    int4 x[kSgdVecs]; float4 g0[kSgdVecs], g1[kSgdVecs];
+    int4 x[VECS]; float4 g0[VECS], g1[VECS];
 #pragma unroll
-    for (int u = 0; u < kSgdVecs; ++u) {
+    for (int u = 0; u < VECS; ++u) {
       const int64_t i = base + u * 256;
       if (i < n8) {
         x[u] = *reinterpret_cast<const int4*>(p + i * 8);
@@ -90,7 +93,7 @@ __device__ __forceinline__ void sgd_range(__nv_bfloat16* __restrict__ p, const f
       }
     }
 #pragma unroll
-    for (int u = 0; u < kSgdVecs; ++u) {
+    for (int u = 0; u < VECS; ++u) {
       const int64_t i = base + u * 256;
       if (i >= n8) break;
       __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&x[u]);
@@ -106,18 +109,19 @@ __device__ __forceinline__ void sgd_range(__nv_bfloat16* __restrict__ p, const f
   }
 }
 
-__global__ void __launch_bounds__(256) sgd_kernel(__nv_bfloat16* p, const float* g, float lr, int64_t n8) { sgd_range(p, g, lr, n8); }
+template <int VECS> __global__ void __launch_bounds__(256) sgd_kernel(__nv_bfloat16* p, const float* g, float lr, int64_t n8) { sgd_range<VECS>(p, g, lr, n8); }
 
 struct SgdPack { __nv_bfloat16* p[4]; const float* g[4]; int64_t n8[4]; };
-__global__ void __launch_bounds__(256) sgd_many_kernel(SgdPack k, float lr) { sgd_range(k.p[blockIdx.y], k.g[blockIdx.y], lr, k.n8[blockIdx.y]); }
+template <int VECS> __global__ void __launch_bounds__(256) sgd_many_kernel(SgdPack k, float lr) { sgd_range<VECS>(k.p[blockIdx.y], k.g[blockIdx.y], lr, k.n8[blockIdx.y]); }
 
 // The same update for the groups of a [G, n] tensor whose mask word is zero (`want` = 0) or non-zero (1):
 // used for the experts that the weight-gradient GEMM did not already update in its epilogue.
+template <int VECS>
 __global__ void __launch_bounds__(256) sgd_groups_kernel(__nv_bfloat16* __restrict__ p, const float* __restrict__ g, float lr,
                                                          int64_t n8, const int32_t* __restrict__ mask, int want) {
   const int grp = blockIdx.y;
   if ((mask[grp] != 0) != (want != 0)) return;
-  sgd_range(p + (int64_t)grp * n8 * 8, g + (int64_t)grp * n8 * 8, lr, n8);
+  sgd_range<VECS>(p + (int64_t)grp * n8 * 8, g + (int64_t)grp * n8 * 8, lr, n8);
 }
 
 // For tests: compares the branch-free forms with the division for the `n` floats whose bits start at `first`;
@@ -146,12 +150,12 @@ extern "C" int mep_swiglu_bwd(const void* dA, const void* gu, const float* w, vo
 }
 
 // `num_blocks` of the three: blocks of a tensor or group, 0: one for each chunk.
-static int sgd_blocks(int num_blocks, int64_t n) { return num_blocks > 0 ? num_blocks : (int)((n / 8 + mep::kSgdChunk - 1) / mep::kSgdChunk); }
+static int sgd_blocks(int num_blocks, int64_t n) { return num_blocks > 0 ? num_blocks : (int)((n / 8 + 256 * mep::kSgdVecs - 1) / (256 * mep::kSgdVecs)); }
 
 extern "C" int mep_sgd_step(void* p, const float* g, float lr, int64_t n, int num_blocks, cudaStream_t stream) {
   MEP_REQUIRE(n % 8 == 0, "sgd_step: element count must be a multiple of 8");
   if (n == 0) return 0;
-  return mep::launch_plain(mep::sgd_kernel, dim3(sgd_blocks(num_blocks, n)), dim3(256), 0, stream, (__nv_bfloat16*)p, g, lr, n / 8);
+  return mep::launch_plain(num_blocks > 0 ? mep::sgd_kernel<1> : mep::sgd_kernel<mep::kSgdVecs>, dim3(sgd_blocks(num_blocks, n)), dim3(256), 0, stream, (__nv_bfloat16*)p, g, lr, n / 8);
 }
 
 // sgd_step of up to four tensors in one launch.
@@ -165,13 +169,13 @@ extern "C" int mep_sgd_step_many(int count, void* const* p, const float* const* 
     if (n[i] > most) most = n[i];
   }
   if (most == 0) return 0;
-  return mep::launch_plain(mep::sgd_many_kernel, dim3(sgd_blocks(num_blocks, most), count), dim3(256), 0, stream, k, lr);
+  return mep::launch_plain(num_blocks > 0 ? mep::sgd_many_kernel<1> : mep::sgd_many_kernel<mep::kSgdVecs>, dim3(sgd_blocks(num_blocks, most), count), dim3(256), 0, stream, k, lr);
 }
 
 extern "C" int mep_sgd_step_groups(void* p, const float* g, float lr, int64_t n_per_group, int G, const int32_t* mask, int want,
                                    int num_blocks, cudaStream_t stream) {
   MEP_REQUIRE(n_per_group % 8 == 0 && G >= 1 && G <= 65535, "sgd_step_groups: %d groups of %lld elements", G, (long long)n_per_group);
   if (n_per_group == 0) return 0;
-  return mep::launch_plain(mep::sgd_groups_kernel, dim3(sgd_blocks(num_blocks, n_per_group), G), dim3(256), 0, stream, (__nv_bfloat16*)p, g, lr,
+  return mep::launch_plain(num_blocks > 0 ? mep::sgd_groups_kernel<1> : mep::sgd_groups_kernel<mep::kSgdVecs>, dim3(sgd_blocks(num_blocks, n_per_group), G), dim3(256), 0, stream, (__nv_bfloat16*)p, g, lr,
                            n_per_group / 8, mask, want);
 }

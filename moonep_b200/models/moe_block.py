@@ -220,12 +220,13 @@ class MoEBlock:
         if lr is None:
             moe.on_grad_ready = None
         elif moe.epilogue_lr is None:
-            moe.on_grad_ready = lambda n: gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr)
+            beside = 8 * moe._total_sms             # blocks that find room next to the GEMMs on the other streams
+            moe.on_grad_ready = lambda n: gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr, num_blocks=beside)
         elif self.world == 1:
             moe.on_grad_ready = no_update           # no replicas: the epilogues have updated every expert
         else:
             moe.on_grad_ready = lambda n: gg.sgd_step_groups(self.pools.local_weight(n), self.pools.local_grad(n), lr,
-                                                             moe._upd_mask, want=False)
+                                                             moe._upd_mask, want=False, num_blocks=2 * moe._total_sms)
 
     def sgd_step(self, lr: float):
         if self.moe.on_grad_ready is None:

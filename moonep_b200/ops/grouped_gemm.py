@@ -361,7 +361,8 @@ def swiglu_bwd(dA, gu, w, dgu, dw, cu, num_blocks=None):
 
 
 def sgd_step_groups(p, g, lr, mask, want: bool, num_blocks=None):
-    """``sgd_step`` for the groups ``i`` of ``p [G, ...]`` with ``(mask[i] != 0) == want`` only (``mask``: int32
+    """``num_blocks`` (of a group here, of a tensor below): blocks that share an SM with a GEMM; by default many short ones that
+    want the GPU to themselves.  ``sgd_step`` for the groups ``i`` of ``p [G, ...]`` with ``(mask[i] != 0) == want`` only (``mask``: int32
     ``[>= G]`` on the device): the complement of what ``wgrad(update=...)`` has already updated."""
     lib = _native.load()
     assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.shape == g.shape
