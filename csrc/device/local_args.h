@@ -59,7 +59,8 @@ struct MoeLocal {
   int32_t* status;
   int32_t* status_host;
   uint64_t budget_ns;
-  int32_t token_padding, reserved;
+  int32_t token_padding;
+  int32_t last_first;            // combine call: the rows were dispatched in the order of the tokens (see local_combine_kernel)
 };
 
 }  // namespace mep

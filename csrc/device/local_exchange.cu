@@ -345,14 +345,15 @@ __device__ __forceinline__ void add_bf16x8(float* acc, const int4& x) {
 // out[s] = sum over k, ascending, of the rows of token s, in fp32, rounded once: what the duplicate reduction
 // followed by the combine computes, without the intermediate row. A warp works on (token, column part) units: one
 // bulk load per row brings a unit into one half of the warp's stage while the other half is summed, and the plan
-// entries of the unit behind that one are already being fetched. `last_first`: units come from the last to the
-// first. Where nothing has touched the rows of a large batch since its dispatch, which goes through the tokens in order, the last
-// ones are still in L2: saved dispatch and combine of S=4096, H=7168, K=8 187.8 -> 182.3 us.
+// entries of the unit behind that one are already being fetched. LAST_FIRST: units come from the last to the
+// first. Where nothing has touched the rows of a large batch since a saved plan's dispatch, which goes through the tokens in order,
+// the last ones are still in L2 (behind a fresh plan, whose CTAs have a range of tokens each, it costs 0.6 %): saved dispatch and combine of S=4096, H=7168, K=8 187.8 -> 182.3 us.
 // Bound by HBM: (K + 1) rows per token. Loading into registers instead kept too little in flight: 138 us at
 // S=4096, H=7168, K=8 with 32 warps per SM and 218 us with 8 (twice the loads per lane).
 constexpr int kLcWarps = 12, kLcHalf = 8192;
 
-__global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts, int last_first) {
+template <bool LAST_FIRST>
+__global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts) {
   pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLcWarps * 2];
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   uint64_t* bars = s_bar + warp * 2;
   const int units = cp->S * nparts, step = gridDim.x * kLcWarps;
   int u = blockIdx.x * kLcWarps + warp;
-  auto unit = [&](int x) { return last_first ? units - 1 - x : x; };
+  auto unit = [&](int x) { return LAST_FIRST ? units - 1 - x : x; };
   auto fetch = [&](int x) { return x < units && lane < K ? __ldg(a.dst + (size_t)(unit(x) / nparts) * K + lane) : 0; };
   // loads of unit x (plan entry d in lane k) into half h; returns the lanes whose entry names a row
   auto issue = [&](int at, int d, int h) {
@@ -452,7 +453,7 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
 }
 
 extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalCombineArgs* args, int num_blocks,
-                                        int S, int H, int K, int pdl, cudaStream_t stream) {
+                                        int S, int H, int K, int pdl, int last_first, cudaStream_t stream) {
   using namespace mep;
   const int nvec = H / 8;
   // a unit is what fits half a warp's stage, or less while that leaves warps without work
@@ -463,6 +464,7 @@ extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalC
   const int nparts = (nvec + part - 1) / part;
   MEP_REQUIRE((long long)S * nparts < (1ll << 30), "combine: S=%d, H=%d is too large", S, H);
   const int grid = (int)(((long long)S * nparts + kLcWarps - 1) / kLcWarps);
-  return launch_plain_pdl(local_combine_kernel, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
-                          stream, pdl != 0, ctx, *args, part, nparts, (long long)S * (K + 1) * H * 2 >= kLocLarge ? 1 : 0);
+  const bool last = last_first && (long long)S * (K + 1) * H * 2 >= kLocLarge;
+  return launch_plain_pdl(last ? local_combine_kernel<true> : local_combine_kernel<false>, dim3(grid < num_blocks ? grid : num_blocks), dim3(kLcWarps * 32), (size_t)kLcWarps * 2 * kLcHalf,
+                          stream, pdl != 0, ctx, *args, part, nparts);
 }

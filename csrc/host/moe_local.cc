@@ -6,7 +6,7 @@
 
 extern "C" {
 int mep_launch_local_dispatch(const MepRankCtx*, const mep::LocalDispatchArgs*, int, int, int, int, int, int, cudaStream_t);
-int mep_launch_local_combine(const MepRankCtx*, const mep::LocalCombineArgs*, int, int, int, int, int, cudaStream_t);
+int mep_launch_local_combine(const MepRankCtx*, const mep::LocalCombineArgs*, int, int, int, int, int, int, cudaStream_t);
 int mep_grouped_gemm_2cta(int, const void*, int64_t, int64_t, int64_t, const void*, const void*, int64_t, int64_t, int64_t,
                           const mep::GemmArgs*, int, cudaStream_t);
 int mep_grouped_wgrad_2cta(const void*, int64_t, int64_t, const void*, int64_t, const mep::GemmArgs*, int, cudaStream_t);
@@ -74,7 +74,7 @@ extern "C" int mep_local_combine_call(const mep::MoeLocal* mp, const int32_t* ds
   using namespace mep;
   const MoeLocal& m = *mp;
   LocalCombineArgs c = {dst, (const __nv_bfloat16*)rows, row_w, (__nv_bfloat16*)out, out_w};
-  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 0, stream);
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 0, m.last_first, stream);
 }
 
 extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden, const float* route_w, const int32_t* topk,
@@ -94,7 +94,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   g.N = m.H; g.K = m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DOWN, m.act, m.Hp, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, nullptr, (__nv_bfloat16*)out, nullptr};
-  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, stream);
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, 0, stream);
 }
 
 // `update`: lr and the group mask of the update in the weight-gradient epilogues, or mask = null (gradients are stored).
@@ -122,7 +122,7 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   g.N = m.H; g.K = 2 * m.Hp; g.out = m.shard; g.ldo = m.H;
   if (gemm(m, GEMM_DGRAD_GU, m.dgu, 2 * (int64_t)m.Hp, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
   LocalCombineArgs c = {slab + m.plan_off[0], m.shard, m.shard_w, (__nv_bfloat16*)dx, d_route_w};
-  if (mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, stream)) return -1;
+  if (mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, 0, stream)) return -1;
   // Gate and up in one launch: x is read from DRAM once and there is one ramp and one last round. 16 groups of 4096 tokens, 2048 x 768: 323 -> 307 us
   // (with the update 318 -> 302); 24 of 700, 1792 x 1280: 196 -> 181; 16 of 300, 1024 x 512: 44 -> 30. An update of their weights has to wait for dgrad(gate/up), which reads them.
   return wgrad(m.x, m.H, m.dgu, 2 * (int64_t)m.Hp, m.Hp, m.dw_gate, m.w_gate, m.dw_up, m.w_up);
