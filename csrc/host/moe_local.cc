@@ -1,5 +1,5 @@
-// Forward and backward pass of a single-rank MoE layer, each one call: the same launches, in the same order, as
-// moonep_b200/moe_layer.py issues one by one (about 15 us of Python each), for callers without hooks between them.
+// Forward and backward pass of a single-rank MoE layer, each one call: the launches that moonep_b200/moe_layer.py issues one by
+// one (about 15 us of Python each), with the weight gradients of gate and up as the last one, for callers without hooks between them.
 #include "../device/gemm_args.h"
 #include "../device/local_args.h"
 #include "launch.h"
