@@ -33,12 +33,12 @@ constexpr int kLocMaxSlots = 8;            // row slots per copying warp
 constexpr int kLocDirect = 24576;
 
 // A large batch of a saved plan is copied by many short CTAs, two or three to an SM, that the hardware hands out as SMs come free: SMs
-// are not equally far from memory, and with one CTA for each the last was done 10 % after the average. Bytes that a CTA moves, times
-// 148, and least bytes of a large batch. One CTA per SM against short ones, in us: S=4096, H=7168, K=8 101.6 / 89.2; 8192, 7168, 4 109.2 /
+// are not equally far from memory, and with one CTA for each the last was done 10 % after the average. Bytes that a CTA moves, and
+// least bytes of a large batch; a caller that wants fewer CTAs than there are SMs gets its number instead. One CTA per SM against short ones, in us: S=4096, H=7168, K=8 101.6 / 89.2; 8192, 7168, 4 109.2 /
 // 95.4; 8192, 2048, 8 58.8 / 53.8. Below 200 MB the gain is gone in a combine right behind, whose rows were in L2 (3001, 4096, 6 with its
 // combine 65.8 / 66.9). Not for a fresh plan: planners and copiers in one launch hand over in 10 us, which only the largest
 // batches win back (4096, 7168, 8 107.6 / 103.4; 1531, 7168, 8 48.1 / 55).
-constexpr long long kLocShort = 45ll << 20, kLocLarge = 200ll << 20;
+constexpr long long kLocShort = 311ll << 10, kLocLarge = 200ll << 20;
 
 // Padding rows that are cleared behind row `first` of a group's `n` (see LocalDispatchArgs.pad_step).
 __device__ __forceinline__ int local_pads(int first, int n, int step) { return step ? min(n, -first & (step - 1)) : n; }
@@ -426,14 +426,15 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
 
 }  // namespace mep
 
-// `num_blocks`: CTAs (one per SM). fresh: plan from topk / tpe as well; else a.dst / a.zero_fill are read.
+// `num_blocks`: most CTAs; from `sms` on (those of the device, with a CTA for each) the launch may have more, see kLocShort. fresh: plan from
+// topk / tpe as well; else a.dst / a.zero_fill are read.
 extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::LocalDispatchArgs* args, int fresh,
-                                         int num_blocks, int S, int K, int H, int E, cudaStream_t stream) {
+                                         int num_blocks, int sms, int S, int K, int H, int E, cudaStream_t stream) {
   using namespace mep;
   const size_t row = (size_t)H * 2;
   const size_t tables = (size_t)(fresh ? 3 : 4) * E * sizeof(int);
   const long long bytes = (long long)S * (K + 1) * (long long)row;
-  const bool large = !fresh && bytes >= kLocLarge && tables + kLocZeroBytes + 2 * row <= 104 * 1024;
+  const bool large = !fresh && num_blocks >= sms && bytes >= kLocLarge && tables + kLocZeroBytes + 2 * row <= 104 * 1024;
   const size_t budget = (large ? 104 : 208) * 1024, ring = (large ? 52 : 96) * 1024;
   MEP_REQUIRE(tables + kLocZeroBytes + 2 * row <= budget, "dispatch: H=%d rows (%zu B) with E=%d do not fit shared memory", H, row, E);
   const int all = (int)((budget - tables - kLocZeroBytes) / row);           // row slots that fit
@@ -443,7 +444,7 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
   while (slots > 2 && (size_t)warps * (slots - 1) * row >= ring) --slots;
   const size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
   if (large) {                               // the same number of tokens for each warp
-    const long long each = kLocShort / 148 / ((long long)row * (K + 1) * warps);
+    const long long each = kLocShort / ((long long)row * (K + 1) * warps);
     const int tokens = warps * (each < 1 ? 1 : (int)each);
     num_blocks = (S + tokens - 1) / tokens;
   }

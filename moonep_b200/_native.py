@@ -72,7 +72,7 @@ class MoeLocal(C.Structure):
                 + [("plan_off", C.c_int64 * 8)]
                 + [(n, C.c_void_p) for n in ("w_gate", "w_up", "w_down", "shard", "shard_w", "srcinfo", "x", "w", "act", "gu", "dA",
                                              "dgu", "dw_gate", "dw_up", "dw_down", "sync", "hist", "status", "status_host")]
-                + [("budget_ns", C.c_uint64), ("token_padding", C.c_int32), ("last_first", C.c_int32)])
+                + [("budget_ns", C.c_uint64), ("token_padding", C.c_int32), ("sms", C.c_int32), ("last_first", C.c_int32)])
 
 
 class SendOrderArgs(C.Structure):

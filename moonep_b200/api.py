@@ -59,7 +59,8 @@ def validate_num_sms(num_sms, max_sms_fn):
 
 
 def num_sms_dedup_from_env(max_sms: int) -> int:
-    """``MOONEP_NUM_SMS_DEDUP``: CTA count of the two local duplicate kernels (default all SMs)."""
+    """``MOONEP_NUM_SMS_DEDUP``: most CTAs of the two local duplicate kernels, and of dispatch and combine of a group of one rank
+    (default all SMs; only then may a large dispatch of a saved plan have more, short ones)."""
     raw = os.environ.get("MOONEP_NUM_SMS_DEDUP")
     if raw is None or raw == "":
         return max_sms

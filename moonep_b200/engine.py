@@ -237,7 +237,7 @@ class LocalExchange:
         g, a = st.geo, _native.MoeLocal()
         a.ctx = st.ctx_ptr
         a.S, a.H, a.K, a.E, a.NvS, a.token_padding = g.S, g.H, g.K, g.E, g.NvS, g.token_padding
-        a.blocks, a.combine_blocks = min(blocks, st.local_blocks), blocks
+        a.blocks, a.combine_blocks, a.sms = min(blocks, st.local_blocks), blocks, st.local_blocks
         _, self._total, first = _plan_layout(st)
         a.plan_off = (C.c_int64 * 8)(*first)
         self._cu_first, self._cu_shape = first[7], (2 * g.epn,)

@@ -150,3 +150,25 @@ LARGE_CASES = [
 @pytest.mark.parametrize("case", LARGE_CASES, ids=lambda c: "S%d_K%d_E%d_H%d" % c[:4])
 def test_local_exchange_of_large_batches(case, cuda_device):
     test_local_exchange(case, cuda_device)
+
+
+@pytest.mark.parametrize("limit", [None, 12])
+def test_saved_plan_of_a_large_batch_keeps_to_the_sm_limit(limit, cuda_device, monkeypatch):
+    """``MOONEP_NUM_SMS_DEDUP`` bounds the CTAs of every dispatch, also of one that would be copied by many short ones."""
+    from moonep_b200 import engine
+    monkeypatch.setenv("MOONEP_TRACE", "1")
+    if limit is not None:
+        monkeypatch.setenv("MOONEP_NUM_SMS_DEDUP", str(limit))
+    S, K, E, H = 2048, 8, 48, 5696
+    topk, tpe = (t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=7))
+    buf = Buffer(S, H, K, E, 1)
+    x = traceable_hidden(S, H, 0).cuda()
+    h, _, _, plan = buf.dispatch(x, None, topk, tpe)
+    engine.read_trace(buf._states[0])
+    again, _, _, _ = buf.dispatch(x, plan=plan)
+    ctas = {r[3] for r in engine.read_trace(buf._states[0])}
+    buf.check()
+    assert len(ctas) <= limit if limit else len(ctas) > torch.cuda.get_device_properties(0).multi_processor_count
+    rows = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long()
+    assert torch.equal(again.view(torch.int16)[rows], h.view(torch.int16)[rows])
+    buf.destroy()
