@@ -66,7 +66,10 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   // Tile list: a thread for each group. Groups with more tokens come first, as their tiles take longer: a launch then ends with
   // the shortest tiles, and the pairs finish together (16 groups of 4096 tokens on average and up to
   // three times as many, 2048 x 768: 164 -> 146 us).
-  int* s_key = reinterpret_cast<int*>(smem);      // the ring is not in use yet
+  // The keys lie in the epilogue's slabs, which ordinary stores write first: in the ring, the first TMA loads would follow ordinary accesses
+  // to the same bytes with no proxy fence between them.
+  int* s_key = reinterpret_cast<int*>(smem + (size_t)kRing * kStageBytes);
+  static_assert(kMaxGroups * sizeof(int) <= (size_t)kEpiWarps * 2 * kSlabBytes, "keys of all groups");
   bool act = false;
   const int tg = threadIdx.x;
   int beg, rows, units;

@@ -276,3 +276,26 @@ def test_sgd_at_the_edges_of_its_chunks(blocks, cuda_device):
     got = p.clone()
     gg.sgd_step_groups(got, d, 0.125, mask, True, num_blocks=blocks)
     assert torch.equal(got[0], want[5]) and torch.equal(got[1], p[1]) and torch.equal(got[2], want[5])
+
+
+@pytest.mark.parametrize("ctas", [2, 12, 148])
+def test_weight_gradients_of_many_uneven_groups(ctas, cuda_device):
+    """189 groups of 0 to 512 rows, larger ones first in the tile list, every other round backwards: the bits of each group alone. What a
+    CTA orders its list with must not reach the operands of its first tile."""
+    from moonep_b200.ops import grouped_gemm as gg
+    n, M, N = [128 * (7 * i * i % 6) for i in range(189)], 256, 256
+    cu = torch.tensor(n).cumsum(0).to(torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, dy = ((torch.randn(sum(n), c, device="cuda", generator=g)).to(torch.bfloat16) for c in (M, N))
+    full = lambda: torch.full((len(n), M, N), 7.0, device="cuda")     # noqa: E731
+    want = full()
+    for i in range(len(n)):
+        gg.wgrad(x, dy, cu, want, zero_empty_below=100, groups=(i, i + 1))
+    for dynamic in (False, True):
+        got = full()
+        gg.wgrad(x, dy, cu, got, zero_empty_below=100, num_ctas=ctas, dynamic=dynamic)
+        torch.cuda.synchronize()
+        gg.check_status()
+        assert torch.equal(got, want)
+    a = sum(n[:5])
+    assert n[5] and _rel(want[5], x[a:a + n[5]].float().T @ dy[a:a + n[5]].float()) < 1e-5       # fp32 sums of the same products
