@@ -168,6 +168,7 @@ wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
       tq::Snake seq(pair, npairs, ntiles);
+      if (args.early) pdl_wait();       // its waits have their limit from when the operands may come
       for (;; ++tcnt) {
         int t = -1;
         if (!dyn) { if (!s_abort) t = seq.next(); }

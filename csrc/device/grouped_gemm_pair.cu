@@ -289,6 +289,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
       tq::Snake seq(pair, npairs, ntiles);
+      if (args.early) pdl_wait();       // no MMA can start before; the limits of its waits run from here, as everyone's do
       for (;; ++tcnt) {
         int t = -1;
         if (!dyn) { if (!s_abort) t = seq.next(); }

@@ -299,3 +299,57 @@ def test_weight_gradients_of_many_uneven_groups(ctas, cuda_device):
         assert torch.equal(got, want)
     a = sum(n[:5])
     assert n[5] and _rel(want[5], x[a:a + n[5]].float().T @ dy[a:a + n[5]].float()) < 1e-5       # fp32 sums of the same products
+
+
+class _Early:
+    """Launches made inside set themselves up while the kernel before them runs, as those of a layer's native pass do, with the given limit of
+    their waits."""
+
+    def __init__(self, monkeypatch, budget_ns=None, **fields):
+        self.mp, self.fields = monkeypatch, dict(early=1, pdl=1, **fields)
+        if budget_ns is not None:
+            self.fields["budget_ns"] = budget_ns
+
+    def __enter__(self):
+        from moonep_b200.ops import grouped_gemm as gg
+        new = gg._new_args
+
+        def early(device, cu, pad):
+            args = new(device, cu, pad)
+            for k, v in self.fields.items():
+                setattr(args, k, v)
+            return args
+        self.ctx = self.mp.context()
+        self.ctx.__enter__().setattr(gg, "_new_args", early)
+
+    def __exit__(self, *exc):
+        self.ctx.__exit__(*exc)
+
+
+@pytest.mark.parametrize("kind", ["down", "gate_up", "wgrad"])
+def test_early_launch_waits_for_the_kernel_before_without_limit(kind, cuda_device, monkeypatch):
+    """The kernel before holds one pair of SMs for about 25 ms; the next launch starts beside it, on all others, with waits of 1 ms.
+    Those count from the end of the kernel before, whose output it reads."""
+    from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
+    S, K, N = 8192, 7168, 2048
+    cu = torch.tensor([S], dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(10)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, wg, wu, w, w2, dy = bf(S, K), bf(1, K, N, sc=0.02), bf(1, K, N, sc=0.02), bf(1, N, 512, sc=0.05), bf(1, N, 512, sc=0.05), bf(S, 256)
+    act = torch.zeros(S, N, dtype=torch.bfloat16, device="cuda")
+    out = {"wgrad": lambda: torch.full((1, N, 256), 7.0, device="cuda")}.get(kind, lambda: torch.full((S, 512), 7.0, dtype=torch.bfloat16, device="cuda"))
+    call = {"down": lambda o: gg.down(act, w, cu, o), "gate_up": lambda o: gg.gate_up(act, w, w2, cu, o), "wgrad": lambda o: gg.wgrad(act, dy, cu, o)}[kind]
+    got, want = out(), out()
+    torch.cuda.synchronize()
+    t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    t[0].record()
+    gg.gate_up(x, wg, wu, cu, act, num_ctas=2)
+    with _Early(monkeypatch, budget_ns=1_000_000):
+        call(got)
+    t[1].record()
+    call(want)
+    torch.cuda.synchronize()
+    gg.check_status()
+    assert t[0].elapsed_time(t[1]) > 8, "the kernel before is meant to outlast the limit several times over"
+    assert torch.equal(got, want)
