@@ -348,6 +348,7 @@ extern "C" int mep_grouped_wgrad_2cta(const void* x, int64_t rows, int64_t x_ld,
   num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "wgrad (2-CTA): needs at least two CTAs");
   MEP_REQUIRE(args.n_each == 0 || (args.N == 2 * args.n_each && args.n_each % 256 == 0 && args.out_b), "wgrad (2-CTA): two matrices of %d columns in %d", args.n_each, args.N);
+  MEP_REQUIRE(!args.upd_mask || (args.upd_w && (!args.n_each || args.upd_w_b)), "wgrad (2-CTA): an update without the weights of every matrix");
   const int pitch = args.n_each ? args.n_each : args.N;
   CUtensorMap ma, mb, mo, mo_b;
   if (tmap_rows(&ma, x, rows, args.M_w, x_ld, 64, 64)) return -1;

@@ -308,8 +308,10 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
     of 256 (the CTA-pair kernel).
 
     ``out_b``: a second tensor like ``out``, for the second half of ``dy``'s columns (gate and up in one launch);
-    ``update_b``: its weights, if ``update`` is given."""
+    ``update_b``: its weights, with ``update`` and only then.  A layer's native pass makes this launch by itself; here it is for
+    callers that issue theirs one by one."""
     G, M, N = out.shape
+    assert (update_b is not None) == (update is not None and out_b is not None), "update_b comes with update and out_b, and they with it"
     assert out.dtype == torch.float32 and out.is_contiguous()
     if out_b is not None:
         assert out_b.dtype == torch.float32 and out_b.is_contiguous() and out_b.shape == out.shape and wgrad_update_supported(M, N)
@@ -334,7 +336,6 @@ def wgrad(x, dy, cu, out, accumulate=False, zero_empty_below=0, groups=None, num
             assert w.dtype == torch.bfloat16 and tuple(w.shape) == tuple(out.shape) and w.is_contiguous()
             assert mask.dtype == torch.int32 and mask.numel() == G and mask.is_cuda
             args.upd_w, args.upd_mask, args.upd_lr = w.data_ptr(), mask.data_ptr(), float(lr)
-            assert (update_b is None) == (out_b is None)
         if out_b is not None:
             args.n_each, args.out_b = N // 2, out_b.data_ptr()
             if update is not None:

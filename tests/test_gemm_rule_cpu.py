@@ -44,3 +44,29 @@ def test_a_ticket_of_any_size_has_a_kernel(total, monkeypatch):
     for mode in MODES:
         for rows, K in ((0, 64), (128, 64), (6144, 2048), (40000, 7168)):
             assert _on_pairs(mode, rows, 16, 16, 768, K, False, total, True) in (True, False)
+
+
+@pytest.mark.parametrize("upd_w,upd_w_b,n_each", [(0, 0, 0), (4096, 0, 256), (0, 4096, 256)])
+def test_an_update_needs_the_weights_of_every_matrix(upd_w, upd_w_b, n_each):
+    """The launcher refuses a mask without weights, of one matrix or of two, before it looks at anything else of the call."""
+    import ctypes as C
+
+    from moonep_b200 import _native
+    from moonep_b200.ops.grouped_gemm import GemmArgs
+    a = GemmArgs()
+    a.G, a.M_w, a.N, a.g_end, a.out, a.n_each = 1, 256, 2 * n_each or 256, 1, 4096, n_each
+    a.out_b, a.upd_mask, a.upd_w, a.upd_w_b = 4096 if n_each else 0, 4096, upd_w, upd_w_b
+    with pytest.raises(_native.MoonEPNativeError, match="without the weights of every matrix"):
+        p = C.c_void_p(4096)
+        _native.check(_native.load().mep_grouped_wgrad_2cta(p, C.c_int64(128), C.c_int64(256), p, C.c_int64(512), C.byref(a), 148, None))
+
+
+def test_a_second_update_comes_with_the_first_and_a_second_matrix():
+    import torch
+
+    from moonep_b200.ops import grouped_gemm as gg
+    w, out, cu, x = torch.zeros(1, 256, 256, dtype=torch.bfloat16), torch.zeros(1, 256, 256), torch.tensor([128], dtype=torch.int32), torch.zeros(128, 256)
+    up = (w, 0.1, torch.ones(1, dtype=torch.int32))
+    for kw in (dict(update_b=w), dict(update_b=w, out_b=out), dict(update_b=w, update=up), dict(update=up, out_b=out)):
+        with pytest.raises(AssertionError, match="update_b comes with"):
+            gg.wgrad(x, x, cu, out, **kw)
