@@ -235,9 +235,9 @@ class MoEBlock:
                 ps = self.pools
                 ps.kept("sgd", lambda: gg.SgdMany([ps.local_weight(n) for n in names], [ps.local_grad(n) for n in names])).step(lr)
             else:
-                for n in names:                  # ``up`` last: its cross-rank reduction may still be running
+                for n in names:                  # ``up`` last: its cross-rank reduction may still be running, and these beside it
                     self.moe.wait_grads(n)
-                    gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr)
+                    gg.sgd_step(self.pools.local_weight(n), self.pools.local_grad(n), lr, num_blocks=8 * self.moe._total_sms)
         else:
             assert lr == self._fused_lr, "the experts were already updated with another learning rate"
             self.moe.wait_grads()       # the last reduction and the update behind it may still be running

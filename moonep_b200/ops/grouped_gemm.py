@@ -362,9 +362,9 @@ def swiglu_bwd(dA, gu, w, dgu, dw, cu, num_blocks=None):
 
 
 def sgd_step_groups(p, g, lr, mask, want: bool, num_blocks=None):
-    """``num_blocks`` (of a group here, of a tensor below): blocks that share an SM with a GEMM; by default many short ones that
-    want the GPU to themselves.  ``sgd_step`` for the groups ``i`` of ``p [G, ...]`` with ``(mask[i] != 0) == want`` only (``mask``: int32
-    ``[>= G]`` on the device): the complement of what ``wgrad(update=...)`` has already updated."""
+    """``sgd_step`` for the groups ``i`` of ``p [G, ...]`` with ``(mask[i] != 0) == want`` only (``mask``: int32
+    ``[>= G]`` on the device): the complement of what ``wgrad(update=...)`` has already updated.  ``num_blocks``: of a group, else as
+    in ``sgd_step``."""
     lib = _native.load()
     assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.shape == g.shape
     assert p.is_contiguous() and g.is_contiguous() and mask.dtype == torch.int32 and mask.numel() >= p.shape[0]
@@ -375,6 +375,10 @@ def sgd_step_groups(p, g, lr, mask, want: bool, num_blocks=None):
 
 
 def sgd_step(p, g, lr, num_blocks=None):
+    """``p -= lr * g`` (``p`` bf16, ``g`` fp32, a multiple of eight elements).  By default a short block for each 8192 elements, for an update that
+    has the GPU to itself: 7 to 10 % faster there, and level beside the GEMMs of a backward pass on a side stream (a step of 4096 tokens,
+    7168 x 2048, 32 experts 9758-10324 us, with a loop 10181-10356).  ``num_blocks``: that many blocks of few registers in a loop, which find
+    room beside whatever else holds the SMs."""
     lib = _native.load()
     assert p.dtype == torch.bfloat16 and g.dtype == torch.float32 and p.numel() == g.numel()
     assert p.is_contiguous() and g.is_contiguous()
@@ -384,7 +388,8 @@ def sgd_step(p, g, lr, num_blocks=None):
 
 
 class SgdMany:
-    """``sgd_step`` of up to four tensors in one launch; the tensors are fixed, so their addresses are gathered once."""
+    """``sgd_step`` of up to four tensors in one launch (``num_blocks``: as there, of each tensor); the tensors are fixed, so their
+    addresses are gathered once."""
 
     def __init__(self, ps, gs, num_blocks=None):
         n = len(ps)
