@@ -154,6 +154,7 @@ static int sgd_blocks(int num_blocks, int64_t n) { return num_blocks > 0 ? num_b
 
 extern "C" int mep_sgd_step(void* p, const float* g, float lr, int64_t n, int num_blocks, cudaStream_t stream) {
   MEP_REQUIRE(n % 8 == 0, "sgd_step: element count must be a multiple of 8");
+  MEP_REQUIRE(num_blocks >= 0, "sgd_step: %d blocks", num_blocks);
   if (n == 0) return 0;
   return mep::launch_plain(num_blocks > 0 ? mep::sgd_kernel<1> : mep::sgd_kernel<mep::kSgdVecs>, dim3(sgd_blocks(num_blocks, n)), dim3(256), 0, stream, (__nv_bfloat16*)p, g, lr, n / 8);
 }
@@ -161,6 +162,7 @@ extern "C" int mep_sgd_step(void* p, const float* g, float lr, int64_t n, int nu
 // sgd_step of up to four tensors in one launch.
 extern "C" int mep_sgd_step_many(int count, void* const* p, const float* const* g, const int64_t* n, float lr, int num_blocks, cudaStream_t stream) {
   MEP_REQUIRE(count >= 1 && count <= 4, "sgd_step: %d tensors", count);
+  MEP_REQUIRE(num_blocks >= 0, "sgd_step: %d blocks", num_blocks);
   mep::SgdPack k = {};
   int64_t most = 0;
   for (int i = 0; i < count; ++i) {
@@ -175,6 +177,7 @@ extern "C" int mep_sgd_step_many(int count, void* const* p, const float* const* 
 extern "C" int mep_sgd_step_groups(void* p, const float* g, float lr, int64_t n_per_group, int G, const int32_t* mask, int want,
                                    int num_blocks, cudaStream_t stream) {
   MEP_REQUIRE(n_per_group % 8 == 0 && G >= 1 && G <= 65535, "sgd_step_groups: %d groups of %lld elements", G, (long long)n_per_group);
+  MEP_REQUIRE(num_blocks >= 0, "sgd_step_groups: %d blocks", num_blocks);
   if (n_per_group == 0) return 0;
   return mep::launch_plain(num_blocks > 0 ? mep::sgd_groups_kernel<1> : mep::sgd_groups_kernel<mep::kSgdVecs>, dim3(sgd_blocks(num_blocks, n_per_group), G), dim3(256), 0, stream, (__nv_bfloat16*)p, g, lr,
                            n_per_group / 8, mask, want);

@@ -16,3 +16,14 @@ def test_update_beside_a_reduction_names_its_blocks(monkeypatch):
     blk.router, blk.shared = torch.zeros(1), None
     blk.sgd_step(0.5)
     assert calls == [c for n in ("down", "gate", "up") for c in (("wait", n), ("sgd", "w_" + n, "d_" + n, 0.5, 8 * 148))]
+
+
+def test_a_negative_number_of_blocks_is_refused():
+    import ctypes as C
+
+    from moonep_b200 import _native
+    lib, p, n, lr = _native.load(), C.c_void_p(4096), C.c_int64(64), C.c_float(0.5)
+    many = (C.c_void_p * 1)(4096), (C.c_void_p * 1)(4096), (C.c_int64 * 1)(64)
+    for call in (lambda b: lib.mep_sgd_step(p, p, lr, n, b, None), lambda b: lib.mep_sgd_step_many(1, *many, lr, b, None),
+                 lambda b: lib.mep_sgd_step_groups(p, p, lr, n, 1, p, 1, b, None)):
+        assert call(-1) != 0 and lib.mep_last_error().endswith(b"-1 blocks")
