@@ -61,7 +61,6 @@ struct MoeLocal {
   uint64_t budget_ns;
   int32_t token_padding;
   int32_t sms;                   // of the device
-  int32_t last_first;            // combine call: the rows were dispatched in the order of the tokens (see local_combine_kernel)
 };
 
 }  // namespace mep

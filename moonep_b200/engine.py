@@ -268,7 +268,6 @@ class LocalExchange:
         """A fresh plan (in one allocation: what a small dispatch would otherwise wait for) and the K rows of every
         token; returns ``(plan, cu_seqlens)``.  ``out_hidden`` / ``out_w``: any tensors of the shard's shape."""
         slab = torch.empty(self._total, dtype=torch.int32, device=self._dev)
-        self._args.last_first = 0        # each CTA copies a range of its own
         rc = self._lib.mep_local_dispatch_call(self._ref, hidden.data_ptr(), None if route_w is None else route_w.data_ptr(),
                                                topk.data_ptr(), tpe.data_ptr(), slab.data_ptr(), None, None, out_hidden.data_ptr(),
                                                None if out_w is None else out_w.data_ptr(), _native.raw_stream())
@@ -278,7 +277,7 @@ class LocalExchange:
 
     def dispatch_again(self, hidden, route_w, plan, out_hidden, out_w):
         """The rows of a saved plan."""
-        self._args.last_first = 1        # a hint for the combine; either order gives the same sums
+        plan.__dict__["_in_order"] = 1   # a hint for the combine of these rows; either order gives the same sums
         rc = self._lib.mep_local_dispatch_call(self._ref, hidden.data_ptr(), None if route_w is None else route_w.data_ptr(), None, None,
                                                None, self._dst(plan), plan.zero_fill_ranges.data_ptr(), out_hidden.data_ptr(),
                                                None if out_w is None else out_w.data_ptr(), _native.raw_stream())
@@ -296,7 +295,8 @@ class LocalExchange:
         out = torch.empty_like(self._rows_like)
         out_w = None if row_w is None else torch.empty_like(self._weights_like)
         rc = self._lib.mep_local_combine_call(self._ref, self._dst(plan), rows.data_ptr(), None if row_w is None else row_w.data_ptr(),
-                                              out.data_ptr(), None if out_w is None else out_w.data_ptr(), _native.raw_stream())
+                                              out.data_ptr(), None if out_w is None else out_w.data_ptr(), plan.__dict__.get("_in_order", 0),
+                                              _native.raw_stream())
         if rc:
             _native.check(rc, "combine")
         return out, out_w
