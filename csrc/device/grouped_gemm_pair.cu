@@ -39,6 +39,13 @@ constexpr int kMaxGroups = 192;
 // 1.55 ms, down 0.91 -> 0.74; groups of 4000, 4096 x 1024: gate/up 0.471 -> 0.440, dgrad 0.237 -> 0.226. Below the line the
 // weights would be read again for nothing (4096 tokens, 4096 deep, 32 MB: 1.445 -> 1.481).
 constexpr int kBand = 8, kXBytes = 36 << 20;
+// Up to this many rounds of tiles over the pairs, groups with larger tiles come first, so that the launch ends with the shortest and the pairs
+// finish together; with more rounds the groups keep their order. Forward passes in long loops, in us, never sorted / by this rule: 1531 tokens,
+// 2048 x 768, 16 experts (5 and 6 rounds) 147.1 / 143.6; 1000, 7168 x 512, 32 (2 and 16) 285.3 / 278.6; 1000, 4096 x 1024, 24 (5 and 9) 254.1 /
+// 251.7. Always sorted / by this rule: 4096, 7168 x 2048, 32 (31 and 54) 2669 / 2619, a captured training step of it 8990 / 8800; from 8 to
+// 24 rounds the two are within 1 % of each other. Every round runs forwards: backwards in odd ones, the pairs that the hardware starts last
+// had the tiles left over in a short last round (64 tokens, 2048 x 768, two rounds, 57.4 / 51.7).
+constexpr int kSortRounds = 12;
 constexpr int kStgSet = 4 * kStgBytes;                 // GATE_UP: act twice, gate, up; else: two buffers for each 64-column side
 constexpr size_t kEpiBytes = 2 * kStgSet + kEpiWarps * kXchBytes;
 constexpr size_t kSmem = (size_t)kRingBytes + kEpiBytes + 1024;
@@ -108,22 +115,24 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     tc::prefetch_tmap(&tma_out); tc::prefetch_tmap(&tma_out2);
   }
   if (!args.early) pdl_wait();           // the tables below may come from the kernel right before
-  // Tile list: a thread for each group. Groups with larger tiles come first, so that the launch ends with the shortest and the
-  // pairs finish together -- unless the rows or weights are still arriving, in the order of the groups.
+  // Tile list: a thread for each group. Groups are ordered by the size of their tiles where the launch has few of them (see kSortRounds) --
+  // unless the rows or weights are still arriving, in the order of the groups. A key: size, group, number of token tiles.
+  const int few = kSortRounds * ((args.sched_ctas > 0 ? args.sched_ctas : (int)gridDim.x) >> 1);      // alike for all launches on one ticket
   const int tg = threadIdx.x;
-  int units, beg, rows, key = -1;
+  int units, beg, rows, key = 0;
   group_rows(args, s_key, beg, rows, units);
   if (tg < kMaxGroups) {
     if (tg < G) {
       if (tg < args.g_begin || tg >= args.g_end) units = 0;
       const int mt = (units + 7) >> 3;
-      key = (units && !args.tile_done && !args.group_flags ? (units + mt - 1) / mt : 0) * 256 + (255 - tg);
+      key = ((units && !args.tile_done && !args.group_flags ? (units + mt - 1) / mt : 0) * 256 + (255 - tg)) << 16 | min(mt, 0xffff);
     }
     s_key[tg] = key;
   }
   __syncthreads();
   if (tg < G) {
-    const int at = rank_of(key, s_key, G);
+    int tiles = 0;
+    const int place = rank_of(key, s_key, G, &tiles), at = (int64_t)tiles * (args.N / kCols) > few ? tg : place;
     s_grp[at] = tg; s_beg[at] = beg; s_units[at] = units;
   }
   __syncthreads();
@@ -191,7 +200,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     bool early = args.early != 0;        // the kernel before has not been waited for yet
     tq::Scheduler<true> sched; tq::Consumer<true> follow;
     if (dyn && lane == 0) { if (leader) sched.setup(&s_ring, args.sched, ntiles); else follow.setup(&s_ring); }
-    tq::Snake seq(pair, npairs, ntiles);
+    tq::Strided seq{pair, npairs, ntiles};
     const uint32_t tile_ep = args.tile_done ? *(volatile const uint32_t*)args.tile_epoch : 0u;
     const uint32_t group_ep = args.group_flags ? *(volatile const uint32_t*)args.group_epoch : 0u;
     int seen_row = -1, seen_group = -1;              // flags known to be up: first row of the last tile, last group
@@ -288,7 +297,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       uint32_t stage = 0, phase = 0;
       bool ready = false;
       tq::Consumer<true> tiles; tiles.setup(&s_ring);
-      tq::Snake seq(pair, npairs, ntiles);
+      tq::Strided seq{pair, npairs, ntiles};
       if (args.early) pdl_wait();       // no MMA can start before; the limits of its waits run from here, as everyone's do
       for (;; ++tcnt) {
         int t = -1;
@@ -339,7 +348,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     int chunk_no = 0;
     int tcnt = 0, gcur = 0; Tile ti;
     tq::Consumer<true> tiles; tiles.setup(&s_ring);
-    tq::Snake seq(pair, npairs, ntiles);
+    tq::Strided seq{pair, npairs, ntiles};
     auto stage = [&](uint32_t buf, const uint32_t* lo, const uint32_t* hi, float sc[4]) {
 #pragma unroll
       for (int b = 0; b < 2; ++b) {

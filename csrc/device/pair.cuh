@@ -53,13 +53,14 @@ struct Divisor {
   }
 };
 // Place of `key` among the first `n` of `keys` in falling order (keys differ, those of groups that do not count are negative;
-// `keys` 16-byte aligned and filled up to a multiple of four).
-__device__ __forceinline__ int rank_of(int key, const int* keys, int n) {
+// `keys` 16-byte aligned and filled up to a multiple of four). `low`: the sum of the keys' low 16 bits is added there.
+__device__ __forceinline__ int rank_of(int key, const int* keys, int n, int* low = nullptr) {
   int r = 0;
 #pragma unroll 4
   for (int j = 0; j < n; j += 4) {
     const int4 k = *reinterpret_cast<const int4*>(keys + j);
     r += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
+    if (low) *low += (k.x & 0xffff) + (k.y & 0xffff) + (k.z & 0xffff) + (k.w & 0xffff);
   }
   return r;
 }

@@ -353,3 +353,36 @@ def test_early_launch_waits_for_the_kernel_before_without_limit(kind, cuda_devic
     gg.check_status()
     assert t[0].elapsed_time(t[1]) > 8, "the kernel before is meant to outlast the limit several times over"
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("split", [(2,), (28,), (30,), (148,), (10, 138)], ids=str)
+def test_token_major_tiles_of_uneven_groups(split, cuda_device, monkeypatch):
+    """Groups of 0 to 1000 rows, ordered by the size of their tiles up to twelve rounds (gate/up from 15 pairs on, the others from 8) and by number above: the
+    bits of each group alone, with tickets too. Launches on one ticket order their list alike, although alone they would not."""
+    from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
+    K, N, n = 256, 512, [[40, 0, 1000, 257, 33, 512, 128, 700, 1][i % 9] for i in range(27)]
+    p = [(r + 127) // 128 * 128 for r in n]
+    ends = torch.tensor(p).cumsum(0)
+    cu = ends.to(torch.int32).cuda()
+    pad = torch.tensor([[int(e) - q + r, q - r] if q > r else [0, 0] for r, q, e in zip(n, p, ends)], dtype=torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(11)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, x2, w, wu, scale = bf(sum(p), K), bf(sum(p), 2 * K), bf(27, K, N, sc=0.05), bf(27, K, N, sc=0.05), torch.rand(sum(p), device="cuda", generator=g)
+    calls = [lambda o, **kw: gg.gate_up(x, w, wu, cu, o, row_scale=scale, pad=pad, **kw), lambda o, **kw: gg.down(x, w, cu, o, pad=pad, **kw),
+             lambda o, **kw: gg.dgrad(x, w.view(27, N, K), cu, o, pad=pad, **kw), lambda o, **kw: gg.dgrad_gate_up(x2, w.view(27, N, K), wu.view(27, N, K), cu, o, pad=pad, **kw)]
+    for call in calls:
+        want, *got = (torch.full((sum(p), N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(3))
+        for i in range(27):
+            call(want, groups=(i, i + 1))
+        if len(split) == 1:
+            call(got[0], num_ctas=split[0])
+            call(got[1], num_ctas=split[0], dynamic=True)
+        else:
+            for o in got:
+                tk = gg.Ticket(x.device, sum(split))
+                for c in split:
+                    call(o, num_ctas=c, ticket=tk)
+        torch.cuda.synchronize()
+        gg.check_status()
+        assert all(torch.equal(o.view(torch.int16), want.view(torch.int16)) for o in got)
