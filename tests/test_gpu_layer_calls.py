@@ -237,3 +237,41 @@ def test_native_calls_follow_the_launch_switch(cuda_device):
     blk.buf.check()
     assert all(torch.equal(a, b) for a, b in zip(*got))
     blk.destroy()
+
+
+@pytest.mark.parametrize("lr", [None, 0.05], ids=["gradients", "update"])
+@pytest.mark.parametrize("ctas", [None, 6])
+def test_native_passes_give_the_bits_of_single_launches(ctas, lr, cuda_device):
+    """16 to 40 blocks of depth (more than a ring holds), 26 experts of which six are empty, more tiles than pairs: the native passes, whose GEMMs start
+    early and share launches, against the same operators issued one by one from Python."""
+    from moonep_b200.models.moe_block import MoEBlock, MoEConfig
+    blk = MoEBlock(MoEConfig("t", H=1024, Hp=1280, K=4, epn=26, shared_experts=0, S=700), num_sms=4, seed=3)
+    if lr is not None:
+        blk.fuse_optimizer(lr, in_epilogue=True)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    p = torch.rand(700, 26, device="cuda", generator=g) * torch.linspace(0.2, 2, 26, device="cuda")
+    p[:, [0, 5, 6, 13, 20, 25]] = -1
+    w, topk = torch.topk(p, 4, dim=1)
+    topk = topk.to(torch.int32).contiguous()
+    tpe = torch.bincount(topk.flatten().long(), minlength=26).to(torch.int32)
+    x, dy = normal((700, 1024), 1), normal((700, 1024), 2)
+    names, got = ("gate", "up", "down"), []
+    before = [blk.pools.local_weight(n).clone() for n in names]
+    native = blk.moe._native
+    assert native is not None
+    for use in (native, None):
+        blk.moe._native = use
+        if use is not None and ctas is not None:
+            use._args.num_ctas = ctas
+        for n, b in zip(names, before):
+            blk.pools.local_weight(n).copy_(b)
+            blk.pools.local_grad(n).fill_(7.0)
+        infer, _ = blk.moe.forward(x, w, topk, tpe, need_backward=False)
+        y, ctx = blk.moe.forward(x, w, topk, tpe)
+        dx, dw = blk.moe.backward(ctx, dy)
+        torch.cuda.synchronize()
+        blk.buf.check()
+        got.append([infer, y, dx, dw] + [blk.pools.local_grad(n).clone() for n in names] + [blk.pools.local_weight(n).clone() for n in names])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    assert (lr is None) == all(torch.equal(a, b) for a, b in zip(got[0][7:], before))
+    blk.destroy()

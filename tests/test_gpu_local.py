@@ -138,7 +138,7 @@ def test_padding_rows_are_counted(cuda_device):
 
 
 # Large batches (200 MiB moved): the saved plan's rows come from many short CTAs and the combine begins with the last tokens. Just above
-# the line with fresh plans on both sides of the hand-over, one entry per token, fewer tokens than CTAs with rows of which three fit.
+# the line with fresh plans on both sides of the hand-over, one entry per token, a token for each CTA with rows of which three fit.
 LARGE_CASES = [
     (2048, 8,  48,   5696,  16,  "random"),
     (5003, 5,  40,   3496,  128, "biased"),

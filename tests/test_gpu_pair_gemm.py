@@ -386,3 +386,72 @@ def test_token_major_tiles_of_uneven_groups(split, cuda_device, monkeypatch):
         torch.cuda.synchronize()
         gg.check_status()
         assert all(torch.equal(o.view(torch.int16), want.view(torch.int16)) for o in got)
+
+
+@pytest.mark.parametrize("tokens", [False, True], ids=["cu", "tokens"])
+@pytest.mark.parametrize("most,depths", [(32, (9, 10, 11, 20)), (128, (7, 8, 9)), (300, (1, 5, 6, 7, 13))], ids=["ring10", "ring8", "ring6"])
+def test_early_launches_around_the_depth_of_the_ring(most, depths, tokens, cuda_device, monkeypatch):
+    """A launch that fills its ring with weights while the kernel before still writes its rows: fewer 64-deep blocks than stages, as many, more;
+    27 groups, some empty, on two pairs (many tiles each) and on all (some without one); tiles from token counts or from cu_seqlens.
+    The bits of an ordinary launch behind the kernel before."""
+    from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
+    E, N, wide = 27, 256, 64 * max(depths) * 2 + 256
+    wide = (wide + 255) // 256 * 256
+    n = [(most, 0, 1, most // 2, 32, 0, most - 1)[i % 7] for i in range(E)]
+    p = [(r + 127) // 128 * 128 for r in n]
+    ends = torch.tensor(p).cumsum(0)
+    rows, cu = sum(p), ends.to(torch.int32).cuda()
+    pad = torch.tensor([[int(e) - q + r, q - r] if q > r else [0, 0] for r, q, e in zip(n, p, ends)], dtype=torch.int32).cuda()
+    tpe = torch.tensor(n, dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(12)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    src, w_src = bf(rows, 512), bf(E, 512, wide, sc=0.05)
+    whole = torch.tensor([rows] + [rows] * (E - 1), dtype=torch.int32, device="cuda")
+    x = torch.zeros(rows, wide, dtype=torch.bfloat16, device="cuda")
+    before = lambda: gg.down(src, w_src, whole, x, num_ctas=2)     # noqa: E731
+    fields = dict(tokens=tpe.data_ptr(), tokens_n=E, token_padding=128) if tokens else {}
+    for d in depths:
+        K = 64 * d
+        w, wu, dy = bf(E, K, N, sc=0.05), bf(E, K, N, sc=0.05), bf(rows, N)
+        for r, q, e in zip(n, p, ends.tolist()):
+            dy[e - q + r:e] = 0
+        calls = {"gate_up": lambda o, **kw: gg.gate_up(x[:, :K], w, wu, cu, o, pad=pad, **kw), "down": lambda o, **kw: gg.down(x[:, :K], w, cu, o, pad=pad, **kw),
+                 "dgrad": lambda o, **kw: gg.dgrad(x[:, :K], w.view(E, N, K), cu, o, pad=pad, **kw),
+                 "dgrad_gu": lambda o, **kw: gg.dgrad_gate_up(x[:, :2 * K], w.view(E, N, K), wu.view(E, N, K), cu, o, pad=pad, **kw)}
+        if d == depths[0]:
+            calls["wgrad"] = lambda o, **kw: gg.wgrad(x[:, :512], dy, cu, o, pad=pad, zero_empty_below=E, **kw)
+        for name, call in calls.items():
+            shape, dt = ((E, 512, N), torch.float32) if name == "wgrad" else ((rows, N), torch.bfloat16)
+            want, *got = (torch.full(shape, 7.0, dtype=dt, device="cuda") for _ in range(3))
+            before()
+            call(want)
+            for o, ctas in zip(got, (4, 148)):
+                x.zero_()
+                before()
+                with _Early(monkeypatch, **fields):
+                    call(o, num_ctas=ctas)
+            torch.cuda.synchronize()
+            gg.check_status()
+            assert all(torch.equal(o, want) for o in got), f"{name}, {d} blocks"
+
+
+def test_counts_that_fall_give_no_tiles(cuda_device):
+    """Ends of groups that fall, as a corrupt table may have them: such a group has no tiles, the others have theirs, and every access stays inside
+    the tensors (all ends do)."""
+    from moonep_b200.ops import grouped_gemm as gg
+    cu = torch.tensor([256, 128, 384], dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(13)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, w, wt, dy = bf(384, 256), bf(3, 256, 512, sc=0.05), bf(3, 512, 256, sc=0.05), bf(384, 256)
+    y, dA, dW = (torch.full(s, 7.0, dtype=t, device="cuda") for s, t in (((384, 512), torch.bfloat16), ((384, 512), torch.bfloat16), ((3, 256, 256), torch.float32)))
+    pad = torch.zeros(3, 2, dtype=torch.int32, device="cuda")
+    gg.down(x, w, cu, y, pad=pad)
+    gg.dgrad(x, wt, cu, dA, pad=pad)
+    gg.wgrad(x, dy, cu, dW, pad=pad)
+    torch.cuda.synchronize()
+    gg.check_status()
+    for out, ref in ((y, w), (dA, wt.transpose(1, 2))):      # rows 128 to 255 belong to two groups
+        assert _rel(out[:128], x[:128].float() @ ref[0].float()) < 4e-3 and _rel(out[256:], x[256:].float() @ ref[2].float()) < 4e-3
+    assert _rel(dW[0], x[:256].float().T @ dy[:256].float()) < 1e-4 and _rel(dW[2], x[128:].float().T @ dy[128:].float()) < 1e-4
+    assert bool((dW[1] == 7.0).all())
