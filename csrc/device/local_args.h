@@ -61,6 +61,8 @@ struct MoeLocal {
   uint64_t budget_ns;
   int32_t token_padding;
   int32_t sms;                   // of the device
+  int32_t in_order, reserved;    // combine call: the rows come from a saved plan's dispatch, which on a whole device goes through a large
+                                 // batch in the order of the tokens (see local_combine_kernel)
 };
 
 }  // namespace mep

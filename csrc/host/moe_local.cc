@@ -56,8 +56,7 @@ static int gemm(const MoeLocal& m, GemmMode mode, const void* a, int64_t a_cols,
 }  // namespace mep
 
 // Dispatch and combine alone, for a Buffer whose caller computes the experts. Dispatch plans into `slab` when `topk` is
-// given and reads the plan from it otherwise; `dst` / `zero_fill` may come from another plan's tensors instead. in_order: the rows come
-// from a saved plan's dispatch, which on a whole device goes through a large batch in the order of the tokens (see local_combine_kernel).
+// given and reads the plan from it otherwise; `dst` / `zero_fill` may come from another plan's tensors instead.
 extern "C" int mep_local_dispatch_call(const mep::MoeLocal* mp, const void* hidden, const float* route_w, const int32_t* topk, const int32_t* tpe,
                                        int32_t* slab, int32_t* dst, int32_t* zero_fill, void* rows, float* row_w, cudaStream_t stream) {
   using namespace mep;
@@ -71,11 +70,11 @@ extern "C" int mep_local_dispatch_call(const mep::MoeLocal* mp, const void* hidd
 }
 
 extern "C" int mep_local_combine_call(const mep::MoeLocal* mp, const int32_t* dst, const void* rows, const float* row_w, void* out, float* out_w,
-                                      int in_order, cudaStream_t stream) {
+                                      cudaStream_t stream) {
   using namespace mep;
   const MoeLocal& m = *mp;
   LocalCombineArgs c = {dst, (const __nv_bfloat16*)rows, row_w, (__nv_bfloat16*)out, out_w};
-  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 0, in_order && m.combine_blocks >= m.sms, stream);
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 0, m.in_order && m.combine_blocks >= m.sms, stream);
 }
 
 extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden, const float* route_w, const int32_t* topk,

@@ -72,7 +72,7 @@ class MoeLocal(C.Structure):
                 + [("plan_off", C.c_int64 * 8)]
                 + [(n, C.c_void_p) for n in ("w_gate", "w_up", "w_down", "shard", "shard_w", "srcinfo", "x", "w", "act", "gu", "dA",
                                              "dgu", "dw_gate", "dw_up", "dw_down", "sync", "hist", "status", "status_host")]
-                + [("budget_ns", C.c_uint64), ("token_padding", C.c_int32), ("sms", C.c_int32)])
+                + [("budget_ns", C.c_uint64), ("token_padding", C.c_int32), ("sms", C.c_int32), ("in_order", C.c_int32), ("reserved", C.c_int32)])
 
 
 class SendOrderArgs(C.Structure):
@@ -155,7 +155,7 @@ def load(build_if_missing: bool = True):
     lib.mep_swiglu.argtypes = [vp, vp, C.c_int64, i32, vp]
     lib.mep_silu_sweep.argtypes = [C.c_uint32, C.c_uint32, vp, vp, vp]
     lib.mep_local_dispatch_call.argtypes = [vp] * 11
-    lib.mep_local_combine_call.argtypes = [vp] * 6 + [i32, vp]
+    lib.mep_local_combine_call.argtypes = [vp] * 7
     lib.mep_moe_local_forward.argtypes = [vp] * 7 + [i32, vp]
     lib.mep_moe_local_backward.argtypes = [vp] * 5 + [i32, C.c_float, vp, vp]
     _LIB = lib

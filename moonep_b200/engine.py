@@ -244,6 +244,11 @@ class LocalExchange:
         a.shard, a.shard_w, a.srcinfo = st.hidden_local.data_ptr(), st.weights_local.data_ptr(), ptr(st.srcinfo_local)
         a.sync, a.hist = st.scratch["loc_sync"].data_ptr(), st.scratch["loc_hist"].data_ptr()
         self._args, self._ref, self._dev = a, C.addressof(a), st.device
+        # the block of a combine whose rows a saved plan has brought (an argument for it and
+        # its lookup cost a decode batch of 64 0.4 us of 23.4)
+        self._args_in_order = _native.MoeLocal.from_buffer_copy(a)
+        self._args_in_order.in_order = 1
+        self._ref_in_order = C.addressof(self._args_in_order)
         self._ints = dict(N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K)
         # shape, strides and first element of each part: one as_strided call costs a third of narrow and view
         self._fields = dict(dst=((g.N,), (1,), first[0]), experts_to_copy=((1, g.epn), (g.epn, 1), first[1]),
@@ -277,7 +282,7 @@ class LocalExchange:
 
     def dispatch_again(self, hidden, route_w, plan, out_hidden, out_w):
         """The rows of a saved plan."""
-        plan.__dict__["_in_order"] = 1   # a hint for the combine of these rows; either order gives the same sums
+        plan.__dict__["_in_order"] = True   # a hint for the combine of these rows; either order gives the same sums
         rc = self._lib.mep_local_dispatch_call(self._ref, hidden.data_ptr(), None if route_w is None else route_w.data_ptr(), None, None,
                                                None, self._dst(plan), plan.zero_fill_ranges.data_ptr(), out_hidden.data_ptr(),
                                                None if out_w is None else out_w.data_ptr(), _native.raw_stream())
@@ -294,9 +299,11 @@ class LocalExchange:
         read."""
         out = torch.empty_like(self._rows_like)
         out_w = None if row_w is None else torch.empty_like(self._weights_like)
-        rc = self._lib.mep_local_combine_call(self._ref, self._dst(plan), rows.data_ptr(), None if row_w is None else row_w.data_ptr(),
-                                              out.data_ptr(), None if out_w is None else out_w.data_ptr(), plan.__dict__.get("_in_order", 0),
-                                              _native.raw_stream())
+        d = plan.__dict__
+        slab = d.get("_slab")
+        rc = self._lib.mep_local_combine_call(self._ref_in_order if "_in_order" in d else self._ref,
+                                              plan.dst.data_ptr() if slab is None else slab.data_ptr(), rows.data_ptr(), None if row_w is None else row_w.data_ptr(),
+                                              out.data_ptr(), None if out_w is None else out_w.data_ptr(), _native.raw_stream())
         if rc:
             _native.check(rc, "combine")
         return out, out_w

@@ -14,7 +14,7 @@ def test_the_hint_for_the_order_of_a_combine_belongs_to_its_plan(monkeypatch):
                          scratch={k: torch.empty(4, dtype=torch.int32) for k in ("loc_sync", "loc_hist")})
     monkeypatch.setattr(engine._native, "raw_stream", lambda: 0)
     ex, hints = engine.LocalExchange(st, 148), []
-    ex._lib = SimpleNamespace(mep_local_dispatch_call=lambda *a: 0, mep_local_combine_call=lambda *a: hints.append(a[-2]) or 0)
+    ex._lib = SimpleNamespace(mep_local_dispatch_call=lambda *a: 0, mep_local_combine_call=lambda *a: hints.append(engine._native.MoeLocal.from_address(a[0]).in_order) or 0)
     x, rows, topk, tpe = torch.empty(g.S, g.H, dtype=torch.bfloat16), st.hidden_local, torch.empty(g.N, dtype=torch.int32), torch.empty(g.E, dtype=torch.int32)
     (a, _), (b, _) = (ex.dispatch(x, None, topk, tpe, rows, None) for _ in range(2))
     ex.combine(a, rows, None)
