@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 // A block's loads of a chunk are all in flight before the first is used, and by default a block has one chunk: short blocks
 // that the hardware hands out even out the SMs' unequal distance from memory. 3 x 705 M parameters: 2324 us (7.28 TB/s), where
 // 1184 blocks in a loop of single vectors took 2496; 3 x 34 M: 115 against 130. Two chunks a block take 2400, loads that are
-// marked as streaming 2480. Callers that name a number of blocks run beside a GEMM: single vectors in a loop need 32 registers
-// instead of 72 and find room next to its CTAs.
+// marked as streaming 2480. Callers that name a number of blocks run beside a GEMM: single vectors in a loop need 29 to 48
+// registers instead of 62 to 72 and find room next to its CTAs.
 constexpr int kSgdVecs = 4;                                  // vectors of eight parameters
 
 template <int VECS>
