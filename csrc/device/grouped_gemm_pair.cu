@@ -33,7 +33,7 @@ constexpr int kChunk = 16;                             // tokens per epilogue st
 constexpr int kStgBytes = kChunk * 128;                // staging: 16 tokens x 64 columns
 constexpr int kXchBytes = 32 * 32;                     // half of a warp's fp32 fragments of a chunk (GATE_UP)
 constexpr int kMaxGroups = 192;
-// BANDS: a group with more than kXBytes of token rows is walked in bands of at most kBand token tiles, all weight columns for
+// BANDED: a group with more than kXBytes of token rows is walked in bands of at most kBand token tiles, all weight columns for
 // a band, then the next band. 74 pairs then read 8 + 9 operand slabs at a time and fetch each token row from DRAM once; DRAM
 // traffic also costs clock, the kernels being at the power limit. One group of 32768 tokens, 7168 x 2048: gate/up 1.85 ->
 // 1.55 ms, down 0.91 -> 0.74; groups of 4000, 4096 x 1024: gate/up 0.471 -> 0.440, dgrad 0.237 -> 0.226. Below the line the
@@ -46,11 +46,20 @@ constexpr int kBand = 8, kXBytes = 36 << 20;
 // 24 rounds the two are within 1 % of each other. Every round runs forwards: backwards in odd ones, the pairs that the hardware starts last
 // had the tiles left over in a short last round (64 tokens, 2048 x 768, two rounds, 57.4 / 51.7).
 constexpr int kSortRounds = 12;
+// STREAM: weights of a group with one token tile are read once: their lines leave L2 first, so that rows, tables and above all the kernels' code, which
+// every launch fetches anew, stay there. Where the groups' matrices, one for each, have this many bytes: a layer of three of less than 100 MB
+// keeps its weights in L2 from one pass to the next. Forward passes with / without, in us: 64 tokens, 2048 x 768, 16 experts (50 MB) 49.2 / 52.5; 700,
+// 2048 x 768, 24 (75) 74.0 / 80.9; 300, 4096 x 1024, 16 (134) 84.8 / 93.0; 256, 7168 x 2048, 32 (940) 477 / 483; but 16 tokens,
+// 2048 x 768, 8 (25) 36.5 / 34.9. Only where few groups have more than one tile (kStreamRows rows in a group on average; a layer allows 127 for padding):
+// the hint costs the others 1 % (1531, 2048 x 768, 16 152.2 / 150.2), and not for tiles that share weights, as pairs are not in step: gate/up of 32 experts and 4096
+// tokens x 8, 7168 x 2048, then reads 6.2 GB instead of 3.4 and takes 2.04 ms instead of 1.80.
+constexpr int64_t kStreamBytes = 32 << 20, kStreamRows = 320;
+enum Kind { PLAIN, BANDED, STREAM };                   // a kernel each: code that a launch does not need costs it 1 to 2 us of 50
 constexpr int kStgSet = 4 * kStgBytes;                 // GATE_UP: act twice, gate, up; else: two buffers for each 64-column side
 constexpr size_t kEpiBytes = 2 * kStgSet + kEpiWarps * kXchBytes;
 constexpr size_t kSmem = (size_t)kRingBytes + kEpiBytes + 1024;
 
-struct Tile { int g, row0, n, n0; };                   // n tokens from row0 (a multiple of 32, at most 256)
+struct Tile { int g, row0, n, n0; bool once; };        // n tokens from row0 (a multiple of 32, at most 256); all of their group's
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -77,7 +86,7 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t epoch, 
   }
 }
 
-template <int MODE, bool BANDS>
+template <int MODE, int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
 tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_x64,
                 const __grid_constant__ CUtensorMap tma_x16, const __grid_constant__ CUtensorMap tma_w0, const __grid_constant__ CUtensorMap tma_w1,
@@ -177,7 +186,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     while (s_start[g + 1] <= t) ++g;
     const int units = s_units[g], mt = (units + 7) >> 3, local = t - s_start[g];
     int cb, pt;
-    if (BANDS && (int64_t)mt * args.K > kXBytes / 512) {
+    if (KIND == BANDED && (int64_t)mt * args.K > kXBytes / 512) {
       const int nblk = args.N / kCols, bands = quotient(mt - 1, kBand) + 1, bw = quotient(mt - 1, bands) + 1;
       const int b = quotient(local, bw * nblk), in = local - b * bw * nblk, w = min(bw, mt - b * bw);
       cb = quotient(in, w); pt = b * bw + in - cb * w;
@@ -188,6 +197,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     ti.g = s_grp[g]; ti.n0 = cb * kCols;
     ti.row0 = s_beg[g] + 32 * (pt * base + min(pt, rem));
     ti.n = 32 * (base + (pt < rem ? 1 : 0));
+    ti.once = mt == 1;
   };
 
   if (warp == 0) {
@@ -203,6 +213,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     tq::Strided seq{pair, npairs, ntiles};
     const uint32_t tile_ep = args.tile_done ? *(volatile const uint32_t*)args.tile_epoch : 0u;
     const uint32_t group_ep = args.group_flags ? *(volatile const uint32_t*)args.group_epoch : 0u;
+    const uint64_t streamed = tc::evict_first(), kept = tc::evict_normal();
     int seen_row = -1, seen_group = -1;              // flags known to be up: first row of the last tile, last group
     const uint32_t smem0 = smem_u32(smem), full0 = mapa(smem_u32(&full_bar[0]), 0);
     for (;;) {
@@ -232,19 +243,26 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       }
       const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
       const uint32_t bytes = (uint32_t)kWBytes + (small ? (uint32_t)half * 128u : half > 64 ? 16384u : 8192u);
+      const uint64_t policy = ti.once ? streamed : kept;
+      auto atoms = [&](uint32_t dst, const CUtensorMap* map, int k, int atom, uint32_t bar) {
+        if (KIND == STREAM) tma_load_3d_bar(dst, map, 0, k, atom, bar, policy); else tma_load_3d_bar(dst, map, 0, k, atom, bar);
+      };
+      auto rows = [&](uint32_t dst, const CUtensorMap* map, int k, int row, uint32_t bar) {
+        if (KIND == STREAM) tma_load_2d_bar(dst, map, k, row, bar, policy); else tma_load_2d_bar(dst, map, k, row, bar);
+      };
       auto load_w = [&](int kb, uint32_t st) {
         const uint32_t sw = smem0 + st * stage_bytes, bar = full0 + st * 8u;
         const int k0 = kb * kBK;
         if (leader) mbar_expect_tx(&full_bar[st], 2 * bytes);
         if (MODE == GEMM_GATE_UP) {
-          tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
-          tma_load_3d_bar(sw + kAtomBytes, &tma_w1, 0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+          atoms(sw, &tma_w0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+          atoms(sw + kAtomBytes, &tma_w1, wrow + k0, ti.n0 / 64 + (int)cr, bar);
         } else if (MODE == GEMM_DOWN) {
-          tma_load_3d_bar(sw, &tma_w0, 0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
+          atoms(sw, &tma_w0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
         } else {
           const int kh = args.K / 2;               // DGRAD_GU: first half of K from Wg, second from Wu
-          if (MODE == GEMM_DGRAD_GU && k0 >= kh) tma_load_2d_bar(sw, &tma_w1, k0 - kh, wrow + ti.n0 + (int)cr * 128, bar);
-          else tma_load_2d_bar(sw, &tma_w0, k0, wrow + ti.n0 + (int)cr * 128, bar);
+          if (MODE == GEMM_DGRAD_GU && k0 >= kh) rows(sw, &tma_w1, k0 - kh, wrow + ti.n0 + (int)cr * 128, bar);
+          else rows(sw, &tma_w0, k0, wrow + ti.n0 + (int)cr * 128, bar);
         }
       };
       auto load_x = [&](int kb, uint32_t st) {
@@ -532,9 +550,12 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   // groups are half as large as the line on average, so that some may be above it. All G groups count: a layer passes its
   // slots for replicas too, which hold no row on one rank, so that there the average expert has to reach the line itself.
   const bool bands = a_rows * args.K * 2 > (int64_t)args.G * (tp::kXBytes / 2);
+  const int64_t groups = args.tokens_n > 0 ? args.tokens_n : args.G;
+  const bool streams = groups * (mode == GEMM_DGRAD_GU ? args.K / 2 : args.K) * args.N * 2 >= tp::kStreamBytes && a_rows <= groups * tp::kStreamRows;
 #define MEP_TP_CASE(M)                                                                                          \
   case M: {                                                                                                     \
-    auto* kernel = bands ? tp::tok_pair_kernel<M, true> : tp::tok_pair_kernel<M, false>;                           \
+    auto* kernel = bands ? tp::tok_pair_kernel<M, tp::BANDED>                                                        \
+                         : streams ? tp::tok_pair_kernel<M, tp::STREAM> : tp::tok_pair_kernel<M, tp::PLAIN>; \
     if (allow_smem((const void*)kernel, tp::kSmem)) return -1;                                                  \
     MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, mx, mx64, mx16, mw0, mw1, mo, mo2, args));                  \
     break;                                                                                                      \

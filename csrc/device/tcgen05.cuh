@@ -94,6 +94,7 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sm
 }
 // The same for data that nobody reads soon: its lines leave L2 before those of the operands.
 __device__ __forceinline__ uint64_t evict_first() { uint64_t p; asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p)); return p; }
+__device__ __forceinline__ uint64_t evict_normal() { uint64_t p; asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p)); return p; }
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t smem_src, int c0, int c1, uint64_t policy) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%1, %2}], [%3], %4;"
                :: "l"(map), "r"(c0), "r"(c1), "r"(smem_src), "l"(policy) : "memory");

@@ -455,3 +455,39 @@ def test_counts_that_fall_give_no_tiles(cuda_device):
         assert _rel(out[:128], x[:128].float() @ ref[0].float()) < 4e-3 and _rel(out[256:], x[256:].float() @ ref[2].float()) < 4e-3
     assert _rel(dW[0], x[:256].float().T @ dy[:256].float()) < 1e-4 and _rel(dW[2], x[128:].float().T @ dy[128:].float()) < 1e-4
     assert bool((dW[1] == 7.0).all())
+
+
+@pytest.mark.parametrize("K", [1984, 2048], ids=["kept", "streamed"])
+def test_weights_that_are_read_once(K, cuda_device):
+    """From 32 MiB of matrices on (8 of 2048 x 1024) the weights of groups with one token tile leave L2 first: the same bits as group by group, where
+    they never do, with tiles that share their weights in between."""
+    from moonep_b200.ops import grouped_gemm as gg
+    N, n = 1024, [1, 32, 256, 257, 0, 600, 255, 512]
+    p = [(r + 127) // 128 * 128 for r in n]
+    ends = torch.tensor(p).cumsum(0)
+    pad = torch.tensor([[int(e) - q + r, q - r] if q > r else [0, 0] for r, q, e in zip(n, p, ends)], dtype=torch.int32)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    x, h, w, wu = bf(sum(p), K), bf(sum(p), 2 * N), bf(8, K, N, sc=0.02), bf(8, K, N, sc=0.02)
+    wt = w.transpose(1, 2).contiguous()
+
+    def run(x, h, w, wu, wt, cu, pad):
+        out = [torch.zeros(len(x), c, dtype=torch.bfloat16, device="cuda") for c in (N, 2 * N, N, N)]
+        kw = dict(pad=pad.cuda())
+        gg.gate_up(x, w, wu, cu.cuda(), out[0], out[1], **kw)
+        gg.down(x, w, cu.cuda(), out[2], **kw)
+        gg.dgrad(x, wt, cu.cuda(), out[3], **kw)
+        if K % 256 == 0:
+            out.append(torch.zeros(len(x), K, dtype=torch.bfloat16, device="cuda"))
+            gg.dgrad_gate_up(h, w, wu, cu.cuda(), out[4], **kw)
+        return out
+
+    got = run(x, h, w, wu, wt, ends.to(torch.int32), pad)
+    for i, (q, e) in enumerate(zip(p, ends.tolist())):
+        if q:
+            s, one = slice(e - q, e), torch.tensor([q], dtype=torch.int32)
+            table = torch.tensor([[n[i], q - n[i]] if q > n[i] else [0, 0]], dtype=torch.int32)
+            for a, b in zip(got, run(x[s].contiguous(), h[s].contiguous(), w[i:i + 1], wu[i:i + 1], wt[i:i + 1], one, table)):
+                assert torch.equal(a[s], b), f"group {i} ({n[i]} rows)"
+    torch.cuda.synchronize()
+    gg.check_status()
