@@ -22,15 +22,16 @@ constexpr int kLocMaxSlots = 8;            // row slots per copying warp
 
 // Up to this many entries every CTA counts all entries before its own by itself, above it the CTAs hand over their
 // histograms. Counting costs a CTA all entries before its own, the hand-over two round trips to L2 and CTAs x E counts. Own
-// count against hand-over (K=8, caches flushed), in us:
-//   entries                12288        20480        24576        28672        32768        49152
-//   H=512,  E=64        16.4 / 23.6  20.5 / 24.6  24.6 / 26.6  26.6 / 27.5  28.7 / 29.7  38.9 / 33.7
-//   H=2048, E=16        22.5 / 28.7  29.6 / 32.9  34.9 / 37.8  38.9 / 41.0  45.2 / 45.1  65.5 / 61.4
-//   H=2048, E=256       35.8 / 45.1  42.0 / 50.2  47.2 / 51.2  49.2 / 54.3  55.3 / 55.3  74.8 / 70.7
-//   H=7168, E=16        45.1 / 49.2  73.7 / 75.8  88.1 / 90.1   102 / 102    115 / 112    168 / 163
-//   H=7168, E=64        53.2 / 53.3  79.0 / 77.8  92.2 / 88.2   107 / 105    119 / 117    174 / 166
-// The two cross between 24576 and 32768 for short rows and between 16384 and 28672 for long ones, whatever E is.
-constexpr int kLocDirect = 24576;
+// count against hand-over, a dispatch with K=8 among others of its kind, in us:
+//   entries             12288        18432        24576        32768        49152        65536        131072
+//   H=512,  E=64      9.9 / 18.3  11.8 / 19.7  14.0 / 21.0  16.8 / 21.9  23.4 / 27.7  29.0 / 32.3  61.8 / 53.8
+//   H=2048, E=16     14.5 / 22.5  19.9 / 25.0  27.5 / 33.9  35.7 / 42.1  52.9 / 57.3  67.9 / 71.5   134 / 129
+//   H=2048, E=256    30.5 / 41.4  35.1 / 47.3  40.7 / 47.8  47.7 / 53.8  66.3 / 69.9  80.9 / 83.5   148 / 146
+//   H=4096, E=60     29.3 / 32.7  38.3 / 42.0  51.6 / 53.1  66.0 / 68.0  96.8 / 96.8   125 / 124    245 / 239
+//   H=7168, E=32     41.1 / 43.4  61.2 / 62.9  78.8 / 82.0   105 / 106    155 / 155    204 / 204
+// So the line is lower for long rows, at this many elements of all rows (4096, 7168, 8, E=32 with its combine: 197.0 / 195.8).
+constexpr int kLocDirect = 65536, kLocDepth = 16;      // kLocDepth: entries that a thread has on their way when it counts
+constexpr long long kLocDirectElems = 24576ll * 7168;
 
 // A large batch of a saved plan is copied by many short CTAs, two or three to an SM, that the hardware hands out as SMs come free: SMs
 // are not equally far from memory, and with one CTA for each the last was done 10 % after the average. Bytes that a CTA moves, and
@@ -136,11 +137,27 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
         if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
         else report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, i, (uint32_t)e, (uint32_t)E);
       }
-    } else if (t0 < t1) {                    // all entries before them
+    } else if (t0 < t1) {
+      // All entries before them. The CTAs read the same ones: each begins at another place, else the slices of L2 that hold the first entries
+      // serve 148 SMs at once and the others none. That and sixteen loads in flight instead of eight: 18432 entries, H=4096, E=60 41.1 -> 38.3 us;
+      // 32768, H=2048, E=16 47 -> 35.7. (Counting by ballots over the bits of the numbers, without atomics: 39.0.)
+      const int n = t0 * K, rounds = n <= 8 * kLocThreads ? 0 : (n + kLocThreads * kLocDepth - 1) / (kLocThreads * kLocDepth);
+      if (!rounds) {                         // a decode batch: without the code for sixteen loads, which every launch would fetch anew
 #pragma unroll 8
-      for (int i = tid; i < t0 * K; i += kLocThreads) {
-        const int e = __ldg(a.topk + i);
-        if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
+        for (int i = tid; i < n; i += kLocThreads) {
+          const int e = __ldg(a.topk + i);
+          if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
+        }
+      }
+      int at = rounds ? vb % rounds : 0;
+      for (int r = 0; r < rounds; ++r) {
+        const int i0 = at * (kLocThreads * kLocDepth) + tid;
+        if (++at == rounds) at = 0;
+        int e[kLocDepth];
+#pragma unroll
+        for (int d = 0; d < kLocDepth; ++d) e[d] = i0 + d * kLocThreads < n ? __ldg(a.topk + i0 + d * kLocThreads) : -1;
+#pragma unroll
+        for (int d = 0; d < kLocDepth; ++d) if ((unsigned)e[d] < (unsigned)E) atomicAdd(&s_cnt[e[d]], 1);
       }
     }
     total_pad = local_layout(a.tpe, E, pad, a.pad_step, s_start, s_padpre, s_warp);
@@ -448,7 +465,7 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
     const int tokens = warps * (each < 1 ? 1 : (int)each);
     num_blocks = (S + tokens - 1) / tokens;
   }
-  if (fresh && S * K <= kLocDirect) return launch_plain(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+  if (fresh && S * K <= kLocDirect && (long long)S * K * H <= kLocDirectElems) return launch_plain(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
   if (fresh) return launch_plain(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
   return launch_plain(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
 }

@@ -22,8 +22,8 @@ CASES = [
     (333,    5,  5,    7168,  128, "single_expert"),
     (64,     8,  8,    15360, 128, "biased"),
     (20000,  8,  32,   64,    128, "biased"),
-    (3072,   8,  64,   128,   16,  "random"),     # 24576 entries: the last size at which every CTA counts for itself
-    (3511,   7,  64,   128,   16,  "random"),     # 24577: the first with the hand-over
+    (3072,   8,  64,   128,   16,  "random"),     # 24576 entries: counted in six whole rounds of 4096
+    (3511,   7,  64,   128,   16,  "random"),     # 24577
 ]
 
 
@@ -135,6 +135,20 @@ def test_padding_rows_are_counted(cuda_device):
         blk.forward(y)
     assert blk.buf.counters()["padding_rows_cleared"] == int((-tpe % 32).sum())
     blk.destroy()
+
+
+# Every CTA counts the entries before its own up to 65536 of them, in rounds of 4096; above that the CTAs hand over their histograms.
+COUNT_CASES = [
+    (4097,   1,  8,    64,    16,  "random"),
+    (4213,   2,  300,  16,    1,   "biased"),
+    (8192,   8,  64,   128,   16,  "random"),
+    (9363,   7,  64,   64,    16,  "biased"),
+]
+
+
+@pytest.mark.parametrize("case", COUNT_CASES, ids=lambda c: "S%d_K%d_E%d_H%d" % c[:4])
+def test_local_exchange_at_the_ends_of_counting(case, cuda_device):
+    test_local_exchange(case, cuda_device)
 
 
 # Large batches (200 MiB moved): the saved plan's rows come from many short CTAs and the combine begins with the last tokens. Just above
