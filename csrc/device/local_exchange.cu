@@ -15,10 +15,13 @@
 
 namespace mep {
 
+// Tables and weights are read by ordinary loads: a launch may begin while the kernel that writes them still runs, and the read-only path (ld.nc) asks
+// for memory that nobody writes while the kernel is there.
 constexpr int kLocThreads = 256, kLocWarps = kLocThreads / 32;
 constexpr int kLocEntries = 1024;          // top-k entries ranked and copied at a time by one CTA
 constexpr int kLocZeroBytes = 4096;        // zeroed shared memory the padding rows are stored from
 constexpr int kLocMaxSlots = 8;            // row slots per copying warp
+constexpr size_t kLocAlone = 115 * 1024;   // dynamic shared memory of which an SM has no room for two CTAs
 
 // Up to this many entries every CTA counts all entries before its own by itself, above it the CTAs hand over their
 // histograms. Counting costs a CTA all entries before its own, the hand-over two round trips to L2 and CTAs x E counts. Own
@@ -50,7 +53,7 @@ __device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int per = (E + kLocThreads - 1) / kLocThreads, e0 = tid * per, e1 = min(e0 + per, E);
   int rows = 0, pads = 0;
-  for (int e = e0; e < e1; ++e) { const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad; rows += p; pads += local_pads(n, p - n, step); }
+  for (int e = e0; e < e1; ++e) { const int n = tpe[e], p = (n + pad - 1) / pad * pad; rows += p; pads += local_pads(n, p - n, step); }
   int ri = warp_incl_scan(rows), pi = warp_incl_scan(pads);
   if (lane == 31) { s_warp[warp] = ri; s_warp[kLocWarps + warp] = pi; }
   __syncthreads();
@@ -61,7 +64,7 @@ __device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, 
   }
   rb += ri - rows; pb += pi - pads;
   for (int e = e0; e < e1; ++e) {
-    const int n = __ldg(tpe + e), p = (n + pad - 1) / pad * pad;
+    const int n = tpe[e], p = (n + pad - 1) / pad * pad;
     start[e] = rb; padpre[e] = pb; rb += p; pb += local_pads(n, p - n, step);
   }
   return total;
@@ -81,7 +84,6 @@ template <int MODE>                        // 0: saved plan
 __global__ void __launch_bounds__(kLocThreads, MODE ? 1 : 3)
 local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, int copy_warps, int slots) {
   constexpr bool FRESH = MODE != 0, SHARED = MODE == 2;
-  pdl_trigger();                             // a GEMM behind this kernel may set itself up meanwhile
   const MepRankCtx c = *cp;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLocWarps * kLocMaxSlots];
@@ -98,16 +100,19 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   int* s_padpre = s_start + ngroups;
   int* s_cnt = s_padpre + ngroups;           // FRESH [E]: histogram, then next free row of expert e for this CTA's entries
 
-  if (tid == 0) {
-    s_fail = 0;
-    s_vb = SHARED ? (int)atomicAdd(&a.sync[1], 1u) : (int)blockIdx.x;
-    trace_mark(c, MEP_K_DISPATCH, 1);
-  }
   if (tid < kLocWarps * kLocMaxSlots) mbar_init(&s_bar[tid], 1);
   fence_mbar_init();
   for (int i = tid; i < kLocZeroBytes / 16; i += kLocThreads) reinterpret_cast<int4*>(s_zero)[i] = make_int4(0, 0, 0, 0);
   fence_proxy_async();
   if (FRESH) for (int e = tid; e < E; e += kLocThreads) s_cnt[e] = 0;
+  // Up to here the kernel right before may still run, whatever it is. A GEMM behind this kernel may set itself up and load weights as soon as that one is done.
+  pdl_wait();
+  pdl_trigger();
+  if (tid == 0) {
+    s_fail = 0;
+    s_vb = SHARED ? (int)atomicAdd(&a.sync[1], 1u) : (int)blockIdx.x;
+    trace_mark(c, MEP_K_DISPATCH, 1);
+  }
   __syncthreads();
   const int vb = s_vb;
   const uint32_t ep = SHARED ? *(volatile uint32_t*)&a.sync[0] + 1u : 0u;
@@ -133,7 +138,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   if (FRESH) {
     if (SHARED) {                            // own entries
       for (int i = t0 * K + tid; i < t1 * K; i += kLocThreads) {
-        const int e = __ldg(a.topk + i);
+        const int e = a.topk[i];
         if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
         else report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, i, (uint32_t)e, (uint32_t)E);
       }
@@ -143,11 +148,11 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
       // 32768, H=2048, E=16 47 -> 35.7. (Counting by ballots over the bits of the numbers, without atomics: 39.0.)
       const int n = t0 * K, rounds = n <= 8 * kLocThreads ? 0 : (n + kLocThreads * kLocDepth - 1) / (kLocThreads * kLocDepth);
       if (!rounds) {                         // a decode batch: without the code for sixteen loads, which every launch would fetch anew
-#pragma unroll 8
-        for (int i = tid; i < n; i += kLocThreads) {
-          const int e = __ldg(a.topk + i);
-          if ((unsigned)e < (unsigned)E) atomicAdd(&s_cnt[e], 1);
-        }
+        int e[8];
+#pragma unroll
+        for (int d = 0; d < 8; ++d) e[d] = tid + d * kLocThreads < n ? a.topk[tid + d * kLocThreads] : -1;
+#pragma unroll
+        for (int d = 0; d < 8; ++d) if ((unsigned)e[d] < (unsigned)E) atomicAdd(&s_cnt[e[d]], 1);
       }
       int at = rounds ? vb % rounds : 0;
       for (int r = 0; r < rounds; ++r) {
@@ -155,7 +160,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
         if (++at == rounds) at = 0;
         int e[kLocDepth];
 #pragma unroll
-        for (int d = 0; d < kLocDepth; ++d) e[d] = i0 + d * kLocThreads < n ? __ldg(a.topk + i0 + d * kLocThreads) : -1;
+        for (int d = 0; d < kLocDepth; ++d) e[d] = i0 + d * kLocThreads < n ? a.topk[i0 + d * kLocThreads] : -1;
 #pragma unroll
         for (int d = 0; d < kLocDepth; ++d) if ((unsigned)e[d] < (unsigned)E) atomicAdd(&s_cnt[e[d]], 1);
       }
@@ -170,7 +175,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
     if (vb == nb - 1) {          // the CTA with the least to copy writes the tables that only depend on the counts
       for (int g = tid; g < 2 * E; g += kLocThreads) {
         const int e = g < E ? g : E - 1;
-        const int n = __ldg(a.tpe + e), p = (n + pad - 1) / pad * pad;
+        const int n = a.tpe[e], p = (n + pad - 1) / pad * pad;
         a.cu_seqlens[g] = s_start[e] + p;
         const bool has = g < E && p > n;
         a.zero_fill[2 * g] = has ? s_start[e] + n : 0;
@@ -184,8 +189,8 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
     int run = 0;
     for (int g0 = 0; g0 < ngroups; g0 += kLocThreads) {
       const int g = g0 + tid;
-      const int first = g < ngroups ? __ldg(a.zero_fill + 2 * g) : 0;
-      const int n = g < ngroups ? local_pads(first, __ldg(a.zero_fill + 2 * g + 1), a.pad_step) : 0;
+      const int first = g < ngroups ? a.zero_fill[2 * g] : 0;
+      const int n = g < ngroups ? local_pads(first, a.zero_fill[2 * g + 1], a.pad_step) : 0;
       if (g < ngroups) s_start[g] = first;
       const int incl = warp_incl_scan(n);
       if (lane == 31) s_warp[warp] = incl;
@@ -204,7 +209,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
       int lo = 0, hi = ngroups - 1;          // last group with padpre <= z
       while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (s_padpre[mid] <= z) lo = mid; else hi = mid - 1; }
       int row = s_start[lo] + (z - s_padpre[lo]);
-      if (FRESH) row += __ldg(a.tpe + lo);
+      if (FRESH) row += a.tpe[lo];
       if ((unsigned)row >= (unsigned)NvS) report(c, MEP_ERR_BOUNDS, MEP_K_DISPATCH, 40, lo, (uint32_t)row, (uint32_t)NvS);
       else {
         char* p = (char*)a.out_hidden + (size_t)row * row_bytes;
@@ -257,7 +262,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
     if (FRESH) {
       for (int i0 = 0; i0 < n; i0 += kLocThreads) {
         const int i = i0 + tid;
-        int e = i < n ? __ldg(a.topk + (size_t)c0 * K + i) : -1;
+        int e = i < n ? a.topk[(size_t)c0 * K + i] : -1;
         if ((unsigned)e >= (unsigned)E) {
           if (MODE == 1 && i < n) report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 1, c0 * K + i, (uint32_t)e, (uint32_t)E);
           e = -1;
@@ -276,7 +281,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
           __syncthreads();
         }
         if (i < n) {
-          if (e >= 0 && (row >= s_start[e] + __ldg(a.tpe + e) || (unsigned)row >= (unsigned)NvS)) {   // counts that are not those of topk
+          if (e >= 0 && (row >= s_start[e] + a.tpe[e] || (unsigned)row >= (unsigned)NvS)) {   // counts that are not those of topk
             report(c, MEP_ERR_BOUNDS, MEP_K_PLANNING, 2, c0 * K + i, (uint32_t)row, (uint32_t)NvS);
             row = -1;
           }
@@ -285,7 +290,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
       }
     } else {
       for (int i = tid; i < n; i += kLocThreads) {
-        const int d = __ldg(a.dst + (size_t)c0 * K + i);
+        const int d = a.dst[(size_t)c0 * K + i];
         int row = d >= 0 ? d : -d - 1;
         if (row >= NvS) { report(c, MEP_ERR_BOUNDS, MEP_K_DISPATCH, 41, c0 + i / K, (uint32_t)row, (uint32_t)NvS); row = -1; }
         s_slot[i] = row;
@@ -386,7 +391,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   const int units = cp->S * nparts, step = gridDim.x * kLcWarps;
   int u = blockIdx.x * kLcWarps + warp;
   auto unit = [&](int x) { return LAST_FIRST ? units - 1 - x : x; };
-  auto fetch = [&](int x) { return x < units && lane < K ? __ldg(a.dst + (size_t)(unit(x) / nparts) * K + lane) : 0; };
+  auto fetch = [&](int x) { return x < units && lane < K ? a.dst[(size_t)(unit(x) / nparts) * K + lane] : 0; };
   // loads of unit x (plan entry d in lane k) into half h; returns the lanes whose entry names a row
   auto issue = [&](int at, int d, int h) {
     const int x = unit(at);
@@ -394,7 +399,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
     const uint32_t bytes = (uint32_t)min(part_vecs, nvec - vb) * 16u;
     const int row = d >= 0 ? d : -d - 1;
     const unsigned valid = __ballot_sync(0xffffffffu, lane < K && row < NvS);
-    if (a.out_weights && part == 0 && lane < K) a.out_weights[(size_t)(x / nparts) * K + lane] = row < NvS ? __ldg(a.weights + row) : 0.f;
+    if (a.out_weights && part == 0 && lane < K) a.out_weights[(size_t)(x / nparts) * K + lane] = row < NvS ? a.weights[row] : 0.f;
     if (lane == 0) mbar_expect_tx(&bars[h], bytes * (uint32_t)__popc(valid));
     __syncwarp();                              // also: every lane has finished reading this half
     if ((valid >> lane) & 1u)
@@ -446,7 +451,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
 // `num_blocks`: most CTAs; from `sms` on (those of the device, with a CTA for each) the launch may have more, see kLocShort. fresh: plan from
 // topk / tpe as well; else a.dst / a.zero_fill are read.
 extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::LocalDispatchArgs* args, int fresh,
-                                         int num_blocks, int sms, int S, int K, int H, int E, cudaStream_t stream) {
+                                         int num_blocks, int sms, int S, int K, int H, int E, int pdl, cudaStream_t stream) {
   using namespace mep;
   const size_t row = (size_t)H * 2;
   const size_t tables = (size_t)(fresh ? 3 : 4) * E * sizeof(int);
@@ -459,15 +464,18 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
   int slots = all / warps < kLocMaxSlots ? all / warps : kLocMaxSlots;
   // the fewest slots that still hold `ring` bytes of rows per CTA: more buys nothing, and a smaller footprint starts sooner
   while (slots > 2 && (size_t)warps * (slots - 1) * row >= ring) --slots;
-  const size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
+  size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
+  // A programmatic launch is placed as the SMs of the kernel before come free: without this the first of them would get two CTAs and the last none
+  // (8000 x 8, H=1024 with its combine 80.6 us instead of 71)
+  if (pdl && !large && smem < kLocAlone) smem = kLocAlone;
   if (large) {                               // the same number of tokens for each warp
     const long long each = kLocShort / ((long long)row * (K + 1) * warps);
     const int tokens = warps * (each < 1 ? 1 : (int)each);
     num_blocks = (S + tokens - 1) / tokens;
   }
-  if (fresh && S * K <= kLocDirect && (long long)S * K * H <= kLocDirectElems) return launch_plain(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
-  if (fresh) return launch_plain(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
-  return launch_plain(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, ctx, *args, warps, slots);
+  if (fresh && S * K <= kLocDirect && (long long)S * K * H <= kLocDirectElems) return launch_plain_pdl(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, *args, warps, slots);
+  if (fresh) return launch_plain_pdl(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, *args, warps, slots);
+  return launch_plain_pdl(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, *args, warps, slots);
 }
 
 extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalCombineArgs* args, int num_blocks,

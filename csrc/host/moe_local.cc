@@ -5,7 +5,7 @@
 #include "launch.h"
 
 extern "C" {
-int mep_launch_local_dispatch(const MepRankCtx*, const mep::LocalDispatchArgs*, int, int, int, int, int, int, int, cudaStream_t);
+int mep_launch_local_dispatch(const MepRankCtx*, const mep::LocalDispatchArgs*, int, int, int, int, int, int, int, int, cudaStream_t);
 int mep_launch_local_combine(const MepRankCtx*, const mep::LocalCombineArgs*, int, int, int, int, int, int, cudaStream_t);
 int mep_grouped_gemm_2cta(int, const void*, int64_t, int64_t, int64_t, const void*, const void*, int64_t, int64_t, int64_t,
                           const mep::GemmArgs*, int, cudaStream_t);
@@ -15,7 +15,7 @@ int mep_swiglu_bwd(const void*, const void*, const float*, void*, float*, const 
 
 namespace mep {
 
-// A pass begins with a dispatch, an ordinary launch that begins when everything before it in the stream is done. Weights, and the
+// A pass begins with a dispatch, which lets the next launch begin when everything before it in the stream is done. Weights, and the
 // plan of a backward pass, are therefore complete before any GEMM of the pass begins, and so are the token counts that a forward
 // pass is given (`tpe`; its plan is written by the dispatch).
 static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab, const int32_t* tpe = nullptr) {
@@ -66,7 +66,7 @@ extern "C" int mep_local_dispatch_call(const mep::MoeLocal* mp, const void* hidd
   d.out_hidden = (__nv_bfloat16*)rows; d.out_weights = row_w; d.out_srcinfo = m.srcinfo;
   d.dst = dst; d.zero_fill = zero_fill;
   if (topk) plan_into(m, topk, tpe, slab, &d);
-  return mep_launch_local_dispatch(m.ctx, &d, topk ? 1 : 0, m.blocks, m.sms, m.S, m.K, m.H, m.E, stream);
+  return mep_launch_local_dispatch(m.ctx, &d, topk ? 1 : 0, m.blocks, m.sms, m.S, m.K, m.H, m.E, m.pdl, stream);
 }
 
 extern "C" int mep_local_combine_call(const mep::MoeLocal* mp, const int32_t* dst, const void* rows, const float* row_w, void* out, float* out_w,
@@ -74,7 +74,7 @@ extern "C" int mep_local_combine_call(const mep::MoeLocal* mp, const int32_t* ds
   using namespace mep;
   const MoeLocal& m = *mp;
   LocalCombineArgs c = {dst, (const __nv_bfloat16*)rows, row_w, (__nv_bfloat16*)out, out_w};
-  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, 0, m.in_order && m.combine_blocks >= m.sms, stream);
+  return mep_launch_local_combine(m.ctx, &c, m.combine_blocks, m.S, m.H, m.K, m.pdl, m.in_order && m.combine_blocks >= m.sms, stream);
 }
 
 extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden, const float* route_w, const int32_t* topk,
@@ -86,7 +86,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   LocalDispatchArgs d = dispatch_args(m, hidden, slab);
   d.weights = route_w; d.out_hidden = x; d.out_weights = w;
   plan_into(m, topk, tpe, slab, &d);
-  if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.sms, m.S, m.K, m.H, m.E, stream)) return -1;
+  if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.sms, m.S, m.K, m.H, m.E, m.pdl, stream)) return -1;
   GemmArgs g = gemm_args(m, slab, tpe);
   g.N = m.Hp; g.K = m.H; g.out = m.act; g.out2 = keep ? m.gu : nullptr; g.row_scale = w; g.ldo = m.Hp;
   if (gemm(m, GEMM_GATE_UP, x, m.H, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
@@ -104,7 +104,7 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   const MoeLocal& m = *mp;
   LocalDispatchArgs d = dispatch_args(m, dy, slab);
   d.out_hidden = m.shard;
-  if (mep_launch_local_dispatch(m.ctx, &d, 0, m.blocks, m.sms, m.S, m.K, m.H, m.E, stream)) return -1;
+  if (mep_launch_local_dispatch(m.ctx, &d, 0, m.blocks, m.sms, m.S, m.K, m.H, m.E, m.pdl, stream)) return -1;
   GemmArgs g = gemm_args(m, slab);
   g.N = m.Hp; g.K = m.H; g.out = m.dA; g.ldo = m.Hp;
   if (gemm(m, GEMM_DGRAD, m.shard, m.H, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;

@@ -194,6 +194,9 @@ class OpsMixin:
         ex = getattr(self, "_local_ex", None)
         if ex is None:
             ex = self._local_ex = engine.LocalExchange(self._states[0], self._num_sms_dedup)
+        pdl = getattr(self, "enable_pdl", False)
+        if ex.pdl is not pdl:
+            ex.set_pdl(pdl)
         return ex
 
     def _dispatch_local(self, hidden, weights, topk, tpe, plan, zero_copy=False, w_zero_copy=False, out=None):

@@ -249,6 +249,7 @@ class LocalExchange:
         self._args_in_order = _native.MoeLocal.from_buffer_copy(a)
         self._args_in_order.in_order = 1
         self._ref_in_order = C.addressof(self._args_in_order)
+        self.pdl = False                    # see set_pdl
         self._ints = dict(N=g.N, R=g.R, E=g.E, NvS=g.NvS, K=g.K)
         # shape, strides and first element of each part: one as_strided call costs a third of narrow and view
         self._fields = dict(dst=((g.N,), (1,), first[0]), experts_to_copy=((1, g.epn), (g.epn, 1), first[1]),
@@ -258,6 +259,10 @@ class LocalExchange:
         self._rows_like = st.hidden_local.narrow(0, 0, g.S)
         self._weights_like = st.weights_local.as_strided((g.S, g.K), (g.K, 1))
         self._lib = _native.load()
+
+    def set_pdl(self, pdl: bool):
+        """Whether a call's kernel may set itself up while the kernel before it in the stream still runs."""
+        self.pdl = self._args.pdl = self._args_in_order.pdl = bool(pdl)
 
     def _name_part(self, slab, name):
         f = self._fields.get(name)

@@ -186,3 +186,36 @@ def test_saved_plan_of_a_large_batch_keeps_to_the_sm_limit(limit, cuda_device, m
     rows = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long()
     assert torch.equal(again.view(torch.int16)[rows], h.view(torch.int16)[rows])
     buf.destroy()
+
+
+@pytest.mark.parametrize("pdl", [False, True], ids=["plain", "pdl"])
+@pytest.mark.parametrize("shape", [(64, 8, 16, 256), (4000, 4, 32, 1024), (9000, 8, 16, 64), (2048, 8, 48, 5696)], ids=str)
+def test_queued_calls_see_what_the_kernel_before_wrote(shape, pdl, cuda_device):
+    """Launches may begin while the one before still runs: batches queued without a pause, each routed and filled by kernels right in front of its
+    calls, give what they give one at a time. ``enable_pdl`` may be changed in between."""
+    S, K, E, H = shape
+    buf = Buffer(S, H, K, E, 1, token_padding=16, enable_pdl=not pdl)
+    buf.enable_pdl = pdl
+    base = torch.randn(S, H, device="cuda").to(torch.bfloat16)
+    tables = [tuple(t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=s)) for s in (1, 2, 3)]
+    x, topk, tpe = torch.empty_like(base), torch.empty_like(tables[0][0]), torch.empty_like(tables[0][1])
+
+    def batch(i):
+        torch.mul(base, 1.0 + 0.25 * (i % 5), out=x)
+        tpe.copy_(tables[i % 3][1])
+        torch.add(tables[i % 3][0], 0, out=topk)
+        h, _, _, plan = buf.dispatch(x, None, topk, tpe, zero_copy=True)
+        y = buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)[0]
+        h, _, _, _ = buf.dispatch(y, plan=plan, zero_copy=True)
+        return y, buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)[0]
+
+    want = []
+    for i in range(12):
+        want.append([t.clone() for t in batch(i)])
+        torch.cuda.synchronize()
+    got = [batch(i) for i in range(12)]
+    torch.cuda.synchronize()
+    buf.check()
+    for a, b in zip(got, want):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    buf.destroy()
