@@ -53,6 +53,9 @@ constexpr int kSortRounds = 12;
 // 2048 x 768, 8 (25) 36.5 / 34.9. Only where few groups have more than one tile (kStreamRows rows in a group on average; a layer allows 127 for padding):
 // the hint costs the others 1 % (1531, 2048 x 768, 16 152.2 / 150.2), and not for tiles that share weights, as pairs are not in step: gate/up of 32 experts and 4096
 // tokens x 8, 7168 x 2048, then reads 6.2 GB instead of 3.4 and takes 2.04 ms instead of 1.80.
+// Its stages are 128 deep: one load brings a column atom's weights of both k-blocks and one pair of barriers serves them. What a round that does not fill
+// the GPU takes is the producer's issue (about 450 cycles a k-block and 58 GB/s per SM before): 64 tokens, 2048 x 768, 16 experts 45.1 -> 43.8
+// us; 8 tokens, 4096 x 1536, 32 162.6 -> 156.1; 256, 7168 x 2048, 32 462.1 -> 459.2.
 constexpr int64_t kStreamBytes = 32 << 20, kStreamRows = 320;
 enum Kind { PLAIN, BANDED, STREAM };                   // a kernel each: code that a launch does not need costs it 1 to 2 us of 50
 constexpr int kStgSet = 4 * kStgBytes;                 // GATE_UP: act twice, gate, up; else: two buffers for each 64-column side
@@ -108,7 +111,8 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   __shared__ float s_scale[2][2][128];   // [set][accumulator]: row factors of the set's chunks
   __shared__ int s_half;                 // most token rows a CTA stages for a tile of this launch
-  const int G = args.G, kblocks = args.K / kBK;
+  constexpr int kSub = KIND == STREAM ? 2 : 1;           // 64-deep k-blocks of a stage
+  const int G = args.G, kblocks = args.K / (kSub * kBK);
   pdl_trigger();
 
   if (warp == 1) {
@@ -170,7 +174,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   // weights, and what an SM has in flight is its bandwidth.
   const bool small = s_half <= 48;
   const uint32_t x_bytes = small ? max(s_half, 16) * 128u : s_half <= 64 ? 8192u : 16384u;
-  const uint32_t stage_bytes = ((uint32_t)kWBytes + x_bytes + 1023u) & ~1023u;
+  const uint32_t stage_bytes = kSub * (((uint32_t)kWBytes + x_bytes + 1023u) & ~1023u);
   const uint32_t nstages = min((uint32_t)kMaxRing, (uint32_t)kRingBytes / stage_bytes);
 
   auto note = [&](int site, int tile, int code) {
@@ -242,7 +246,7 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         fence_proxy_async();
       }
       const int half = ti.n >> 1, xrow = ti.row0 + (int)cr * half, wrow = ti.g * args.b_group_rows;
-      const uint32_t bytes = (uint32_t)kWBytes + (small ? (uint32_t)half * 128u : half > 64 ? 16384u : 8192u);
+      const uint32_t bytes = kSub * ((uint32_t)kWBytes + (small ? (uint32_t)half * 128u : half > 64 ? 16384u : 8192u));
       const uint64_t policy = ti.once ? streamed : kept;
       auto atoms = [&](uint32_t dst, const CUtensorMap* map, int k, int atom, uint32_t bar) {
         if (KIND == STREAM) tma_load_3d_bar(dst, map, 0, k, atom, bar, policy); else tma_load_3d_bar(dst, map, 0, k, atom, bar);
@@ -252,28 +256,36 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       };
       auto load_w = [&](int kb, uint32_t st) {
         const uint32_t sw = smem0 + st * stage_bytes, bar = full0 + st * 8u;
-        const int k0 = kb * kBK;
+        const int k0 = kb * kSub * kBK;
         if (leader) mbar_expect_tx(&full_bar[st], 2 * bytes);
         if (MODE == GEMM_GATE_UP) {
           atoms(sw, &tma_w0, wrow + k0, ti.n0 / 64 + (int)cr, bar);
-          atoms(sw + kAtomBytes, &tma_w1, wrow + k0, ti.n0 / 64 + (int)cr, bar);
+          atoms(sw + kSub * kAtomBytes, &tma_w1, wrow + k0, ti.n0 / 64 + (int)cr, bar);
         } else if (MODE == GEMM_DOWN) {
           atoms(sw, &tma_w0, wrow + k0, ti.n0 / 64 + 2 * (int)cr, bar);
         } else {
           const int kh = args.K / 2;               // DGRAD_GU: first half of K from Wg, second from Wu
-          if (MODE == GEMM_DGRAD_GU && k0 >= kh) rows(sw, &tma_w1, k0 - kh, wrow + ti.n0 + (int)cr * 128, bar);
-          else rows(sw, &tma_w0, k0, wrow + ti.n0 + (int)cr * 128, bar);
+#pragma unroll
+          for (int i = 0; i < kSub; ++i) {
+            const int k = k0 + i * kBK;
+            if (MODE == GEMM_DGRAD_GU && k >= kh) rows(sw + i * kWBytes, &tma_w1, k - kh, wrow + ti.n0 + (int)cr * 128, bar);
+            else rows(sw + i * kWBytes, &tma_w0, k, wrow + ti.n0 + (int)cr * 128, bar);
+          }
         }
       };
       auto load_x = [&](int kb, uint32_t st) {
-        const uint32_t sx = smem0 + st * stage_bytes + kWBytes, bar = full0 + st * 8u;
-        const int k0 = kb * kBK;
-        if (small) {
-          for (int i = 0; i < half; i += 16) tma_load_2d_bar(sx + i * 128, &tma_x16, k0, xrow + i, bar);
-        } else if (half > 64) {
-          tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
-        } else {
-          tma_load_2d_bar(sx, &tma_x64, k0, xrow, bar);
+        const uint32_t bar = full0 + st * 8u;
+#pragma unroll
+        for (int j = 0; j < kSub; ++j) {
+          const uint32_t sx = smem0 + st * stage_bytes + kSub * kWBytes + j * x_bytes;
+          const int k0 = (kb * kSub + j) * kBK;
+          if (small) {
+            for (int i = 0; i < half; i += 16) tma_load_2d_bar(sx + i * 128, &tma_x16, k0, xrow + i, bar);
+          } else if (half > 64) {
+            tma_load_2d_bar(sx, &tma_x, k0, xrow, bar);
+          } else {
+            tma_load_2d_bar(sx, &tma_x64, k0, xrow, bar);
+          }
         }
       };
       int kb = 0;
@@ -308,8 +320,9 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     // loop took 673 cycles per k-block, 512 of which the tensor cores need.
     if (leader) {
       const uint32_t smem0 = smem_u32(smem);
-      const uint64_t wdesc0 = W_MN ? tc::smem_desc(smem0, kAtomBytes, 1024) : tc::smem_desc(smem0, 16, 1024);
-      const uint64_t xdesc0 = tc::smem_desc(smem0 + kWBytes, 16, 1024);
+      const uint64_t wdesc0 = W_MN ? tc::smem_desc(smem0, kSub * kAtomBytes, 1024) : tc::smem_desc(smem0, 16, 1024);
+      const uint64_t xdesc0 = tc::smem_desc(smem0 + kSub * kWBytes, 16, 1024);
+      constexpr uint32_t kWSub = (W_MN ? kAtomBytes : kWBytes) >> 4;
       constexpr uint32_t kWStep = W_MN ? 2048 >> 4 : 32 >> 4, kXStep = 32 >> 4;      // one 16-deep step in a descriptor's address field
       int tcnt = 0, gcur = 0; Tile ti;
       uint32_t stage = 0, phase = 0;
@@ -341,7 +354,10 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
           if (elect_one()) {
             const uint64_t wd = wdesc0 + stage * (stage_bytes >> 4), xd = xdesc0 + stage * (stage_bytes >> 4);
 #pragma unroll
-            for (int k = 0; k < kBK / 16; ++k) mma2_bf16(d_tmem, wd + k * kWStep, xd + k * kXStep, idesc, (kb | k) ? 1u : 0u);
+            for (int i = 0; i < kSub; ++i)
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k)
+                mma2_bf16(d_tmem, wd + i * kWSub + k * kWStep, xd + i * (x_bytes >> 4) + k * kXStep, idesc, (kb | i | k) ? 1u : 0u);
             mma2_commit_both(smem_u32(&empty_bar[stage]));
           }
           __syncwarp();
@@ -524,12 +540,18 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   MEP_REQUIRE(args.K % 64 == 0 && args.N % (mode == GEMM_GATE_UP ? 128 : 256) == 0, "gemm (CTA pairs): K=%d N=%d not tileable", args.K, args.N);
   num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "gemm (CTA pairs): needs at least two CTAs");
+  // Group sizes are only known on the device, and the code for bands costs a launch of few tiles 1 us of 20: it is there where
+  // groups are half as large as the line on average, so that some may be above it. All G groups count: a layer passes its
+  // slots for replicas too, which hold no row on one rank, so that there the average expert has to reach the line itself.
+  const bool bands = a_rows * args.K * 2 > (int64_t)args.G * (tp::kXBytes / 2);
+  const int64_t groups = args.tokens_n > 0 ? args.tokens_n : args.G;
+  const bool streams = !bands && args.K % 128 == 0 && groups * (mode == GEMM_DGRAD_GU ? args.K / 2 : args.K) * args.N * 2 >= tp::kStreamBytes && a_rows <= groups * tp::kStreamRows;
   CUtensorMap mx, mx64, mx16, mw0, mw1, mo, mo2;
   if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 128) || tmap_rows(&mx64, a, a_rows, a_cols, a_ld, 64, 64) ||
       tmap_rows(&mx16, a, a_rows, a_cols, a_ld, 64, 16)) return -1;
   auto weights = [&](CUtensorMap* m, const void* b) {
-    if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1);
-    if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2);
+    if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1, streams ? 128 : 64);
+    if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2, streams ? 128 : 64);
     return tmap_rows(m, b, b_rows, b_cols, b_ld, 64, 128);
   };
   if (weights(&mw0, b0)) return -1;
@@ -546,12 +568,6 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
-  // Group sizes are only known on the device, and the code for bands costs a launch of few tiles 1 us of 20: it is there where
-  // groups are half as large as the line on average, so that some may be above it. All G groups count: a layer passes its
-  // slots for replicas too, which hold no row on one rank, so that there the average expert has to reach the line itself.
-  const bool bands = a_rows * args.K * 2 > (int64_t)args.G * (tp::kXBytes / 2);
-  const int64_t groups = args.tokens_n > 0 ? args.tokens_n : args.G;
-  const bool streams = groups * (mode == GEMM_DGRAD_GU ? args.K / 2 : args.K) * args.N * 2 >= tp::kStreamBytes && a_rows <= groups * tp::kStreamRows;
 #define MEP_TP_CASE(M)                                                                                          \
   case M: {                                                                                                     \
     auto* kernel = bands ? tp::tok_pair_kernel<M, tp::BANDED>                                                        \

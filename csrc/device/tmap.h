@@ -24,7 +24,7 @@ inline int tmap_get(CUtensorMap* m, const TmapKey& k) {
   if (k.kind == 2) {
     MEP_REQUIRE(k.cols % 64 == 0, "gemm: MN-major operand width %lld must be a multiple of 64", (long long)k.cols);
     cuuint64_t dims[3] = {64, (cuuint64_t)k.rows, (cuuint64_t)(k.cols / 64)}, strides[2] = {(cuuint64_t)k.ld * 2, 128};
-    cuuint32_t box[3] = {64, 64, (cuuint32_t)k.box0};
+    cuuint32_t box[3] = {64, (cuuint32_t)k.box1, (cuuint32_t)k.box0};
     MEP_CU_CHECK(d->TensorMapEncodeTiled(&s.map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(k.base), dims, strides, box, es,
                                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
@@ -45,10 +45,10 @@ inline int tmap_rows(CUtensorMap* m, const void* base, int64_t rows, int64_t col
   return tmap_get(m, k);
 }
 // MN-major bf16 operand [rows (k), cols (m or n)] viewed as (64 elements, rows, cols / 64): one box of `atoms` 64-wide
-// atoms x 64 rows lands in shared memory atom after atom.
-inline int tmap_atoms(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld, int atoms) {
+// atoms x `box_rows` rows lands in shared memory atom after atom.
+inline int tmap_atoms(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld, int atoms, int box_rows = 64) {
   TmapKey k; memset(&k, 0, sizeof(k));
-  k.base = base; k.rows = rows; k.cols = cols; k.ld = ld; k.box0 = atoms; k.kind = 2;
+  k.base = base; k.rows = rows; k.cols = cols; k.ld = ld; k.box0 = atoms; k.box1 = box_rows; k.kind = 2;
   return tmap_get(m, k);
 }
 
