@@ -38,6 +38,12 @@ static LocalDispatchArgs dispatch_args(const MoeLocal& m, const void* hidden, in
   return d;
 }
 
+// Whether a pass's dispatch may begin while the kernel before still runs. A programmatic launch finds the SMs in the order in which that kernel leaves
+// them, and the GEMM pairs behind it inherit the order; after an ordinary one neighbours in the tile list are close to each other and read the
+// same lines of L2. That is worth 1.5 % of a forward pass of 4096 tokens, 7168 x 2048, 32 experts (2736 / 2782 us, six alternations); the launch
+// 1.5 to 4 us of a small one.
+static int early_dispatch(const MoeLocal& m) { return m.pdl && (int64_t)m.S * (m.K + 1) * m.H * 2 < (40ll << 20); }
+
 static void plan_into(const MoeLocal& m, const int32_t* topk, const int32_t* tpe, int32_t* slab, LocalDispatchArgs* d) {
   d->topk = topk; d->tpe = tpe;
   d->dst = slab + m.plan_off[0]; d->experts_to_copy = slab + m.plan_off[1]; d->zero_fill = slab + m.plan_off[2];
@@ -86,7 +92,7 @@ extern "C" int mep_moe_local_forward(const mep::MoeLocal* mp, const void* hidden
   LocalDispatchArgs d = dispatch_args(m, hidden, slab);
   d.weights = route_w; d.out_hidden = x; d.out_weights = w;
   plan_into(m, topk, tpe, slab, &d);
-  if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.sms, m.S, m.K, m.H, m.E, m.pdl, stream)) return -1;
+  if (mep_launch_local_dispatch(m.ctx, &d, 1, m.blocks, m.sms, m.S, m.K, m.H, m.E, early_dispatch(m), stream)) return -1;
   GemmArgs g = gemm_args(m, slab, tpe);
   g.N = m.Hp; g.K = m.H; g.out = m.act; g.out2 = keep ? m.gu : nullptr; g.row_scale = w; g.ldo = m.Hp;
   if (gemm(m, GEMM_GATE_UP, x, m.H, m.w_gate, m.w_up, m.H, m.Hp, g, stream)) return -1;
@@ -104,7 +110,7 @@ extern "C" int mep_moe_local_backward(const mep::MoeLocal* mp, const void* dy, i
   const MoeLocal& m = *mp;
   LocalDispatchArgs d = dispatch_args(m, dy, slab);
   d.out_hidden = m.shard;
-  if (mep_launch_local_dispatch(m.ctx, &d, 0, m.blocks, m.sms, m.S, m.K, m.H, m.E, m.pdl, stream)) return -1;
+  if (mep_launch_local_dispatch(m.ctx, &d, 0, m.blocks, m.sms, m.S, m.K, m.H, m.E, early_dispatch(m), stream)) return -1;
   GemmArgs g = gemm_args(m, slab);
   g.N = m.Hp; g.K = m.H; g.out = m.dA; g.ldo = m.Hp;
   if (gemm(m, GEMM_DGRAD, m.shard, m.H, m.w_down, nullptr, m.Hp, m.H, g, stream)) return -1;
