@@ -27,7 +27,7 @@ struct LocalDispatchArgs {
   int32_t* hist;                 // [grid, E] expert histogram of each CTA's tokens
   int32_t pad_step;              // 0: every padding row is cleared; else those up to the next multiple of this (a power of
                                  // two that divides token_padding), which is as far as the CTA-pair GEMMs read
-  int32_t reserved;
+  int32_t early;                 // a programmatic launch (set by the launcher)
 };
 
 struct LocalCombineArgs {

@@ -84,6 +84,7 @@ template <int MODE>                        // 0: saved plan
 __global__ void __launch_bounds__(kLocThreads, MODE ? 1 : 3)
 local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, int copy_warps, int slots) {
   constexpr bool FRESH = MODE != 0, SHARED = MODE == 2;
+  if (!a.early) pdl_trigger();               // a GEMM behind this kernel may set itself up meanwhile
   const MepRankCtx c = *cp;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLocWarps * kLocMaxSlots];
@@ -107,7 +108,7 @@ local_dispatch_kernel(const MepRankCtx* __restrict__ cp, LocalDispatchArgs a, in
   if (FRESH) for (int e = tid; e < E; e += kLocThreads) s_cnt[e] = 0;
   // Up to here the kernel right before may still run, whatever it is. A GEMM behind this kernel may set itself up and load weights as soon as that one is done.
   pdl_wait();
-  pdl_trigger();
+  if (a.early) pdl_trigger();
   if (tid == 0) {
     s_fail = 0;
     s_vb = SHARED ? (int)atomicAdd(&a.sync[1], 1u) : (int)blockIdx.x;
@@ -453,6 +454,8 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
 extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::LocalDispatchArgs* args, int fresh,
                                          int num_blocks, int sms, int S, int K, int H, int E, int pdl, cudaStream_t stream) {
   using namespace mep;
+  LocalDispatchArgs a = *args;
+  a.early = pdl;
   const size_t row = (size_t)H * 2;
   const size_t tables = (size_t)(fresh ? 3 : 4) * E * sizeof(int);
   const long long bytes = (long long)S * (K + 1) * (long long)row;
@@ -473,9 +476,9 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
     const int tokens = warps * (each < 1 ? 1 : (int)each);
     num_blocks = (S + tokens - 1) / tokens;
   }
-  if (fresh && S * K <= kLocDirect && (long long)S * K * H <= kLocDirectElems) return launch_plain_pdl(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, *args, warps, slots);
-  if (fresh) return launch_plain_pdl(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, *args, warps, slots);
-  return launch_plain_pdl(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, *args, warps, slots);
+  if (fresh && S * K <= kLocDirect && (long long)S * K * H <= kLocDirectElems) return launch_plain_pdl(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
+  if (fresh) return launch_plain_pdl(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
+  return launch_plain_pdl(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
 }
 
 extern "C" int mep_launch_local_combine(const MepRankCtx* ctx, const mep::LocalCombineArgs* args, int num_blocks,
