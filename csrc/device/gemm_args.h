@@ -65,9 +65,11 @@ struct GemmArgs {
   // optional [G, 2] table (first padding row, padding rows) of the groups, as a plan carries it: rows behind the real
   // ones, rounded up to 32, are then neither computed nor read (null: all padded rows are). CTA-pair kernels only.
   const int32_t* pad_rows;
-  // CTA-pair kernels. early: everything a launch reads besides the rows of `a` (WGRAD: besides both operands) and row_scale was there
-  // before the kernel right before it in the stream BEGAN: the tables below or cu_seqlens and pad_rows, the weights, upd_mask. It then
-  // sets up its tiles and loads the first weights while that kernel still runs.
+  // CTA-pair kernels. early: what a launch reads besides the rows of `a` (WGRAD: besides both operands) and row_scale -- the tables below or cu_seqlens and
+  // pad_rows, the weights, upd_mask -- was complete before the kernel right before it in the stream let its dependents launch. The launch then
+  // sets up its tiles and loads the first weights while that kernel still runs. A programmatic dispatch or combine of one rank lets them in when everything
+  // before it is done, so behind it that holds of whatever was queued before it; the GEMMs and the SwiGLU kernel let them in at their own
+  // start, so behind those it holds of what was complete before the first of an unbroken row of them.
   // tokens, optional: token counts of groups 0 to tokens_n - 1 (the others are empty), instead of cu_seqlens and pad_rows; groups are padded to
   // multiples of token_padding rows.
   const int32_t* tokens;

@@ -377,7 +377,6 @@ constexpr int kLcWarps = 12, kLcHalf = 8192;
 
 template <bool LAST_FIRST>
 __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const MepRankCtx* __restrict__ cp, LocalCombineArgs a, int part_vecs, int nparts) {
-  pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[kLcWarps * 2];
   const int K = cp->K, NvS = cp->NvS, nvec = cp->H >> 3;
@@ -386,6 +385,7 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   if (tid < kLcWarps * 2) mbar_init(&s_bar[tid], 1);
   fence_mbar_init();
   pdl_wait();                                  // the rows may come from the kernel right before
+  pdl_trigger();                               // only now: what an early launch behind this one reads ahead of its own wait may come from the kernel before, too
   __syncthreads();
   unsigned char* stage = smem + (size_t)warp * 2 * kLcHalf;
   uint64_t* bars = s_bar + warp * 2;

@@ -355,6 +355,42 @@ def test_early_launch_waits_for_the_kernel_before_without_limit(kind, cuda_devic
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("call", ["dispatch", "again", "combine"])
+def test_early_launch_behind_an_exchange_call_finds_what_came_before_it(call, cuda_device, monkeypatch):
+    """A dispatch or combine that set itself up beside the kernel before lets the next launch begin only when that kernel is done: weights which a kernel
+    in front of the exchange call writes, on one pair of SMs for about half a millisecond, are there when an early launch behind the call loads them."""
+    from moonep_b200 import Buffer, routing
+    from moonep_b200.ops import grouped_gemm as gg
+    monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
+    S, H, K, E = 40, 256, 2, 4                          # fewer CTAs than SMs: all of them run beside the kernel before
+    buf = Buffer(S, H, K, E, 1)
+    topk, _, tpe = routing.softmax_topk(S, K, E, 0.5, 3, 0, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(14)
+    bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
+    hid, src, w_src, x = bf(S, H), bf(2048, 7168), bf(1, 7168, 512, sc=0.02), bf(384, 2048)
+    cu_src, cu = (torch.tensor([n], dtype=torch.int32, device="cuda") for n in (2048, 384))
+    w, out = torch.zeros(1, 2048, 512, dtype=torch.bfloat16, device="cuda"), torch.empty(384, 512, dtype=torch.bfloat16, device="cuda")
+    rows, _, _, plan = buf.dispatch(hid, None, topk, tpe)
+    calls = dict(dispatch=lambda: buf.dispatch(hid, None, topk, tpe, zero_copy=True), again=lambda: buf.dispatch(hid, plan=plan, zero_copy=True),
+                 combine=lambda: buf.combine(plan=plan, hidden_nvsh=rows))
+    gg.down(src, w_src, cu_src, w[0])
+    gg.down(x, w, cu, out)
+    want = out.clone()
+    for _ in range(5):
+        w.zero_()
+        out.zero_()
+        torch.cuda.synchronize()
+        gg.down(src, w_src, cu_src, w[0], num_ctas=2)
+        calls[call]()
+        with _Early(monkeypatch):
+            gg.down(x, w, cu, out)
+        torch.cuda.synchronize()
+        gg.check_status()
+        buf.check()
+        assert torch.equal(out, want)
+    buf.destroy()
+
+
 @pytest.mark.parametrize("split", [(2,), (28,), (30,), (148,), (10, 138)], ids=str)
 def test_token_major_tiles_of_uneven_groups(split, cuda_device, monkeypatch):
     """Groups of 0 to 1000 rows, ordered by the size of their tiles up to twelve rounds (gate/up from 15 pairs on, the others from 8) and by number above: the
