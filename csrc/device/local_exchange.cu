@@ -385,7 +385,6 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   if (tid < kLcWarps * 2) mbar_init(&s_bar[tid], 1);
   fence_mbar_init();
   pdl_wait();                                  // the rows may come from the kernel right before
-  pdl_trigger();                               // only now: what an early launch behind this one reads ahead of its own wait may come from the kernel before, too
   __syncthreads();
   unsigned char* stage = smem + (size_t)warp * 2 * kLcHalf;
   uint64_t* bars = s_bar + warp * 2;
@@ -413,6 +412,9 @@ __global__ void __launch_bounds__(kLcWarps * 32, 1) local_combine_kernel(const M
   uint32_t phase = 0;                          // parity of both halves: they are used in turn
   if (u < units) cur = issue(u, fetch(u), 0);
   int dn = fetch(u + step);
+  // Only now: what an early launch behind this one reads ahead of its own wait may come from the kernel before this one, too. In front of the first loads it
+  // delayed them: dispatch and combine of 3000 x 4, H=512 14.64 us instead of 14.54 (as long as from the kernel's start), 500 x 4, H=1024 10.62 instead of 10.42.
+  pdl_trigger();
   bool ok = true;
   for (; u < units; u += step) {
     const int un = u + step;
