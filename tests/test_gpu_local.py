@@ -219,3 +219,28 @@ def test_queued_calls_see_what_the_kernel_before_wrote(shape, pdl, cuda_device):
     for a, b in zip(got, want):
         assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
     buf.destroy()
+
+
+def test_calls_on_the_communication_stream_are_ordinary_launches(cuda_device):
+    """They follow an event and no kernel, and share the SMs with what runs on other streams; calls on the caller's stream follow the switch again."""
+    S, K, E, H = 300, 4, 16, 256
+    buf = Buffer(S, H, K, E, 1, token_padding=16)
+    topk, tpe = (t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=5))
+    x = torch.randn(S, H, device="cuda").to(torch.bfloat16)
+    seen = []
+    for enabled in (True, False):
+        for asynchronous in (False, True, False):
+            buf.enable_pdl = enabled
+            h, _, _, plan, *ev = buf.dispatch(x, None, topk, tpe, async_finish=asynchronous)
+            seen.append(buf._local_ex._args.pdl)
+            for e in ev:
+                torch.cuda.current_stream().wait_event(e)
+            y, _, e = buf.combine(plan=plan, hidden_nvsh=h, async_finish=asynchronous)
+            seen.append(buf._local_ex._args.pdl)
+            if e is not None:
+                torch.cuda.current_stream().wait_event(e)
+            torch.cuda.synchronize()
+            assert torch.equal(y, x * 4)               # four equal numbers: exact
+    buf.check()
+    assert seen == [1, 1, 0, 0, 1, 1] + [0] * 6
+    buf.destroy()
