@@ -25,14 +25,20 @@ constexpr size_t kLocAlone = 115 * 1024;   // dynamic shared memory of which an 
 
 // Up to this many entries every CTA counts all entries before its own by itself, above it the CTAs hand over their
 // histograms. Counting costs a CTA all entries before its own, the hand-over two round trips to L2 and CTAs x E counts. Own
-// count against hand-over, a dispatch with K=8 among others of its kind, in us:
-//   entries             12288        18432        24576        32768        49152        65536        131072
-//   H=512,  E=64      9.9 / 18.3  11.8 / 19.7  14.0 / 21.0  16.8 / 21.9  23.4 / 27.7  29.0 / 32.3  61.8 / 53.8
-//   H=2048, E=16     14.5 / 22.5  19.9 / 25.0  27.5 / 33.9  35.7 / 42.1  52.9 / 57.3  67.9 / 71.5   134 / 129
-//   H=2048, E=256    30.5 / 41.4  35.1 / 47.3  40.7 / 47.8  47.7 / 53.8  66.3 / 69.9  80.9 / 83.5   148 / 146
-//   H=4096, E=60     29.3 / 32.7  38.3 / 42.0  51.6 / 53.1  66.0 / 68.0  96.8 / 96.8   125 / 124    245 / 239
-//   H=7168, E=32     41.1 / 43.4  61.2 / 62.9  78.8 / 82.0   105 / 106    155 / 155    204 / 204
+// count against hand-over, a dispatch with K=8 among others of its kind (programmatic launches), in us:
+//   entries                 12288         18432         24576         32768         49152         65536        131072
+//   H=64,   E=64      8.5 / 15.6   10.0 / 15.7   11.8 / 17.4   13.9 / 18.6   19.4 / 22.1   23.4 / 23.9   42.8 / 35.5
+//   H=512,  E=64      9.1 / 16.2   11.3 / 17.6   13.2 / 19.1   15.9 / 21.6   22.4 / 26.0   27.8 / 28.8   62.5 / 53.8
+//   H=2048, E=16     13.8 / 20.3   19.0 / 24.9   25.8 / 31.9   34.8 / 39.7   51.8 / 52.5   67.4 / 69.7     135 / 127
+//   H=2048, E=256    14.7 / 22.3   20.8 / 28.8   27.6 / 36.3   35.8 / 44.0   54.8 / 60.8   69.8 / 71.9     141 / 138
+//   H=4096, E=60     24.2 / 31.5   35.5 / 42.1   47.0 / 51.4   61.4 / 67.6   93.3 / 97.8     122 / 124             -
+//   H=7168, E=32     37.6 / 44.6   56.5 / 60.3   75.3 / 82.1     101 / 101     153 / 157     202 / 196             -
 // So the line is lower for long rows, at this many elements of all rows (4096, 7168, 8, E=32 with its combine: 197.0 / 195.8).
+// With few CTAs each has as many entries before it, but there are fewer histograms to add up: below two thirds of the SMs the line is at five
+// eighths. K=8, E=64 with 64 and with 32 CTAs: 32768 entries, H=64 20.1 / 21.1 and 31.8 / 33.0, H=1024 33.9 / 35.9 and 59.8 / 61.3; 40960, H=64 24.6
+// / 25.3 and 39.4 / 39.8, H=1024 43.7 / 44.3 and 77.6 / 76.2; 49152, H=64 28.2 / 27.7 and 46.2 / 45.4, H=1024 53.1 / 51.5 and 91.5 / 90.0; 65536,
+// H=64 36.3 / 33.7 and 60.1 / 58.0, H=1024 66.4 / 65.4 and 124 / 117. With 100: 49152, H=64 22.1 / 22.6, H=1024 37.6 / 40.4; 65536 28.6 / 26.6, 49.2
+// / 50.6.
 constexpr int kLocDirect = 65536, kLocDepth = 16;      // kLocDepth: entries that a thread has on their way when it counts
 constexpr long long kLocDirectElems = 24576ll * 7168;
 
@@ -478,7 +484,8 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
     const int tokens = warps * (each < 1 ? 1 : (int)each);
     num_blocks = (S + tokens - 1) / tokens;
   }
-  if (fresh && S * K <= kLocDirect && (long long)S * K * H <= kLocDirectElems) return launch_plain_pdl(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
+  const int direct = 3ll * num_blocks >= 2ll * sms ? kLocDirect : kLocDirect / 8 * 5;
+  if (fresh && S * K <= direct && (long long)S * K * H <= kLocDirectElems) return launch_plain_pdl(local_dispatch_kernel<1>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
   if (fresh) return launch_plain_pdl(local_dispatch_kernel<2>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
   return launch_plain_pdl(local_dispatch_kernel<0>, dim3(num_blocks), dim3(kLocThreads), smem, stream, pdl != 0, ctx, a, warps, slots);
 }

@@ -244,3 +244,26 @@ def test_calls_on_the_communication_stream_are_ordinary_launches(cuda_device):
     buf.check()
     assert seen == [1, 1, 0, 0, 1, 1] + [0] * 6
     buf.destroy()
+
+
+@pytest.mark.parametrize("limit,shapes", [(None, {(8192, 8, 64): 0, (8193, 8, 64): 1}), (99, {(8192, 8, 64): 0}), (98, {(5120, 8, 64): 0, (5121, 8, 64): 1}),
+                                          (16, {(5120, 8, 64): 0, (8192, 8, 64): 1})], ids=str)
+def test_which_dispatches_hand_over(limit, shapes, cuda_device, monkeypatch):
+    """Up to 65536 entries every CTA counts for itself, up to 40960 where it may use less than two thirds of the (148) SMs; only the hand-over numbers its launches."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the limits are those of 148 SMs")
+    if limit is not None:
+        monkeypatch.setenv("MOONEP_NUM_SMS_DEDUP", str(limit))
+    for (S, K, H), launches in shapes.items():
+        topk, tpe = make_topk("biased", S, K, 24, 1, seed=5)
+        cp = plan_cluster(np.stack([t.numpy() for t in topk]), 24, 16)
+        buf = Buffer(S, H, K, 24, 1, token_padding=16)
+        x = traceable_hidden(S, H, 0).cuda()
+        h, _, cu, plan = buf.dispatch(x, None, topk[0].cuda(), tpe[0].cuda(), zero_copy=True)
+        torch.cuda.synchronize()
+        buf.check()
+        check_plans([plan], [cu], cp, 1)
+        rows = torch.where(plan.dst < 0, -plan.dst - 1, plan.dst).long()
+        assert torch.equal(h.view(torch.int16)[rows], x.view(torch.int16).repeat_interleave(K, 0))
+        assert int(buf._states[0].scratch["loc_sync"][0]) == launches
+        buf.destroy()
