@@ -477,8 +477,10 @@ extern "C" int mep_launch_local_dispatch(const MepRankCtx* ctx, const mep::Local
   while (slots > 2 && (size_t)warps * (slots - 1) * row >= ring) --slots;
   size_t smem = kLocZeroBytes + (size_t)warps * slots * row + tables;
   // A programmatic launch is placed as the SMs of the kernel before come free: without this the first of them would get two CTAs and the last none
-  // (8000 x 8, H=1024 with its combine 80.6 us instead of 71)
-  if (pdl && !large && smem < kLocAlone) smem = kLocAlone;
+  // (8000 x 8, H=1024 with its combine 80.0 us instead of 65.6, 3000 x 4, H=512 17.7 instead of 14.5). It costs two Buffers on streams of their own, whose
+  // dispatches then share no SM: of 3000 x 4, H=256 each with its combine 21.1 us instead of 16.9 with ordinary launches. Not with a token
+  // for each CTA at most, where two CTAs on an SM are as good as one (148 x 8, H=1024 9.4 / 9.5, 64 x 8 9.3 / 9.2; beside another Buffer's 13.8 / 9.3 and 10.3 / 8.8).
+  if (pdl && !large && S > num_blocks && smem < kLocAlone) smem = kLocAlone;
   if (large) {                               // the same number of tokens for each warp
     const long long each = kLocShort / ((long long)row * (K + 1) * warps);
     const int tokens = warps * (each < 1 ? 1 : (int)each);
