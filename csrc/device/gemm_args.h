@@ -78,6 +78,9 @@ struct GemmArgs {
   // gives the gradient (update) of another matrix of the same shape, out_b (upd_w_b).
   int32_t n_each;
   void *out_b, *upd_w_b;
+  // Token-major CTA-pair kernels: groups that hold rows, as far as the caller knows, and their rows without padding; 0: all G, and the rows of `a`. They
+  // only decide which kernel runs.
+  int32_t held, held_rows;
 };
 
 // CTAs of a pair launch that was asked for `n`. On a counter shared with other launches the grid accounts for all `n`.

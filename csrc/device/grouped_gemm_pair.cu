@@ -47,16 +47,27 @@ constexpr int kBand = 8, kXBytes = 36 << 20;
 // had the tiles left over in a short last round (64 tokens, 2048 x 768, two rounds, 57.4 / 51.7).
 constexpr int kSortRounds = 12;
 // STREAM: weights of a group with one token tile are read once: their lines leave L2 first, so that rows, tables and above all the kernels' code, which
-// every launch fetches anew, stay there. Where the groups' matrices, one for each, have this many bytes: a layer of three of less than 100 MB
-// keeps its weights in L2 from one pass to the next. Forward passes with / without, in us: 64 tokens, 2048 x 768, 16 experts (50 MB) 49.2 / 52.5; 700,
-// 2048 x 768, 24 (75) 74.0 / 80.9; 300, 4096 x 1024, 16 (134) 84.8 / 93.0; 256, 7168 x 2048, 32 (940) 477 / 483; but 16 tokens,
-// 2048 x 768, 8 (25) 36.5 / 34.9. Only where few groups have more than one tile (kStreamRows rows in a group on average; a layer allows 127 for padding):
-// the hint costs the others 1 % (1531, 2048 x 768, 16 152.2 / 150.2), and not for tiles that share weights, as pairs are not in step: gate/up of 32 experts and 4096
-// tokens x 8, 7168 x 2048, then reads 6.2 GB instead of 3.4 and takes 2.04 ms instead of 1.80.
-// Its stages are 128 deep: one load brings a column atom's weights of both k-blocks and one pair of barriers serves them. What a round that does not fill
-// the GPU takes is the producer's issue (about 450 cycles a k-block and 58 GB/s per SM before): 64 tokens, 2048 x 768, 16 experts 45.1 -> 43.8
-// us; 8 tokens, 4096 x 1536, 32 162.6 -> 156.1; 256, 7168 x 2048, 32 462.1 -> 459.2.
-constexpr int64_t kStreamBytes = 32 << 20, kStreamRows = 320;
+// every launch fetches anew, stay there. Its stages are 128 deep: one load brings a column atom's weights of both k-blocks and one pair of barriers
+// serves them. What a round that does not fill the GPU takes is the producer's issue (about 450 cycles a k-block and 58 GB/s per SM before). Not for
+// tiles that share weights, as pairs are not in step: gate/up of 32 experts and 4096 tokens x 8, 7168 x 2048, then reads 6.2 GB instead of 3.4 and takes 2.04
+// ms instead of 1.80. Without / with, in us:
+//   rows of an expert                                        32            64           128           192           256           384           512
+//   2048 x 768, 16 experts, forward                 46.9 / 44.2   53.2 / 47.3   57.1 / 54.6   62.8 / 61.6   69.4 / 69.4   82.9 / 84.1  100.0 / 102.3
+//   (two layers in turn)    both dgrads             45.3 / 42.9   47.1 / 43.1   51.3 / 48.7   60.1 / 57.9   61.6 / 62.6   75.9 / 78.0   87.1 / 89.6
+//   4096 x 1536, 32 experts, forward                 211 / 200     222 / 208     253 / 249     309 / 301     362 / 353     479 / 502     605 / 606
+//   rows of an expert, captured steps                        96           112           128           144           160
+//   4096 x 1536, 32 experts                         1015 / 1008   1026 / 1016   1037 / 1028   1069 / 1069   1080 / 1089
+//   with the update in the epilogue                 1166 / 1158   1179 / 1165   1213 / 1198   1220 / 1232   1238 / 1261
+//   7168 x 2048, 32 experts                         2196 / 2193   2212 / 2215   2286 / 2239   2391 / 2381   2477 / 2474
+//   with the update in the epilogue                 2466 / 2466   2487 / 2473   2496 / 2500   2533 / 2543   2567 / 2577
+// kStreamRows: so many rows (without padding) a group that holds any has at most on average. A direct call counts the rows of `a`, which may have room for more
+// (kStreamRoom): dgrads of 16 groups of 66, 2048 x 768, in a table of 320 rows for each 47.3 / 43.1.
+// kStreamBytes: those groups' matrices, one for each. A smaller layer whose forward pass is called over and over keeps its weights in L2: 2048 x 768, 8 experts
+// (24 MiB), 32 and 128 rows 31.8 / 31.4 and 39.9 / 41.7, 1536 x 1024, 10 (30 MiB), 10 rows 33.7 / 35.2; captured steps with the update in the epilogue, dgrads
+// of 512 x 1024, 19 (19 MiB), 116 rows 120.6 / 123.1, 512 x 1280, 17 (21 MiB), 16 rows 107.2 / 105.5. Half of it for a layer's
+// launches that do not start early (kStreamBytesLate): nobody has loaded their first weights for them. Passes issued from Python, 2048 x 768, 8 experts:
+// backward, 4 and 64 rows 88.4 / 83.9 and 95.9 / 88.2, forward, 64 rows 38.2 / 37.1.
+constexpr int64_t kStreamBytes = 32 << 20, kStreamBytesLate = 16 << 20, kStreamRows = 128, kStreamRoom = 320;
 enum Kind { PLAIN, BANDED, STREAM };                   // a kernel each: code that a launch does not need costs it 1 to 2 us of 50
 constexpr int kStgSet = 4 * kStgBytes;                 // GATE_UP: act twice, gate, up; else: two buffers for each 64-column side
 constexpr size_t kEpiBytes = 2 * kStgSet + kEpiWarps * kXchBytes;
@@ -529,6 +540,17 @@ tok_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
 }  // namespace tp
 }  // namespace mep
 
+// Which kernel a launch takes (see Kind). Group sizes are only known on the device, and the code for bands costs a launch of few tiles 1 us of 20: it is there
+// where groups are half as large as the line on average, so that some may be above it. All G groups count: a layer passes its slots for replicas
+// too, which hold no row on one rank, so that there the average expert has to reach the line itself.
+extern "C" int mep_pair_kind(int mode, int64_t a_rows, int G, int N, int K, int held, int held_rows, int early) {
+  using namespace mep;
+  if (a_rows * K * 2 > (int64_t)G * (tp::kXBytes / 2)) return tp::BANDED;
+  const int64_t groups = held > 0 ? held : G, bytes = groups * (mode == GEMM_DGRAD_GU ? K / 2 : K) * N * 2;
+  const bool few = held > 0 ? held_rows <= groups * tp::kStreamRows : a_rows <= groups * tp::kStreamRoom;
+  return K % 128 == 0 && few && bytes >= (held > 0 && !early ? tp::kStreamBytesLate : tp::kStreamBytes) ? tp::STREAM : tp::PLAIN;
+}
+
 // One grouped GEMM launch on CTA pairs; same contract as mep_grouped_gemm for modes 0-3.
 extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, int64_t a_cols, int64_t a_ld,
                                      const void* b0, const void* b1, int64_t b_rows, int64_t b_cols, int64_t b_ld,
@@ -540,18 +562,13 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   MEP_REQUIRE(args.K % 64 == 0 && args.N % (mode == GEMM_GATE_UP ? 128 : 256) == 0, "gemm (CTA pairs): K=%d N=%d not tileable", args.K, args.N);
   num_ctas = pair_ctas(&args, num_ctas);
   MEP_REQUIRE(num_ctas >= 2, "gemm (CTA pairs): needs at least two CTAs");
-  // Group sizes are only known on the device, and the code for bands costs a launch of few tiles 1 us of 20: it is there where
-  // groups are half as large as the line on average, so that some may be above it. All G groups count: a layer passes its
-  // slots for replicas too, which hold no row on one rank, so that there the average expert has to reach the line itself.
-  const bool bands = a_rows * args.K * 2 > (int64_t)args.G * (tp::kXBytes / 2);
-  const int64_t groups = args.tokens_n > 0 ? args.tokens_n : args.G;
-  const bool streams = !bands && args.K % 128 == 0 && groups * (mode == GEMM_DGRAD_GU ? args.K / 2 : args.K) * args.N * 2 >= tp::kStreamBytes && a_rows <= groups * tp::kStreamRows;
+  const int kind = mep_pair_kind(mode, a_rows, args.G, args.N, args.K, args.held, args.held_rows, args.early), deep = kind == tp::STREAM ? 128 : 64;
   CUtensorMap mx, mx64, mx16, mw0, mw1, mo, mo2;
   if (tmap_rows(&mx, a, a_rows, a_cols, a_ld, 64, 128) || tmap_rows(&mx64, a, a_rows, a_cols, a_ld, 64, 64) ||
       tmap_rows(&mx16, a, a_rows, a_cols, a_ld, 64, 16)) return -1;
   auto weights = [&](CUtensorMap* m, const void* b) {
-    if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1, streams ? 128 : 64);
-    if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2, streams ? 128 : 64);
+    if (mode == GEMM_GATE_UP) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 1, deep);
+    if (mode == GEMM_DOWN) return tmap_atoms(m, b, b_rows, b_cols, b_ld, 2, deep);
     return tmap_rows(m, b, b_rows, b_cols, b_ld, 64, 128);
   };
   if (weights(&mw0, b0)) return -1;
@@ -570,8 +587,8 @@ extern "C" int mep_grouped_gemm_2cta(int mode, const void* a, int64_t a_rows, in
   cfg.attrs = attr; cfg.numAttrs = args.pdl ? 2 : 1;
 #define MEP_TP_CASE(M)                                                                                          \
   case M: {                                                                                                     \
-    auto* kernel = bands ? tp::tok_pair_kernel<M, tp::BANDED>                                                        \
-                         : streams ? tp::tok_pair_kernel<M, tp::STREAM> : tp::tok_pair_kernel<M, tp::PLAIN>; \
+    auto* kernel = kind == tp::BANDED ? tp::tok_pair_kernel<M, tp::BANDED>                                                \
+                   : kind == tp::STREAM ? tp::tok_pair_kernel<M, tp::STREAM> : tp::tok_pair_kernel<M, tp::PLAIN>; \
     if (allow_smem((const void*)kernel, tp::kSmem)) return -1;                                                  \
     MEP_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, mx, mx64, mx16, mw0, mw1, mo, mo2, args));                  \
     break;                                                                                                      \

@@ -25,6 +25,7 @@ static GemmArgs gemm_args(const MoeLocal& m, const int32_t* slab, const int32_t*
   a.G = 2 * m.E; a.g_end = 2 * m.E;
   a.early = 1; a.tokens = tpe; a.tokens_n = m.E; a.token_padding = m.token_padding;
   a.pdl = m.pdl;                 // behind another kernel of the same call
+  a.held = m.E; a.held_rows = m.S * m.K;
   a.status = m.status; a.status_host = m.status_host; a.budget_ns = m.budget_ns;
   return a;
 }

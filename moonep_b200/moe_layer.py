@@ -117,6 +117,7 @@ class ExpertParallelMoE:
         if ready_flags is None:             # MOONEP_READY_FLAGS=0: the GEMMs wait for the whole dispatch
             ready_flags = os.environ.get("MOONEP_READY_FLAGS", "1") != "0"
         self.ready_flags = ready_flags
+        self._held = (g.epn, g.N)        # what the GEMMs may count on: every rank gets as many rows as it sends, most of them for its own experts
         self._skip_pad = gg.skips_padding() and self.H % 256 == 0 and self.Hp % 256 == 0
         self._local = buffer._states[0].local       # single rank: see _forward_local
         dev = buffer.hidden_nvsh_buffer_view.device
@@ -203,11 +204,11 @@ class ExpertParallelMoE:
         gu = self._gu if need_backward else None
         Wg, Wu, pad = self._W("gate"), self._W("up"), self._pad(plan)
         if ev is not None:
-            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(0, epn), pad=pad)
+            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(0, epn), pad=pad, held=self._held)
             torch.cuda.current_stream().wait_event(ev)
-            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(epn, 2 * epn), pad=pad)
+            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, groups=(epn, 2 * epn), pad=pad, held=self._held)
         else:
-            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, pad=pad)
+            gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, pad=pad, held=self._held)
         return self._forward_tail(plan, cu, stashed, need_backward)
 
     def _forward_local(self, hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, need_backward):
@@ -228,8 +229,8 @@ class ExpertParallelMoE:
             w = None
         _, _, cu, plan = buf._dispatch_local(hidden_sh, route_weights_sk, topk_sk, tokens_per_expert, None, out=(x, w))
         pad = self._pad(plan)
-        gg.gate_up(x, self._W("gate"), self._W("up"), cu, self._act, self._gu if need_backward else None, row_scale=w, pad=pad)
-        gg.down(self._act, self._W("down"), cu, st.hidden_local, pad=pad)
+        gg.gate_up(x, self._W("gate"), self._W("up"), cu, self._act, self._gu if need_backward else None, row_scale=w, pad=pad, held=self._held)
+        gg.down(self._act, self._W("down"), cu, st.hidden_local, pad=pad, held=self._held)
         out, _ = buf._combine_local(plan, st.hidden_local, None)
         return out, MoEContext(plan, cu, x, w, self._act, self._gu) if need_backward else None
 
@@ -257,10 +258,10 @@ class ExpertParallelMoE:
         tk = gg.Ticket(self._act.device, self._total_sms)
         free = min(ready.free_sms, self._total_sms - self._comm_sms) & ~1      # CTA pairs
         gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, num_ctas=free, ticket=tk, ready=ready, slots=slots,
-                   pad=self._pad(plan))
+                   pad=self._pad(plan), held=self._held)
         with torch.cuda.stream(comm):
             gg.gate_up(x, Wg, Wu, cu, self._act, gu, row_scale=w, num_ctas=self._total_sms - free, ticket=tk,
-                       ready=ready, slots=slots, pad=self._pad(plan))
+                       ready=ready, slots=slots, pad=self._pad(plan), held=self._held)
             joined = comm.record_event()
         main.wait_event(joined)
         return self._forward_tail(plan, cu, stashed, need_backward)
@@ -273,10 +274,10 @@ class ExpertParallelMoE:
         if g.off_push:
             # push-combine: the down GEMM's epilogue sends every row to its source rank while the
             # GEMM is still running; what is left of the combine is a barrier and a local sum
-            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, push=buf.push_target(), pad=self._pad(plan))
+            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, push=buf.push_target(), pad=self._pad(plan), held=self._held)
             out, _, _ = buf.combine_pushed()
         else:
-            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, pad=self._pad(plan))
+            gg.down(self._act, Wd, cu, buf.hidden_nvsh_buffer_view, pad=self._pad(plan), held=self._held)
             out, _, _ = buf.combine(plan=plan, hidden_nvsh=buf.hidden_nvsh_buffer_view, zero_copy=True)
         ctx = MoEContext(plan, cu, self._x, self._w, self._act, self._gu) if need_backward else None
         return out, ctx
@@ -345,7 +346,7 @@ class ExpertParallelMoE:
         if self._local:
             dy = shard
             buf._dispatch_local(grad_out_sh, None, None, None, ctx.plan, out=(shard, None))
-            gg.dgrad(dy, Wd, ctx.cu, self._dA, pad=pad)
+            gg.dgrad(dy, Wd, ctx.cu, self._dA, pad=pad, held=self._held)
         elif self.ready_flags and ctx.plan.send_list is not None:
             # dgrad(down) starts on the tiles of the re-dispatched output grad as they complete
             dy, _, _, _, ready, _ = buf.dispatch_ready(grad_out_sh, plan=ctx.plan)
@@ -354,9 +355,9 @@ class ExpertParallelMoE:
                 slots = buf.slot_ready()
             tk = gg.Ticket(self._act.device, self._total_sms)
             free = min(ready.free_sms, self._total_sms - self._comm_sms) & ~1      # CTA pairs
-            gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=free, ticket=tk, ready=ready, slots=slots, pad=pad)
+            gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=free, ticket=tk, ready=ready, slots=slots, pad=pad, held=self._held)
             with torch.cuda.stream(buf.comm_stream):
-                gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=self._total_sms - free, ticket=tk, ready=ready, slots=slots, pad=pad)
+                gg.dgrad(dy, Wd, ctx.cu, self._dA, num_ctas=self._total_sms - free, ticket=tk, ready=ready, slots=slots, pad=pad, held=self._held)
                 joined = buf.comm_stream.record_event()
             main.wait_event(joined)
         else:
@@ -364,7 +365,7 @@ class ExpertParallelMoE:
             if refetch:
                 ev_pf = buf.prefetch_weight(plan=ctx.plan, async_finish=True, **pools.prefetch_kwargs())
                 slots = buf.slot_ready()
-            gg.dgrad(dy, Wd, ctx.cu, self._dA, slots=slots, pad=pad)
+            gg.dgrad(dy, Wd, ctx.cu, self._dA, slots=slots, pad=pad, held=self._held)
         if ev_pf is not None:
             main.wait_event(ev_pf)      # dgrad(gate/up) further down reads the other two projections' slots
         dw_view = buf.router_weight_buffer_view
@@ -394,10 +395,10 @@ class ExpertParallelMoE:
             ev_red = buf.reduce_grad_subset(ctx.plan, first, async_finish=ov, clear_slots=acc)
             self._optimizer("down", ev_red if ov else main)
         if ov and multi:
-            ev = self._beside_comm(lambda n, tk: gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, num_ctas=n, ticket=tk, pad=pad))
+            ev = self._beside_comm(lambda n, tk: gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, num_ctas=n, ticket=tk, pad=pad, held=self._held))
             main.wait_event(ev)
         else:
-            gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, pad=pad)
+            gg.dgrad_gate_up(self._dgu, Wg, Wu, ctx.cu, shard, pad=pad, held=self._held)
         if not gate_late:
             self._optimizer("gate", main, *([ev_red] if ev_red is not None else []))
         grad_hidden, grad_w, ev_comb = buf.combine(plan=ctx.plan, hidden_nvsh=shard, route_weights_nvs=dw_view,

@@ -39,7 +39,8 @@ class GemmArgs(C.Structure):
                 ("push_rows", C.c_int32), ("push_ranks", C.c_int32), ("group_first", C.c_int32), ("sched_ctas", C.c_int32),
                 ("upd_w", C.c_void_p), ("upd_mask", C.c_void_p), ("upd_lr", C.c_float), ("sched_odd", C.c_int32),
                 ("pad_rows", C.c_void_p), ("tokens", C.c_void_p), ("tokens_n", C.c_int32), ("token_padding", C.c_int32),
-                ("early", C.c_int32), ("n_each", C.c_int32), ("out_b", C.c_void_p), ("upd_w_b", C.c_void_p)]
+                ("early", C.c_int32), ("n_each", C.c_int32), ("out_b", C.c_void_p), ("upd_w_b", C.c_void_p),
+                ("held", C.c_int32), ("held_rows", C.c_int32)]
 
 
 class PushTarget:
@@ -184,7 +185,7 @@ def _on_pairs(mode, rows, ngroups, G, N, K, skips_pad, ctas, shared) -> bool:
 
 def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=None, row_scale=None, ldo=0,
             accumulate=False, zero_empty_below=0, a_cols=None, b_rows=None, b_cols=None, b_ld=None, groups=None, num_ctas=None,
-            dynamic=False, ticket=None, push=None, push_w=None, ready=None, slots=None, pad=None):
+            dynamic=False, ticket=None, push=None, push_w=None, ready=None, slots=None, pad=None, held=None):
     lib = _native.load()
     assert a.dtype == torch.bfloat16 and b0.dtype == torch.bfloat16
     assert cu.dtype == torch.int32 and cu.is_contiguous()
@@ -197,6 +198,8 @@ def _launch(mode, a, b0, b1, cu, *, N, K=0, M_w=0, b_group_rows=0, out, out2=Non
     args.zero_empty_below = zero_empty_below
     args.out, args.out2 = out.data_ptr(), _native.ptr(out2)
     args.row_scale, args.ldo = _native.ptr(row_scale), ldo
+    if held is not None:
+        args.held, args.held_rows = held
     if ticket is not None:
         args.sched, args.sched_ctas = ticket.ptr, ticket.total_ctas
     else:
@@ -234,7 +237,7 @@ def _w2d(w):
 
 
 def gate_up(x, wg, wu, cu, act_out, gu_out=None, row_scale=None, groups=None, num_ctas=None, dynamic=False, ticket=None,
-            ready=None, slots=None, pad=None):
+            ready=None, slots=None, pad=None, held=None):
     """``act_out[r] = row_scale[r] * silu(x[r] Wg[g]) * (x[r] Wu[g])``; optionally stores the
     pre-activations ``gu_out = [x Wg | x Wu]`` (``[NvS, 2*out]``) for the backward pass.
     ``ready`` (a ``TileReady`` from ``Buffer.dispatch_ready``): ``x`` is still being filled by that
@@ -243,36 +246,39 @@ def gate_up(x, wg, wu, cu, act_out, gu_out=None, row_scale=None, groups=None, nu
     ``slots`` (a ``SlotReady`` from ``Buffer.slot_ready``): the weights of the groups ``>= slots.first`` are
     prefetched experts that may still be on their way; each such group is loaded once its slot is complete.
     ``pad`` (every GEMM of this module; int32 ``[G, 2]``, a plan's ``zero_fill_ranges``): rows behind a group's real ones,
-    rounded up to 32, are then neither computed nor read."""
+    rounded up to 32, are then neither computed nor read.
+    ``held`` (every token-major GEMM): ``(groups, rows)``, how many groups hold rows and how many those are without padding, as far as the caller
+    knows (default: all groups, and the rows of ``x``); it decides which kernel runs and nothing else."""
     G, K, N = wg.shape
     assert wu.shape == wg.shape and x.shape[1] == K and N % 128 == 0 and K % 64 == 0
     rows, cols = _w2d(wg)
     _launch(GATE_UP, x, wg, wu, cu, N=N, K=K, b_group_rows=K, out=act_out, out2=gu_out, row_scale=row_scale,
             ldo=act_out.stride(0), b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket,
-            ready=ready, slots=slots, pad=pad)
+            ready=ready, slots=slots, pad=pad, held=held)
 
 
-def down(act, wd, cu, out, row_scale=None, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, pad=None):
+def down(act, wd, cu, out, row_scale=None, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, pad=None, held=None):
     """``out[r] = row_scale[r] * (act[r] Wd[g])`` with ``Wd [G, inner, hidden]``.  With ``push`` (a
     ``PushTarget``) the rows are not written to ``out`` but sent to the ranks their tokens came from."""
     G, K, N = wd.shape
     assert act.shape[1] == K and N % 256 == 0 and K % 64 == 0
     rows, cols = _w2d(wd)
     _launch(DOWN, act, wd, None, cu, N=N, K=K, b_group_rows=K, out=out, row_scale=row_scale, ldo=out.stride(0),
-            b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, push=push, pad=pad)
+            b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, push=push, pad=pad,
+            held=held)
 
 
-def dgrad(dy, w, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, ready=None, slots=None, pad=None):
+def dgrad(dy, w, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, ready=None, slots=None, pad=None, held=None):
     """``out[r] = dy[r] W[g]^T`` with ``W [G, in, out]`` -> ``out [NvS, in]``.  ``ready`` / ``slots``: as in ``gate_up``."""
     G, N, K = w.shape
     assert dy.shape[1] == K and N % 256 == 0 and K % 64 == 0
     rows, cols = _w2d(w)
     _launch(DGRAD, dy, w, None, cu, N=N, K=K, b_group_rows=N, out=out, ldo=out.stride(0),
             b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket, ready=ready,
-            slots=slots, pad=pad)
+            slots=slots, pad=pad, held=held)
 
 
-def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, push_w=None, pad=None):
+def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=False, ticket=None, push=None, push_w=None, pad=None, held=None):
     """``out[r] = dG[r] Wg[g]^T + dU[r] Wu[g]^T`` with ``dgu = [dG | dU]`` (``[NvS, 2*inner]``).  With
     ``push`` the rows (and ``push_w[r]``, e.g. the route-weight grads) go to their source ranks."""
     G, N, Kh = wg.shape
@@ -280,7 +286,7 @@ def dgrad_gate_up(dgu, wg, wu, cu, out, groups=None, num_ctas=None, dynamic=Fals
     rows, cols = _w2d(wg)
     _launch(DGRAD_GU, dgu, wg, wu, cu, N=N, K=2 * Kh, b_group_rows=N, out=out, ldo=out.stride(0),
             b_rows=rows, b_cols=cols, b_ld=cols, groups=groups, num_ctas=num_ctas, dynamic=dynamic, ticket=ticket,
-            push=push, push_w=push_w, pad=pad)
+            push=push, push_w=push_w, pad=pad, held=held)
 
 
 def skips_padding() -> bool:

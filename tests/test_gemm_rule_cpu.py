@@ -70,3 +70,44 @@ def test_a_second_update_comes_with_the_first_and_a_second_matrix():
     for kw in (dict(update_b=w), dict(update_b=w, out_b=out), dict(update_b=w, update=up), dict(update=up, out_b=out)):
         with pytest.raises(AssertionError, match="update_b comes with"):
             gg.wgrad(x, x, cu, out, **kw)
+
+
+PLAIN, BANDED, STREAM = range(3)
+
+
+@pytest.mark.parametrize("H,Hp,E,K,S,early,late", [
+    (2048, 768, 16, 8, 64, STREAM, STREAM), (2048, 768, 16, 8, 256, STREAM, STREAM), (2048, 768, 16, 8, 257, PLAIN, PLAIN),      # 128 rows an expert, one more
+    (2048, 768, 11, 1, 64, STREAM, STREAM), (2048, 768, 10, 1, 64, PLAIN, STREAM), (2048, 768, 8, 8, 64, PLAIN, STREAM),          # 33, 30 and 24 MiB of matrices
+    (2048, 768, 5, 1, 64, PLAIN, PLAIN), (1024, 1024, 16, 4, 200, STREAM, STREAM), (960, 1024, 16, 4, 200, PLAIN, STREAM),
+    (1024, 1024, 8, 4, 200, PLAIN, STREAM), (960, 1024, 8, 4, 200, PLAIN, PLAIN), (7168, 2048, 32, 8, 256, STREAM, STREAM), (2048, 768, 16, 8, 1531, PLAIN, PLAIN)])
+def test_which_gemms_stream_their_weights(H, Hp, E, K, S, early, late):
+    """What decides is the experts at home and the batch's rows, on one rank in a table of 2E groups with room for all their padding, in a native pass
+    (early) as in one issued from Python (late)."""
+    from moonep_b200 import _native
+    kind, room = _native.load().mep_pair_kind, S * K + 127 * 2 * E
+    for mode, N, k in ((GATE_UP, Hp, H), (DOWN, H, Hp), (DGRAD, Hp, H), (DGRAD_GU, H, 2 * Hp)):
+        deep = k % 128 == 0
+        assert kind(mode, _i64(room), 2 * E, N, k, E, S * K, 1) == (early if deep else PLAIN)
+        assert kind(mode, _i64(room), 2 * E, N, k, E, S * K, 0) == (late if deep else PLAIN)
+
+
+def test_a_direct_call_counts_its_groups_and_the_room_for_their_rows():
+    from moonep_b200 import _native
+    kind = _native.load().mep_pair_kind
+    for early in (0, 1):
+        for G, rows, want in ((11, 11 * 320, STREAM), (11, 11 * 320 + 1, PLAIN), (10, 10, PLAIN)):
+            for mode, N, k in ((GATE_UP, 768, 2048), (DOWN, 2048, 768), (DGRAD, 768, 2048), (DGRAD_GU, 2048, 1536)):
+                assert kind(mode, _i64(rows), G, N, k, 0, 0, early) == want
+
+
+def test_large_groups_are_banded_whoever_holds_them():
+    from moonep_b200 import _native
+    kind = _native.load().mep_pair_kind
+    for held in ((0, 0), (1, 1000), (32, 100000)):           # 18 MiB of rows for each of 64 groups, whether they hold any or not
+        assert kind(GATE_UP, _i64(32 * 4096), 64, 2048, 4608, *held, 0) == PLAIN
+        assert kind(GATE_UP, _i64(32 * 4096 + 1), 64, 2048, 4608, *held, 0) == BANDED
+
+
+def _i64(n):
+    import ctypes as C
+    return C.c_int64(n)

@@ -275,3 +275,33 @@ def test_native_passes_give_the_bits_of_single_launches(ctas, lr, cuda_device):
     assert all(torch.equal(a, b) for a, b in zip(*got))
     assert (lr is None) == all(torch.equal(a, b) for a, b in zip(got[0][7:], before))
     blk.destroy()
+
+
+@pytest.mark.parametrize("flags", [False, True], ids=["local", "ranks"])
+def test_a_layers_launches_say_which_groups_hold_rows(flags, cuda_device, monkeypatch):
+    """With a hook the GEMMs are issued one by one; they name the experts and rows that the native passes name, forwards (without route weights) and
+    backwards, and so does the code for several ranks."""
+    from moonep_b200.ops import grouped_gemm as gg
+    blk, seen, launch = make_block(), [], gg._launch
+
+    def spy(mode, *a, **kw):
+        seen.append((mode, kw.get("held")))
+        return launch(mode, *a, **kw)
+    monkeypatch.setattr(gg, "_launch", spy)
+    if flags:
+        blk.moe._local, blk.moe._native = False, None
+    blk.moe.on_grad_ready = lambda n: None
+    x, dy = normal((130, 256), 1), normal((130, 256), 2)
+    with torch.no_grad():
+        w, topk, tpe = blk.route(x)
+    if not flags:
+        blk.moe.forward(x, None, topk, tpe, need_backward=False)
+    _, ctx = blk.moe.forward(x, w, topk, tpe)
+    blk.moe.backward(ctx, dy)
+    torch.cuda.synchronize()
+    blk.buf.check()
+    assert {m for m, _ in seen} >= {gg.GATE_UP, gg.DOWN, gg.DGRAD, gg.DGRAD_GU}
+    assert {h for m, h in seen if m != gg.WGRAD} == {(4, 260)}
+    native = blk.moe._native_layer()._args
+    assert (native.E, native.S * native.K) == (4, 260)
+    blk.destroy()
