@@ -305,3 +305,54 @@ def test_a_layers_launches_say_which_groups_hold_rows(flags, cuda_device, monkey
     native = blk.moe._native_layer()._args
     assert (native.E, native.S * native.K) == (4, 260)
     blk.destroy()
+
+
+@pytest.mark.parametrize("last", ["weights", "counts"])
+def test_queued_passes_see_what_the_kernel_before_wrote(last, cuda_device):
+    """The GEMMs of a pass load weights and token counts while its dispatch still runs, and the dispatch sets itself up beside the kernel before: weights or
+    counts written by the kernel right in front of a pass, passes queued without a pause, give what ordinary launches give with a pause behind everything."""
+    from moonep_b200.models.moe_block import MoEBlock, MoEConfig
+    names = ("gate", "up", "down")
+    blk = MoEBlock(MoEConfig("t", H=512, Hp=512, K=4, epn=8, shared_experts=0, S=600), num_sms=4, seed=3, router_skew=0.5)
+    assert blk.moe._native is not None
+    xs, dys = [normal((600, 512), i) for i in (1, 2)], [normal((600, 512), i) for i in (3, 4)]
+    with torch.no_grad():
+        routes = [tuple(t.clone() for t in blk.route(x)) for x in xs]
+    assert not torch.equal(routes[0][2], routes[1][2])
+    base = {n: blk.pools.local_weight(n).clone() for n in names}
+    zero = torch.zeros_like(routes[0][2])
+    w, topk, tpe = (t.clone() for t in routes[0])
+    x, dy = xs[0].clone(), dys[0].clone()
+
+    def write(i, order):
+        todo = {"inputs": lambda: [torch.add(a, 0, out=b) for a, b in zip((xs[i % 2], dys[i % 2], *routes[i % 2][:2]), (x, dy, w, topk))],
+                "counts": lambda: torch.add(routes[i % 2][2], zero, out=tpe),
+                "weights": lambda: [torch.mul(base[n], 1.0 + 0.125 * (i % 3), out=blk.pools.local_weight(n)) for n in order]}
+        for k in sorted(todo, key=lambda k: k == last):
+            todo[k]()
+
+    def one(i, pause):
+        write(i, ("up", "down", "gate"))               # gate/up is the first GEMM of a forward pass
+        pause()
+        out, _ = blk.moe.forward(x, w, topk, tpe, need_backward=False)
+        pause()
+        write(i + 1, ("down", "gate", "up"))
+        pause()
+        y, ctx = blk.moe.forward(x, w, topk, tpe)
+        pause()
+        for n in ("gate", "up", "down"):                # dgrad(down) the first of a backward pass
+            torch.mul(base[n], 1.0 + 0.125 * ((i + 2) % 3), out=blk.pools.local_weight(n))
+        pause()
+        dx, dw = blk.moe.backward(ctx, dy)
+        pause()
+        return [out, y, dx, dw] + [blk.pools.local_grad(n).clone() for n in names]
+
+    blk.buf.enable_pdl = False
+    want = [one(i, torch.cuda.synchronize) for i in range(6)]
+    blk.buf.enable_pdl = True
+    got = [one(i % 6, lambda: None) for i in range(12)]
+    torch.cuda.synchronize()
+    blk.buf.check()
+    for i, g in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(g, want[i % 6])), f"pass {i}"
+    blk.destroy()

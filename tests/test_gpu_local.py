@@ -137,22 +137,30 @@ def test_padding_rows_are_counted(cuda_device):
     blk.destroy()
 
 
-# Every CTA counts the entries before its own up to 65536 of them, in rounds of 4096; above that the CTAs hand over their histograms.
+# Every CTA counts the entries before its own up to 65536 of them, in rounds of 4096; above that the CTAs hand over their histograms (COUNT_CASES), and
+# from 24576 * 7168 elements of rows on (ROW_CASES: the last batch below and the first above, with two slots a warp).
 COUNT_CASES = [
     (4097,   1,  8,    64,    16,  "random"),
     (4213,   2,  300,  16,    1,   "biased"),
     (8192,   8,  64,   128,   16,  "random"),
     (9363,   7,  64,   64,    16,  "biased"),
+    (9400,   7,  700,  16,    1,   "random"),     # the hand-over with more experts than a CTA has threads
 ]
 
 
-@pytest.mark.parametrize("case", COUNT_CASES, ids=lambda c: "S%d_K%d_E%d_H%d" % c[:4])
+ROW_CASES = [
+    (2194,   11, 24,   7296,  16,  "random"),
+    (2195,   11, 24,   7296,  16,  "random"),
+]
+
+
+@pytest.mark.parametrize("case", COUNT_CASES + ROW_CASES, ids=lambda c: "S%d_K%d_E%d_H%d" % c[:4])
 def test_local_exchange_at_the_ends_of_counting(case, cuda_device):
     test_local_exchange(case, cuda_device)
 
 
 # Large batches (200 MiB moved): the saved plan's rows come from many short CTAs and the combine begins with the last tokens. Just above
-# the line with fresh plans on both sides of the hand-over, one entry per token, a token for each CTA with rows of which three fit.
+# the line, one entry per token, a token for each CTA with rows of which three fit. Their fresh plans are counted; ROW_CASES has large ones with the hand-over.
 LARGE_CASES = [
     (2048, 8,  48,   5696,  16,  "random"),
     (5003, 5,  40,   3496,  128, "biased"),
@@ -188,36 +196,44 @@ def test_saved_plan_of_a_large_batch_keeps_to_the_sm_limit(limit, cuda_device, m
     buf.destroy()
 
 
-@pytest.mark.parametrize("pdl", [False, True], ids=["plain", "pdl"])
+@pytest.mark.parametrize("pdl", [(True,), (False,), (True, False)], ids=["pdl", "plain", "in_turn"])
 @pytest.mark.parametrize("shape", [(64, 8, 16, 256), (4000, 4, 32, 1024), (9000, 8, 16, 64), (2048, 8, 48, 5696)], ids=str)
 def test_queued_calls_see_what_the_kernel_before_wrote(shape, pdl, cuda_device):
     """Launches may begin while the one before still runs: batches queued without a pause, each routed and filled by kernels right in front of its
-    calls, give what they give one at a time. ``enable_pdl`` may be changed in between."""
+    calls, give what ordinary launches give with a pause behind every one. ``enable_pdl`` may be changed from one batch to the next."""
     S, K, E, H = shape
-    buf = Buffer(S, H, K, E, 1, token_padding=16, enable_pdl=not pdl)
-    buf.enable_pdl = pdl
-    base = torch.randn(S, H, device="cuda").to(torch.bfloat16)
+    buf = Buffer(S, H, K, E, 1, token_padding=16)
+    base, scale = torch.randn(S, H, device="cuda").to(torch.bfloat16), torch.rand(S, K, device="cuda")
     tables = [tuple(t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=s)) for s in (1, 2, 3)]
-    x, topk, tpe = torch.empty_like(base), torch.empty_like(tables[0][0]), torch.empty_like(tables[0][1])
+    x, w, topk, tpe = torch.empty_like(base), torch.empty_like(scale), torch.empty_like(tables[0][0]), torch.empty_like(tables[0][1])
 
-    def batch(i):
-        torch.mul(base, 1.0 + 0.25 * (i % 5), out=x)
-        tpe.copy_(tables[i % 3][1])
-        torch.add(tables[i % 3][0], 0, out=topk)
-        h, _, _, plan = buf.dispatch(x, None, topk, tpe, zero_copy=True)
-        y = buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)[0]
+    def batch(i, pause):
+        """The producer in front of the first call is another one in every third batch."""
+        fill = [lambda: torch.mul(base, 1.0 + 0.25 * (i % 5), out=x), lambda: torch.add(tables[i % 3][1], 0, out=tpe),
+                lambda: torch.add(tables[i % 3][0], 0, out=topk), lambda: torch.mul(scale, 1.0 + i, out=w)]
+        for f in fill[i % 4:] + fill[:i % 4]:
+            f()
+            pause()
+        h, wn, cu, plan = buf.dispatch(x, w, topk, tpe, zero_copy=True, router_weights_zero_copy=True)
+        pause()
+        y, wb, _ = buf.combine(plan=plan, hidden_nvsh=h, route_weights_nvs=wn, zero_copy=True, router_weights_zero_copy=True)
+        pause()
         h, _, _, _ = buf.dispatch(y, plan=plan, zero_copy=True)
-        return y, buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)[0]
+        pause()
+        z = buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)[0]
+        pause()
+        return y, wb, z, cu, plan.dst, plan.zero_fill_ranges
 
-    want = []
-    for i in range(12):
-        want.append([t.clone() for t in batch(i)])
-        torch.cuda.synchronize()
-    got = [batch(i) for i in range(12)]
+    buf.enable_pdl = False
+    want = [batch(i, torch.cuda.synchronize) for i in range(12)]
+    got = []
+    for i in range(24):
+        buf.enable_pdl = pdl[i % len(pdl)]
+        got.append(batch(i % 12, lambda: None))
     torch.cuda.synchronize()
     buf.check()
-    for a, b in zip(got, want):
-        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    for i, g in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(g, want[i % 12])), f"batch {i}"
     buf.destroy()
 
 
@@ -246,10 +262,61 @@ def test_calls_on_the_communication_stream_are_ordinary_launches(cuda_device):
     buf.destroy()
 
 
-@pytest.mark.parametrize("limit,shapes", [(None, {(8192, 8, 64): 0, (8193, 8, 64): 1}), (99, {(8192, 8, 64): 0}), (98, {(5120, 8, 64): 0, (5121, 8, 64): 1}),
+@pytest.mark.parametrize("pdl", [False, True], ids=["plain", "pdl"])
+@pytest.mark.parametrize("before", ["copy", "memset", "kernel", "join"])
+def test_captured_calls_behind_nodes_of_every_kind(before, pdl, cuda_device):
+    """The first exchange call of a captured graph right behind a copy, a memset, a kernel, and a join of two streams whose last nodes are a kernel and a
+    copy; replayed back to back with new inputs."""
+    S, K, E, H = 300, 4, 16, 512
+    buf = Buffer(S, H, K, E, 1, token_padding=16, enable_pdl=pdl)
+    tables = [tuple(t[0].cuda() for t in make_topk("random", S, K, E, 1, seed=s)) for s in (1, 2, 3)]
+    xs = [torch.randn(S, H, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    src_x, src_k, src_t = xs[0].clone(), tables[0][0].clone(), tables[0][1].clone()
+    x, topk, tpe, junk = torch.empty_like(src_x), src_k.clone(), src_t.clone(), torch.empty(1 << 22, dtype=torch.uint8, device="cuda")
+    side = torch.cuda.Stream()
+
+    def body():
+        if before == "join":
+            cur = torch.cuda.current_stream()
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                x.copy_(src_x)
+            torch.add(src_k, 0, out=topk)
+            torch.add(src_t, 0, out=tpe)
+            cur.wait_stream(side)
+        else:
+            torch.add(src_k, 0, out=topk)
+            torch.add(src_t, 0, out=tpe)
+            torch.add(src_x, 0, out=x) if before == "kernel" else x.copy_(src_x)
+            if before == "memset":
+                junk.zero_()
+        h, _, _, plan = buf.dispatch(x, None, topk, tpe, zero_copy=True)
+        return buf.combine(plan=plan, hidden_nvsh=h, zero_copy=True)[0]
+
+    body()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = body()
+    for i in range(9):
+        src_x.copy_(xs[i % 3])
+        src_k.copy_(tables[i // 3][0])
+        src_t.copy_(tables[i // 3][1])
+        graph.replay()
+        graph.replay()
+        got = y.clone()
+        torch.cuda.synchronize()
+        # every token's row comes back K = 4 times: the sum of four equal numbers is exact
+        assert torch.equal(got, xs[i % 3] * 4)
+    buf.check()
+    del graph
+    buf.destroy()
+
+
+@pytest.mark.parametrize("limit,shapes", [(None, {(8192, 8, 64): 0, (8193, 8, 64): 1, (2194, 11, 7296): 0, (2195, 11, 7296): 1}), (99, {(8192, 8, 64): 0}), (98, {(5120, 8, 64): 0, (5121, 8, 64): 1}),
                                           (16, {(5120, 8, 64): 0, (8192, 8, 64): 1})], ids=str)
 def test_which_dispatches_hand_over(limit, shapes, cuda_device, monkeypatch):
-    """Up to 65536 entries every CTA counts for itself, up to 40960 where it may use less than two thirds of the (148) SMs; only the hand-over numbers its launches."""
+    """Up to 65536 entries and 24576 * 7168 elements every CTA counts for itself, up to 40960 where it may use less than two thirds of the (148) SMs; only the hand-over numbers its launches."""
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the limits are those of 148 SMs")
     if limit is not None:

@@ -202,13 +202,14 @@ def test_pushed_rows_and_flagged_tiles_on_both_kernels(pairs, cuda_device, monke
     test_gemm_consumes_tiles_while_dispatch_runs(4, "gate_up", cuda_device)
 
 
+@pytest.mark.parametrize("H,E", [(256, 4), (768, 16)], ids=["small", "streamed"])
 @pytest.mark.parametrize("pairs", ["0", "1"], ids=["single", "pairs"])
-def test_dgrad_pushes_rows_and_their_scalars(pairs, cuda_device, monkeypatch):
+def test_dgrad_pushes_rows_and_their_scalars(pairs, H, E, cuda_device, monkeypatch):
     """dgrad(gate/up) with identity weights: every dispatched row and its scalar go back to the token that it came from."""
     from moonep_b200 import Buffer, routing
     from moonep_b200.ops import grouped_gemm as gg
     monkeypatch.setenv("MOONEP_GEMM_2CTA", pairs)
-    S, H, K, E = 96, 256, 4, 4
+    S, K = 96, 4
     topk, w, tpe = routing.softmax_topk(S, K, E, 1.0, 5, 0, device="cuda")
     g = torch.Generator(device="cuda").manual_seed(7)
     x = torch.randn(S, H, device="cuda", generator=g).to(torch.bfloat16)
@@ -424,21 +425,23 @@ def test_token_major_tiles_of_uneven_groups(split, cuda_device, monkeypatch):
         assert all(torch.equal(o.view(torch.int16), want.view(torch.int16)) for o in got)
 
 
-@pytest.mark.parametrize("tokens", [False, True], ids=["cu", "tokens"])
-@pytest.mark.parametrize("most,depths", [(32, (9, 10, 11, 20)), (128, (7, 8, 9)), (300, (1, 5, 6, 7, 13))], ids=["ring10", "ring8", "ring6"])
-def test_early_launches_around_the_depth_of_the_ring(most, depths, tokens, cuda_device, monkeypatch):
-    """A launch that fills its ring with weights while the kernel before still writes its rows: fewer 64-deep blocks than stages, as many, more;
+def _around_the_depth_of_the_ring(most, depths, block, columns, tokens, check, monkeypatch):
+    """A launch that fills its ring with weights while the kernel before still writes its rows: fewer blocks of depth than stages, as many, more;
     27 groups, some empty, on two pairs (many tiles each) and on all (some without one); tiles from token counts or from cu_seqlens.
-    The bits of an ordinary launch behind the kernel before."""
+    The bits of an ordinary launch behind the kernel before; with `check` of single CTAs, too, and of launches that stream their weights."""
+    import ctypes as C
+
+    from moonep_b200 import _native
     from moonep_b200.ops import grouped_gemm as gg
     monkeypatch.setenv("MOONEP_GEMM_2CTA", "1")
-    E, N, wide = 27, 256, 64 * max(depths) * 2 + 256
-    wide = (wide + 255) // 256 * 256
+    E = 27
+    wide = (2 * block * max(depths) + 256 + 255) // 256 * 256
     n = [(most, 0, 1, most // 2, 32, 0, most - 1)[i % 7] for i in range(E)]
     p = [(r + 127) // 128 * 128 for r in n]
     ends = torch.tensor(p).cumsum(0)
     rows, cu = sum(p), ends.to(torch.int32).cuda()
     pad = torch.tensor([[int(e) - q + r, q - r] if q > r else [0, 0] for r, q, e in zip(n, p, ends)], dtype=torch.int32).cuda()
+    real = torch.cat([torch.arange(e - q, e - q + r) for r, q, e in zip(n, p, ends.tolist())]).cuda()
     tpe = torch.tensor(n, dtype=torch.int32, device="cuda")
     g = torch.Generator(device="cuda").manual_seed(12)
     bf = lambda *s, sc=1.0: (torch.randn(*s, device="cuda", generator=g) * sc).to(torch.bfloat16)     # noqa: E731
@@ -448,14 +451,15 @@ def test_early_launches_around_the_depth_of_the_ring(most, depths, tokens, cuda_
     before = lambda: gg.down(src, w_src, whole, x, num_ctas=2)     # noqa: E731
     fields = dict(tokens=tpe.data_ptr(), tokens_n=E, token_padding=128) if tokens else {}
     for d in depths:
-        K = 64 * d
+        K = block * d
+        N = columns(E * K)
         w, wu, dy = bf(E, K, N, sc=0.05), bf(E, K, N, sc=0.05), bf(rows, N)
         for r, q, e in zip(n, p, ends.tolist()):
             dy[e - q + r:e] = 0
         calls = {"gate_up": lambda o, **kw: gg.gate_up(x[:, :K], w, wu, cu, o, pad=pad, **kw), "down": lambda o, **kw: gg.down(x[:, :K], w, cu, o, pad=pad, **kw),
                  "dgrad": lambda o, **kw: gg.dgrad(x[:, :K], w.view(E, N, K), cu, o, pad=pad, **kw),
                  "dgrad_gu": lambda o, **kw: gg.dgrad_gate_up(x[:, :2 * K], w.view(E, N, K), wu.view(E, N, K), cu, o, pad=pad, **kw)}
-        if d == depths[0]:
+        if d == depths[0] and block == 64:
             calls["wgrad"] = lambda o, **kw: gg.wgrad(x[:, :512], dy, cu, o, pad=pad, zero_empty_below=E, **kw)
         for name, call in calls.items():
             shape, dt = ((E, 512, N), torch.float32) if name == "wgrad" else ((rows, N), torch.bfloat16)
@@ -470,6 +474,28 @@ def test_early_launches_around_the_depth_of_the_ring(most, depths, tokens, cuda_
             torch.cuda.synchronize()
             gg.check_status()
             assert all(torch.equal(o, want) for o in got), f"{name}, {d} blocks"
+            if check and name != "wgrad":
+                mode, k = dict(gate_up=(gg.GATE_UP, K), down=(gg.DOWN, K), dgrad=(gg.DGRAD, K), dgrad_gu=(gg.DGRAD_GU, 2 * K))[name]
+                assert _native.load().mep_pair_kind(mode, C.c_int64(rows), E, N, k, 0, 0, 1) == 2, "not the kernel that streams"
+                single = torch.empty_like(want)
+                with monkeypatch.context() as m:
+                    m.setenv("MOONEP_GEMM_2CTA", "0")
+                    call(single)
+                assert torch.equal(single[real], want[real]), f"{name}, {d} blocks: single CTAs"
+
+
+@pytest.mark.parametrize("tokens", [False, True], ids=["cu", "tokens"])
+@pytest.mark.parametrize("most,depths", [(32, (9, 10, 11, 20)), (128, (7, 8, 9)), (300, (1, 5, 6, 7, 13))], ids=["ring10", "ring8", "ring6"])
+def test_early_launches_around_the_depth_of_the_ring(most, depths, tokens, cuda_device, monkeypatch):
+    """64-deep blocks."""
+    _around_the_depth_of_the_ring(most, depths, 64, lambda k: 256, tokens, False, monkeypatch)
+
+
+@pytest.mark.parametrize("tokens", [False, True], ids=["cu", "tokens"])
+@pytest.mark.parametrize("most,depths", [(32, (1, 2, 4, 5, 6, 11)), (96, (3, 4, 5)), (128, (3, 4, 5, 9)), (255, (1, 2, 3, 4, 7))], ids=["ring5", "ring4_16", "ring4", "ring3"])
+def test_early_launches_of_streamed_weights_around_the_depth_of_the_ring(most, depths, tokens, cuda_device, monkeypatch):
+    """128-deep blocks: 27 matrices of 32 MiB, the narrowest that are so large."""
+    _around_the_depth_of_the_ring(most, depths, 128, lambda k: -(-(32 << 20) // (2 * k * 256)) * 256, tokens, True, monkeypatch)
 
 
 def test_counts_that_fall_give_no_tiles(cuda_device):
@@ -493,12 +519,18 @@ def test_counts_that_fall_give_no_tiles(cuda_device):
     assert bool((dW[1] == 7.0).all())
 
 
+@pytest.mark.parametrize("n", [[1, 32, 256, 257, 0, 600, 255, 512], [1, 32, 96, 64, 0, 33, 16, 95], [1, 128, 97, 64, 0, 127, 128, 33]], ids=["rows128", "rows16", "rows64"])
 @pytest.mark.parametrize("K", [1984, 2048], ids=["kept", "streamed"])
-def test_weights_that_are_read_once(K, cuda_device):
-    """From 32 MiB of matrices on (8 of 2048 x 1024) the weights of groups with one token tile leave L2 first: the same bits as group by group, where
-    they never do, with tiles that share their weights in between."""
+def test_weights_that_are_read_once(K, n, cuda_device):
+    """From 32 MiB of matrices on (8 of 2048 x 1024) the weights of groups with one token tile leave L2 first, in stages of 128: the same bits as group by
+    group, where they never do, with tiles that share their weights in between; with rows in boxes of 128, 64 and 16, in both tile orders, and behind flags
+    of tiles and groups (which are all up)."""
+    import ctypes as C
+
+    from moonep_b200 import _native
+    from moonep_b200.api import SlotReady, TileReady
     from moonep_b200.ops import grouped_gemm as gg
-    N, n = 1024, [1, 32, 256, 257, 0, 600, 255, 512]
+    N = 1024
     p = [(r + 127) // 128 * 128 for r in n]
     ends = torch.tensor(p).cumsum(0)
     pad = torch.tensor([[int(e) - q + r, q - r] if q > r else [0, 0] for r, q, e in zip(n, p, ends)], dtype=torch.int32)
@@ -507,18 +539,25 @@ def test_weights_that_are_read_once(K, cuda_device):
     x, h, w, wu = bf(sum(p), K), bf(sum(p), 2 * N), bf(8, K, N, sc=0.02), bf(8, K, N, sc=0.02)
     wt = w.transpose(1, 2).contiguous()
 
-    def run(x, h, w, wu, wt, cu, pad):
+    up = torch.full((64,), 5, dtype=torch.int32, device="cuda")          # flags and their epoch
+    flags = dict(ready=TileReady(up.data_ptr(), up.data_ptr(), 148), slots=SlotReady(up.data_ptr(), up.data_ptr(), 3))
+
+    def run(x, h, w, wu, wt, cu, pad, dynamic=False, gated={}):
         out = [torch.zeros(len(x), c, dtype=torch.bfloat16, device="cuda") for c in (N, 2 * N, N, N)]
-        kw = dict(pad=pad.cuda())
-        gg.gate_up(x, w, wu, cu.cuda(), out[0], out[1], **kw)
+        kw = dict(pad=pad.cuda(), dynamic=dynamic)
+        gg.gate_up(x, w, wu, cu.cuda(), out[0], out[1], **kw, **gated)
         gg.down(x, w, cu.cuda(), out[2], **kw)
-        gg.dgrad(x, wt, cu.cuda(), out[3], **kw)
+        gg.dgrad(x, wt, cu.cuda(), out[3], **kw, **gated)
         if K % 256 == 0:
             out.append(torch.zeros(len(x), K, dtype=torch.bfloat16, device="cuda"))
             gg.dgrad_gate_up(h, w, wu, cu.cuda(), out[4], **kw)
         return out
 
-    got = run(x, h, w, wu, wt, ends.to(torch.int32), pad)
+    args = x, h, w, wu, wt, ends.to(torch.int32), pad
+    assert _native.load().mep_pair_kind(gg.DOWN, C.c_int64(sum(p)), 8, N, K, 0, 0, 0) == (2 if K == 2048 else 0)
+    got = run(*args)
+    for kw in (dict(dynamic=True), dict(gated=flags), dict(dynamic=True, gated=flags)):
+        assert all(torch.equal(a, b) for a, b in zip(got, run(*args, **kw)))
     for i, (q, e) in enumerate(zip(p, ends.tolist())):
         if q:
             s, one = slice(e - q, e), torch.tensor([q], dtype=torch.int32)
