@@ -84,7 +84,7 @@ __device__ __forceinline__ int local_layout(const int32_t* tpe, int E, int pad, 
 // already running and no cooperative launch is needed. Then, from `dst` alone, each row goes through a warp's slot in shared memory
 // with one bulk load and K bulk stores (lane k issues the store of entry k); rows of the next tokens are in
 // flight meanwhile, in the fresh case already during the ranking.
-// Bound by HBM: (1 + K) rows per token; 106 us at S=4096, H=7168, K=8 (5.0 TB/s, mostly stores) where planning, dispatch
+// Bound by HBM: (1 + K) rows per token; 103 us at S=4096, H=7168, K=8 (5.1 TB/s, mostly stores) where planning, dispatch
 // and duplicate expansion took 185.
 template <int MODE>                        // 0: saved plan
 __global__ void __launch_bounds__(kLocThreads, MODE ? 1 : 3)

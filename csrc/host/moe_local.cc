@@ -41,8 +41,10 @@ static LocalDispatchArgs dispatch_args(const MoeLocal& m, const void* hidden, in
 
 // Whether a pass's dispatch may begin while the kernel before still runs. A programmatic launch finds the SMs in the order in which that kernel leaves
 // them, and the GEMM pairs behind it inherit the order; after an ordinary one neighbours in the tile list are close to each other and read the
-// same lines of L2. That is worth 1.5 % of a forward pass of 4096 tokens, 7168 x 2048, 32 experts (2736 / 2782 us, six alternations); the launch
-// 1.5 to 4 us of a small one.
+// same lines of L2. Forward passes that begin with a programmatic / an ordinary dispatch, in us, by MiB of rows moved, six alternations: 2 (2048 x 768,
+// 64 tokens) 43.5 / 47.3; 18 (512) 69.0 / 75.6; 36 (1024) 99.3 / 106.5; 39 (7168 x 2048, 320) 498 / 500; 54 (2048 x 768, 1531) 131.0 / 140.0 and
+// 128.6 / 130.3 on another box; 63 (7168 x 2048, 512) 583 / 567; 126 (1024) 799 / 834 and 852 / 798; 252 (2048) 1465 / 1454; 504 (4096) 2682 / 2701 and 2782 / 2736.
+// So from the line on neither is better by more than runs and boxes differ.
 static int early_dispatch(const MoeLocal& m) { return m.pdl && (int64_t)m.S * (m.K + 1) * m.H * 2 < (40ll << 20); }
 
 static void plan_into(const MoeLocal& m, const int32_t* topk, const int32_t* tpe, int32_t* slab, LocalDispatchArgs* d) {
